@@ -1155,3 +1155,27 @@ def test_product_on_pairs_of_sms_with_k_split(shape):
     close(out, want.to(torch.bfloat16), torch.bfloat16)
     assert not gemm_tc.gave_up()
     assert gemm_tc.k_splits_for(512, 2304, 9216, ops.EPI_NONE) > 1 and gemm_tc.k_splits_for(2048, 2304, 9216, ops.EPI_NONE) == 1
+
+
+@pytest.mark.parametrize("shape", [(1, 64, 32), (2, 1, 4), (16, 65, 132), (17, 2304, 512), (33, 130, 36), (49, 31, 1028), (95, 200, 260),
+                                   (97, 33, 2052), (128, 64, 4096), (129, 100, 68), (300, 96, 128)])
+def test_gemm_f32(shape):
+    """The 32-bit product with rows of whole 16-byte pieces: every tile height, remainders of rows, columns and k, tiles
+    shared by a cluster.  A sum of K products of numbers of size 1 and K^-1/2, each rounded to 2^-24 of it, is off by less than
+    2^-24 K of sum |a w| <= 2^-24 K x (some) K^1/2; 3e-6 x sqrt(K) is far above what random signs leave of it."""
+    from hos_b200 import ops
+    M, N, K = shape
+    a = torch.randn(M, K, device=DEV)
+    w = torch.randn(2 * N, K, device=DEV) / math.sqrt(K)
+    bias = torch.randn(N, device=DEV)
+    g, u = a.double() @ w[:N].double().T, a.double() @ w[N:].double().T
+    one = w[:N].contiguous()
+    out = torch.empty(M, N, device=DEV)
+    for want, weight, kw in ((g, one, {}), (0.7 * torch.tanh(g / 0.7), one, dict(epilogue=ops.EPI_SOFTCAP, cap=0.7)),
+                             (torch.nn.functional.gelu(g + bias, approximate="tanh"), one,
+                              dict(epilogue=ops.EPI_BIAS, act=ops.BIAS_ACTIVATIONS["gelu_tanh"], bias=bias)),
+                             (torch.nn.functional.silu(g) * u, w, dict(epilogue=ops.EPI_GATED, act=ops.ACT_SILU))):
+        out.fill_(float("nan"))
+        ops.gemm_plain(a, weight, out, **kw)
+        err = (out.double() - want).abs().max().item()
+        assert err <= 3e-6 * math.sqrt(K) + 1e-6, (kw, err)
