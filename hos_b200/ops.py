@@ -167,8 +167,9 @@ def call_times() -> dict:
 _launch_ahead = False
 
 _ERROR_WORD_SETTERS = ("hos_gemm_tc_set_error_word", "hos_attn_decode_set_error_word",
-                       "hos_attn_prefill_tc_set_error_word")
-GIVE_UP_CODES = {1: "the tcgen05 matrix product", 2: "the decode attention", 3: "the tcgen05 prompt attention"}
+                       "hos_attn_prefill_tc_set_error_word", "hos_latent_prompt_set_error_word")
+GIVE_UP_CODES = {1: "the tcgen05 matrix product", 2: "the decode attention", 3: "the tcgen05 prompt attention",
+                 4: "the tcgen05 prompt attention over latent rows"}
 _error_word_tensor: Optional[torch.Tensor] = None
 _after_give_up = []        # callables that put shared scratch state right after a kernel gave up
 
@@ -695,6 +696,34 @@ def latent_attn(q_lat: torch.Tensor, q: torch.Tensor, dq: int, inv_freq: Optiona
                   _ptr(step.token_pos), _ptr(step.token_seq), _ptr(step.cu_seqlens), _ptr(step.seq_slot),
                   int(row0), int(rows), heads, rank, d, float(scale), int(window) if window else 0,
                   1 if tensor_cores else 0, _stream())
+
+
+LATENT_PROMPT_SIZES = (64, 64, 128)      # a key's unrotated and rotated numbers, a value's, that latent_prompt takes at most
+
+
+def latent_prompt(q: torch.Tensor, dq: int, vd: int, inv_freq: Optional[torch.Tensor], rot_dims: int, style: int, kv: torch.Tensor,
+                  kc: torch.Tensor, sink: Optional[torch.Tensor], out: torch.Tensor, step, rows: int, rank: int, scale: float,
+                  window: Optional[int]) -> None:
+    """Rows 0 .. rows-1 of the step (sequences from position 0) over keys and values that were formed: kv float32 [rows, heads x dq +
+    heads x vd], the latents times the heads' W_uk and W_uv; kc: the latent rows, whose last numbers are the keys' rotated
+    part; q: rows of the heads' queries as projected (dq unrotated and then the rotated numbers each).  out [N, heads x vd]."""
+    _check(q, "query rows", torch.bfloat16, 2)
+    _check(kv, "expanded latents", torch.float32, 2)
+    _check(kc, "latent rows", torch.bfloat16, 2)
+    _check(out, "attention outputs", torch.bfloat16, 2)
+    heads, rot = out.shape[1] // vd, kc.shape[1] - rank
+    if kv.shape != (rows, heads * (dq + vd)) or q.shape[1] < heads * (dq + rot) or min(q.shape[0], kc.shape[0], out.shape[0]) < rows:
+        raise KernelError("latent_prompt: sizes disagree")
+    a, b, c = LATENT_PROMPT_SIZES
+    ws = torch.empty((3 * a + 2 * a + c) * heads * rows, dtype=torch.bfloat16, device=q.device)
+    k_ws, v_ws = ws[3 * a * heads * rows:], ws[5 * a * heads * rows:]
+    n_seqs = step.fresh_seqs or step.n_seqs
+    lens = [step.cu_host[i + 1] - step.cu_host[i] for i in range(n_seqs)] if step.cu_host else []
+    tiles = sum((n + 127) // 128 for n in lens) if lens else (rows + 127) // 128 + n_seqs
+    blocks().call("hos_latent_prompt", _ptr(q), q.shape[1], _ptr(kv), _ptr(kc), _ptr(inv_freq), int(rot_dims) if inv_freq is not None else 0,
+                  int(style), _ptr(sink), _ptr(step.token_pos), _ptr(step.token_seq), _ptr(step.cu_seqlens), n_seqs, tiles, int(rows),
+                  heads, int(dq), rot, int(vd), int(rank), float(scale), int(window) if window else 0, _ptr(ws), _ptr(k_ws), _ptr(v_ws),
+                  _ptr(out), _stream())
 
 
 def heads_product(x: torch.Tensor, x_off: int, lda: int, a_head: int, w: torch.Tensor, out: torch.Tensor, out_off: int,

@@ -7,7 +7,8 @@ numbers, not normed).  A head's key is [W_uk_h c | rotated part], its value W_uv
 mask is causal with an optional window of the last `window` keys; with `sink`, a learned number
 per head joins the softmax's denominator as exp(sink_h) (no key, no value, unscaled).
 
-Neither keys nor values are formed: the query absorbs W_uk (q'_h = W_uk_h^T q_h, `kv_rank`
+Prompts of 64 rows or more whose sizes fit form keys and values (one product of the latents, then the tcgen05 walk of
+csrc/latent_prompt.cu: less arithmetic per pair).  Elsewhere neither is formed: the query absorbs W_uk (q'_h = W_uk_h^T q_h, `kv_rank`
 numbers) and W_uv is applied to the weighted sum of latents, so the attention kernel reads
 `kv_rank + rot_dim` numbers per key for all heads.  Everything between the projections (norm of
 c, angles, scores, softmax, weighted sums) is 32-bit; with bfloat16 rows the two products run on the
@@ -39,6 +40,12 @@ from ..errors import KernelError, SpecError
 from ..registry import part_impl, register_part
 from . import linear
 from .base import CallStore, KVNeed, Mixer, StepInfo, WeightSpec
+
+
+# From so many rows that start at position 0 on their keys and values are formed.  Measured against the absorbed form (eight
+# layers of Nuvivik, one prompt): 64 rows 0.97 against 1.03 ms, 128 rows 1.12 / 1.24, 512 rows 1.67 / 2.36, 4,000 rows 7.1 / 19.3;
+# fewer rows have their keys cut into shares there, which this walk does not do.
+PROMPT_ROWS = 64
 
 
 class LatentAttention(Mixer):
@@ -108,6 +115,12 @@ class LatentAttention(Mixer):
         uk = self._matrix(tensors[w["uk"]]).view(self.n_heads, self.dim, self.rank)
         self.w_uk_t = uk.transpose(1, 2).contiguous()                # [heads, rank, dim]: q'_h = W_uk_h^T q_h
         self.w_uv = self._matrix(tensors[w["uv"]]).view(self.n_heads, self.vdim, self.rank).contiguous()
+        # a prompt's keys and values as one product of its latent rows [c | rotated part]: the heads' W_uk, then their W_uv,
+        # with zeros under the rotated part
+        self.w_expand = None
+        if self._prompt_sizes_fit() and uk.dtype == torch.bfloat16 and self.w_uv.dtype == torch.bfloat16:
+            both = torch.cat([uk.reshape(-1, self.rank), self.w_uv.reshape(-1, self.rank)])
+            self.w_expand = torch.cat([both, both.new_zeros((both.shape[0], self.rot_dim))], dim=1).contiguous()
         self.w_o = self._matrix(tensors[w["o"]])
         self.sink = self._vector32(tensors[w["sink"]]) if self.has_sink else None
 
@@ -127,6 +140,12 @@ class LatentAttention(Mixer):
         keys = min(int(self.window), longest) if self.window else longest
         return max(1, min(32, (keys + 63) // 64, (2 * sms + blocks - 1) // blocks)), 1
 
+    def _prompt_sizes_fit(self) -> bool:
+        """Whether a prompt's keys and values may be formed and walked over by the tcgen05 kernel (csrc/latent_prompt.cu)."""
+        sizes = (self.dim, self.rot_dim, self.vdim)
+        return (not self.rt.is_fp32 and not self.shares_kv and self.scale > 0 and self.rank % 8 == 0 and
+                all(n % 8 == 0 and n <= most for n, most in zip(sizes, ops.LATENT_PROMPT_SIZES)))
+
     def forward(self, h: torch.Tensor, step: StepInfo, store: CallStore) -> torch.Tensor:
         return self._run(h, step, store, False)
 
@@ -144,7 +163,6 @@ class LatentAttention(Mixer):
         H, R, D = self.n_heads, self.rank, self.row
         proj = linear.matmul(h, self.w_in)
         kc = None if self.shares_kv else torch.empty((n, D), dtype=h.dtype, device=h.device)
-        q_lat = torch.empty((n, H, R), dtype=torch.float32, device=h.device)
         inv_freq, rot_dims, style = self.position.kernel_args() if self.position else (None, 0, 1)
         q_first = self.q_rank or self.q_cols                # the column where the down projection's part of `proj` begins
         parts = {} if self.shares_kv else dict(down=(proj, q_first), w_norm=self.w_norm, kc=kc, cache=cache)
@@ -156,12 +174,28 @@ class LatentAttention(Mixer):
             ops.latent_prep(step, R, self.rot_dim, self.eps, inv_freq, rot_dims, style, **parts)
         if self.q_rank:
             q = linear.matmul(cq, self.w_uq)
-        # q'_h = W_uk_h^T q_h
-        ops.heads_product(q, 0, q.shape[1], self.dim + self.rot_dim, self.w_uk_t, q_lat, 0, H * R, R, n)
-        attend = functools.partial(ops.latent_attn, q_lat, q, self.dim, inv_freq, rot_dims, style)
-        o_lat = torch.empty((n, H, R), dtype=h.dtype, device=h.device)      # what the value expansion reads
+        att = torch.empty((n, H * self.vdim), dtype=h.dtype, device=h.device)
         nf = 0 if self.shares_kv else (n if step.from_zero else step.fresh_tokens)
-        if nf > 0:
+        done = 0
+        if nf >= PROMPT_ROWS and self.w_expand is not None and self.use_tensor_cores and not step.single_token:
+            kv = linear.matmul(kc[:nf], self.w_expand, out_dtype=torch.float32)
+            ops.latent_prompt(q, self.dim, self.vdim, inv_freq, rot_dims, style, kv, kc, self.sink, att, step, nf, R, self.scale,
+                              self.window)
+            done = nf
+        if done < n:
+            self._run_absorbed(q, kc, att, done, nf, step, cache, (inv_freq, rot_dims, style))
+        return linear.matmul_or_partials(att, self.w_o) if partial_ok else linear.matmul(att, self.w_o)
+
+    def _run_absorbed(self, q, kc, att, first: int, nf: int, step: StepInfo, cache, rot) -> None:
+        """Rows first .. of `att` from the queries taken to the latent: rows up to nf attend over the step's own latent
+        rows kc, the others over the cache."""
+        n, H, R = q.shape[0], self.n_heads, self.rank
+        q_lat = torch.empty((n, H, R), dtype=torch.float32, device=q.device)
+        o_lat = torch.empty((n, H, R), dtype=q.dtype, device=q.device)      # what the value expansion reads
+        # q'_h = W_uk_h^T q_h
+        ops.heads_product(q, first * q.shape[1], q.shape[1], self.dim + self.rot_dim, self.w_uk_t, q_lat, first * H * R, H * R, R, n - first)
+        attend = functools.partial(ops.latent_attn, q_lat, q, self.dim, *rot)
+        if nf > first:
             shares, per_block = self.plan(nf, step)
             attend(kc, None, self.sink, o_lat, step, 0, nf, R, self.scale, self.window, paged=False,
                    n_splits=shares, rows_per_block=per_block, tensor_cores=self.use_tensor_cores)
@@ -177,9 +211,7 @@ class LatentAttention(Mixer):
             shares, per_block = self.plan(rows, step)
             attend(None, cache, self.sink, o_lat, step, nf, rows, R, self.scale, self.window, paged=True,
                    n_splits=shares, rows_per_block=per_block, tensor_cores=self.use_tensor_cores)
-        att = torch.empty((n, H * self.vdim), dtype=h.dtype, device=h.device)
-        ops.heads_product(o_lat, 0, H * R, R, self.w_uv, att, 0, H * self.vdim, self.vdim, n)
-        return linear.matmul_or_partials(att, self.w_o) if partial_ok else linear.matmul(att, self.w_o)
+        ops.heads_product(o_lat, first * H * R, H * R, R, self.w_uv, att, first * H * self.vdim, H * self.vdim, self.vdim, n - first)
 
 
 register_part("mixer", "latent_attention", LatentAttention)

@@ -1179,3 +1179,55 @@ def test_gemm_f32(shape):
         ops.gemm_plain(a, weight, out, **kw)
         err = (out.double() - want).abs().max().item()
         assert err <= 3e-6 * math.sqrt(K) + 1e-6, (kw, err)
+
+
+@pytest.mark.parametrize("sizes", [(64, 64, 128, 512, 0), (64, 64, 128, 512, 100), (48, 32, 64, 72, 0), (8, 16, 40, 64, 65)])
+@pytest.mark.parametrize("lens", [(64,), (1, 63, 130, 257), (500, 128)])
+def test_latent_prompt(sizes, lens):
+    """The walk over formed keys and values against the same in 64 bits, with the values rounded to bfloat16 as the kernel
+    reads them: what is left is the output's own rounding (eight bits of significand: up to 2^-8 of it) and terms of 16 bits in
+    keys and weights (2^-16 of a score of size ten, so 2^-12 of a value).  Padding rows
+    lie behind the sequences, and a sequence's infinite values must not reach its neighbour."""
+    from types import SimpleNamespace
+    from hos_b200 import ops
+    dq, P, vd, R, window = sizes
+    H, n, pad = 3, sum(lens), 5
+    rows = n + pad
+    inv_freq = (10000.0 ** (-torch.arange(P // 2 - 2, device=DEV) / 16.0)).float()
+    rot_dims, style, scale = P - 4, 0, 0.2
+    q = torch.randn(rows, H * (dq + P) + 8, device=DEV).bfloat16()
+    kc = torch.randn(rows, R + P, device=DEV).bfloat16()
+    kv = torch.randn(rows, H * (dq + vd), device=DEV)
+    kv[n:] = float("nan")
+    if len(lens) > 1:
+        kv[lens[0], H * dq:] = float("inf")                    # the second sequence's first values
+    sink = torch.randn(H, device=DEV)
+    cu = [0]
+    for x in lens:
+        cu.append(cu[-1] + x)
+    pos = torch.cat([torch.arange(x) for x in lens] + [torch.zeros(pad, dtype=torch.int64)]).int().to(DEV)
+    seq = torch.cat([torch.full((x,), i) for i, x in enumerate(lens)] + [torch.full((pad,), -1)]).int().to(DEV)
+    step = SimpleNamespace(cu_host=tuple(cu), n_seqs=len(lens), fresh_seqs=0, token_pos=pos, token_seq=seq,
+                           cu_seqlens=torch.tensor(cu, dtype=torch.int32, device=DEV))
+    out = torch.full((rows, H * vd), 7.0, device=DEV).bfloat16()
+    ops.latent_prompt(q, dq, vd, inv_freq, rot_dims, style, kv, kc, sink, out, step, rows, R, scale, window)
+    assert torch.all(out[n:] == 7.0)
+    for i, x in enumerate(lens):
+        s = slice(cu[i], cu[i + 1])
+        qq = q[s, : H * (dq + P)].double().view(x, H, dq + P)
+        a = pos[s].float()[:, None] * inv_freq
+        c, z = a.cos().double()[:, None], a.sin().double()[:, None]
+        r, half = qq[..., dq:].clone(), rot_dims // 2
+        r[..., :half] = qq[..., dq:dq + half] * c - qq[..., dq + half:dq + rot_dims] * z
+        r[..., half:rot_dims] = qq[..., dq + half:dq + rot_dims] * c + qq[..., dq:dq + half] * z
+        k = kv[s, : H * dq].double().view(x, H, dq)
+        v = kv[s, H * dq:].bfloat16().double().view(x, H, vd)
+        score = (torch.einsum("ihd,jhd->hij", qq[..., :dq], k) + torch.einsum("ihd,jd->hij", r, kc[s, R:].double())) * scale
+        d = torch.arange(x, device=DEV)[:, None] - torch.arange(x, device=DEV)[None]
+        hidden = (d < 0) | ((d >= window) if window else torch.zeros_like(d, dtype=torch.bool))
+        score = torch.cat([score.masked_fill(hidden, -math.inf), sink.double()[:, None, None].expand(H, x, 1)], 2)
+        want = torch.einsum("hij,jhd->ihd", score.softmax(2)[..., :-1], v).reshape(x, H * vd)
+        if i == 1:
+            continue                                           # infinite itself
+        err = (out[s].double() - want).abs()
+        assert torch.all(err <= want.abs() * 2.0 ** -8 + 2.0 ** -12 * v.abs().max()), err.max().item()
