@@ -1,4 +1,4 @@
-// Plain attention: one warp per (token, query head), keys visited one by one with a
+// Plain attention: one warp per (token, query head), keys visited a few at a time with a
 // running maximum and sum, everything in 32-bit with precise tanhf and expf.  Any
 // head size up to 1024, any number of heads and groups.  It is the 32-bit path's
 // attention, the reference of the tensor-core attention kernels, and the kernel for
@@ -53,43 +53,62 @@ attn_plain_kernel(const T* __restrict__ q, int q_stride, const T* __restrict__ k
     const int slot = PAGED ? seq_slot[seq] : 0;
     const size_t row0 = PAGED ? 0 : (size_t)cu_seqlens[seq];
 
-    for (int t = lo; t <= pos; ++t) {
-        const T* kp;
-        const T* vp;
-        int r = 0;
-        if (PAGED) {
-            const int lp = t / kPageTokens;
-            r = t % kPageTokens;
-            const int page = cache.page_table[(size_t)slot * cache.table_stride + kv_table_entry(cache, lp)];
-            const size_t tile = kv_tile_offset(cache, page, kvh);
-            kp = (const T*)cache.k_pages + tile;
-            vp = (const T*)cache.v_pages + tile;
-        } else {
-            kp = k_rows + (row0 + t) * kv_stride + (size_t)kvh * head_dim;
-            vp = v_rows + (row0 + t) * kv_stride + (size_t)kvh * head_dim;
+    // Keys four at a time (two of large heads): their loads, dot products and exponentials do not wait for one another, and the
+    // running sums are scaled once for all of them.  The 121-token prompt of an 8-head layer with 256 numbers a head
+    // takes 47 us so and 114 us with one key at a time, which is one chain of load, warp sum and exponential per key (165 us
+    // where the values are only asked for once the weights are there).
+    constexpr int KEYS = PL <= 8 ? 4 : 2;
+    for (int t = lo; t <= pos; t += KEYS) {
+        float s[KEYS], p[KEYS], v[KEYS][PL];
+#pragma unroll
+        for (int u = 0; u < KEYS; ++u) {
+            const int key = min(t + u, pos);       // beyond the last: read again, weight 0
+            const T* kp;
+            const T* vp;
+            int r = 0;
+            if (PAGED) {
+                const int lp = key / kPageTokens;
+                r = key % kPageTokens;
+                const int page = cache.page_table[(size_t)slot * cache.table_stride + kv_table_entry(cache, lp)];
+                const size_t tile = kv_tile_offset(cache, page, kvh);
+                kp = (const T*)cache.k_pages + tile;
+                vp = (const T*)cache.v_pages + tile;
+            } else {
+                kp = k_rows + (row0 + key) * kv_stride + (size_t)kvh * head_dim;
+                vp = v_rows + (row0 + key) * kv_stride + (size_t)kvh * head_dim;
+            }
+            float dot = 0.f;
+#pragma unroll
+            for (int i = 0; i < per_lane; ++i) {
+                const int d = lane + 32 * i;
+                v[u][i] = 0.f;
+                if (d < head_dim) {
+                    const int off = PAGED ? kv_elem_offset(r, d, head_dim) : d;
+                    dot = fmaf(qreg[i], to_float(kp[off]), dot);
+                    v[u][i] = to_float(vp[off]);        // on its way while the scores are formed
+                }
+            }
+            s[u] = dot;
         }
-        float dot = 0.f;
+        float m_new = m;
+#pragma unroll
+        for (int u = 0; u < KEYS; ++u) {
+            s[u] = softcap_precise(warp_sum(s[u]) * scale, cap);
+            m_new = fmaxf(m_new, s[u]);
+        }
+        const float corr = expf(m - m_new);      // exp(-inf) = 0 on the first keys
+        l *= corr;
+#pragma unroll
+        for (int u = 0; u < KEYS; ++u) {
+            p[u] = t + u <= pos ? expf(s[u] - m_new) : 0.f;
+            l += p[u];
+        }
 #pragma unroll
         for (int i = 0; i < per_lane; ++i) {
-            const int d = lane + 32 * i;
-            if (d < head_dim) {
-                const int off = PAGED ? kv_elem_offset(r, d, head_dim) : d;
-                dot = fmaf(qreg[i], to_float(kp[off]), dot);
-            }
-        }
-        dot = warp_sum(dot);
-        const float s = softcap_precise(dot * scale, cap);
-        const float m_new = fmaxf(m, s);
-        const float corr = expf(m - m_new);      // exp(-inf) = 0 on the first key
-        const float p = expf(s - m_new);
-        l = l * corr + p;
+            acc[i] *= corr;
 #pragma unroll
-        for (int i = 0; i < per_lane; ++i) {
-            const int d = lane + 32 * i;
-            if (d < head_dim) {
-                const int off = PAGED ? kv_elem_offset(r, d, head_dim) : d;
-                acc[i] = acc[i] * corr + p * to_float(vp[off]);
-            }
+            for (int u = 0; u < KEYS; ++u)
+                if (t + u <= pos) acc[i] = fmaf(p[u], v[u][i], acc[i]);
         }
         m = m_new;
     }
