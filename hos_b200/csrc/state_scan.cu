@@ -27,12 +27,15 @@
 // conv_act_rows: the short convolution with a bias and an activation on a run of columns, many tokens to a thread; with
 //   per-head step sizes: dt = softplus(raw + dt_bias) and the decay exp(-exp(A_log) dt) in the same launch.
 // channel_decay: logistic(W z + b)^(1 / tau) per key channel from a low-rank row z.
+#include <type_traits>
+
 #include "common.cuh"
 #include "short_conv.cuh"
 
 namespace hos {
 
 constexpr int kScanChunk = 8;       // tokens staged at a time
+constexpr int kDeepRing = 6;        // chunks in shared memory of a walk that has its SM to itself
 constexpr int kPad = 4;             // floats after every DR staged numbers: 16-byte reads of R neighbours miss each other's banks
 
 __device__ __forceinline__ float silu_precise(float x) { return x / (1.f + expf(-x)); }
@@ -44,7 +47,7 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit_all() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // x <- x logistic(x) on the first `cols` numbers of every row (the decay rule's q, k, v before the scan)
 __global__ void act_rows_kernel(float* __restrict__ x, long long ld, int cols, long long n) {
@@ -124,7 +127,7 @@ struct Segments {
     int len, count;
 };
 
-// A thread's cells: DR rows of DC neighbouring columns (DC > 1, the walks by segments: what is read of k, q and the decays
+// A thread's cells: DR rows of DC neighbouring columns (DC > 1, the walks by segments and the delta rule's long ones: what is read of k, q and the decays
 // serves DC columns).
 template <int DR, int R, int DC, int RULE, bool LOCAL>
 __global__ void __launch_bounds__(256)
@@ -133,7 +136,7 @@ state_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
                   long long beta_ld, float* __restrict__ state, const int* __restrict__ token_pos,
                   const int* __restrict__ token_seq, const int* __restrict__ cu_seqlens, const int* __restrict__ seq_slot,
                   float* __restrict__ out, int H, int Gk, int dim, int vdim, int CC, const float* __restrict__ rot_freq,
-                  int rot_dims, int rot_style, float k_mult, float o_mult, Segments sg) {
+                  int rot_dims, int rot_style, float k_mult, float o_mult, Segments sg, int n_buf) {
     constexpr bool DELTA = RULE == kDeltaRule, CHANNEL = RULE == kChannelRule;
     pdl_enter();
     extern __shared__ __align__(16) float sm[];
@@ -158,7 +161,7 @@ state_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
     const int n_cols = CC / DC;                  // threads' columns of this block
     auto live = [&](int j) { return c < n_cols && col + j < vdim; };
     const int dpad = R * (DR + kPad);
-    // two buffers of staged tokens: while one chunk is walked the next one's rows are on their way (cp.async)
+    // a ring of n_buf (2 or kDeepRing) buffers of staged tokens: while one chunk is walked the next ones' rows are on their way (cp.async)
     const int per_buf = kScanChunk * ((CHANNEL ? 3 : 2) * dpad + 2 * CC) + 2 * kScanChunk;      // q, k, (g,) v, o, g, beta
     const bool v_aligned = DC == 4 && (vdim & 3) == 0 && (ld & 3) == 0 && ((uintptr_t)v & 15) == 0;
     const bool v_scaled = RULE == kDecayRule && beta != nullptr;
@@ -188,8 +191,8 @@ state_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
             for (int i = 0; i < DR; ++i) S[j][i] = (!zero && live(j) && r * DR + i < dim) ? from[i] : 0.f;
         }
     }
-    uint64_t P[DC][DR / 2];                      // four columns: the cells as pairs of rows
-    if (DC == 4) {
+    uint64_t P[DC][DR / 2];                      // four columns, and the delta rule: the cells as pairs of rows
+    if (DC == 4 || DELTA) {
 #pragma unroll
         for (int j = 0; j < DC; ++j)
 #pragma unroll
@@ -197,7 +200,7 @@ state_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
     }
     // rows beyond dim and columns beyond vdim are read by the walk and never staged: they stay zero for good
     if (R * DR != dim || col0 + CC > vdim) {
-        for (int i = threadIdx.x; i < 2 * per_buf; i += blockDim.x) sm[i] = 0.f;
+        for (int i = threadIdx.x; i < n_buf * per_buf; i += blockDim.x) sm[i] = 0.f;
         __syncthreads();
     }
 
@@ -242,17 +245,23 @@ state_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
             if (!CHANNEL) cp_async4(gs + threadIdx.x, g + (size_t)(t0 + threadIdx.x) * g_ld + head);
             if (DELTA || v_scaled) cp_async4(bs + threadIdx.x, beta + (size_t)(t0 + threadIdx.x) * beta_ld + head);
         }
-        cp_async_commit_all();
     };
 
-    stage(lo, min(kScanChunk, hi - lo), sm);
+    for (int b = 0; b < n_buf - 1; ++b) {
+        const int t0 = lo + b * kScanChunk;
+        if (t0 < hi) stage(t0, min(kScanChunk, hi - t0), sm + b * per_buf);
+        cp_async_commit_all();
+    }
     int which = 0;
     float dec[kDecayPerThread] = {1.f, 1.f, 1.f, 1.f};       // first walks: the product of the segment's decays
-    for (int t0 = lo; t0 < hi; t0 += kScanChunk, which ^= 1) {
+    for (int t0 = lo; t0 < hi; t0 += kScanChunk, which = which + 1 == n_buf ? 0 : which + 1) {
         const int nt = min(kScanChunk, hi - t0);
-        cp_async_wait_all();
-        __syncthreads();            // this chunk has landed; everyone is done with the other buffer
-        if (t0 + kScanChunk < hi) stage(t0 + kScanChunk, min(kScanChunk, hi - t0 - kScanChunk), sm + (which ^ 1) * per_buf);
+        if (n_buf == 2) cp_async_wait<0>();
+        else cp_async_wait<kDeepRing - 2>();
+        __syncthreads();            // this chunk has landed; everyone is done with the buffer before it
+        const int ahead = t0 + (n_buf - 1) * kScanChunk;
+        if (ahead < hi) stage(ahead, min(kScanChunk, hi - ahead), sm + (which == 0 ? n_buf - 1 : which - 1) * per_buf);
+        cp_async_commit_all();
         float* qs = sm + which * per_buf;
         float* ks = qs + kScanChunk * dpad;
         if (!LOCAL && rot_in_walk) {
@@ -343,6 +352,97 @@ state_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
                 for (int o = R / 8; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
                 if ((r & (R / 4 - 1)) == 0 && c < n_cols) os[t * CC + c * DC + (up ? 2 : 0) + (up2 ? 1 : 0)] = acc * o_mult;
             }
+        } else if constexpr (DELTA) {
+            // Every thread walks (a warp's shuffles want all its lanes); only live columns are written.  A chain per token: the
+            // dot product over the column's threads, then the update.  Whole chunks have no branch in them, so that the
+            // tokens' reads and the products with q run beside the chain.
+            auto walk = [&](auto whole_chunk) {
+                constexpr bool FULL = decltype(whole_chunk)::value;
+                float part[DC][kScanChunk];   // the read-outs' partial sums: added up after the walk, off its chain
+#pragma unroll
+                for (int t = 0; t < kScanChunk; ++t) {
+                    if (!FULL && t >= nt) continue;
+                    const ulonglong2* k4 = (const ulonglong2*)(ks + t * dpad + r * (DR + kPad));
+                    const ulonglong2* q4 = (const ulonglong2*)(qs + t * dpad + r * (DR + kPad));
+                    const uint64_t gt = pair_of(gs[t], gs[t]);
+                    ulonglong2 kk[DR / 4];
+                    float dot[DC];
+                    uint64_t d01[DC], d23[DC];          // four chains a column, not one of DR links
+#pragma unroll
+                    for (int i = 0; i < DR / 4; ++i) {
+                        kk[i] = k4[i];
+#pragma unroll
+                        for (int j = 0; j < DC; ++j) {
+                            P[j][2 * i] = mul_pair(gt, P[j][2 * i]);
+                            P[j][2 * i + 1] = mul_pair(gt, P[j][2 * i + 1]);
+                            d01[j] = fma_pair(P[j][2 * i], kk[i].x, i == 0 ? 0 : d01[j]);
+                            d23[j] = fma_pair(P[j][2 * i + 1], kk[i].y, i == 0 ? 0 : d23[j]);
+                        }
+                    }
+#pragma unroll
+                    for (int j = 0; j < DC; ++j) {
+                        float d0, d1, d2, d3;
+                        halves_of(d01[j], d0, d1);
+                        halves_of(d23[j], d2, d3);
+                        dot[j] = (d0 + d1) + (d2 + d3);
+                    }
+#pragma unroll
+                    for (int o = 1; o < R; o <<= 1)
+#pragma unroll
+                        for (int j = 0; j < DC; ++j) dot[j] += __shfl_xor_sync(0xffffffffu, dot[j], o);
+#pragma unroll
+                    for (int j = 0; j < DC; ++j) {
+                        const float u = bs[t] * ((c < n_cols ? vs[t * CC + c * DC + j] : 0.f) - dot[j]);
+                        const uint64_t uu = pair_of(u, u);
+                        uint64_t a01 = 0, a23 = 0;
+#pragma unroll
+                        for (int i = 0; i < DR / 4; ++i) {
+                            const ulonglong2 qq = q4[i];
+                            P[j][2 * i] = fma_pair(kk[i].x, uu, P[j][2 * i]);
+                            P[j][2 * i + 1] = fma_pair(kk[i].y, uu, P[j][2 * i + 1]);
+                            a01 = fma_pair(P[j][2 * i], qq.x, a01);
+                            a23 = fma_pair(P[j][2 * i + 1], qq.y, a23);
+                        }
+                        float a0, a1, a2, a3;
+                        halves_of(a01, a0, a1);
+                        halves_of(a23, a2, a3);
+                        part[j][t] = (a0 + a1) + (a2 + a3);
+                    }
+                }
+                if constexpr (FULL && R >= kScanChunk) {
+                    // eight tokens' sums over R threads: with every turn a thread hands on half of the tokens it still has
+                    static_assert(kScanChunk == 8, "three turns");
+#pragma unroll
+                    for (int j = 0; j < DC; ++j) {
+                        const float(&p)[kScanChunk] = part[j];
+                        float four[4], two[2];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            four[i] = ((r & 1) ? p[i + 4] : p[i]) + __shfl_xor_sync(0xffffffffu, (r & 1) ? p[i] : p[i + 4], 1);
+#pragma unroll
+                        for (int i = 0; i < 2; ++i)
+                            two[i] = ((r & 2) ? four[i + 2] : four[i]) + __shfl_xor_sync(0xffffffffu, (r & 2) ? four[i] : four[i + 2], 2);
+                        float acc = ((r & 4) ? two[1] : two[0]) + __shfl_xor_sync(0xffffffffu, (r & 4) ? two[0] : two[1], 4);
+#pragma unroll
+                        for (int o = 8; o < R; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+                        const int t = (r & 1) * 4 + (r & 2) + ((r & 4) >> 2);
+                        if (r < 8 && c < n_cols) os[t * CC + c * DC + j] = acc * o_mult;
+                    }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < DC; ++j)
+#pragma unroll
+                        for (int t = 0; t < kScanChunk; ++t) {
+                            if (!FULL && t >= nt) break;
+                            float acc = part[j][t];
+#pragma unroll
+                            for (int o = 1; o < R; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+                            if (r == 0 && c < n_cols) os[t * CC + c * DC + j] = acc * o_mult;
+                        }
+                }
+            };
+            if (nt == kScanChunk) walk(std::true_type{});
+            else walk(std::false_type{});
         } else {       // every thread walks (a warp's shuffles want all its lanes); only live columns are written
             float part[kScanChunk];       // the read-outs' partial sums: added up after the walk, off its chain
 #pragma unroll
@@ -356,22 +456,6 @@ state_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
                 float u = c < n_cols ? vs[t * CC + c] : 0.f;
                 if (RULE == kDecayRule && act_in_walk) u = silu_precise(u);      // single tokens: the activation rides here
                 if (v_scaled) u *= bs[t];
-                if (DELTA) {
-                    float d0 = 0.f, d1 = 0.f, d2 = 0.f, d3 = 0.f;       // four chains, not one of DR links
-#pragma unroll
-                    for (int i = 0; i < DR / 4; ++i) {
-                        const float4 kk = k4[i];
-                        S[0][4 * i] *= gt; S[0][4 * i + 1] *= gt; S[0][4 * i + 2] *= gt; S[0][4 * i + 3] *= gt;
-                        d0 = fmaf(S[0][4 * i], kk.x, d0);
-                        d1 = fmaf(S[0][4 * i + 1], kk.y, d1);
-                        d2 = fmaf(S[0][4 * i + 2], kk.z, d2);
-                        d3 = fmaf(S[0][4 * i + 3], kk.w, d3);
-                    }
-                    float dot = (d0 + d1) + (d2 + d3);
-#pragma unroll
-                    for (int o = 1; o < R; o <<= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-                    u = bs[t] * (u - dot);
-                }
                 float a[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
                 for (int i = 0; i < DR / 4; ++i) {
@@ -382,17 +466,10 @@ state_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
                     }
                     const float4 gg = CHANNEL ? g4[i] : make_float4(gt, gt, gt, gt);
                     float* s4 = &S[0][4 * i];
-                    if (DELTA) {
-                        s4[0] = fmaf(kk.x, u, s4[0]);
-                        s4[1] = fmaf(kk.y, u, s4[1]);
-                        s4[2] = fmaf(kk.z, u, s4[2]);
-                        s4[3] = fmaf(kk.w, u, s4[3]);
-                    } else {
-                        s4[0] = fmaf(gg.x, s4[0], kk.x * u);
-                        s4[1] = fmaf(gg.y, s4[1], kk.y * u);
-                        s4[2] = fmaf(gg.z, s4[2], kk.z * u);
-                        s4[3] = fmaf(gg.w, s4[3], kk.w * u);
-                    }
+                    s4[0] = fmaf(gg.x, s4[0], kk.x * u);
+                    s4[1] = fmaf(gg.y, s4[1], kk.y * u);
+                    s4[2] = fmaf(gg.z, s4[2], kk.z * u);
+                    s4[3] = fmaf(gg.w, s4[3], kk.w * u);
                     if (LOCAL) continue;
                     a[0] = fmaf(s4[0], qq.x, a[0]);
                     a[1] = fmaf(s4[1], qq.y, a[1]);
@@ -440,7 +517,7 @@ state_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
     } else if (!last) {
         return;                                  // only the last segment's state is the sequence's
     }
-    if (DC == 4) {
+    if (DC == 4 || DELTA) {
 #pragma unroll
         for (int j = 0; j < DC; ++j)
 #pragma unroll
@@ -694,7 +771,7 @@ namespace hos {
 // How a walk is cut: DR rows of a column to a thread, R threads to a column, CC columns to a block.
 struct ScanShape {
     int DR, R, CC, DC = 1;
-    ScanShape(int dim, int vdim, bool segments = false) {
+    ScanShape(int dim, int vdim, bool segments = false, bool long_delta = false) {
         // short runs of rows per thread: a token's walk is a chain of dependent instructions (scale, dot, sum over the
         // runs, update, read-out, sum), and with few (sequence, head) pairs nothing else hides its latency; the sums over
         // 16 or 32 runs are shuffles
@@ -706,6 +783,7 @@ struct ScanShape {
         if (DR == 8 && R < 4) R = 4;          // the compiled shapes (rows beyond dim are zeros)
         if (DR >= 16) R = 32;
         if (segments && DR == 8) DC = 4;      // the shapes that are compiled for four columns to a thread
+        if (long_delta && DR == 8) DC = 2;    // and for two
         CC = 256 / R * DC;
         if (CC > vdim) CC = (vdim + DC - 1) / DC * DC;
     }
@@ -751,7 +829,12 @@ extern "C" int hos_state_scan(const float* q, const float* k, const float* v, lo
     if (Gk <= 0 || H % Gk != 0) HOS_REFUSE("state_scan: %d heads are not a multiple of %d key heads", H, Gk);
     if (dim <= 0 || dim > 1024 || vdim <= 0) HOS_REFUSE("state_scan: heads of %d x %d", dim, vdim);
     const bool segments = seg_count > 1;
-    const ScanShape shape(dim, vdim, segments);
+    const bool long_walk = n_rows >= 4ll * kScanChunk * n_seqs;
+    // The delta rule's long walks, where they fill the SMs several times over: two columns to a thread share what is read of k and
+    // q (four prompts of 300 to 1,000 tokens: a layer's walk goes with the step from 5.89 to 5.67 ms; a walk that has its SM to
+    // itself is bound by its chain and has nothing of it: 504 us for 2,048 tokens with one column, 521 with two).
+    const bool many = (long long)n_seqs * H * vdim * 16 > 2ll * 256 * sm_count_cached();
+    const ScanShape shape(dim, vdim, segments, rule == kDeltaRule && long_walk && many);
     const int DR = shape.DR, R = shape.R, DC = shape.DC;
     int CC = shape.CC;
     // single tokens and few (sequence, head) pairs: fewer columns to a block, so that the blocks fill the GPU (columns
@@ -768,10 +851,17 @@ extern "C" int hos_state_scan(const float* q, const float* k, const float* v, lo
         HOS_REFUSE("state_scan: rule %d and its inputs do not fit", rule);
     if (rule == kChannelRule && Gk != H) HOS_REFUSE("state_scan: the channel rule has a key head per head");
     const int wide_rows = rule == kChannelRule ? 3 : 2;
-    const size_t smem = (size_t)2 * (wide_rows * kScanChunk * dpad + 2 * kScanChunk * CC + 2 * kScanChunk) * sizeof(float);
+    const size_t per_buf = (size_t)(wide_rows * kScanChunk * dpad + 2 * kScanChunk * CC + 2 * kScanChunk) * sizeof(float);
     const int aligned = (dim % 4 == 0 && ld % 4 == 0 && (uintptr_t)q % 16 == 0 && (uintptr_t)k % 16 == 0 &&
                          (rule != kChannelRule || (g_ld % 4 == 0 && (uintptr_t)g % 16 == 0))) ? 1 : 0;
     const dim3 grid(n_seqs * sg.count, H, (vdim + CC - 1) / CC);
+    // Few long walks have an SM (almost) to themselves, and nothing but the ring hides the way of their rows from memory: two
+    // chunks of eight tokens are not enough (the delta rule, 16 heads of 128 x 128, 2,048 tokens: with a deeper ring and pairs
+    // of rows in one instruction 723 -> 504 us).  More walks than that hide one another's loads, and shared memory for more of
+    // them at once is worth more.
+    const bool alone = (long long)grid.x * grid.y * grid.z <= 2ll * sm_count_cached() && long_walk;
+    const int n_buf = alone && kDeepRing * per_buf <= 100 * 1024 ? kDeepRing : 2;
+    const size_t smem = n_buf * per_buf;
     if (rule != kDecayRule && act_in_walk) HOS_REFUSE("state_scan: the activation in the walk is the decay rule's");
     if (smem > 200 * 1024) HOS_REFUSE("state_scan: heads of %d x %d do not fit a block's shared memory", dim, vdim);
 #define HOS_SCAN(DRv, Rv, DCv, DL, LOC)                                                                                   \
@@ -780,7 +870,7 @@ extern "C" int hos_state_scan(const float* q, const float* k, const float* v, lo
             cudaFuncSetAttribute(state_scan_kernel<DRv, Rv, DCv, DL, LOC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
         launch_pdl(state_scan_kernel<DRv, Rv, DCv, DL, LOC>, grid, dim3(threads), smem, stream, q, k, v, ld, aligned, act_in_walk, g, g_ld, beta, \
                    beta_ld, state, token_pos, token_seq, cu_seqlens, seq_slot, out, H, Gk, dim, vdim, CC, rot_freq,  \
-                   rot_dims, rot_style, k_mult, o_mult, sg);                                                         \
+                   rot_dims, rot_style, k_mult, o_mult, sg, n_buf);                                                         \
     } while (0)
 #define HOS_SCAN_S(DRv, Rv, DL)                                                                                      \
     do {                                                                                                             \
@@ -796,7 +886,9 @@ extern "C" int hos_state_scan(const float* q, const float* k, const float* v, lo
     } while (0)
 #define HOS_SCAN_D(DRv, Rv)                                                                                          \
     do {                                                                                                             \
-        if (rule == kDeltaRule) HOS_SCAN(DRv, Rv, 1, kDeltaRule, false);                                              \
+        constexpr int DCd = DRv == 8 ? 2 : 1;                                                                        \
+        if (rule == kDeltaRule && DC == 1) HOS_SCAN(DRv, Rv, 1, kDeltaRule, false);                                  \
+        else if (rule == kDeltaRule) HOS_SCAN(DRv, Rv, DCd, kDeltaRule, false);                                      \
         else if (rule == kChannelRule) HOS_SCAN_S(DRv, Rv, kChannelRule);                                            \
         else HOS_SCAN_S(DRv, Rv, kDecayRule);                                                                        \
     } while (0)
