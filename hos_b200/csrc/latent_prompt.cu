@@ -7,18 +7,17 @@
 //   a key's unrotated part [W_uk_h c]   two bfloat16 terms (16 bits of mantissa), as the absorbed query has there
 //   a query's rotated part              two terms
 //   a query's unrotated part, a key's rotated part (the cache's own row)   bfloat16 as projected or stored: exact
-//   the weights                         two terms
-// and the values W_uv_h c are rounded to bfloat16 where the absorbed form rounds its weighted sums of latents.
+//   a value W_uv_h c, the weights       two terms
 //
 // The kernel is the walk of attention_prefill_tc.cu: one CTA takes 128 consecutive queries of one sequence and one head and
 // walks over tiles of 64 keys; S = Q K^T from four products of 64 numbers (q k_hi, q k_lo, r_hi r_key, r_lo r_key) into tensor
-// memory (two buffers), eight softmax warps (two threads per row), O += P_hi V + P_lo V.  Sizes up to 64 + 64 numbers a key and 128
-// a value fit: smaller ones are padded with zeros as they are written.
+// memory (two buffers), eight softmax warps (two threads per row), O += P_hi V_hi + P_lo V_hi + P_hi V_lo.
+// Sizes up to 64 + 64 numbers a key and 128 a value fit: smaller ones are padded with zeros as they are written.
 //
-// Measured (B200, 16 heads, 64 + 64 and 128 numbers, rank 512, a window of 1,024 of 2,048 tokens): product 24 us, expansion 22,
-// walk 53 (what bounds it: 256 CTAs of up to 18 tiles on 148 SMs, one at a time, about 1.3 us a tile); the absorbed form took 117 + 943 +
-// 38 us with its products before and after.  Nuvivik's prompt of 2,048 tokens 9.50 -> 3.91 ms, of 4,000 19.3 -> 7.1, of 512 2.36
-// -> 1.67, of 64 1.03 -> 0.97.
+// Measured (B200, 16 heads, 64 + 64 and 128 numbers, rank 512, a window of 1,024 of 2,048 tokens): product 19 us, expansion 12,
+// walk 57 (50 with the values as one term; what bounds it: 256 CTAs of up to 18 tiles on 148 SMs, one at a time, 1.4 us a tile); the
+// absorbed form took 117 + 943 + 38 us with its products before and after.  Nuvivik's prompt of 2,048 tokens 9.50 -> 3.95 ms, of 4,000
+// 19.3 -> 7.1, of 512 2.36 -> 1.67, of 64 1.03 -> 0.97.
 #include "common.cuh"
 #include "latent_rot.cuh"
 #include "mma_utils.cuh"
@@ -28,9 +27,9 @@ namespace hos {
 
 constexpr int LQ = 128, LK = 64;                        // queries of a CTA, keys of a tile
 constexpr int LDIM = 64, LVDIM = 128;                   // numbers of a key's two parts, of a value, as laid out
-constexpr int kLqCols = 3 * LDIM, kLkCols = 2 * LDIM;   // [q | r_hi | r_lo], [k_hi | k_lo] of a row and head
+constexpr int kLqCols = 3 * LDIM, kLkCols = 2 * LDIM, kLvCols = 2 * LVDIM;    // [q | r_hi | r_lo], [k_hi | k_lo], [v_hi | v_lo]
 constexpr int kLqBlock = LQ * 128, kLkBlock = LK * 128; // a column block of 64 numbers of the queries, of a tile
-constexpr int kLqBytes = 3 * kLqBlock, kLkBytes = 3 * kLkBlock, kLvBytes = LVDIM / 64 * kLkBlock;
+constexpr int kLqBytes = 3 * kLqBlock, kLkBytes = 3 * kLkBlock, kLvTerm = LVDIM / 64 * kLkBlock, kLvBytes = 2 * kLvTerm;
 constexpr int kLStages = 2, kLpBytes = 2 * LQ * 128;    // the weights' two terms
 constexpr int kLSmem = kLqBytes + kLStages * (kLkBytes + kLvBytes) + 2 * kLpBytes + 2 * LQ * 4 + 160 + 976;
 constexpr int kLThreads = 320;
@@ -68,7 +67,7 @@ struct LatentExpand {
     const int* token_seq;
     bf16* q_out;                // [n][H][192]
     bf16* k_out;                // [n][H][128]
-    bf16* v_out;                // [n][H][128]
+    bf16* v_out;                // [n][H][256]
 };
 
 __device__ __forceinline__ void split4(const float (&x)[4], uint2& hi, uint2& lo) {
@@ -82,9 +81,9 @@ __global__ void __launch_bounds__(256) latent_expand_kernel(LatentExpand a) {
     pdl_enter();
     __shared__ float2 sincos_tab[LDIM / 2];
     const int n = blockIdx.x, H = a.H;
-    bf16* v_out = a.v_out + (size_t)n * H * LVDIM;
+    bf16* v_out = a.v_out + (size_t)n * H * kLvCols;
     if (a.token_seq[n] < 0) {   // padding: nobody's key, but its values may lie in a tile with weight 0
-        for (int i = threadIdx.x; i < H * LVDIM / 4; i += blockDim.x) reinterpret_cast<uint2*>(v_out)[i] = make_uint2(0u, 0u);
+        for (int i = threadIdx.x; i < H * kLvCols / 4; i += blockDim.x) reinterpret_cast<uint2*>(v_out)[i] = make_uint2(0u, 0u);
         return;
     }
     const float pos = (float)a.token_pos[n];
@@ -123,12 +122,14 @@ __global__ void __launch_bounds__(256) latent_expand_kernel(LatentExpand a) {
     const float* v = kv + (size_t)H * a.dq;
     for (int i = threadIdx.x; i < H * LVDIM / 4; i += blockDim.x) {
         const int h = i / (LVDIM / 4), c = i % (LVDIM / 4) * 4;
-        uint2 out = make_uint2(0u, 0u);
+        uint2 hi = make_uint2(0u, 0u), lo = hi;
         if (c < a.vd) {
-            const float4 x = *reinterpret_cast<const float4*>(v + (size_t)h * a.vd + c);
-            out = make_uint2(pack_bf16(x.x, x.y), pack_bf16(x.z, x.w));
+            const float4 t = *reinterpret_cast<const float4*>(v + (size_t)h * a.vd + c);
+            const float x[4] = {t.x, t.y, t.z, t.w};
+            split4(x, hi, lo);
         }
-        reinterpret_cast<uint2*>(v_out)[i] = out;
+        *reinterpret_cast<uint2*>(v_out + h * kLvCols + c) = hi;
+        *reinterpret_cast<uint2*>(v_out + h * kLvCols + LVDIM + c) = lo;
     }
 }
 
@@ -225,8 +226,8 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap map_q,      // queries,
                 tc_tma_2d(kd + 2 * kLkBlock, &map_r, a.rank, krow, &k_full[s]);
                 if (j >= kLStages && !latent_wait(&v_empty[s], ((j / kLStages) - 1) & 1)) { ok = false; break; }
                 mbar_expect_tx(&v_full[s], kLvBytes);
-                for (int c = 0; c < LVDIM / 64; ++c)
-                    tc_tma_2d(vd + c * kLkBlock, &map_v, head * LVDIM + 64 * c, krow, &v_full[s]);
+                for (int c = 0; c < kLvCols / 64; ++c)
+                    tc_tma_2d(vd + c * kLkBlock, &map_v, head * kLvCols + 64 * c, krow, &v_full[s]);
             }
             if (!ok) latent_give_up();
         }
@@ -265,11 +266,11 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap map_q,      // queries,
                 tc_fence_after_sync();
                 const uint32_t v_addr = smem_u32(v_s + s * kLvBytes), p_addr = smem_u32(p_s + pb * kLpBytes);
 #pragma unroll
-                for (int term = 0; term < 2; ++term)
+                for (int term = 0; term < 3; ++term)                 // P_hi V_hi, P_lo V_hi, P_hi V_lo
 #pragma unroll
                     for (int ks = 0; ks < LK / 16; ++ks)
-                        tc_mma(tmem_base + kLColO, desc_kmajor(p_addr + term * LQ * 128) + 2 * ks,
-                               desc_mnmajor(v_addr + ks * 16 * 128, kLkBlock), idesc_o, (j > 0 || term > 0 || ks > 0) ? 1u : 0u);
+                        tc_mma(tmem_base + kLColO, desc_kmajor(p_addr + (term == 1 ? LQ * 128 : 0)) + 2 * ks,
+                               desc_mnmajor(v_addr + (term == 2 ? kLvTerm : 0) + ks * 16 * 128, kLkBlock), idesc_o, (j > 0 || term > 0 || ks > 0) ? 1u : 0u);
                 tc_commit(&v_empty[s]);
                 tc_commit(&pv_done[pb]);      // this P buffer has been read, O holds tile j
             }
@@ -363,7 +364,7 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap map_q,      // queries,
                 const int s = j % kLStages, vr = (int)(threadIdx.x - 64) >> 2, part = threadIdx.x & 3;
                 if (!latent_wait(&v_full[s], (j / kLStages) & 1)) { ok = false; break; }
                 if (kt0 + vr >= len)
-                    for (int c = part * 4; c < part * 4 + 4; ++c)
+                    for (int c = part * 8; c < part * 8 + 8; ++c)
                         *reinterpret_cast<uint4*>(v_s + s * kLvBytes + (c >> 3) * kLkBlock + vr * 128 + (c & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // generic writes -> visible to the tensor core
@@ -420,7 +421,7 @@ extern "C" int hos_latent_prompt_set_error_word(int* word) {
 
 // Rows 0 .. n_rows - 1 of a step whose sequences all start at position 0 (sequence s has the rows cu_seqlens[s] ..).
 // q: row n, head h at q + n * ldq + h * (dq + P); kv: 32-bit [n_rows][H * dq + H * vd], the latents expanded; kc: the latent
-// rows [n_rows][rank + P].  q_ws [n_rows][H][192], k_ws and v_ws [n_rows][H][128] bfloat16: scratch.  out [n_rows][H * vd].
+// rows [n_rows][rank + P].  q_ws [n_rows][H][192], k_ws [n_rows][H][128] and v_ws [n_rows][H][256] bfloat16: scratch.  out [n_rows][H * vd].
 // n_q_tiles: at least the sum over the sequences of ceil(rows / 128).
 extern "C" int hos_latent_prompt(const void* q, long long ldq, const float* kv, const void* kc, const float* inv_freq, int rot_dims,
                                  int style, const float* sink, const int* token_pos, const int* token_seq, const int* cu_seqlens,
@@ -439,7 +440,7 @@ extern "C" int hos_latent_prompt(const void* q, long long ldq, const float* kv, 
     if ((rc = tc_make_map(&mq, q_ws, n_rows, H * kLqCols, H * kLqCols, LQ))) return rc;
     if ((rc = tc_make_map(&mk, k_ws, n_rows, H * kLkCols, H * kLkCols, LK))) return rc;
     if ((rc = tc_make_map(&mr, kc, n_rows, rank + P, rank + P, LK))) return rc;
-    if ((rc = tc_make_map(&mv, v_ws, n_rows, H * LVDIM, H * LVDIM, LK))) return rc;
+    if ((rc = tc_make_map(&mv, v_ws, n_rows, H * kLvCols, H * kLvCols, LK))) return rc;
     if (cudaFuncSetAttribute(latent_prompt_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kLSmem) != cudaSuccess)
         HOS_REFUSE("latent_prompt: cannot get %d bytes of shared memory", kLSmem);
     LatentExpand e = {(const bf16*)q, kv, ldq, H, dq, P, vd, {inv_freq, inv_freq != nullptr ? rot_dims : 0, style}, token_pos, token_seq,

@@ -715,7 +715,7 @@ def latent_prompt(q: torch.Tensor, dq: int, vd: int, inv_freq: Optional[torch.Te
     if kv.shape != (rows, heads * (dq + vd)) or q.shape[1] < heads * (dq + rot) or min(q.shape[0], kc.shape[0], out.shape[0]) < rows:
         raise KernelError("latent_prompt: sizes disagree")
     a, b, c = LATENT_PROMPT_SIZES
-    ws = torch.empty((3 * a + 2 * a + c) * heads * rows, dtype=torch.bfloat16, device=q.device)
+    ws = torch.empty((3 * a + 2 * a + 2 * c) * heads * rows, dtype=torch.bfloat16, device=q.device)
     k_ws, v_ws = ws[3 * a * heads * rows:], ws[5 * a * heads * rows:]
     n_seqs = step.fresh_seqs or step.n_seqs
     lens = [step.cu_host[i + 1] - step.cu_host[i] for i in range(n_seqs)] if step.cu_host else []

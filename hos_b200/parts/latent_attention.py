@@ -7,7 +7,7 @@ numbers, not normed).  A head's key is [W_uk_h c | rotated part], its value W_uv
 mask is causal with an optional window of the last `window` keys; with `sink`, a learned number
 per head joins the softmax's denominator as exp(sink_h) (no key, no value, unscaled).
 
-Prompts of 64 rows or more whose sizes fit form keys and values (one product of the latents, then the tcgen05 walk of
+Prompts of many rows whose sizes fit form keys and values (one product of the latents, then the tcgen05 walk of
 csrc/latent_prompt.cu: less arithmetic per pair).  Elsewhere neither is formed: the query absorbs W_uk (q'_h = W_uk_h^T q_h, `kv_rank`
 numbers) and W_uv is applied to the weighted sum of latents, so the attention kernel reads
 `kv_rank + rot_dim` numbers per key for all heads.  Everything between the projections (norm of
@@ -42,10 +42,12 @@ from . import linear
 from .base import CallStore, KVNeed, Mixer, StepInfo, WeightSpec
 
 
-# From so many rows that start at position 0 on their keys and values are formed.  Measured against the absorbed form (eight
-# layers of Nuvivik, one prompt): 64 rows 0.97 against 1.03 ms, 128 rows 1.12 / 1.24, 512 rows 1.67 / 2.36, 4,000 rows 7.1 / 19.3;
-# fewer rows have their keys cut into shares there, which this walk does not do.
+# From so many rows that start at position 0 on their keys and values are formed, if there are also PROMPT_WORK numbers of
+# latents: what the absorbed form pays grows with the rank, the formed one's walk does not.  Measured, absorbed / formed: eight
+# layers of Nuvivik (rank 512) with 64 rows 1.03 / 0.97 ms, 128 rows 1.24 / 1.12, 512 rows 2.36 / 1.67, 4,000 rows 19.3 / 7.1; one
+# layer's attention at 256 rows with rank 512, 256 and 128: 69 / 51, 43 / 37 and 37 / 43 us; at 1,024 rows with rank 24: 161 / 53.
 PROMPT_ROWS = 64
+PROMPT_WORK = 64 * 512
 
 
 class LatentAttention(Mixer):
@@ -177,7 +179,7 @@ class LatentAttention(Mixer):
         att = torch.empty((n, H * self.vdim), dtype=h.dtype, device=h.device)
         nf = 0 if self.shares_kv else (n if step.from_zero else step.fresh_tokens)
         done = 0
-        if nf >= PROMPT_ROWS and self.w_expand is not None and self.use_tensor_cores and not step.single_token:
+        if nf >= PROMPT_ROWS and nf * R >= PROMPT_WORK and self.w_expand is not None and self.use_tensor_cores and not step.single_token:
             kv = linear.matmul(kc[:nf], self.w_expand, out_dtype=torch.float32)
             ops.latent_prompt(q, self.dim, self.vdim, inv_freq, rot_dims, style, kv, kc, self.sink, att, step, nf, R, self.scale,
                               self.window)

@@ -1184,9 +1184,8 @@ def test_gemm_f32(shape):
 @pytest.mark.parametrize("sizes", [(64, 64, 128, 512, 0), (64, 64, 128, 512, 100), (48, 32, 64, 72, 0), (8, 16, 40, 64, 65)])
 @pytest.mark.parametrize("lens", [(64,), (1, 63, 130, 257), (500, 128)])
 def test_latent_prompt(sizes, lens):
-    """The walk over formed keys and values against the same in 64 bits, with the values rounded to bfloat16 as the kernel
-    reads them: what is left is the output's own rounding (eight bits of significand: up to 2^-8 of it) and terms of 16 bits in
-    keys and weights (2^-16 of a score of size ten, so 2^-12 of a value).  Padding rows
+    """The walk over formed keys and values against the same in 64 bits: what is left is the output's own rounding (eight bits of
+    significand: up to 2^-8 of it) and terms of 16 bits in keys, values and weights (2^-16 of a score of size ten, so 2^-12 of a value).  Padding rows
     lie behind the sequences, and a sequence's infinite values must not reach its neighbour."""
     from types import SimpleNamespace
     from hos_b200 import ops
@@ -1221,7 +1220,7 @@ def test_latent_prompt(sizes, lens):
         r[..., :half] = qq[..., dq:dq + half] * c - qq[..., dq + half:dq + rot_dims] * z
         r[..., half:rot_dims] = qq[..., dq + half:dq + rot_dims] * c + qq[..., dq:dq + half] * z
         k = kv[s, : H * dq].double().view(x, H, dq)
-        v = kv[s, H * dq:].bfloat16().double().view(x, H, vd)
+        v = kv[s, H * dq:].double().view(x, H, vd)
         score = (torch.einsum("ihd,jhd->hij", qq[..., :dq], k) + torch.einsum("ihd,jd->hij", r, kc[s, R:].double())) * scale
         d = torch.arange(x, device=DEV)[:, None] - torch.arange(x, device=DEV)[None]
         hidden = (d < 0) | ((d >= window) if window else torch.zeros_like(d, dtype=torch.bool))
