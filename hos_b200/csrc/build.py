@@ -54,7 +54,7 @@ _STATIC_LIBS: Dict[str, Tuple[List[str], List[str]]] = {
     "gemm_tc": (["gemm_tc.cu"], []),
     "gemm_skinny": (["gemm_skinny.cu"], []),
     "rows": (["embed_pair.cu", "dyt_norm.cu"], []),
-    "experts": (["moe.cu"], []),
+    "experts": (["moe.cu", "moe_grouped.cu"], []),
     "blocks": (["latent_attention.cu", "latent_prompt.cu", "wkv.cu"], []),
     "gated_attn": (["gated_attention.cu", "gated_attention_mma.cu"], []),
     "mixers": (["postnorm.cu", "state_scan.cu", "hyper.cu"], []),

@@ -7,7 +7,7 @@
 //             The last `n_identity` router outputs are experts without tensors: their output is
 //             the row itself.
 //   align     the chosen (row, choice) pairs listed expert by expert, each expert's list padded to
-//             whole tiles of kTile rows, and the expert of every tile.
+//             whole tiles, and the expert of every tile.
 //   gate_up   per tile, the expert's gate and up products of the listed rows and the activation
 //             y = g' * sigmoid(alpha * g') * (u' + 1), g' = min(g, limit), u' = clamp(u, -limit, limit)
 //             (limit <= 0: no clamp; the 1 is `up_shift`, 0 for the plain gated form g' sigmoid(alpha g') u').  With
@@ -20,8 +20,10 @@
 //             as weight * row, plus the row of `extra` if given (an expert that every row uses).
 // The grid of the tiled kernels is the most tiles the step can have; tiles beyond the real ones
 // leave at once, so nothing depends on the host knowing the counts.  Products accumulate in 32-bit;
-// a warp whose rows of a tile are all padding skips the arithmetic.
+// a warp whose rows of a tile are all padding skips the arithmetic.  In bfloat16 with more pairs than a handful the two products
+// are those of moe_grouped.cu; the tiled kernels here are the 32-bit path's and take the sizes that one refuses.
 #include "common.cuh"
+#include "expert_act.cuh"
 #include "mma_tile.cuh"
 
 namespace hos {
@@ -31,22 +33,6 @@ __device__ __forceinline__ float4 route_load4(const bf16* p) {
     const uint2 u = *(const uint2*)p;
     return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16),
                        __uint_as_float(u.y & 0xffff0000u));
-}
-
-enum ExpertAct : int { kGatedSwish = 0, kReluSquare = 1 };
-
-// y of an expert's inner number from its 32-bit gate and up products (kReluSquare: from the up product, given as g)
-template <int ACT>
-__device__ __forceinline__ float expert_act(float g, float u, float limit, float alpha, float up_shift) {
-    if (ACT == kReluSquare) {
-        const float r = fmaxf(g, 0.f);
-        return r * r;
-    }
-    if (limit > 0.f) {
-        g = fminf(g, limit);
-        u = fminf(fmaxf(u, -limit), limit);
-    }
-    return g / (1.f + expf(-alpha * g)) * (u + up_shift);
 }
 
 // One warp: the outputs outside the `keep` best of `groups` equal groups are marked as taken.  gs: [groups] in shared memory;
@@ -297,7 +283,7 @@ moe_choose_kernel(const float* __restrict__ logits, const float* __restrict__ co
 // One block.  listed: [cap] pair ids (row * top + choice) expert by expert, -1 where a tile is padded;
 // tile_expert: [max_tiles], -1 beyond the real tiles.
 __global__ void moe_align_kernel(const int* __restrict__ choice, int n_pairs, int n_experts, int* __restrict__ listed,
-                                 int cap, int* __restrict__ tile_expert, int max_tiles) {
+                                 int cap, int* __restrict__ tile_expert, int max_tiles, int tile_rows) {
     pdl_enter();
     extern __shared__ int sh[];                // count[n_experts], start[n_experts + 1], cursor[n_experts]
     int* count = sh;
@@ -314,13 +300,13 @@ __global__ void moe_align_kernel(const int* __restrict__ choice, int n_pairs, in
         int at = 0;
         for (int e = 0; e < n_experts; ++e) {
             start[e] = at;
-            const int tiles = (count[e] + kTile - 1) / kTile;
+            const int tiles = (count[e] + tile_rows - 1) / tile_rows;
             for (int t = 0; t < tiles; ++t)
-                if (at / kTile + t < max_tiles) tile_expert[at / kTile + t] = e;
-            at += tiles * kTile;
+                if (at / tile_rows + t < max_tiles) tile_expert[at / tile_rows + t] = e;
+            at += tiles * tile_rows;
         }
         start[n_experts] = at;
-        for (int t = at / kTile; t < max_tiles; ++t) tile_expert[t] = -1;
+        for (int t = at / tile_rows; t < max_tiles; ++t) tile_expert[t] = -1;
     }
     __syncthreads();
     const int used = min(start[n_experts], cap);
@@ -795,12 +781,13 @@ extern "C" int hos_moe_route(const void* h, int dtype, const float* router, cons
 }
 
 extern "C" int hos_moe_align(const int* choice, int n_pairs, int n_experts, int* listed, int cap, int* tile_expert,
-                             int max_tiles, cudaStream_t stream) {
+                             int max_tiles, int tile_rows, cudaStream_t stream) {
     if (n_pairs <= 0) return 0;
+    if (tile_rows <= 0) HOS_REFUSE("moe_align: tiles of %d rows", tile_rows);
     const size_t smem = (size_t)(3 * n_experts + 1) * sizeof(int);
     if (smem > 48 * 1024) HOS_REFUSE("moe_align: %d experts are more than a block's shared memory holds", n_experts);
     launch_pdl(moe_align_kernel, dim3(1), dim3(1024), smem, stream, choice, n_pairs, n_experts, listed, cap, tile_expert,
-               max_tiles);
+               max_tiles, tile_rows);
     return check_launch("moe_align");
 }
 

@@ -167,9 +167,9 @@ def call_times() -> dict:
 _launch_ahead = False
 
 _ERROR_WORD_SETTERS = ("hos_gemm_tc_set_error_word", "hos_attn_decode_set_error_word",
-                       "hos_attn_prefill_tc_set_error_word", "hos_latent_prompt_set_error_word")
+                       "hos_attn_prefill_tc_set_error_word", "hos_latent_prompt_set_error_word", "hos_moe_grouped_set_error_word")
 GIVE_UP_CODES = {1: "the tcgen05 matrix product", 2: "the decode attention", 3: "the tcgen05 prompt attention",
-                 4: "the tcgen05 prompt attention over latent rows"}
+                 4: "the tcgen05 prompt attention over latent rows", 5: "the tcgen05 products of the routed experts"}
 _error_word_tensor: Optional[torch.Tensor] = None
 _after_give_up = []        # callables that put shared scratch state right after a kernel gave up
 
@@ -800,9 +800,28 @@ def moe_route(h, router, correction, token_seq, choice, weight, top: int, scorin
                   -1.0 if renormalise is None else float(renormalise), float(weight_scale), *(groups or (0, 0)), _stream())
 
 
-def moe_align(choice, n_experts: int, listed, tile_expert) -> None:
+def moe_align(choice, n_experts: int, listed, tile_expert, tile_rows: Optional[int] = None) -> None:
+    """Every expert's pairs, its list padded to whole tiles of tile_rows (None: moe_tile_rows())."""
     experts().call("hos_moe_align", _ptr(choice), choice.numel(), int(n_experts), _ptr(listed), listed.numel(),
-                  _ptr(tile_expert), tile_expert.numel(), _stream())
+                  _ptr(tile_expert), tile_expert.numel(), int(tile_rows or moe_tile_rows()), _stream())
+
+
+MOE_GROUPED_ROWS = 128      # rows of a tile of the lists that moe_grouped takes
+
+
+def moe_grouped(h, w_up, w_down, listed, tile_expert, rows, y, pair_out, top: int, limit: float, alpha: float, up_shift: float,
+                in_weight: Optional[torch.Tensor], out_weight: Optional[torch.Tensor], act: int) -> None:
+    """Both products of the experts over lists padded to MOE_GROUPED_ROWS; rows [places, D] and y [places, F] are scratch.  The
+    other arguments as moe_gate_up's and moe_down's.  bfloat16, D and F multiples of 8."""
+    for t, what in ((h, "rows"), (w_up, "expert gate/up weights"), (w_down, "expert down weights"), (rows, "gathered rows"), (y, "inner rows")):
+        _check(t, what, torch.bfloat16)
+    e, d, f = w_down.shape
+    if w_up.shape != (e, f * (2 if act == 0 else 1), d) or h.shape[1] != d or rows.shape[1] != d or y.shape[1] != f \
+            or min(rows.shape[0], y.shape[0], listed.numel()) < tile_expert.numel() * MOE_GROUPED_ROWS:
+        raise KernelError("moe_grouped: sizes disagree")
+    experts().call("hos_moe_grouped", _ptr(h), _ptr(w_up), _ptr(w_down), _ptr(listed), _ptr(tile_expert), _ptr(rows), _ptr(y),
+                  _ptr(pair_out), tile_expert.numel(), e, d, f, int(top), float(limit), float(alpha), float(up_shift),
+                  _ptr(in_weight), _ptr(out_weight), int(act), _stream())
 
 
 def moe_gate_up(h, w, listed, tile_expert, y, top: int, limit: float, alpha: float, up_shift: float = 1.0,

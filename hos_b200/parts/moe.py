@@ -27,6 +27,7 @@ from ..registry import part_impl, register_part
 from .base import FeedForward, StepInfo, WeightSpec
 
 
+GROUPED = True          # bfloat16 with more pairs: the tcgen05 products of csrc/moe_grouped.cu; tests switch it off to compare
 FEW_PAIRS = 32          # up to this many (row, choice) pairs take the kernels without lists and tiles
 
 
@@ -101,7 +102,7 @@ class RoutedExperts(FeedForward):
 
     def forward(self, h: torch.Tensor, step: StepInfo = None) -> torch.Tensor:
         n, dev = h.shape[0], h.device
-        top, tile = self.top, ops.moe_tile_rows()
+        top = self.top
         pairs = n * top
         choice = torch.empty(pairs, dtype=torch.int32, device=dev)
         weight = torch.empty(pairs, dtype=torch.float32, device=dev)
@@ -119,14 +120,23 @@ class RoutedExperts(FeedForward):
                                    self.limit, self.alpha, self.up_shift, self.weight_on_input, self.act)
             if not done:
                 # every expert's list is padded to whole tiles: at most this many tiles whatever the router chooses
+                grouped = (GROUPED and h.dtype == torch.bfloat16 and self.width % 8 == 0 and self.inner % 8 == 0
+                           and h.data_ptr() % 16 == 0)
+                tile = ops.MOE_GROUPED_ROWS if grouped else ops.moe_tile_rows()
                 max_tiles = min(pairs, self.n_experts) + pairs // tile
                 listed = torch.empty(max_tiles * tile, dtype=torch.int32, device=dev)
                 tile_expert = torch.empty(max_tiles, dtype=torch.int32, device=dev)
-                ops.moe_align(choice, self.n_experts, listed, tile_expert)
+                ops.moe_align(choice, self.n_experts, listed, tile_expert, tile)
                 y = torch.empty((max_tiles * tile, self.inner), dtype=h.dtype, device=dev)
-                ops.moe_gate_up(h, self.w_gate_up, listed, tile_expert, y, top, self.limit, self.alpha, self.up_shift,
-                                weight if self.weight_on_input else None, self.act)
-                ops.moe_down(y, self.w_down, listed, tile_expert, None if self.weight_on_input else weight, pair_out)
+                weights = (weight, None) if self.weight_on_input else (None, weight)
+                if grouped:
+                    rows = torch.empty((max_tiles * tile, self.width), dtype=h.dtype, device=dev)
+                    ops.moe_grouped(h, self.w_gate_up, self.w_down, listed, tile_expert, rows, y, pair_out, top, self.limit,
+                                    self.alpha, self.up_shift, *weights, self.act)
+                else:
+                    ops.moe_gate_up(h, self.w_gate_up, listed, tile_expert, y, top, self.limit, self.alpha, self.up_shift,
+                                    weights[0], self.act)
+                    ops.moe_down(y, self.w_down, listed, tile_expert, weights[1], pair_out)
         extra = self.shared.forward(h, step) if self.shared is not None else None
         ops.moe_combine(pair_out, choice, weight, h, out, top, self.n_experts, extra)
         return out

@@ -1230,3 +1230,44 @@ def test_latent_prompt(sizes, lens):
             continue                                           # infinite itself
         err = (out[s].double() - want).abs()
         assert torch.all(err <= want.abs() * 2.0 ** -8 + 2.0 ** -12 * v.abs().max()), err.max().item()
+
+
+@pytest.mark.parametrize("act", ["gated_swish", "relu_square"])
+@pytest.mark.parametrize("sizes", [(40, 3, 8, 8, 8), (70, 2, 5, 136, 264), (300, 3, 4, 264, 136), (900, 1, 3, 520, 312)])
+def test_moe_grouped(act, sizes):
+    """The experts' products over tiles of 128 listed pairs: an expert that nobody chose, pairs of no expert, remainders of rows, k and
+    output numbers, more tiles than one round of CTAs has; the weight on the input and on the output.  Against 64 bits with the inner
+    rows rounded to bfloat16 (eight bits of significand) where the kernels round them: each of F products is then off by up to
+    2^-8 of itself, with random signs a few 2^-8 of the result's root mean square."""
+    from hos_b200 import ops
+    n, top, E, D, F = sizes
+    code, gated = ops.EXPERT_ACTIVATIONS[act], act == "gated_swish"
+    pairs, tile = n * top, ops.MOE_GROUPED_ROWS
+    h = torch.randn(n, D, device=DEV).bfloat16()
+    up = (torch.randn(E, F * (2 if gated else 1), D, device=DEV) / math.sqrt(D)).bfloat16()
+    down = (torch.randn(E, D, F, device=DEV) / math.sqrt(F)).bfloat16()
+    choice = torch.stack([torch.randperm(E - 1)[:top] for _ in range(n)]).int().view(-1).to(DEV)       # the last expert is never chosen
+    choice[::7] = -1
+    weight = torch.rand(pairs, device=DEV) + 0.25
+    tiles = min(pairs, E) + pairs // tile
+    listed, owner = (torch.empty(k, dtype=torch.int32, device=DEV) for k in (tiles * tile, tiles))
+    ops.moe_align(choice, E, listed, owner, tile)
+    for on_input in (False, True):
+        rows, y = (torch.full((tiles * tile, k), float("nan"), device=DEV).bfloat16() for k in (D, F))
+        out = torch.full((pairs, D), 7.0, device=DEV)
+        ops.moe_grouped(h, up, down, listed, owner, rows, y, out, top, 2.0, 1.5, 1.0, weight if on_input else None,
+                        None if on_input else weight, code)
+        assert torch.all(out[choice < 0] == 7.0)
+        for e in range(E):
+            at = (choice == e).nonzero()[:, 0]
+            if not len(at):
+                continue
+            z = h[at // top].double() @ up[e].double().T * (weight[at, None].double() if on_input else 1.0)
+            if gated:
+                g, u = z[:, :F].clamp(max=2.0), z[:, F:].clamp(-2.0, 2.0)
+                z = g * torch.sigmoid(1.5 * g) * (u + 1.0)
+            else:
+                z = torch.relu(z) ** 2
+            want = z @ down[e].double().T * (1.0 if on_input else weight[at, None].double())
+            err = (out[at].double() - want).abs().max().item()
+            assert err <= 6 * 2.0 ** -8 * (z @ down[e].double().T).square().mean().sqrt().item() + 1e-6, (on_input, e, err)
