@@ -167,12 +167,19 @@ __global__ void norm_add_norm_vec_kernel(const TY* __restrict__ y, int n_parts, 
     for (int c = 0; c < CH; ++c) {
         const int i = (c * blockDim.x + threadIdx.x) * 4;
         if (i < D) {
-            yv[c] = load4(y + base + i);
-            for (int p = 1; p < n_parts; ++p) {
-                const float4 t = load4(y + p * part_stride + base + i);
-                yv[c].x += t.x; yv[c].y += t.y; yv[c].z += t.z; yv[c].w += t.w;
-            }
             xv[c] = load4(x + base + i);
+            // The parts of a K-split product, eight asked for before any is added (as they came, one or two at a time were
+            // under way: a prompt of 97 tokens 2.26 -> 2.23 ms, eight sequences' decode steps 0.5% faster).
+            yv[c] = load4(y + base + i);
+            for (int p0 = 1; p0 < n_parts; p0 += 8) {
+                float4 t[8];
+#pragma unroll
+                for (int p = 0; p < 8; ++p)
+                    if (p0 + p < n_parts) t[p] = load4(y + (p0 + p) * part_stride + base + i);
+#pragma unroll
+                for (int p = 0; p < 8; ++p)
+                    if (p0 + p < n_parts) { yv[c].x += t[p].x; yv[c].y += t[p].y; yv[c].z += t[p].z; yv[c].w += t[p].w; }
+            }
             ss += yv[c].x * yv[c].x + yv[c].y * yv[c].y + yv[c].z * yv[c].z + yv[c].w * yv[c].w;
         }
     }
