@@ -127,7 +127,7 @@ struct Segments {
     int len, count;
 };
 
-// A thread's cells: DR rows of DC neighbouring columns (DC > 1, the walks by segments and the delta rule's long ones: what is read of k, q and the decays
+// A thread's cells: DR rows of DC neighbouring columns (DC > 1, the walks by segments: what is read of k, q and the decays
 // serves DC columns).
 template <int DR, int R, int DC, int RULE, bool LOCAL>
 __global__ void __launch_bounds__(256)
@@ -539,6 +539,182 @@ state_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
     }
 }
 
+// ---- the delta rule's long walks ---------------------------------------------------------------------------------------
+// Heads of 8 R key numbers whose rows are whole 16-byte pieces: the same walk as above (and the same bits), with nothing in a
+// chunk of eight tokens but the tokens.  What bounds it is the chain of a token (scale, dot product, sum over the column's R
+// threads, update), about 160 cycles, so everything else has to stay off it: where a thread stages is known once, the ring is
+// deep, a chunk has one barrier, whole chunks have no branch, and the read-outs go from the registers that hold them
+// straight to memory.  A thread holds 8 rows of DC columns.
+// Measured (B200, 16 heads of 128 x 128, 2,048 tokens): 399 us, 195 ns a token; in the general kernel 504, before its ring and pairs 723.
+// Vagonex, prompt of 2,048 tokens 5.05 -> 4.63 ms, four of 300 to 1,000 tokens 5.67 -> 5.43 (two columns to a thread in both).
+constexpr int kDeltaRing = 6;
+
+template <int R, int DC>
+struct DeltaTile {
+    static constexpr int COLS = 256 / R * DC;                        // columns of a block
+    static constexpr int ROW = R * (8 + kPad);                       // a staged row of q or k
+    static constexpr int CHUNK = kScanChunk * (2 * ROW + COLS + 2);  // numbers of a chunk: q, k, v, g, beta
+    static constexpr int SMEM = kDeltaRing * CHUNK * 4;
+    static constexpr int PER_ROW = 2 * R;                            // 16-byte pieces of a row
+};
+
+template <int R, int DC>
+__global__ void __launch_bounds__(256)
+delta_walk_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v, long long ld,
+                  const float* __restrict__ g, long long g_ld, const float* __restrict__ beta, long long beta_ld,
+                  float* __restrict__ state, const int* __restrict__ token_pos, const int* __restrict__ token_seq,
+                  const int* __restrict__ cu_seqlens, const int* __restrict__ seq_slot, float* __restrict__ out, int H, int Gk,
+                  int vdim, float o_mult) {
+    using T = DeltaTile<R, DC>;
+    constexpr int DIM = 8 * R;
+    pdl_enter();
+    extern __shared__ __align__(16) float sm[];
+    const int seq = blockIdx.x, head = blockIdx.y, col0 = blockIdx.z * T::COLS;
+    const int lo = cu_seqlens[seq], hi = cu_seqlens[seq + 1];
+    if (hi <= lo || token_seq[lo] < 0) return;
+    const bool fresh = token_pos[lo] == 0;
+    const int kh = head / (H / Gk);
+    const int r = threadIdx.x % R, c = threadIdx.x / R, col = col0 + c * DC;       // vdim is a multiple of 4, so of DC
+    const bool live = col < vdim;
+
+    // what this thread stages of every chunk: a piece of some of its q and k rows, of its v rows, a decay or a beta
+    const int piece = threadIdx.x % T::PER_ROW, row = threadIdx.x / T::PER_ROW;
+    const int at = row * T::ROW + piece / 2 * (8 + kPad) + piece % 2 * 4;
+    const int vrow = threadIdx.x / (T::COLS / 4), vcol = threadIdx.x % (T::COLS / 4) * 4;
+    const bool stages_v = vrow < kScanChunk && col0 + vcol < vdim;
+    const int tail = 255 - threadIdx.x;                              // the last threads: 8 decays, 8 betas
+    const float* from_q = q + (size_t)kh * DIM + piece * 4;
+    const float* from_k = k + (size_t)kh * DIM + piece * 4;
+    const float* from_v = v + (size_t)head * vdim + col0 + vcol;
+    auto stage = [&](int t0, float* buf) {
+#pragma unroll
+        for (int t = 0; t < kScanChunk; t += 256 / T::PER_ROW) {
+            const int n = t0 + t + row;
+            if (t + row < kScanChunk && n < hi) {
+                cp_async16(buf + t * T::ROW + at, from_q + (size_t)n * ld);
+                cp_async16(buf + (kScanChunk + t) * T::ROW + at, from_k + (size_t)n * ld);
+            }
+        }
+        float* rest = buf + 2 * kScanChunk * T::ROW;
+        if (stages_v && t0 + vrow < hi) cp_async16(rest + vrow * T::COLS + vcol, from_v + (size_t)(t0 + vrow) * ld);
+        if (tail < 16) {
+            const int n = t0 + (tail & 7);
+            float* to = rest + kScanChunk * T::COLS + tail;
+            if (n < hi) cp_async4(to, tail < 8 ? g + (size_t)n * g_ld + head : beta + (size_t)n * beta_ld + head);
+        }
+    };
+
+    float* st = state + (((size_t)seq_slot[seq] * H + head) * vdim + (live ? col : 0)) * DIM + r * 8;
+    uint64_t P[DC][4];
+#pragma unroll
+    for (int j = 0; j < DC; ++j) {
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+        if (!fresh && live) {
+            a = *reinterpret_cast<const float4*>(st + (size_t)j * DIM);
+            b = *reinterpret_cast<const float4*>(st + (size_t)j * DIM + 4);
+        }
+        P[j][0] = pair_of(a.x, a.y); P[j][1] = pair_of(a.z, a.w); P[j][2] = pair_of(b.x, b.y); P[j][3] = pair_of(b.z, b.w);
+    }
+#pragma unroll
+    for (int b = 0; b < kDeltaRing - 1; ++b) {
+        if (lo + b * kScanChunk < hi) stage(lo + b * kScanChunk, sm + b * T::CHUNK);
+        cp_async_commit_all();
+    }
+    int which = 0;
+    for (int t0 = lo; t0 < hi; t0 += kScanChunk) {
+        cp_async_wait<kDeltaRing - 2>();
+        __syncthreads();            // this chunk has landed; everyone is done with the buffer before it
+        const int ahead = t0 + (kDeltaRing - 1) * kScanChunk;
+        if (ahead < hi) stage(ahead, sm + (which == 0 ? kDeltaRing - 1 : which - 1) * T::CHUNK);
+        cp_async_commit_all();
+        const float* qs = sm + which * T::CHUNK + r * (8 + kPad);
+        const float* ks = qs + kScanChunk * T::ROW;
+        const float* vs = sm + which * T::CHUNK + 2 * kScanChunk * T::ROW + c * DC;
+        const float* gs = sm + which * T::CHUNK + 2 * kScanChunk * T::ROW + kScanChunk * T::COLS;
+        which = which + 1 == kDeltaRing ? 0 : which + 1;
+        auto walk = [&](auto whole_chunk) {
+            constexpr bool FULL = decltype(whole_chunk)::value;
+            const int nt = FULL ? kScanChunk : hi - t0;
+            float part[DC][kScanChunk];       // the read-outs' partial sums: added up after the walk, off its chain
+#pragma unroll
+            for (int t = 0; t < kScanChunk; ++t) {
+                if (!FULL && t >= nt) {
+#pragma unroll
+                    for (int j = 0; j < DC; ++j) part[j][t] = 0.f;
+                    continue;
+                }
+                const ulonglong2* k4 = (const ulonglong2*)(ks + t * T::ROW);
+                const ulonglong2* q4 = (const ulonglong2*)(qs + t * T::ROW);
+                const ulonglong2 k0 = k4[0], k1 = k4[1], q0 = q4[0], q1 = q4[1];
+                const float gt = gs[t], bt = gs[8 + t];
+                const uint64_t gg = pair_of(gt, gt);
+                float dot[DC];
+#pragma unroll
+                for (int j = 0; j < DC; ++j) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) P[j][i] = mul_pair(gg, P[j][i]);
+                    const uint64_t d01 = fma_pair(P[j][2], k1.x, fma_pair(P[j][0], k0.x, 0));       // four chains
+                    const uint64_t d23 = fma_pair(P[j][3], k1.y, fma_pair(P[j][1], k0.y, 0));
+                    float d0, d1, d2, d3;
+                    halves_of(d01, d0, d1);
+                    halves_of(d23, d2, d3);
+                    dot[j] = (d0 + d1) + (d2 + d3);
+                }
+#pragma unroll
+                for (int o = 1; o < R; o <<= 1)
+#pragma unroll
+                    for (int j = 0; j < DC; ++j) dot[j] += __shfl_xor_sync(0xffffffffu, dot[j], o);
+#pragma unroll
+                for (int j = 0; j < DC; ++j) {
+                    const float u = bt * (vs[t * T::COLS + j] - dot[j]);
+                    const uint64_t uu = pair_of(u, u);
+                    P[j][0] = fma_pair(k0.x, uu, P[j][0]);
+                    P[j][1] = fma_pair(k0.y, uu, P[j][1]);
+                    P[j][2] = fma_pair(k1.x, uu, P[j][2]);
+                    P[j][3] = fma_pair(k1.y, uu, P[j][3]);
+                    const uint64_t a01 = fma_pair(P[j][2], q1.x, fma_pair(P[j][0], q0.x, 0));
+                    const uint64_t a23 = fma_pair(P[j][3], q1.y, fma_pair(P[j][1], q0.y, 0));
+                    float a0, a1, a2, a3;
+                    halves_of(a01, a0, a1);
+                    halves_of(a23, a2, a3);
+                    part[j][t] = (a0 + a1) + (a2 + a3);
+                }
+            }
+            // eight tokens' sums over R threads: with every turn a thread hands on half of the tokens it still has
+            static_assert(kScanChunk == 8 && R >= 8, "three turns");
+#pragma unroll
+            for (int j = 0; j < DC; ++j) {
+                const float(&p)[kScanChunk] = part[j];
+                float four[4], two[2];
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    four[i] = ((r & 1) ? p[i + 4] : p[i]) + __shfl_xor_sync(0xffffffffu, (r & 1) ? p[i] : p[i + 4], 1);
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+                    two[i] = ((r & 2) ? four[i + 2] : four[i]) + __shfl_xor_sync(0xffffffffu, (r & 2) ? four[i] : four[i + 2], 2);
+                float acc = ((r & 4) ? two[1] : two[0]) + __shfl_xor_sync(0xffffffffu, (r & 4) ? two[0] : two[1], 4);
+#pragma unroll
+                for (int o = 8; o < R; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+                const int t = (r & 1) * 4 + (r & 2) + ((r & 4) >> 2);
+                if (r < 8 && live && (FULL || t < nt)) out[((size_t)(t0 + t) * H + head) * vdim + col + j] = acc * o_mult;
+            }
+        };
+        if (hi - t0 >= kScanChunk) walk(std::true_type{});
+        else walk(std::false_type{});
+    }
+    if (!live) return;
+#pragma unroll
+    for (int j = 0; j < DC; ++j) {
+        float4 a, b;
+        halves_of(P[j][0], a.x, a.y);
+        halves_of(P[j][1], a.z, a.w);
+        halves_of(P[j][2], b.x, b.y);
+        halves_of(P[j][3], b.z, b.w);
+        *reinterpret_cast<float4*>(st + (size_t)j * DIM) = a;
+        *reinterpret_cast<float4*>(st + (size_t)j * DIM + 4) = b;
+    }
+}
+
 // states: what the first walk left, [count][cells] per sequence; becomes the states at the segments' starts (the first one's:
 // the slot's, or zero).  A thread per cell; decays: a number per head, or (channel) per head and key number.
 __global__ void __launch_bounds__(256)
@@ -771,7 +947,7 @@ namespace hos {
 // How a walk is cut: DR rows of a column to a thread, R threads to a column, CC columns to a block.
 struct ScanShape {
     int DR, R, CC, DC = 1;
-    ScanShape(int dim, int vdim, bool segments = false, bool long_delta = false) {
+    ScanShape(int dim, int vdim, bool segments = false) {
         // short runs of rows per thread: a token's walk is a chain of dependent instructions (scale, dot, sum over the
         // runs, update, read-out, sum), and with few (sequence, head) pairs nothing else hides its latency; the sums over
         // 16 or 32 runs are shuffles
@@ -783,13 +959,23 @@ struct ScanShape {
         if (DR == 8 && R < 4) R = 4;          // the compiled shapes (rows beyond dim are zeros)
         if (DR >= 16) R = 32;
         if (segments && DR == 8) DC = 4;      // the shapes that are compiled for four columns to a thread
-        if (long_delta && DR == 8) DC = 2;    // and for two
         CC = 256 / R * DC;
         if (CC > vdim) CC = (vdim + DC - 1) / DC * DC;
     }
     int threads() const { return (CC / DC * R + 31) / 32 * 32; }
 };
 constexpr int kMinSegment = 64;       // tokens
+template <int R, int DC>
+int launch_delta(const float* q, const float* k, const float* v, long long ld, const float* g, long long g_ld, const float* beta,
+                 long long beta_ld, float* state, const int* token_pos, const int* token_seq, const int* cu_seqlens, const int* seq_slot,
+                 float* out, int n_seqs, int H, int Gk, int vdim, float o_mult, cudaStream_t stream) {
+    using T = DeltaTile<R, DC>;
+    if (cudaFuncSetAttribute(delta_walk_kernel<R, DC>, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM) != cudaSuccess)
+        HOS_REFUSE("state_scan: cannot get %d bytes of shared memory", T::SMEM);
+    launch_pdl(delta_walk_kernel<R, DC>, dim3(n_seqs, H, (vdim + T::COLS - 1) / T::COLS), dim3(256), T::SMEM, stream, q, k, v, ld, g, g_ld, beta,
+               beta_ld, state, token_pos, token_seq, cu_seqlens, seq_slot, out, H, Gk, vdim, o_mult);
+    return check_launch("state_scan (delta rule)");
+}
 }  // namespace hos
 
 // How many tokens a segment has where sequences that bring up to max_new tokens are worth walking in segments (see the file's
@@ -830,11 +1016,7 @@ extern "C" int hos_state_scan(const float* q, const float* k, const float* v, lo
     if (dim <= 0 || dim > 1024 || vdim <= 0) HOS_REFUSE("state_scan: heads of %d x %d", dim, vdim);
     const bool segments = seg_count > 1;
     const bool long_walk = n_rows >= 4ll * kScanChunk * n_seqs;
-    // The delta rule's long walks, where they fill the SMs several times over: two columns to a thread share what is read of k and
-    // q (four prompts of 300 to 1,000 tokens: a layer's walk goes with the step from 5.89 to 5.67 ms; a walk that has its SM to
-    // itself is bound by its chain and has nothing of it: 504 us for 2,048 tokens with one column, 521 with two).
-    const bool many = (long long)n_seqs * H * vdim * 16 > 2ll * 256 * sm_count_cached();
-    const ScanShape shape(dim, vdim, segments, rule == kDeltaRule && long_walk && many);
+    const ScanShape shape(dim, vdim, segments);
     const int DR = shape.DR, R = shape.R, DC = shape.DC;
     int CC = shape.CC;
     // single tokens and few (sequence, head) pairs: fewer columns to a block, so that the blocks fill the GPU (columns
@@ -856,14 +1038,28 @@ extern "C" int hos_state_scan(const float* q, const float* k, const float* v, lo
                          (rule != kChannelRule || (g_ld % 4 == 0 && (uintptr_t)g % 16 == 0))) ? 1 : 0;
     const dim3 grid(n_seqs * sg.count, H, (vdim + CC - 1) / CC);
     // Few long walks have an SM (almost) to themselves, and nothing but the ring hides the way of their rows from memory: two
-    // chunks of eight tokens are not enough (the delta rule, 16 heads of 128 x 128, 2,048 tokens: with a deeper ring and pairs
-    // of rows in one instruction 723 -> 504 us).  More walks than that hide one another's loads, and shared memory for more of
+    // chunks of eight tokens are not enough (the delta rule, 16 heads of 128 x 128, 2,048 tokens, before it had a kernel of its own
+    // for such sizes: with a deeper ring and pairs of rows in one instruction 723 -> 504 us).  More walks than that hide one another's loads, and shared memory for more of
     // them at once is worth more.
     const bool alone = (long long)grid.x * grid.y * grid.z <= 2ll * sm_count_cached() && long_walk;
     const int n_buf = alone && kDeepRing * per_buf <= 100 * 1024 ? kDeepRing : 2;
     const size_t smem = n_buf * per_buf;
     if (rule != kDecayRule && act_in_walk) HOS_REFUSE("state_scan: the activation in the walk is the decay rule's");
     if (smem > 200 * 1024) HOS_REFUSE("state_scan: heads of %d x %d do not fit a block's shared memory", dim, vdim);
+    if (rule == kDeltaRule && long_walk && aligned && (dim == 64 || dim == 128 || dim == 256) && vdim % 4 == 0 && (uintptr_t)v % 16 == 0 &&
+        (uintptr_t)state % 16 == 0 && rot_dims == 0 && k_mult == 1.f) {
+        // two columns to a thread where the blocks fill the SMs several times over anyway: the reads of k and q serve both
+        const bool many = (long long)n_seqs * H * vdim * (dim / 8) > 2ll * 256 * sm_count_cached();
+#define HOS_DELTA(Rv)                                                                                                \
+    return many ? launch_delta<Rv, 2>(q, k, v, ld, g, g_ld, beta, beta_ld, state, token_pos, token_seq, cu_seqlens, seq_slot, out, n_seqs, H, Gk, \
+                                      vdim, o_mult, stream)                                                          \
+                : launch_delta<Rv, 1>(q, k, v, ld, g, g_ld, beta, beta_ld, state, token_pos, token_seq, cu_seqlens, seq_slot, out, n_seqs, H, Gk, \
+                                      vdim, o_mult, stream)
+        if (dim == 64) HOS_DELTA(8);
+        if (dim == 128) HOS_DELTA(16);
+        HOS_DELTA(32);
+#undef HOS_DELTA
+    }
 #define HOS_SCAN(DRv, Rv, DCv, DL, LOC)                                                                                   \
     do {                                                                                                             \
         if (smem > 48 * 1024)                                                                                        \
@@ -886,9 +1082,7 @@ extern "C" int hos_state_scan(const float* q, const float* k, const float* v, lo
     } while (0)
 #define HOS_SCAN_D(DRv, Rv)                                                                                          \
     do {                                                                                                             \
-        constexpr int DCd = DRv == 8 ? 2 : 1;                                                                        \
-        if (rule == kDeltaRule && DC == 1) HOS_SCAN(DRv, Rv, 1, kDeltaRule, false);                                  \
-        else if (rule == kDeltaRule) HOS_SCAN(DRv, Rv, DCd, kDeltaRule, false);                                      \
+        if (rule == kDeltaRule) HOS_SCAN(DRv, Rv, 1, kDeltaRule, false);                                              \
         else if (rule == kChannelRule) HOS_SCAN_S(DRv, Rv, kChannelRule);                                            \
         else HOS_SCAN_S(DRv, Rv, kDecayRule);                                                                        \
     } while (0)

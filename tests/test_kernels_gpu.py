@@ -1271,3 +1271,49 @@ def test_moe_grouped(act, sizes):
             want = z @ down[e].double().T * (1.0 if on_input else weight[at, None].double())
             err = (out[at].double() - want).abs().max().item()
             assert err <= 6 * 2.0 ** -8 * (z @ down[e].double().T).square().mean().sqrt().item() + 1e-6, (on_input, e, err)
+
+
+@pytest.mark.parametrize("many", [False, True])
+@pytest.mark.parametrize("dim,vdim", [(64, 36), (128, 128), (256, 20)])
+def test_long_delta_walk(dim, vdim, many):
+    """The delta rule's walk of long sequences: whole chunks of eight tokens and every remainder, columns that do not fill a block,
+    key heads shared by two heads, one and two columns to a thread (`many`: blocks enough), a sequence that starts and ones
+    that go on, against 64 bits.  Keys of length one keep the state's size: rounding (2^-24 a step) adds up over 65 steps at most."""
+    from types import SimpleNamespace
+    from hos_b200 import ops
+    H, Gk = 4, 2
+    lens = ([65, 33, 40, 47] if not many else [33 + i % 16 for i in range(64)])
+    if many:
+        H, Gk = 8, 4
+    n, B = sum(lens), len(lens)
+    cu = [0]
+    for x in lens:
+        cu.append(cu[-1] + x)
+    k = torch.nn.functional.normalize(torch.randn(n, Gk, dim, device=DEV), dim=-1)
+    q = torch.nn.functional.normalize(torch.randn(n, Gk, dim, device=DEV), dim=-1)
+    v = torch.randn(n, H, vdim, device=DEV)
+    rows = torch.cat([q.flatten(1), k.flatten(1), v.flatten(1)], 1).contiguous()
+    g, beta = torch.rand(n, H, device=DEV) * 0.2 + 0.8, torch.rand(n, H, device=DEV)
+    state = torch.randn(B, H, vdim, dim, device=DEV) * 0.1
+    starts = [0 if i == 0 else 70 for i in range(B)]
+    pos = torch.cat([torch.arange(s, s + x) for s, x in zip(starts, lens)]).int().to(DEV)
+    seq = torch.cat([torch.full((x,), i) for i, x in enumerate(lens)]).int().to(DEV)
+    slot = torch.arange(B - 1, -1, -1, dtype=torch.int32, device=DEV)
+    step = SimpleNamespace(token_pos=pos, token_seq=seq, cu_seqlens=torch.tensor(cu, dtype=torch.int32, device=DEV), seq_slot=slot,
+                           n_seqs=B, n_tokens=n, max_new=max(lens))
+    S = state[slot.long()].double()
+    S[0] = 0.0
+    out = torch.full((n, H * vdim), float("nan"), device=DEV)
+    ops.state_scan(rows, 0, Gk * dim, 2 * Gk * dim, False, g, True, beta, state, step, out, H, Gk, dim, vdim)
+    want = torch.zeros(n, H, vdim, dtype=torch.float64, device=DEV)
+    for t in range(max(lens)):
+        on = [i for i in range(B) if t < lens[i]]
+        at = torch.tensor([cu[i] + t for i in on], device=DEV)
+        kk, qq = (x[at].double().repeat_interleave(H // Gk, 1) for x in (k, q))
+        s = S[on] * g[at].double()[..., None, None]
+        u = beta[at].double()[..., None] * (v[at].double() - torch.einsum("bhvd,bhd->bhv", s, kk))
+        s = s + u[..., None] * kk[:, :, None]
+        S[on] = s
+        want[at] = torch.einsum("bhvd,bhd->bhv", s, qq)
+    assert (out.double() - want.flatten(1)).abs().max().item() <= 2e-5
+    assert (state[slot.long()].double() - S).abs().max().item() <= 2e-5
