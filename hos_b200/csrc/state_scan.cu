@@ -49,13 +49,21 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
 __device__ __forceinline__ void cp_async_commit_all() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// x <- x logistic(x) on the first `cols` numbers of every row (the decay rule's q, k, v before the scan)
-__global__ void act_rows_kernel(float* __restrict__ x, long long ld, int cols, long long n) {
+// x <- x logistic(x) on the first `cols` numbers of every row (the decay rule's q, k, v before the scan).  blockIdx.y: the row;
+// a thread takes VEC neighbours (2,048 rows of 6,144: one number a thread, its row found by a 64-bit division, 53 us; four and no
+// division 16).
+template <int VEC>
+__global__ void __launch_bounds__(256) act_rows_kernel(float* __restrict__ x, long long ld, int cols) {
     pdl_enter();
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float* p = x + (i / cols) * ld + (i % cols);
-    *p = silu_precise(*p);
+    const int c = (blockIdx.x * blockDim.x + threadIdx.x) * VEC;
+    if (c >= cols) return;
+    float* p = x + (size_t)blockIdx.y * ld + c;
+    if constexpr (VEC == 4) {
+        const float4 t = *reinterpret_cast<const float4*>(p);
+        *reinterpret_cast<float4*>(p) = make_float4(silu_precise(t.x), silu_precise(t.y), silu_precise(t.z), silu_precise(t.w));
+    } else {
+        *p = silu_precise(*p);
+    }
 }
 
 // x: float32 [N][ld]; from column 0 on `Hq` query heads and then `Hk` key heads of `dim` numbers each.  The first
@@ -1103,9 +1111,13 @@ extern "C" int hos_state_scan(const float* q, const float* k, const float* v, lo
 }
 
 extern "C" int hos_act_rows(float* x, long long ld, int cols, int N, cudaStream_t stream) {
-    const long long n = (long long)N * cols;
-    if (n <= 0) return 0;
-    launch_pdl(act_rows_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, stream, x, ld, cols, n);
+    if (N <= 0 || cols <= 0) return 0;
+    const bool vec = cols % 4 == 0 && ld % 4 == 0 && (uintptr_t)x % 16 == 0;
+    for (int n0 = 0; n0 < N; n0 += 65535) {
+        const int rows = N - n0 < 65535 ? N - n0 : 65535;
+        launch_pdl(vec ? act_rows_kernel<4> : act_rows_kernel<1>, dim3((cols + (vec ? 1024 : 256) - 1) / (vec ? 1024 : 256), rows), dim3(256), 0,
+                   stream, x + (size_t)n0 * ld, ld, cols);
+    }
     return check_launch("act_rows");
 }
 
