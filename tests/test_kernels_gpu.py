@@ -1317,3 +1317,45 @@ def test_long_delta_walk(dim, vdim, many):
         want[at] = torch.einsum("bhvd,bhd->bhv", s, qq)
     assert (out.double() - want.flatten(1)).abs().max().item() <= 2e-5
     assert (state[slot.long()].double() - S).abs().max().item() <= 2e-5
+
+
+@pytest.mark.parametrize("rule", ["decay", "delta"])
+@pytest.mark.parametrize("dim,vdim,B,H", [(64, 36, 3, 4), (128, 128, 24, 16), (128, 20, 9, 4), (256, 72, 40, 4)])
+def test_state_of_single_tokens(rule, dim, vdim, B, H):
+    """One token per sequence: every number of columns to a thread, columns that do not fill a block, key heads shared by two
+    heads, a padding row, a sequence that starts, the activation in the walk.  Against 64 bits: sums of `dim` products of
+    numbers below ten, each rounded to 2^-24 of itself."""
+    from types import SimpleNamespace
+    from hos_b200 import ops
+    delta, Gk = rule == "delta", H // 2
+    rows = torch.randn(B, 2 * Gk * dim + H * vdim, device=DEV) / math.sqrt(dim)
+    per_row = torch.rand(B, H, device=DEV) * 0.2 + 0.8
+    beta = torch.rand(B, H, device=DEV) if delta else None
+    state = torch.randn(B, H, vdim, dim, device=DEV)
+    before = state.clone()
+    pos = torch.full((B,), 70, dtype=torch.int32, device=DEV)
+    pos[0] = 0
+    seq = torch.arange(B, dtype=torch.int32, device=DEV)
+    seq[1] = -1
+    slot = torch.arange(B - 1, -1, -1, dtype=torch.int32, device=DEV)
+    step = SimpleNamespace(token_pos=pos, token_seq=seq, cu_seqlens=torch.arange(B + 1, dtype=torch.int32, device=DEV), seq_slot=slot,
+                           n_seqs=B, n_tokens=B, max_new=1)
+    x = rows.double()
+    out = torch.full((B, H * vdim), 7.0, device=DEV)
+    ops.state_scan(rows, 0, Gk * dim, 2 * Gk * dim, not delta, per_row if delta else per_row[0].contiguous(), delta, beta, state, step, out,
+                   H, Gk, dim, vdim, o_mult=0.5)
+    if not delta:
+        x = x * torch.sigmoid(x)
+    q, k = (x[:, i * Gk * dim:(i + 1) * Gk * dim].view(B, Gk, dim).repeat_interleave(H // Gk, 1) for i in (0, 1))
+    v = x[:, 2 * Gk * dim:].view(B, H, vdim)
+    S = before[slot.long()].double()
+    S[0] = 0.0
+    S = S * (per_row if delta else per_row[:1].expand(B, H)).double()[..., None, None]
+    u = beta.double()[..., None] * (v - torch.einsum("bhvd,bhd->bhv", S, k)) if delta else v
+    S = S + u[..., None] * k[:, :, None]
+    want = 0.5 * torch.einsum("bhvd,bhd->bhv", S, q).flatten(1)
+    live = [i for i in range(B) if i != 1]
+    assert torch.all(out[1] == 7.0) and torch.equal(state[slot[1].long()], before[slot[1].long()])
+    tol = dim * 2.0 ** -24 * 10
+    assert (out.double() - want)[live].abs().max().item() <= tol
+    assert (state[slot.long()].double() - S)[live].abs().max().item() <= tol
