@@ -129,13 +129,13 @@ static int launch_plain(const void* A, const void* W, void* out, int M, int N, i
 // by cp.async through a ring of stages.  A thread's accumulators are pairs, the even and the odd k of a sum: then one
 // fma.rn.f32x2 takes two neighbours of a row of A and two of a row of W as they were read, and nothing is transposed
 // or duplicated.  What a thread reads from shared memory costs as much time as what it multiplies at 8 x 8 sums a thread,
-// and more with fewer sums, so with few rows the warps split a stage's k (WK of them) instead of the tile: up to 16 rows a
-// thread still holds 8 x 4 sums, from 17 on 8 x 8.  Where the tiles of the output are too few for the GPU's SMs, the CTAs of a
-// cluster share one tile by k and add their sums through distributed shared memory, each a slice of the rows, in the
-// order of the ranks.
-// Measured (B200): the gated product of 2 x 9,216 rows of W, K 2,304, at 121 rows 621 us with the 64 x 64 tiles above and 259
-// here (40 TFLOP/s); at 16 rows 48 us, 3.6 TB/s of weights; a 121-token prompt of Gemma-2 2B 81.6 -> 17.5 ms.  Its logits'
-// error against 64 bits went from 9e-6 to 4e-6 (sums of two or more parts instead of one long one).
+// and more with fewer sums, so the four warps split a stage's k instead of the tile: with tiles of 16 rows a thread still
+// holds 8 x 4 sums, with tiles of 32 rows 8 x 8.  Where few rows leave too few tiles for the GPU's SMs, the CTAs of a cluster
+// share one tile by k and add their sums through distributed shared memory, each a slice of the rows, in the order of the
+// ranks.  In what order a sum is added up hangs on N and K alone: a row's results are the same bits whatever rows stand
+// beside it (padding, another batch), so k is always cut for one tile of rows, and there are no tiles of more rows, whose
+// warps would have to share k differently (up to 128 rows by one such tile were 10% faster at 121 rows).
+// Measured (B200): XX
 constexpr int kF32Threads = 128, kF32Cols = 64, kF32Depth = 32;
 
 struct F32Gemm {
@@ -158,18 +158,17 @@ __device__ __forceinline__ float pair_sum(unsigned long long v) {
     return __uint_as_float((uint32_t)v) + __uint_as_float((uint32_t)(v >> 32));
 }
 
-// A tile of BM rows: how the four warps and a warp's lanes share it.
+// A tile of BM rows: how a warp's lanes share it.
 template <int BM>
 struct F32Tile {
-    static constexpr int WK = BM <= 32 ? 4 : (BM <= 64 ? 2 : 1);     // warps that split k
-    static constexpr int ROWS = BM / (4 / WK);                       // rows of a warp
+    static constexpr int WK = kF32Threads / 32;                      // the warps split k
     static constexpr int LC = BM <= 16 ? 16 : 8, LR = 32 / LC;       // lanes along the columns, along the rows
-    static constexpr int RM = ROWS / LR, RN = kF32Cols / LC;         // sums of a thread
+    static constexpr int RM = BM / LR, RN = kF32Cols / LC;         // sums of a thread
     static constexpr int STAGE = (BM + kF32Cols) * kF32Depth;        // numbers of a stage
-    static constexpr int STAGES = BM <= 64 ? 6 : 4;
+    static constexpr int STAGES = 6;
     static constexpr int SMEM = STAGES * STAGE * 4;
     static constexpr int LD = kF32Cols + 1;                          // a row of the sums' tile, which takes the stages' place
-    static_assert(WK * BM * LD <= STAGES * STAGE && RM * LR * (4 / WK) == BM && RM <= 8, "tile");
+    static_assert(WK * BM * LD <= STAGES * STAGE && RM * LR == BM && RM <= 8, "tile");
 };
 
 template <int BM, int EPI>
@@ -177,11 +176,11 @@ __global__ void __launch_bounds__(kF32Threads, BM <= 16 ? 3 : 2) gemm_f32_kernel
     using T = F32Tile<BM>;
     constexpr int STAGE = T::STAGE, STAGES = T::STAGES, RM = T::RM, RN = T::RN, LD = T::LD;
     extern __shared__ __align__(128) float smem[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int tx = lane % T::LC, ty = lane / T::LC;                  // columns tx + LC j, rows first_row + ty + LR i
-    const int kg = warp % T::WK, first_row = warp / T::WK * T::ROWS;
+    const int lane = threadIdx.x & 31, kg = threadIdx.x >> 5;
+    const int tx = lane % T::LC, ty = lane / T::LC;                  // columns tx + LC j, rows ty + LR i
     const int rank = p.splits > 1 ? blockIdx.x % p.splits : 0;       // a cluster is `splits` CTAs along x
-    const int n0 = blockIdx.x / p.splits * (EPI == kEpiGated ? kF32Cols / 2 : kF32Cols), m0 = blockIdx.y * BM;
+    const int tile = blockIdx.x / p.splits, mt = (p.M + BM - 1) / BM;            // tiles of rows side by side: they share W in L2
+    const int n0 = tile / mt * (EPI == kEpiGated ? kF32Cols / 2 : kF32Cols), m0 = tile % mt * BM;
     const int blocks = (p.K + kF32Depth - 1) / kF32Depth;
     const int first = (int)((long long)blocks * rank / p.splits), last = (int)((long long)blocks * (rank + 1) / p.splits);
 
@@ -226,7 +225,7 @@ __global__ void __launch_bounds__(kF32Threads, BM <= 16 ? 3 : 2) gemm_f32_kernel
         const int ahead = block + STAGES - 1;
         if (ahead < last) load(stage == 0 ? STAGES - 1 : stage - 1, ahead);
         asm volatile("cp.async.commit_group;" ::: "memory");
-        const float* a_at = smem + stage * STAGE + (first_row + ty) * kF32Depth;
+        const float* a_at = smem + stage * STAGE + ty * kF32Depth;
         const float* w_at = smem + stage * STAGE + (BM + tx) * kF32Depth;
 #pragma unroll 2
         for (int u = 0; u < kF32Depth / 4 / T::WK; ++u) {
@@ -235,7 +234,7 @@ __global__ void __launch_bounds__(kF32Threads, BM <= 16 ? 3 : 2) gemm_f32_kernel
 #pragma unroll
             for (int i = 0; i < RM; ++i)
                 a[i] = *reinterpret_cast<const ulonglong2*>(a_at + T::LR * i * kF32Depth +
-                                                            ((c ^ ((first_row + ty + T::LR * i) & 7)) << 2));
+                                                            ((c ^ ((ty + T::LR * i) & 7)) << 2));
 #pragma unroll
             for (int j = 0; j < RN; ++j) {
                 const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(w_at + T::LC * j * kF32Depth + ((c ^ (tx & 7)) << 2));
@@ -256,7 +255,7 @@ __global__ void __launch_bounds__(kF32Threads, BM <= 16 ? 3 : 2) gemm_f32_kernel
     for (int i = 0; i < RM; ++i)
 #pragma unroll
         for (int j = 0; j < RN; ++j)
-            smem[(kg * BM + first_row + ty + T::LR * i) * LD + tx + T::LC * j] = pair_sum(acc[i][j]);
+            smem[(kg * BM + ty + T::LR * i) * LD + tx + T::LC * j] = pair_sum(acc[i][j]);
     if (p.splits > 1) {
         asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -292,9 +291,9 @@ __global__ void __launch_bounds__(kF32Threads, BM <= 16 ? 3 : 2) gemm_f32_kernel
 }
 
 template <int BM, int EPI>
-cudaLaunchConfig_t f32_config(int nt, int mt, int splits, cudaLaunchAttribute* attr, cudaStream_t stream) {
+cudaLaunchConfig_t f32_config(long long tiles, int splits, cudaLaunchAttribute* attr, cudaStream_t stream) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(nt * splits, mt);
+    cfg.gridDim = dim3((unsigned)(tiles * splits));
     cfg.blockDim = kF32Threads;
     cfg.dynamicSmemBytes = F32Tile<BM>::SMEM;
     cfg.stream = stream;
@@ -324,7 +323,7 @@ const int* f32_clusters() {
         c.n[1] = per_sm * sm_count_cached();
         for (int s = 2; s <= kF32MaxSplits && c.ok; ++s) {
             cudaLaunchAttribute attr[1];
-            cudaLaunchConfig_t cfg = f32_config<BM, EPI>(1024, 1, s, attr, 0);
+            cudaLaunchConfig_t cfg = f32_config<BM, EPI>(1024, s, attr, 0);
             if (cudaOccupancyMaxActiveClusters(&c.n[s], gemm_f32_kernel<BM, EPI>, &cfg) != cudaSuccess) c.n[s] = 0;
         }
         cudaGetLastError();                                          // a size that does not fit is none to choose, not an error
@@ -334,7 +333,7 @@ const int* f32_clusters() {
     return counts.ok ? counts.n : nullptr;
 }
 
-// In how many parts k is cut.  A CTA's time is its blocks of 32 k, plus about four blocks' worth for filling the ring and
+// In how many parts k is cut, for one tile of rows (so not by M: see above).  A CTA's time is its blocks of 32 k, plus about four blocks' worth for filling the ring and
 // adding up; an SM's time is that of its CTAs together, but a single CTA does not fill it; clusters that do not fit at
 // once wait for a whole one.
 inline int f32_splits(const int* clusters, int tiles, int K) {
@@ -356,31 +355,24 @@ template <int BM, int EPI>
 int launch_f32(F32Gemm p, cudaStream_t stream) {
     const int cols = EPI == kEpiGated ? kF32Cols / 2 : kF32Cols;
     const int nt = (p.N + cols - 1) / cols, mt = (p.M + BM - 1) / BM;
-    const int* clusters = f32_clusters<BM, EPI>();
-    if (clusters == nullptr) HOS_REFUSE("gemm_f32: the kernel does not fit on this GPU");
-    p.splits = (long long)nt * mt >= 4LL * clusters[1] ? 1 : f32_splits(clusters, nt * mt, p.K);
+    const int* clusters = f32_clusters<32, EPI>();       // the larger tiles' for both heights: the same cut of k
+    if (clusters == nullptr || f32_clusters<BM, EPI>() == nullptr) HOS_REFUSE("gemm_f32: the kernel does not fit on this GPU");
+    p.splits = f32_splits(clusters, nt, p.K);
     cudaLaunchAttribute attr[1];
-    cudaLaunchConfig_t cfg = f32_config<BM, EPI>(nt, mt, p.splits, attr, stream);
+    cudaLaunchConfig_t cfg = f32_config<BM, EPI>((long long)nt * mt, p.splits, attr, stream);
     cudaLaunchKernelEx(&cfg, gemm_f32_kernel<BM, EPI>, p);
     return check_launch("gemm_f32");
 }
 
-// Rows of a tile: the smallest that holds them all; above 128 rows the one that computes the fewest rows beyond M, the
-// larger of equals, which reads W fewer times.
 template <int EPI>
 int launch_f32_rows(const F32Gemm& p, cudaStream_t stream) {
-    if (p.M <= 16) return launch_f32<16, EPI>(p, stream);
-    if (p.M <= 32) return launch_f32<32, EPI>(p, stream);
-    if (p.M <= 48) return launch_f32<48, EPI>(p, stream);
-    if (p.M <= 64) return launch_f32<64, EPI>(p, stream);
-    if (p.M <= 96) return launch_f32<96, EPI>(p, stream);
-    const int at128 = (p.M + 127) / 128 * 128, at96 = (p.M + 95) / 96 * 96;
-    return at96 < at128 ? launch_f32<96, EPI>(p, stream) : launch_f32<128, EPI>(p, stream);
+    return p.M <= 16 ? launch_f32<16, EPI>(p, stream) : launch_f32<32, EPI>(p, stream);
 }
 
 // Whether rows are whole 16-byte pieces and the launch's counts fit.
 inline bool f32_can_take(const void* A, const void* W, long long M, long long N, int K, int lda, int ldw) {
-    return (((uintptr_t)A | (uintptr_t)W) & 15) == 0 && ((K | lda | ldw) & 3) == 0 && M <= 64LL * 65535 && N <= (1LL << 28);
+    const long long tiles = (M / 16 + 1) * (N / 32 + 1);
+    return (((uintptr_t)A | (uintptr_t)W) & 15) == 0 && ((K | lda | ldw) & 3) == 0 && tiles <= (1LL << 31) / (2 * kF32MaxSplits) && N <= (1LL << 28);
 }
 
 }  // namespace hos

@@ -1179,6 +1179,10 @@ def test_gemm_f32(shape):
         ops.gemm_plain(a, weight, out, **kw)
         err = (out.double() - want).abs().max().item()
         assert err <= 3e-6 * math.sqrt(K) + 1e-6, (kw, err)
+        for rows in (1, 16, 33):                      # a row's results hang on no other row
+            few = torch.empty(min(rows, M), N, device=DEV)
+            ops.gemm_plain(a[: min(rows, M)], weight, few, **kw)
+            assert torch.equal(few, out[: min(rows, M)]), (kw, rows)
 
 
 @pytest.mark.parametrize("sizes", [(64, 64, 128, 512, 0), (64, 64, 128, 512, 100), (48, 32, 64, 72, 0), (8, 16, 40, 64, 65)])
