@@ -138,8 +138,14 @@ __global__ void rmsnorm_vec_kernel(const TIn* __restrict__ x, const float* __res
     }
 }
 
+// A block has up to kVecThreads threads, so a thread has 64 registers: they hold the rows and both norms' weights of CH = 2
+// chunks, and of four chunks the rows alone (the weights are then read where they are used).  The parts of a K-split product
+// are asked for eight at a time where a thread has room for them, with one chunk (as they came, one or two at a time were
+// under way: a prompt of 97 tokens 2.26 -> 2.23 ms, eight sequences' decode steps 0.5% faster); rows of bfloat16 are never parts.
+constexpr int kVecThreads = 1024;
 template <typename TY, typename TH, int CH>
-__global__ void norm_add_norm_vec_kernel(const TY* __restrict__ y, int n_parts, size_t part_stride,
+__global__ void __launch_bounds__(kVecThreads)
+norm_add_norm_vec_kernel(const TY* __restrict__ y, int n_parts, size_t part_stride,
                                          const float* __restrict__ w_post, float eps_post, float add_one_post,
                                          float* __restrict__ x, const float* __restrict__ w_next, float eps_next,
                                          float add_one_next, TH* __restrict__ h, int D, int late_flag) {
@@ -151,13 +157,17 @@ __global__ void norm_add_norm_vec_kernel(const TY* __restrict__ y, int n_parts, 
     if (!late_x) pdl_launch_dependents();
     __shared__ float scratch[32];
     const size_t base = (size_t)blockIdx.x * D;
-    float4 yv[CH], xv[CH], wp[CH], wn[CH];
+    constexpr bool HELD = CH <= 2;
+    constexpr int AHEAD = sizeof(TY) == 2 ? 0 : (CH == 1 ? 8 : 1);      // parts under way together
+    float4 yv[CH], xv[CH], wp[HELD ? CH : 1], wn[HELD ? CH : 1];
+    if constexpr (HELD) {
 #pragma unroll
-    for (int c = 0; c < CH; ++c) {
-        const int i = (c * blockDim.x + threadIdx.x) * 4;
-        if (i < D) {
-            wp[c] = load4(w_post + i);
-            if (w_next != nullptr) wn[c] = load4(w_next + i);
+        for (int c = 0; c < CH; ++c) {
+            const int i = (c * blockDim.x + threadIdx.x) * 4;
+            if (i < D) {
+                wp[c] = load4(w_post + i);
+                if (w_next != nullptr) wn[c] = load4(w_next + i);
+            }
         }
     }
     pdl_wait();       // the kernels before this one are complete from here on
@@ -168,17 +178,17 @@ __global__ void norm_add_norm_vec_kernel(const TY* __restrict__ y, int n_parts, 
         const int i = (c * blockDim.x + threadIdx.x) * 4;
         if (i < D) {
             xv[c] = load4(x + base + i);
-            // The parts of a K-split product, eight asked for before any is added (as they came, one or two at a time were
-            // under way: a prompt of 97 tokens 2.26 -> 2.23 ms, eight sequences' decode steps 0.5% faster).
             yv[c] = load4(y + base + i);
-            for (int p0 = 1; p0 < n_parts; p0 += 8) {
-                float4 t[8];
+            if constexpr (AHEAD > 0) {
+                for (int p0 = 1; p0 < n_parts; p0 += AHEAD) {
+                    float4 t[AHEAD];
 #pragma unroll
-                for (int p = 0; p < 8; ++p)
-                    if (p0 + p < n_parts) t[p] = load4(y + (p0 + p) * part_stride + base + i);
+                    for (int p = 0; p < AHEAD; ++p)
+                        if (p0 + p < n_parts) t[p] = load4(y + (p0 + p) * part_stride + base + i);
 #pragma unroll
-                for (int p = 0; p < 8; ++p)
-                    if (p0 + p < n_parts) { yv[c].x += t[p].x; yv[c].y += t[p].y; yv[c].z += t[p].z; yv[c].w += t[p].w; }
+                    for (int p = 0; p < AHEAD; ++p)
+                        if (p0 + p < n_parts) { yv[c].x += t[p].x; yv[c].y += t[p].y; yv[c].z += t[p].z; yv[c].w += t[p].w; }
+                }
             }
             ss += yv[c].x * yv[c].x + yv[c].y * yv[c].y + yv[c].z * yv[c].z + yv[c].w * yv[c].w;
         }
@@ -190,10 +200,11 @@ __global__ void norm_add_norm_vec_kernel(const TY* __restrict__ y, int n_parts, 
     for (int c = 0; c < CH; ++c) {
         const int i = (c * blockDim.x + threadIdx.x) * 4;
         if (i < D) {
-            xv[c].x += yv[c].x * r * (wp[c].x + add_one_post);
-            xv[c].y += yv[c].y * r * (wp[c].y + add_one_post);
-            xv[c].z += yv[c].z * r * (wp[c].z + add_one_post);
-            xv[c].w += yv[c].w * r * (wp[c].w + add_one_post);
+            const float4 w = HELD ? wp[HELD ? c : 0] : load4(w_post + i);
+            xv[c].x += yv[c].x * r * (w.x + add_one_post);
+            xv[c].y += yv[c].y * r * (w.y + add_one_post);
+            xv[c].z += yv[c].z * r * (w.z + add_one_post);
+            xv[c].w += yv[c].w * r * (w.w + add_one_post);
             store4(x + base + i, xv[c]);
             if (h != nullptr && w_next == nullptr) store4(h + base + i, xv[c]);
             ss2 += xv[c].x * xv[c].x + xv[c].y * xv[c].y + xv[c].z * xv[c].z + xv[c].w * xv[c].w;
@@ -205,9 +216,11 @@ __global__ void norm_add_norm_vec_kernel(const TY* __restrict__ y, int n_parts, 
 #pragma unroll
     for (int c = 0; c < CH; ++c) {
         const int i = (c * blockDim.x + threadIdx.x) * 4;
-        if (i < D)
-            store4(h + base + i, make_float4(xv[c].x * r2 * (wn[c].x + add_one_next), xv[c].y * r2 * (wn[c].y + add_one_next),
-                                             xv[c].z * r2 * (wn[c].z + add_one_next), xv[c].w * r2 * (wn[c].w + add_one_next)));
+        if (i < D) {
+            const float4 w = HELD ? wn[HELD ? c : 0] : load4(w_next + i);
+            store4(h + base + i, make_float4(xv[c].x * r2 * (w.x + add_one_next), xv[c].y * r2 * (w.y + add_one_next),
+                                             xv[c].z * r2 * (w.z + add_one_next), xv[c].w * r2 * (w.w + add_one_next)));
+        }
     }
 }
 
@@ -305,13 +318,26 @@ __global__ void norm_add_norm_rows_kernel(const TY* __restrict__ y, int n_parts,
     }
 }
 
+// The most threads that a block of it may have: its 69 to 80 registers a thread leave room for fewer than 1,024, so the widest
+// rows (above some 6,100 numbers of 32 bits, 7,100 of bfloat16) take the kernel for few rows.  Asked once.
+template <typename TY, typename TH>
+static int rows_kernel_threads() {
+    static const int most = [] {
+        cudaFuncAttributes at;
+        if (cudaFuncGetAttributes(&at, norm_add_norm_rows_kernel<TY, TH>) == cudaSuccess) return at.maxThreadsPerBlock;
+        cudaGetLastError();
+        return 0;
+    }();
+    return most;
+}
+
 // Threads per row and chunks per thread for the register-resident kernels; chunks 0: use the others.
 static void vec_shape(int D, int* threads, int* chunks) {
     *chunks = 0;
     if (D % 4 != 0) return;
     const int quads = D / 4;
     for (int ch = 1; ch <= 4; ch *= 2) {
-        if (quads <= 1024 * ch) {
+        if (quads <= kVecThreads * ch) {
             *chunks = ch;
             *threads = (((quads + ch - 1) / ch) + 31) / 32 * 32;
             return;
@@ -704,20 +730,22 @@ extern "C" int hos_norm_add_norm(const void* y, int y_dtype, int n_parts, const 
     if (h == nullptr) w_next = nullptr;
     if (h == nullptr) h_dtype = y_dtype == kF32 ? kF32 : kBF16;
     // many rows of a width in steps of 8: CTAs that walk over rows with the next row's loads in flight
-    if (N >= kRowsKernelMinRows && chunks != 0 && D % 8 == 0 && D / 8 <= 1024) {
+    if (N >= kRowsKernelMinRows && chunks != 0 && D % 8 == 0) {
         const int threads_r = (D / 8 + 31) / 32 * 32;
         // about 1024 threads per SM: measured best (3 CTAs of 288 threads at width 2304; more CTAs with fewer rows each
         // lose what the loads in flight across the sums gain)
         const int per_sm = 1024 / threads_r < 1 ? 1 : 1024 / threads_r;
         const int grid_r = N < sm_count_cached() * per_sm ? N : sm_count_cached() * per_sm;
-#define HOS_ROWS(TY, TH) launch_pdl(norm_add_norm_rows_kernel<TY, TH>, dim3(grid_r), dim3(threads_r), 0, stream,            \
-        (const TY*)y, n_parts, ps, w_post, eps_post, a1, x, w_next, eps_next, a2, (TH*)h, D, N)
-        if (y_dtype == kF32 && h_dtype == kF32) HOS_ROWS(float, float);
-        else if (y_dtype == kF32 && h_dtype == kBF16) HOS_ROWS(float, bf16);
-        else if (y_dtype == kBF16 && h_dtype == kBF16) HOS_ROWS(bf16, bf16);
-        else HOS_REFUSE("norm_add_norm: no kernel for dtypes %d -> %d", y_dtype, h_dtype);
+#define HOS_ROWS(TY, TH)                                                                                                        \
+    if (threads_r <= rows_kernel_threads<TY, TH>()) {                                                                           \
+        launch_pdl(norm_add_norm_rows_kernel<TY, TH>, dim3(grid_r), dim3(threads_r), 0, stream,                                 \
+            (const TY*)y, n_parts, ps, w_post, eps_post, a1, x, w_next, eps_next, a2, (TH*)h, D, N);                            \
+        return check_launch("norm_add_norm");                                                                                   \
+    }
+        if (y_dtype == kF32 && h_dtype == kF32) { HOS_ROWS(float, float) }
+        else if (y_dtype == kF32 && h_dtype == kBF16) { HOS_ROWS(float, bf16) }
+        else if (y_dtype == kBF16 && h_dtype == kBF16) { HOS_ROWS(bf16, bf16) }
 #undef HOS_ROWS
-        return check_launch("norm_add_norm");
     }
     if (y_dtype == kF32 && h_dtype == kF32) HOS_LAUNCH(float, float);
     else if (y_dtype == kF32 && h_dtype == kBF16) HOS_LAUNCH(float, bf16);

@@ -92,6 +92,33 @@ def test_norm_add_norm(dtype, shape):
         close(h, norm(want_x, w2, 1e-5).to(dt), dt)
 
 
+@pytest.mark.parametrize("rows", [3, 300])
+@pytest.mark.parametrize("D", [4096, 4100, 5896, 6144, 7168, 8192, 8200, 10240, 12288, 16384])
+@pytest.mark.parametrize("types", [("float32", "float32"), ("float32", "bfloat16"), ("bfloat16", "bfloat16")])
+def test_norm_add_norm_of_wide_rows(types, D, rows):
+    """Widths at which a block has its most threads: every number of chunks to a thread must leave them registers, with one
+    part and with several (fewer and more than are asked for together).  Against 64 bits: sums of D numbers in 32-bit along
+    trees, a few 2^-24 of numbers below 100; the next norm's rows are rounded once to their type (2^-9 of them in bfloat16)."""
+    from hos_b200 import ops
+    ty, th = DT[types[0]], DT[types[1]]
+    x0 = torch.randn(rows, D, device=DEV)
+    w1, w2 = torch.randn(D, device=DEV) * 0.1, torch.randn(D, device=DEV) * 0.1
+
+    def norm(v, w):
+        return v / torch.sqrt((v * v).mean(-1, keepdim=True) + 1e-6) * (1 + w.double())
+    for parts in (1, 3, 12) if ty == torch.float32 else (1,):
+        y = (torch.randn(parts, rows, D, device=DEV) * 2).to(ty)
+        want = x0.double() + norm(y.double().sum(0), w1)
+        x, h = x0.clone(), torch.empty(rows, D, device=DEV, dtype=th)
+        ops.norm_add_norm(y if parts > 1 else y[0], w1, 1e-6, True, x, w2, 1e-6, True, h)
+        assert (x.double() - want).abs().max().item() <= 2e-5, parts
+        nxt = norm(want, w2)
+        assert torch.all((h.double() - nxt).abs() <= 2e-5 + nxt.abs() * (2.0 ** -8 if th == torch.bfloat16 else 0.0)), parts
+        x, h = x0.clone(), torch.empty(rows, D, device=DEV, dtype=th)
+        ops.norm_add_norm(y if parts > 1 else y[0], w1, 1e-6, True, x, h=h)
+        assert (x.double() - want).abs().max().item() <= 2e-5 and torch.equal(h, x.to(th)), parts
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("act", ["gelu_tanh", "silu"])
 def test_gated_act(dtype, act):
