@@ -48,13 +48,6 @@ __device__ __forceinline__ void latent_give_up() {
         __threadfence_system();
     }
 }
-__device__ __forceinline__ bool latent_wait(uint64_t* bar, uint32_t parity) {
-    if (mbar_try_wait(bar, parity)) return true;
-    const long long t0 = clock64();
-    while (!mbar_try_wait(bar, parity))
-        if (clock64() - t0 > kLWaitCycles) return false;
-    return true;
-}
 
 // ---- what the attention reads -------------------------------------------------------------------------------------
 struct LatentExpand {
@@ -141,6 +134,8 @@ struct LatentPrompt {
     const int* token_seq;
     int n_seqs, n_rows, H, vd, rank, window;
     float scale;
+    long long wait_cycles;      // the limit of every wait
+    int stop_tile;              // for tests of the give-up path: the tile at which a softmax warp takes its wait as run out (-1: none)
 };
 
 __global__ void __launch_bounds__(kLThreads, 1)
@@ -207,11 +202,12 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap map_q,      // queries,
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_base_smem;
+    bool ok = true;             // false: a wait of this thread (in the softmax warps: of its warp) ran out
+    auto wait = [&](uint64_t* bar, uint32_t parity) { return mbar_wait_cycles(bar, parity, a.wait_cycles); };
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
         if (lane == 0) {
-            bool ok = true;
             pdl_wait();
             mbar_expect_tx(q_full, kLqBytes);
             for (int c = 0; c < 3; ++c) tc_tma_2d(q_s + c * kLqBlock, &map_q, head * kLqCols + 64 * c, row0 + q0, q_full);
@@ -219,12 +215,12 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap map_q,      // queries,
                 const int s = j % kLStages, krow = row0 + (kt_lo + j) * LK;
                 unsigned char* kd = k_s + s * kLkBytes;
                 unsigned char* vd = v_s + s * kLvBytes;
-                if (j >= kLStages && !latent_wait(&k_empty[s], ((j / kLStages) - 1) & 1)) { ok = false; break; }
+                if (j >= kLStages && !wait(&k_empty[s], ((j / kLStages) - 1) & 1)) { ok = false; break; }
                 mbar_expect_tx(&k_full[s], kLkBytes);
                 tc_tma_2d(kd, &map_k, head * kLkCols, krow, &k_full[s]);
                 tc_tma_2d(kd + kLkBlock, &map_k, head * kLkCols + 64, krow, &k_full[s]);
                 tc_tma_2d(kd + 2 * kLkBlock, &map_r, a.rank, krow, &k_full[s]);
-                if (j >= kLStages && !latent_wait(&v_empty[s], ((j / kLStages) - 1) & 1)) { ok = false; break; }
+                if (j >= kLStages && !wait(&v_empty[s], ((j / kLStages) - 1) & 1)) { ok = false; break; }
                 mbar_expect_tx(&v_full[s], kLvBytes);
                 for (int c = 0; c < kLvCols / 64; ++c)
                     tc_tma_2d(vd + c * kLkBlock, &map_v, head * kLvCols + 64 * c, krow, &v_full[s]);
@@ -237,12 +233,12 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap map_q,      // queries,
         if (lane == 0) {
             constexpr uint32_t idesc_s = tc_idesc(LQ, LK, 0);        // S = Q K^T: both K-major
             constexpr uint32_t idesc_o = tc_idesc(LQ, LVDIM, 1);     // O = P V: V is MN-major
-            bool ok = latent_wait(q_full, 0);
+            ok = wait(q_full, 0);
             tc_fence_after_sync();
             auto issue_s = [&](int j) -> bool {
                 const int s = j % kLStages, sb = j & 1;
-                if (!latent_wait(&k_full[s], (j / kLStages) & 1)) return false;
-                if (j >= 2 && !latent_wait(&s_empty[sb], ((j >> 1) - 1) & 1)) return false;
+                if (!wait(&k_full[s], (j / kLStages) & 1)) return false;
+                if (j >= 2 && !wait(&s_empty[sb], ((j >> 1) - 1) & 1)) return false;
                 tc_fence_after_sync();
                 const uint32_t k_addr = smem_u32(k_s + s * kLkBytes), q_addr = smem_u32(q_s);
 #pragma unroll
@@ -261,8 +257,8 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap map_q,      // queries,
             for (int j = 0; j < n_tiles && ok; ++j) {
                 if (j + 1 < n_tiles && !issue_s(j + 1)) { ok = false; break; }      // the next S runs under this tile's softmax
                 const int pb = j & 1, s = j % kLStages;
-                if (!latent_wait(&p_full[pb], (j >> 1) & 1)) { ok = false; break; }
-                if (!latent_wait(&v_full[s], (j / kLStages) & 1)) { ok = false; break; }
+                if (!wait(&p_full[pb], (j >> 1) & 1)) { ok = false; break; }
+                if (!wait(&v_full[s], (j / kLStages) & 1)) { ok = false; break; }
                 tc_fence_after_sync();
                 const uint32_t v_addr = smem_u32(v_s + s * kLvBytes), p_addr = smem_u32(p_s + pb * kLpBytes);
 #pragma unroll
@@ -287,38 +283,44 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap map_q,      // queries,
         const float c2 = a.scale * 1.4426950408889634f;          // weights are exp2(s c2 - m c2), the maximum over raw s
         const float slack = 8.f / a.scale;                       // the running maximum is raised when exceeded by e^8
         float m_ref = -INFINITY, l_run = 0.f;                    // l_run: this thread's keys only
-        bool ok = true;
+        // The eight warps meet at barriers, twice a tile and twice at the end, so none of them leaves on its own: a warp whose
+        // wait ran out waits for nothing and computes nothing any more, but comes to every barrier that is left.  The others'
+        // waits for what it then does not hand on run out in turn, once for each, so the block ends.
+        auto warp_wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, wait(bar, parity)) != 0; };
         for (int j = 0; j < n_tiles; ++j) {
             const int sb = j & 1, pb = j & 1;
-            if (!latent_wait(&s_full[sb], (j >> 1) & 1)) { ok = false; break; }
-            tc_fence_after_sync();
-            float sc[32];
-            {
-                uint32_t v0[32];
-                tc_ld32(t_lane + kLColS + sb * LK + 32 * half, v0);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                for (int i = 0; i < 32; ++i) sc[i] = __uint_as_float(v0[i]);
-            }
-            tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&s_empty[sb]);
             const int kt0 = (kt_lo + j) * LK, k0 = kt0 + 32 * half;
             float m_half = -INFINITY;
-            const bool whole = kt0 + LK - 1 <= q0 && (a.window <= 0 || kt0 > q0 + LQ - 1 - a.window);
-            if (!whole) {
+            float sc[32];
+            if (ok) ok = warp_wait(&s_full[sb], (j >> 1) & 1);
+            if (ok) {
+                tc_fence_after_sync();
+                {
+                    uint32_t v0[32];
+                    tc_ld32(t_lane + kLColS + sb * LK + 32 * half, v0);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    const int key = k0 + i;
-                    sc[i] = key <= qpos && (a.window <= 0 || key > qpos - a.window) ? sc[i] : -INFINITY;
+                    for (int i = 0; i < 32; ++i) sc[i] = __uint_as_float(v0[i]);
                 }
-            }
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&s_empty[sb]);
+                const bool whole = kt0 + LK - 1 <= q0 && (a.window <= 0 || kt0 > q0 + LQ - 1 - a.window);
+                if (!whole) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) m_half = fmaxf(m_half, sc[i]);
+                    for (int i = 0; i < 32; ++i) {
+                        const int key = k0 + i;
+                        sc[i] = key <= qpos && (a.window <= 0 || key > qpos - a.window) ? sc[i] : -INFINITY;
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < 32; ++i) m_half = fmaxf(m_half, sc[i]);
+            }
             xchg[half * LQ + r] = m_half;
             asm volatile("bar.sync 1, 256;" ::: "memory");
             const float m_tile = fmaxf(m_half, xchg[(half ^ 1) * LQ + r]);
             asm volatile("bar.sync 1, 256;" ::: "memory");       // both have read before the next tile writes
+            if (!ok) continue;
             float factor = 1.f;
             if (m_tile > m_ref + slack || (m_ref == -INFINITY && m_tile > -INFINITY)) {
                 factor = m_ref == -INFINITY ? 0.f : ex2_approx((m_ref - m_tile) * c2);
@@ -335,10 +337,13 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap map_q,      // queries,
                 lo[i / 2] = pack_bf16(w0 - __uint_as_float(hi[i / 2] << 16), w1 - __uint_as_float(hi[i / 2] & 0xffff0000u));
             }
             l_run = l_run * factor + psum;
-            if (j >= 2 && !latent_wait(&pv_done[pb], ((j >> 1) - 1) & 1)) { ok = false; break; }
+            if (j >= 2) ok = warp_wait(&pv_done[pb], ((j >> 1) - 1) & 1);
+            if (j == a.stop_tile && warp == 2) ok = false;
+            if (!ok) continue;
             if (j > 0 && __any_sync(0xffffffffu, factor != 1.f)) {
                 // O is touched only between products: wait for the one of the tile before
-                if (!latent_wait(&pv_done[pb ^ 1], ((j - 1) >> 1) & 1)) { ok = false; break; }
+                ok = warp_wait(&pv_done[pb ^ 1], ((j - 1) >> 1) & 1);
+                if (!ok) continue;
                 tc_fence_after_sync();
 #pragma unroll 1
                 for (int c = half * (LVDIM / 2); c < (half + 1) * (LVDIM / 2); c += 32) {
@@ -362,7 +367,8 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap map_q,      // queries,
             if (kt0 + LK > len) {
                 // the tile's rows beyond the sequence are another's, whose values must not matter (0 times infinity)
                 const int s = j % kLStages, vr = (int)(threadIdx.x - 64) >> 2, part = threadIdx.x & 3;
-                if (!latent_wait(&v_full[s], (j / kLStages) & 1)) { ok = false; break; }
+                ok = warp_wait(&v_full[s], (j / kLStages) & 1);
+                if (!ok) continue;
                 if (kt0 + vr >= len)
                     for (int c = part * 8; c < part * 8 + 8; ++c)
                         *reinterpret_cast<uint4*>(v_s + s * kLvBytes + (c >> 3) * kLkBlock + vr * 128 + (c & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
@@ -373,12 +379,12 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap map_q,      // queries,
             if (lane == 0) mbar_arrive(&p_full[pb]);
         }
         // ---- epilogue: O / l -> bfloat16; each thread half of its row ----
-        if (ok && !latent_wait(&pv_done[(n_tiles - 1) & 1], ((n_tiles - 1) >> 1) & 1)) ok = false;
+        if (ok) ok = warp_wait(&pv_done[(n_tiles - 1) & 1], ((n_tiles - 1) >> 1) & 1);
+        tc_fence_after_sync();
+        asm volatile("bar.sync 1, 256;" ::: "memory");      // every reader of xchg's maxima is done
+        xchg[half * LQ + r] = l_run;
+        asm volatile("bar.sync 1, 256;" ::: "memory");
         if (ok) {
-            tc_fence_after_sync();
-            asm volatile("bar.sync 1, 256;" ::: "memory");      // every reader of xchg's maxima is done
-            xchg[half * LQ + r] = l_run;
-            asm volatile("bar.sync 1, 256;" ::: "memory");
             float l_row = l_run + xchg[(half ^ 1) * LQ + r];
             if (a.sink != nullptr) l_row += expf(a.sink[head] - m_ref * a.scale);
             const float inv = l_row > 0.f ? 1.f / l_row : 0.f;
@@ -403,7 +409,7 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap map_q,      // queries,
         if (!ok && lane == 0) latent_give_up();
     }
     tc_fence_before_sync();
-    __syncthreads();
+    if (__syncthreads_or(!ok)) let_work_under_way_end();
     if (warp == 1)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kLTmemCols) : "memory");
 }
@@ -422,11 +428,13 @@ extern "C" int hos_latent_prompt_set_error_word(int* word) {
 // Rows 0 .. n_rows - 1 of a step whose sequences all start at position 0 (sequence s has the rows cu_seqlens[s] ..).
 // q: row n, head h at q + n * ldq + h * (dq + P); kv: 32-bit [n_rows][H * dq + H * vd], the latents expanded; kc: the latent
 // rows [n_rows][rank + P].  q_ws [n_rows][H][192], k_ws [n_rows][H][128] and v_ws [n_rows][H][256] bfloat16: scratch.  out [n_rows][H * vd].
-// n_q_tiles: at least the sum over the sequences of ceil(rows / 128).
+// n_q_tiles: at least the sum over the sequences of ceil(rows / 128).  wait_cycles, stop_tile: for tests of what happens when a
+// wait runs out (LatentPrompt); 0 and -1 otherwise.
 extern "C" int hos_latent_prompt(const void* q, long long ldq, const float* kv, const void* kc, const float* inv_freq, int rot_dims,
                                  int style, const float* sink, const int* token_pos, const int* token_seq, const int* cu_seqlens,
                                  int n_seqs, int n_q_tiles, int n_rows, int H, int dq, int P, int vd, int rank, float scale, int window,
-                                 void* q_ws, void* k_ws, void* v_ws, void* out, cudaStream_t stream) {
+                                 void* q_ws, void* k_ws, void* v_ws, void* out, long long wait_cycles, int stop_tile,
+                                 cudaStream_t stream) {
     if (n_rows <= 0 || n_seqs <= 0 || n_q_tiles <= 0) return 0;
     if (H <= 0 || dq <= 0 || dq > LDIM || P <= 0 || P > LDIM || vd <= 0 || vd > LVDIM || ((dq | P | vd | rank) & 7) || (ldq & 3))
         HOS_REFUSE("latent_prompt: keys of %d + %d and values of %d numbers (rank %d) are not multiples of 8 up to %d, %d and %d",
@@ -447,7 +455,8 @@ extern "C" int hos_latent_prompt(const void* q, long long ldq, const float* kv, 
                       (bf16*)q_ws, (bf16*)k_ws, (bf16*)v_ws};
     launch_pdl(latent_expand_kernel, dim3(n_rows), dim3(256), 0, stream, e);
     if ((rc = check_launch("latent_prompt (expansion)"))) return rc;
-    LatentPrompt a = {(bf16*)out, sink, cu_seqlens, token_seq, n_seqs, n_rows, H, vd, rank, window, scale};
+    LatentPrompt a = {(bf16*)out, sink, cu_seqlens, token_seq, n_seqs, n_rows, H, vd, rank, window, scale,
+                      wait_cycles > 0 ? wait_cycles : kLWaitCycles, stop_tile};
     launch_pdl(latent_prompt_kernel, dim3(H, n_q_tiles), dim3(kLThreads), kLSmem, stream, mq, mk, mr, mv, a);
     return check_launch("latent_prompt");
 }

@@ -36,12 +36,20 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-// Wait for a phase, but not for ever: after `limit` failed tries the caller gets false,
-// records the fact and leaves (a wait that cannot end must not hang the GPU).
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32_t limit = (1u << 24)) {
-    for (uint32_t i = 0; i < limit; ++i)
-        if (mbar_try_wait(bar, parity)) return true;
-    return false;
+// Wait for a phase, but not for ever: after `limit` clock cycles the caller gets false, records the fact and leaves (a wait
+// that cannot end must not hang the GPU).
+__device__ __forceinline__ bool mbar_wait_cycles(uint64_t* bar, uint32_t parity, long long limit) {
+    if (mbar_try_wait(bar, parity)) return true;
+    const long long t0 = clock64();
+    while (!mbar_try_wait(bar, parity))
+        if (clock64() - t0 > limit) return false;
+    return true;
+}
+// What a block does between the barrier behind which it issues nothing any more and its end, if one of its waits ran out: copies
+// and products that are still under way get about two milliseconds to end, before the memory they write is somebody else's.
+__device__ __forceinline__ void let_work_under_way_end() {
+    const long long t0 = clock64();
+    while (clock64() - t0 < (1ll << 22)) __nanosleep(1000);
 }
 
 // ---- bulk copy global -> shared, completion counted on an mbarrier ---------------------

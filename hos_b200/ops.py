@@ -703,10 +703,11 @@ LATENT_PROMPT_SIZES = (64, 64, 128)      # a key's unrotated and rotated numbers
 
 def latent_prompt(q: torch.Tensor, dq: int, vd: int, inv_freq: Optional[torch.Tensor], rot_dims: int, style: int, kv: torch.Tensor,
                   kc: torch.Tensor, sink: Optional[torch.Tensor], out: torch.Tensor, step, rows: int, rank: int, scale: float,
-                  window: Optional[int]) -> None:
+                  window: Optional[int], wait_cycles: int = 0, stop_tile: int = -1) -> None:
     """Rows 0 .. rows-1 of the step (sequences from position 0) over keys and values that were formed: kv float32 [rows, heads x dq +
     heads x vd], the latents times the heads' W_uk and W_uv; kc: the latent rows, whose last numbers are the keys' rotated
-    part; q: rows of the heads' queries as projected (dq unrotated and then the rotated numbers each).  out [N, heads x vd]."""
+    part; q: rows of the heads' queries as projected (dq unrotated and then the rotated numbers each).  out [N, heads x vd].
+    wait_cycles, stop_tile: for tests of a wait that runs out (the limit of the waits; the tile at which one does)."""
     _check(q, "query rows", torch.bfloat16, 2)
     _check(kv, "expanded latents", torch.float32, 2)
     _check(kc, "latent rows", torch.bfloat16, 2)
@@ -723,7 +724,7 @@ def latent_prompt(q: torch.Tensor, dq: int, vd: int, inv_freq: Optional[torch.Te
     blocks().call("hos_latent_prompt", _ptr(q), q.shape[1], _ptr(kv), _ptr(kc), _ptr(inv_freq), int(rot_dims) if inv_freq is not None else 0,
                   int(style), _ptr(sink), _ptr(step.token_pos), _ptr(step.token_seq), _ptr(step.cu_seqlens), n_seqs, tiles, int(rows),
                   heads, int(dq), rot, int(vd), int(rank), float(scale), int(window) if window else 0, _ptr(ws), _ptr(k_ws), _ptr(v_ws),
-                  _ptr(out), _stream())
+                  _ptr(out), int(wait_cycles), int(stop_tile), _stream())
 
 
 def heads_product(x: torch.Tensor, x_off: int, lda: int, a_head: int, w: torch.Tensor, out: torch.Tensor, out_off: int,

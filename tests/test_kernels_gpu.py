@@ -1263,6 +1263,33 @@ def test_latent_prompt(sizes, lens):
         assert torch.all(err <= want.abs() * 2.0 ** -8 + 2.0 ** -12 * v.abs().max()), err.max().item()
 
 
+@pytest.mark.parametrize("stop_tile", [0, 1, 2, 5])
+def test_latent_prompt_ends_when_a_wait_runs_out(stop_tile):
+    """One softmax warp takes its wait at a tile as run out: the others, which meet it at barriers, end as well, each after one
+    wait of half a millisecond; the host hears of it and the next launch gives what it gave before."""
+    from types import SimpleNamespace
+    from hos_b200 import ops
+    from hos_b200.errors import KernelError
+    H, n, R = 2, 500, 64
+    q = torch.randn(n, H * 128, device=DEV).bfloat16()
+    kc, kv = torch.randn(n, R + 64, device=DEV).bfloat16(), torch.randn(n, H * 192, device=DEV)
+    step = SimpleNamespace(cu_host=(0, n), n_seqs=1, fresh_seqs=0, token_pos=torch.arange(n, dtype=torch.int32, device=DEV),
+                           token_seq=torch.zeros(n, dtype=torch.int32, device=DEV), cu_seqlens=torch.tensor([0, n], dtype=torch.int32, device=DEV))
+
+    def run(**kw):
+        out = torch.zeros(n, H * 128, device=DEV).bfloat16()
+        ops.latent_prompt(q, 64, 128, None, 0, 0, kv, kc, None, out, step, n, R, 0.1, None, **kw)
+        torch.cuda.synchronize()
+        return out
+    want = run()
+    ops.check_errors()
+    run(wait_cycles=1 << 20, stop_tile=stop_tile)
+    with pytest.raises(KernelError, match="latent rows gave up a wait"):
+        ops.check_errors()
+    assert torch.equal(run(), want)
+    ops.check_errors()
+
+
 @pytest.mark.parametrize("act", ["gated_swish", "relu_square"])
 @pytest.mark.parametrize("sizes", [(40, 3, 8, 8, 8), (70, 2, 5, 136, 264), (300, 3, 4, 264, 136), (900, 1, 3, 520, 312)])
 def test_moe_grouped(act, sizes):
