@@ -77,13 +77,6 @@ __device__ __forceinline__ void record_give_up() {
     }
 }
 
-__device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity) {
-    if (mbar_try_wait(bar, parity)) return true;
-    const long long t0 = clock64();
-    while (!mbar_try_wait(bar, parity))
-        if (clock64() - t0 > kTcWaitCycles) return false;
-    return true;
-}
 // ---- tanh and exp2 shared between the MUFU unit and the FMA pipe ----------------------------------
 // Per score the softmax needs a tanh (soft-cap) and an exp2, and the special-function unit takes 16 a clock
 // per SM: with two softmax warps on a scheduler that unit, not the issue slots, sets the pace.  So a fixed
@@ -156,7 +149,13 @@ struct PrefillTcArgs {
     const int* seq_slot;
     const int* page_table;
     int table_stride, ring_pages;
+    long long wait_cycles;      // the limit of every wait
+    int stop_tile;              // for tests of the give-up path: the tile at which a softmax warp takes its wait as run out (-1: none)
 };
+
+// The eight softmax warps of a CTA meet at barriers, twice a tile and twice at the end, so none of them leaves on its own: a warp
+// whose wait ran out waits for nothing and computes nothing any more, but comes to every barrier that is left.  The others' waits
+// for what it then does not hand on run out in turn, once for each, so the kernel ends.
 
 // PAGED: map_kv covers the key pages and map_v the value pages, both as [pages x kv heads x 64 rows][head_dim]
 // without swizzle; otherwise map_kv covers the projection rows (keys and values) and map_v is not used.
@@ -232,11 +231,12 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,      // boxes 
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_base_smem;
+    bool ok = true;             // false: a wait of this thread (in the softmax warps: of its warp) ran out
+    auto tc_wait = [&](uint64_t* bar, uint32_t parity) { return mbar_wait_cycles(bar, parity, a.wait_cycles); };
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
         if (lane == 0) {
-            bool ok = true;
             pdl_wait();       // the projection's rows and the step's keys and values are complete from here on
             mbar_expect_tx(q_full, kQBytesTc);
             for (int c = 0; c < CBLK; ++c)
@@ -272,7 +272,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,      // boxes 
         if (lane == 0) {
             constexpr uint32_t idesc_s = tc_idesc(TQ, TK, 0);        // S = Q K^T: both K-major
             constexpr uint32_t idesc_o = tc_idesc(TQ, THD, 1);       // O = P V: V is MN-major
-            bool ok = tc_wait(q_full, 0);
+            ok = tc_wait(q_full, 0);
             tc_fence_after_sync();
             auto issue_s = [&](int j) -> bool {
                 const int s = j % kKVStages, sb = j & 1;
@@ -327,39 +327,40 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,      // boxes 
         const float c2 = c_logit * 1.4426950408889634f;
         const float slack_t = kRescaleSlack / c_logit;
         float m_ref = -INFINITY, l_run = 0.f;                    // m_ref in units of t; l_run: this thread's keys only
-        bool ok = true;
+        auto warp_wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, tc_wait(bar, parity)) != 0; };
         for (int j = 0; j < n_tiles; ++j) {
             const int sb = j & 1, pb = j & 1;
-            if (!tc_wait(&s_full[sb], (j >> 1) & 1)) { ok = false; break; }
-            tc_fence_after_sync();
-            float sc[32];
-            {
-                uint32_t v0[32];
-                tc_ld32(t_lane + kColS + sb * TK + 32 * half, v0);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                for (int i = 0; i < 32; ++i) sc[i] = __uint_as_float(v0[i]);
-            }
-            tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&s_empty[sb]);            // this warp has its part of the S buffer
-            const int kt0 = (kt_lo + j) * TK;                    // first key of the tile
-            const int k0 = kt0 + 32 * half;
+            const int kt0 = (kt_lo + j) * TK, k0 = kt0 + 32 * half;     // first key of the tile, and of this thread
             float m_half = -INFINITY;
-            if (capped) tanh_scores<32>(sc, pre);
-            // a tile that every query of the block sees whole needs no mask (all but the last one or two of a walk,
-            // and the first ones under a window)
-            const bool whole = kt0 + TK - 1 <= p0 && (a.window <= 0 || kt0 > p0 + TQ - 1 - a.window);
-            if (whole) {
+            float sc[32];
+            if (ok) ok = warp_wait(&s_full[sb], (j >> 1) & 1);
+            if (ok) {
+                tc_fence_after_sync();
+                {
+                    uint32_t v0[32];
+                    tc_ld32(t_lane + kColS + sb * TK + 32 * half, v0);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                for (int i = 0; i < 32; ++i) m_half = fmaxf(m_half, sc[i]);
-            } else {
+                    for (int i = 0; i < 32; ++i) sc[i] = __uint_as_float(v0[i]);
+                }
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&s_empty[sb]);            // this warp has its part of the S buffer
+                if (capped) tanh_scores<32>(sc, pre);
+                // a tile that every query of the block sees whole needs no mask (all but the last one or two of a walk,
+                // and the first ones under a window)
+                const bool whole = kt0 + TK - 1 <= p0 && (a.window <= 0 || kt0 > p0 + TQ - 1 - a.window);
+                if (whole) {
 #pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    const int key = k0 + i;
-                    const bool vis = key <= qpos && (a.window <= 0 || key > qpos - a.window);
-                    sc[i] = vis ? sc[i] : -INFINITY;
-                    m_half = fmaxf(m_half, sc[i]);
+                    for (int i = 0; i < 32; ++i) m_half = fmaxf(m_half, sc[i]);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) {
+                        const int key = k0 + i;
+                        const bool vis = key <= qpos && (a.window <= 0 || key > qpos - a.window);
+                        sc[i] = vis ? sc[i] : -INFINITY;
+                        m_half = fmaxf(m_half, sc[i]);
+                    }
                 }
             }
             // the row's maximum over both halves
@@ -367,6 +368,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,      // boxes 
             asm volatile("bar.sync 1, 256;" ::: "memory");
             const float m_tile = fmaxf(m_half, xchg[(half ^ 1) * TQ + r]);
             asm volatile("bar.sync 1, 256;" ::: "memory");       // both have read before the next tile writes
+            if (!ok) continue;
             // raise the reference maximum only when it is exceeded by a margin (both threads of a row decide alike)
             float factor = 1.f;
             if (m_tile > m_ref + slack_t || (m_ref == -INFINITY && m_tile > -INFINITY)) {
@@ -386,10 +388,13 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,      // boxes 
             }
             l_run = l_run * factor + psum;
             // this P buffer is free once the product of two tiles ago has read it
-            if (j >= 2 && !tc_wait(&pv_done[pb], ((j >> 1) - 1) & 1)) { ok = false; break; }
+            if (j >= 2) ok = warp_wait(&pv_done[pb], ((j >> 1) - 1) & 1);
+            if (j == a.stop_tile && warp == 2) ok = false;
+            if (!ok) continue;
             if (j > 0 && __any_sync(0xffffffffu, factor != 1.f)) {
                 // O is touched only between products: wait for the one of the tile before
-                if (!tc_wait(&pv_done[(j - 1) & 1], ((j - 1) >> 1) & 1)) { ok = false; break; }
+                ok = warp_wait(&pv_done[(j - 1) & 1], ((j - 1) >> 1) & 1);
+                if (!ok) continue;
                 tc_fence_after_sync();
 #pragma unroll 1
                 for (int c = half * (THD / 2); c < (half + 1) * (THD / 2); c += 32) {
@@ -416,12 +421,12 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,      // boxes 
             if (lane == 0) mbar_arrive(&p_full[pb]);
         }
         // ---- epilogue: O / l -> bfloat16 -> global; each thread half of its row ----
-        if (ok && !tc_wait(&pv_done[(n_tiles - 1) & 1], ((n_tiles - 1) >> 1) & 1)) ok = false;
+        if (ok) ok = warp_wait(&pv_done[(n_tiles - 1) & 1], ((n_tiles - 1) >> 1) & 1);
+        tc_fence_after_sync();
+        asm volatile("bar.sync 1, 256;" ::: "memory");      // every reader of xchg's maxima is done
+        xchg[half * TQ + r] = l_run;
+        asm volatile("bar.sync 1, 256;" ::: "memory");
         if (ok) {
-            tc_fence_after_sync();
-            asm volatile("bar.sync 1, 256;" ::: "memory");      // every reader of xchg's maxima is done
-            xchg[half * TQ + r] = l_run;
-            asm volatile("bar.sync 1, 256;" ::: "memory");
             const float l_row = l_run + xchg[(half ^ 1) * TQ + r];
             const float inv = l_row > 0.f ? 1.f / l_row : 0.f;
             bf16* orow = a.out + (size_t)(row0 + q0 + r) * a.out_stride + (size_t)head * THD;
@@ -445,7 +450,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,      // boxes 
         if (!ok && lane == 0) record_give_up();
     }
     tc_fence_before_sync();
-    __syncthreads();
+    if (__syncthreads_or(!ok)) let_work_under_way_end();
     if (warp == 1)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemColsTc) : "memory");
 }
@@ -480,11 +485,11 @@ constexpr int kPairTmemCols = 512;
 static_assert(kPairSmem <= 232448, "the pair kernel's shared memory");
 static_assert(kPairColO + THD <= kPairTmemCols, "the pair kernel's tensor memory");
 
-__device__ __forceinline__ bool tc_wait_cluster(uint64_t* bar, uint32_t parity) {
+__device__ __forceinline__ bool mbar_wait_cluster_cycles(uint64_t* bar, uint32_t parity, long long limit) {
     if (mbar_try_wait_cluster(bar, parity)) return true;
     const long long t0 = clock64();
     while (!mbar_try_wait_cluster(bar, parity))
-        if (clock64() - t0 > kTcWaitCycles) return false;
+        if (clock64() - t0 > limit) return false;
     return true;
 }
 
@@ -554,11 +559,13 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q,      // boxe
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_base_smem;
+    bool ok = true;             // false: a wait of this thread (in the softmax warps: of its warp) ran out
+    auto tc_wait = [&](uint64_t* bar, uint32_t parity) { return mbar_wait_cycles(bar, parity, a.wait_cycles); };
+    auto tc_wait_cluster = [&](uint64_t* bar, uint32_t parity) { return mbar_wait_cluster_cycles(bar, parity, a.wait_cycles); };
 
     if (warp == 0) {
         // ---------------- TMA producer (both CTAs, each its own halves) ----------------
         if (lane == 0) {
-            bool ok = true;
             pdl_wait();       // the projection's rows are complete from here on
             if (leader) mbar_expect_tx(q_full, 2 * kQBytesTc);
             for (int c = 0; c < CBLK; ++c)
@@ -587,7 +594,7 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q,      // boxe
         if (lane == 0 && leader) {
             constexpr uint32_t idesc_s = tc_idesc(2 * TQ, PK, 0);        // S = Q K^T: both K-major
             constexpr uint32_t idesc_o = tc_idesc(2 * TQ, THD, 1);       // O = P V: V is MN-major
-            bool ok = tc_wait(q_full, 0);
+            ok = tc_wait(q_full, 0);
             tc_fence_after_sync();
             auto issue_s = [&](int j) -> bool {
                 const int s = j % kPairStages, sb = j & 1;
@@ -639,44 +646,46 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q,      // boxe
         const float c2 = c_logit * 1.4426950408889634f;
         const float slack_t = kRescaleSlack / c_logit;
         float m_ref = -INFINITY, l_run = 0.f;                    // m_ref in units of t; l_run: this thread's keys only
-        bool ok = true;
+        auto warp_wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, tc_wait(bar, parity)) != 0; };
         for (int j = 0; j < n_tiles; ++j) {
             const int sb = j & 1, pb = j % kPairPBufs;
-            if (!tc_wait(&s_full[sb], (j >> 1) & 1)) { ok = false; break; }
-            tc_fence_after_sync();
-            float sc[64];
-            {
-                uint32_t v0[32], v1[32];
-                tc_ld32(t_lane + kPairColS + sb * PK + 64 * half, v0);
-                tc_ld32(t_lane + kPairColS + sb * PK + 64 * half + 32, v1);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                for (int i = 0; i < 32; ++i) { sc[i] = __uint_as_float(v0[i]); sc[32 + i] = __uint_as_float(v1[i]); }
-            }
-            tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_leader(&s_empty[sb]);     // this warp has its part of the S buffer
-            const int kt0 = (kt_lo + j) * PK;                    // first key of the tile
-            const int k0 = kt0 + 64 * half;
-            if (capped) tanh_scores<64>(sc, pre);
+            const int kt0 = (kt_lo + j) * PK, k0 = kt0 + 64 * half;     // first key of the tile, and of this thread
             float m_half = -INFINITY;
-            const bool whole = kt0 + PK - 1 <= q0 && (a.window <= 0 || kt0 > q0 + TQ - 1 - a.window);
-            if (whole) {
+            float sc[64];
+            if (ok) ok = warp_wait(&s_full[sb], (j >> 1) & 1);
+            if (ok) {
+                tc_fence_after_sync();
+                {
+                    uint32_t v0[32], v1[32];
+                    tc_ld32(t_lane + kPairColS + sb * PK + 64 * half, v0);
+                    tc_ld32(t_lane + kPairColS + sb * PK + 64 * half + 32, v1);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                for (int i = 0; i < 64; ++i) m_half = fmaxf(m_half, sc[i]);
-            } else {
+                    for (int i = 0; i < 32; ++i) { sc[i] = __uint_as_float(v0[i]); sc[32 + i] = __uint_as_float(v1[i]); }
+                }
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_leader(&s_empty[sb]);     // this warp has its part of the S buffer
+                if (capped) tanh_scores<64>(sc, pre);
+                const bool whole = kt0 + PK - 1 <= q0 && (a.window <= 0 || kt0 > q0 + TQ - 1 - a.window);
+                if (whole) {
 #pragma unroll
-                for (int i = 0; i < 64; ++i) {
-                    const int key = k0 + i;
-                    const bool vis = key <= qpos && (a.window <= 0 || key > qpos - a.window);
-                    sc[i] = vis ? sc[i] : -INFINITY;
-                    m_half = fmaxf(m_half, sc[i]);
+                    for (int i = 0; i < 64; ++i) m_half = fmaxf(m_half, sc[i]);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 64; ++i) {
+                        const int key = k0 + i;
+                        const bool vis = key <= qpos && (a.window <= 0 || key > qpos - a.window);
+                        sc[i] = vis ? sc[i] : -INFINITY;
+                        m_half = fmaxf(m_half, sc[i]);
+                    }
                 }
             }
             xchg[half * TQ + r] = m_half;
             asm volatile("bar.sync 1, 256;" ::: "memory");
             const float m_tile = fmaxf(m_half, xchg[(half ^ 1) * TQ + r]);
             asm volatile("bar.sync 1, 256;" ::: "memory");       // both have read before the next tile writes
+            if (!ok) continue;
             float factor = 1.f;
             if (m_tile > m_ref + slack_t || (m_ref == -INFINITY && m_tile > -INFINITY)) {
                 factor = m_ref == -INFINITY ? 0.f : __expf((m_ref - m_tile) * c_logit);
@@ -695,10 +704,13 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q,      // boxe
             }
             l_run = l_run * factor + psum;
             // this P buffer is free once the product that read it last is done
-            if (j >= kPairPBufs && !tc_wait(&pv_done[pb], ((j / kPairPBufs) - 1) & 1)) { ok = false; break; }
+            if (j >= kPairPBufs) ok = warp_wait(&pv_done[pb], ((j / kPairPBufs) - 1) & 1);
+            if (j == a.stop_tile && warp == 2) ok = false;
+            if (!ok) continue;
             if (j > 0 && __any_sync(0xffffffffu, factor != 1.f)) {
                 // O is touched only between products: wait for the one of the tile before
-                if (!tc_wait(&pv_done[(j - 1) % kPairPBufs], ((j - 1) / kPairPBufs) & 1)) { ok = false; break; }
+                ok = warp_wait(&pv_done[(j - 1) % kPairPBufs], ((j - 1) / kPairPBufs) & 1);
+                if (!ok) continue;
                 tc_fence_after_sync();
 #pragma unroll 1
                 for (int c = half * (THD / 2); c < (half + 1) * (THD / 2); c += 32) {
@@ -729,12 +741,12 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q,      // boxe
             if (lane == 0) mbar_arrive_leader(&p_full[pb]);
         }
         // ---- epilogue: O / l -> bfloat16 -> global; each thread half of its row ----
-        if (ok && !tc_wait(&pv_done[(n_tiles - 1) % kPairPBufs], ((n_tiles - 1) / kPairPBufs) & 1)) ok = false;
+        if (ok) ok = warp_wait(&pv_done[(n_tiles - 1) % kPairPBufs], ((n_tiles - 1) / kPairPBufs) & 1);
+        tc_fence_after_sync();
+        asm volatile("bar.sync 1, 256;" ::: "memory");      // every reader of xchg's maxima is done
+        xchg[half * TQ + r] = l_run;
+        asm volatile("bar.sync 1, 256;" ::: "memory");
         if (ok) {
-            tc_fence_after_sync();
-            asm volatile("bar.sync 1, 256;" ::: "memory");      // every reader of xchg's maxima is done
-            xchg[half * TQ + r] = l_run;
-            asm volatile("bar.sync 1, 256;" ::: "memory");
             const float l_row = l_run + xchg[(half ^ 1) * TQ + r];
             const float inv = l_row > 0.f ? 1.f / l_row : 0.f;
             bf16* orow = a.out + (size_t)(row0 + qpos) * a.out_stride + (size_t)head * THD;
@@ -759,7 +771,7 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q,      // boxe
     }
     // ---- teardown: nobody of either CTA touches tensor memory or the other's barriers any more ----
     tc_fence_before_sync();
-    __syncthreads();
+    if (__syncthreads_or(!ok)) let_work_under_way_end();
     cluster_sync_all();
     if (warp == 1) tmem_dealloc_pair(tmem_base, kPairTmemCols);
 }
@@ -808,10 +820,12 @@ extern "C" int hos_attn_prefill_tc_error() {
 
 // rows: the fused projection output [n_rows, row_stride] (q heads, then k heads, then v heads);
 // sequences occupy rows cu_seqlens[s] .. cu_seqlens[s+1]-1, each from position 0; n_q_tiles is the
-// sum over sequences of ceil(len / 128).
+// sum over sequences of ceil(len / 128).  wait_cycles, stop_tile: for tests of what happens when a wait runs out
+// (PrefillTcArgs); 0 and -1 otherwise.
 extern "C" int hos_attn_prefill_tc(const void* rows, long long n_rows, int row_stride, void* out, int out_stride,
                                    const int* cu_seqlens, int n_seqs, int n_q_tiles, int n_heads, int n_kv_heads,
-                                   int head_dim, float scale, float cap, int window, cudaStream_t stream) {
+                                   int head_dim, float scale, float cap, int window, long long wait_cycles, int stop_tile,
+                                   cudaStream_t stream) {
 #if (HOS_HEAD_DIM == 64) || (HOS_HEAD_DIM == 128) || (HOS_HEAD_DIM == 256)
     if (n_q_tiles <= 0 || n_seqs <= 0) return 0;
     if (head_dim != THD) HOS_REFUSE("attn_prefill_tc: built for head_dim %d, asked for %d", THD, head_dim);
@@ -837,6 +851,7 @@ extern "C" int hos_attn_prefill_tc(const void* rows, long long n_rows, int row_s
     a.n_heads = n_heads; a.n_kv_heads = n_kv_heads;
     a.q_col0 = 0; a.k_col0 = n_heads * THD; a.v_col0 = (n_heads + n_kv_heads) * THD;
     a.scale = scale; a.cap = cap; a.window = window;
+    a.wait_cycles = wait_cycles > 0 ? wait_cycles : kTcWaitCycles; a.stop_tile = stop_tile;
     dim3 grid(n_heads, n_q_tiles);
 #if (HOS_HEAD_DIM == 128) || (HOS_HEAD_DIM == 256)
     // pairs of SMs when two query heads share their keys (and nothing switched it off)
@@ -897,6 +912,7 @@ extern "C" int hos_attn_chunk_tc(const void* q, long long n_rows, int row_stride
     a.scale = scale; a.cap = cap; a.window = window;
     a.row_base = row_base; a.token_pos = token_pos; a.seq_slot = seq_slot;
     a.page_table = page_table; a.table_stride = table_stride; a.ring_pages = ring_pages;
+    a.wait_cycles = kTcWaitCycles; a.stop_tile = -1;
     launch_pdl(attn_prefill_tc_kernel<true>, dim3(n_heads, n_q_tiles), dim3(kTcThreads), kTcSmem, stream, mq, mk, mv, a);
     return check_launch("attn_chunk_tc");
 #else

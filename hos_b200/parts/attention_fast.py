@@ -223,11 +223,12 @@ def prompt_blocks(step, block: int):
 
 
 def prefill_tc(rows: torch.Tensor, out, cu_seqlens, n_seqs: int, blocks: int, n_heads, n_kv_heads, head_dim, scale, cap,
-               window, pairs: bool = True) -> None:
+               window, pairs: bool = True, wait_cycles: int = 0, stop_tile: int = -1) -> None:
     """Attention of whole prompts from position 0 on the tcgen05 tensor cores; `rows` is the
     fused projection output [N, (n_heads + 2 n_kv_heads) * head_dim] (head sizes 64, 128, 256).
     `blocks`: at least the sum over sequences of ceil(length / 128).  `pairs`: two query heads that
-    share their keys may run as one pair of SMs (head sizes 128 and 256, an even group)."""
+    share their keys may run as one pair of SMs (head sizes 128 and 256, an even group).
+    wait_cycles, stop_tile: for tests of a wait that runs out (the limit of the waits; the tile at which one does)."""
     lib = lib_for(head_dim)
     want = bool(pairs and enabled["prefill_pair"])
     if _pair_state.get(head_dim) != want:
@@ -235,7 +236,7 @@ def prefill_tc(rows: torch.Tensor, out, cu_seqlens, n_seqs: int, blocks: int, n_
         _pair_state[head_dim] = want
     lib.call("hos_attn_prefill_tc", ops._ptr(rows), rows.shape[0], rows.shape[1], ops._ptr(out), out.shape[1],
              ops._ptr(cu_seqlens), n_seqs, blocks, n_heads, n_kv_heads, head_dim, float(scale), float(cap),
-             int(window) if window else 0, ops._stream())
+             int(window) if window else 0, int(wait_cycles), int(stop_tile), ops._stream())
 
 
 def prefill_tc_gave_up(head_dim: int) -> bool:

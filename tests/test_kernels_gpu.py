@@ -1263,6 +1263,32 @@ def test_latent_prompt(sizes, lens):
         assert torch.all(err <= want.abs() * 2.0 ** -8 + 2.0 ** -12 * v.abs().max()), err.max().item()
 
 
+@pytest.mark.parametrize("stop_tile", [0, 1, 3])
+@pytest.mark.parametrize("hd,pairs", [(64, False), (128, False), (128, True), (256, True)])
+def test_prompt_attention_ends_when_a_wait_runs_out(hd, pairs, stop_tile):
+    """As test_latent_prompt_ends_when_a_wait_runs_out, in the prompt kernels on one SM and on pairs of SMs."""
+    from hos_b200 import ops
+    from hos_b200.errors import KernelError
+    from hos_b200.parts import attention_fast as af
+    nh, nkv, n = 4, 2, 600
+    rows = torch.randn(n, (nh + 2 * nkv) * hd, device=DEV).bfloat16()
+    cu = torch.tensor([0, n], dtype=torch.int32, device=DEV)
+
+    def run(**kw):
+        out = torch.zeros(n, nh * hd, device=DEV).bfloat16()
+        af.prefill_tc(rows, out, cu, 1, (n + 127) // 128, nh, nkv, hd, 0.3 / math.sqrt(hd), 50.0, None, pairs=pairs, **kw)
+        torch.cuda.synchronize()
+        return out
+    want = run()
+    ops.check_errors()
+    run(wait_cycles=1 << 20, stop_tile=stop_tile)
+    with pytest.raises(KernelError, match="prompt attention gave up a wait"):
+        ops.check_errors()
+    assert af.prefill_tc_gave_up(hd) and not af.prefill_tc_gave_up(hd)
+    assert torch.equal(run(), want)
+    ops.check_errors()
+
+
 @pytest.mark.parametrize("stop_tile", [0, 1, 2, 5])
 def test_latent_prompt_ends_when_a_wait_runs_out(stop_tile):
     """One softmax warp takes its wait at a tile as run out: the others, which meet it at barriers, end as well, each after one
