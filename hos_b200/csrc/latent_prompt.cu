@@ -61,6 +61,7 @@ struct LatentExpand {
     bf16* q_out;                // [n][H][192]
     bf16* k_out;                // [n][H][128]
     bf16* v_out;                // [n][H][256]
+    bf16* out;                  // the attention's output [n][H * vd]: zeros in padding rows, which the walk does not visit
 };
 
 __device__ __forceinline__ void split4(const float (&x)[4], uint2& hi, uint2& lo) {
@@ -76,6 +77,8 @@ __global__ void __launch_bounds__(256) latent_expand_kernel(LatentExpand a) {
     const int n = blockIdx.x, H = a.H;
     bf16* v_out = a.v_out + (size_t)n * H * kLvCols;
     if (a.token_seq[n] < 0) {   // padding: nobody's key, but its values may lie in a tile with weight 0
+        uint4* out = reinterpret_cast<uint4*>(a.out + (size_t)n * H * a.vd);
+        for (int i = threadIdx.x; i < H * a.vd / 8; i += blockDim.x) out[i] = make_uint4(0u, 0u, 0u, 0u);
         for (int i = threadIdx.x; i < H * kLvCols / 4; i += blockDim.x) reinterpret_cast<uint2*>(v_out)[i] = make_uint2(0u, 0u);
         return;
     }
@@ -427,7 +430,8 @@ extern "C" int hos_latent_prompt_set_error_word(int* word) {
 
 // Rows 0 .. n_rows - 1 of a step whose sequences all start at position 0 (sequence s has the rows cu_seqlens[s] ..).
 // q: row n, head h at q + n * ldq + h * (dq + P); kv: 32-bit [n_rows][H * dq + H * vd], the latents expanded; kc: the latent
-// rows [n_rows][rank + P].  q_ws [n_rows][H][192], k_ws [n_rows][H][128] and v_ws [n_rows][H][256] bfloat16: scratch.  out [n_rows][H * vd].
+// rows [n_rows][rank + P].  q_ws [n_rows][H][192], k_ws [n_rows][H][128] and v_ws [n_rows][H][256] bfloat16: scratch.  out [n_rows][H * vd], zeros
+// in padding rows (token_seq < 0).
 // n_q_tiles: at least the sum over the sequences of ceil(rows / 128).  wait_cycles, stop_tile: for tests of what happens when a
 // wait runs out (LatentPrompt); 0 and -1 otherwise.
 extern "C" int hos_latent_prompt(const void* q, long long ldq, const float* kv, const void* kc, const float* inv_freq, int rot_dims,
@@ -452,7 +456,7 @@ extern "C" int hos_latent_prompt(const void* q, long long ldq, const float* kv, 
     if (cudaFuncSetAttribute(latent_prompt_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kLSmem) != cudaSuccess)
         HOS_REFUSE("latent_prompt: cannot get %d bytes of shared memory", kLSmem);
     LatentExpand e = {(const bf16*)q, kv, ldq, H, dq, P, vd, {inv_freq, inv_freq != nullptr ? rot_dims : 0, style}, token_pos, token_seq,
-                      (bf16*)q_ws, (bf16*)k_ws, (bf16*)v_ws};
+                      (bf16*)q_ws, (bf16*)k_ws, (bf16*)v_ws, (bf16*)out};
     launch_pdl(latent_expand_kernel, dim3(n_rows), dim3(256), 0, stream, e);
     if ((rc = check_launch("latent_prompt (expansion)"))) return rc;
     LatentPrompt a = {(bf16*)out, sink, cu_seqlens, token_seq, n_seqs, n_rows, H, vd, rank, window, scale,

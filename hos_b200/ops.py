@@ -706,7 +706,8 @@ def latent_prompt(q: torch.Tensor, dq: int, vd: int, inv_freq: Optional[torch.Te
                   window: Optional[int], wait_cycles: int = 0, stop_tile: int = -1) -> None:
     """Rows 0 .. rows-1 of the step (sequences from position 0) over keys and values that were formed: kv float32 [rows, heads x dq +
     heads x vd], the latents times the heads' W_uk and W_uv; kc: the latent rows, whose last numbers are the keys' rotated
-    part; q: rows of the heads' queries as projected (dq unrotated and then the rotated numbers each).  out [N, heads x vd].
+    part; q: rows of the heads' queries as projected (dq unrotated and then the rotated numbers each).  out [N, heads x vd], zeros in
+    padding rows.
     wait_cycles, stop_tile: for tests of a wait that runs out (the limit of the waits; the tile at which one does)."""
     _check(q, "query rows", torch.bfloat16, 2)
     _check(kv, "expanded latents", torch.float32, 2)

@@ -1241,7 +1241,7 @@ def test_latent_prompt(sizes, lens):
                            cu_seqlens=torch.tensor(cu, dtype=torch.int32, device=DEV))
     out = torch.full((rows, H * vd), 7.0, device=DEV).bfloat16()
     ops.latent_prompt(q, dq, vd, inv_freq, rot_dims, style, kv, kc, sink, out, step, rows, R, scale, window)
-    assert torch.all(out[n:] == 7.0)
+    assert torch.all(out[n:] == 0.0)                           # padding rows: a defined output
     for i, x in enumerate(lens):
         s = slice(cu[i], cu[i + 1])
         qq = q[s, : H * (dq + P)].double().view(x, H, dq + P)

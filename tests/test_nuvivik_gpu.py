@@ -733,6 +733,34 @@ def test_the_square_of_relu_experts_alone_against_float64():
             assert float((out[p].double().cpu() - want).abs().max()) < tol * max(1e-2, float(want.abs().max())), (rows, d, f, p)
 
 
+@pytest.mark.parametrize("graph", [False, True])
+def test_a_replayed_prompt_leaves_no_row_undefined(folders, monkeypatch, graph):
+    """A short prompt in a bucket of more rows (95 + 22 tokens in 128), keys and values formed: every row that the attention hands
+    on is written, padding rows as zeros, whatever its buffer held before, and the logits are the oracle's."""
+    from hos_b200 import ops
+    from hos_b200.parts import latent_attention
+    monkeypatch.setattr(latent_attention, "PROMPT_WORK", 0)
+    monkeypatch.setenv("HOS_NO_GRAPH", "" if graph else "1")
+    real, seen = ops.latent_prompt, []
+
+    def filled(*args, **kw):
+        out = args[9]
+        out.fill_(float("nan"))
+        real(*args, **kw)
+        seen.append(out.clone())
+    monkeypatch.setattr(ops, "latent_prompt", filled)
+    seqs = [tokens(i, n, CASES["E"][0]["vocab"]) for i, n in enumerate((95, 22))]
+    want = _oracle(folders["E"], seqs)
+    r = _runner(folders["E"], "bfloat16")
+    for _ in range(2):
+        slots = r.admit(2)
+        got = r.step(slots, seqs).cpu()
+        assert_rows(got, torch.stack([w[-1] for w in want]), "bfloat16", "last tokens")
+        for s in slots:
+            r.release(s)
+    assert seen and all(bool(torch.isfinite(x).all()) and not x[117:].any() for x in seen)
+
+
 def test_products_with_an_activation_and_no_bias():
     """act(x . W^T) with the tanh-form GELU and no bias in every product: few rows, the tcgen05 kernel in both orientations
     and on pairs of SMs, the plain kernel in both types; with a bias as well."""
