@@ -42,13 +42,6 @@ __device__ __forceinline__ void grouped_give_up() {
         __threadfence_system();
     }
 }
-__device__ __forceinline__ bool grouped_wait(uint64_t* bar, uint32_t parity) {
-    if (mbar_try_wait(bar, parity)) return true;
-    const long long t0 = clock64();
-    while (!mbar_try_wait(bar, parity))
-        if (clock64() - t0 > kXWaitCycles) return false;
-    return true;
-}
 
 // A warp per list place.
 __global__ void __launch_bounds__(256)
@@ -72,6 +65,8 @@ struct GroupedArgs {
     void* out;
     int max_tiles, N, K;        // N: numbers of an output row
     float limit, alpha, up_shift;
+    long long wait_cycles;      // the limit of every wait
+    int stop_tile;              // for tests of the give-up path: the CTA's tile at which an epilogue warp takes its wait as run out (-1: none)
 };
 
 template <int STEP>
@@ -111,17 +106,18 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap map_a,      // list place
     }
     const int n_tiles = (p.N + COLS - 1) / COLS, total = used * n_tiles, k_blocks = (p.K + XK - 1) / XK;
     const int rows_per_expert = (GATED ? 2 : 1) * p.N;
+    bool ok = true;                             // false: a wait of this thread (in the epilogue: of its warp) ran out
+    auto wait = [&](uint64_t* bar, uint32_t parity) { return mbar_wait_cycles(bar, parity, p.wait_cycles); };
 
     if (warp == 0) {
         if (lane == 0) {
             int it = 0;
-            bool ok = true;
             for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x) {
                 const int mt = tile % used, n0 = tile / used * COLS;
                 const int w0 = p.tile_expert[mt] * rows_per_expert + n0, w1 = w0 + (GATED ? p.N : XN / 2);
                 for (int kb = 0; kb < k_blocks; ++kb, ++it) {
                     const int s = it % kXStages;
-                    if (it >= kXStages && !grouped_wait(&empty[s], ((it / kXStages) - 1) & 1)) { ok = false; break; }
+                    if (it >= kXStages && !wait(&empty[s], ((it / kXStages) - 1) & 1)) { ok = false; break; }
                     unsigned char* a_dst = stages + s * kXStageBytes;
                     mbar_expect_tx(&full[s], kXStageBytes);
                     tc_tma_2d(a_dst, &map_a, kb * XK, mt * XM, &full[s]);
@@ -136,14 +132,13 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap map_a,      // list place
         if (lane == 0) {
             constexpr uint32_t idesc = tc_idesc(XM, XN, 0);
             int it = 0, local = 0;
-            bool ok = true;
             for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x, ++local) {
                 const int acc = local & 1;
-                if (local >= 2 && !grouped_wait(&acc_empty[acc], ((local >> 1) - 1) & 1)) { ok = false; break; }
+                if (local >= 2 && !wait(&acc_empty[acc], ((local >> 1) - 1) & 1)) { ok = false; break; }
                 tc_fence_after_sync();
                 for (int kb = 0; kb < k_blocks; ++kb, ++it) {
                     const int s = it % kXStages;
-                    if (!grouped_wait(&full[s], (it / kXStages) & 1)) { ok = false; break; }
+                    if (!wait(&full[s], (it / kXStages) & 1)) { ok = false; break; }
                     tc_fence_after_sync();
                     const uint32_t a_addr = smem_u32(stages + s * kXStageBytes);
                     const uint64_t a_desc = desc_kmajor(a_addr), b_desc = desc_kmajor(a_addr + kXABytes);
@@ -160,13 +155,13 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap map_a,      // list place
     } else {
         const int quarter = warp & 3, half = (warp - 2) >> 2, r = quarter * 32 + lane;
         int local = 0;
-        bool ok = true;
         for (int tile = blockIdx.x; tile < total; tile += gridDim.x, ++local) {
             const int mt = tile % used, n_first = tile / used * COLS;
             const int id = p.listed[mt * XM + r];
             const float wt = id >= 0 && p.weight != nullptr ? p.weight[id] : 1.f;
             const int acc = local & 1;
-            if (!grouped_wait(&acc_full[acc], (local >> 1) & 1)) { ok = false; break; }
+            ok = __all_sync(0xffffffffu, wait(&acc_full[acc], (local >> 1) & 1)) && !(local == p.stop_tile && warp == 2);
+            if (!ok) break;
             tc_fence_after_sync();
             const uint32_t t_lane = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * XN;
 #pragma unroll 1
@@ -215,7 +210,7 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap map_a,      // list place
         if (!ok && lane == 0) grouped_give_up();
     }
     tc_fence_before_sync();
-    __syncthreads();
+    if (__syncthreads_or(!ok)) let_work_under_way_end();
     if (warp == 1)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2 * XN) : "memory");
 }
@@ -246,10 +241,12 @@ extern "C" int hos_moe_grouped_set_error_word(int* word) {
 }
 
 // Both products of `max_tiles` listed tiles of 128: rows [max_tiles * 128][D] and y [max_tiles * 128][F] bfloat16 are scratch, pair_out
-// [pairs][D] 32-bit by pair id.  W_up: [experts][2F or F][D], W_down: [experts][D][F].  in_weight or out_weight (by pair, or null).
+// [pairs][D] 32-bit by pair id.  W_up: [experts][2F or F][D], W_down: [experts][D][F].  in_weight or out_weight (by pair, or null).  wait_cycles, stop_tile:
+// for tests of what happens when a wait runs out (GroupedArgs); 0 and -1 otherwise.
 extern "C" int hos_moe_grouped(const void* h, const void* W_up, const void* W_down, const int* listed, const int* tile_expert, void* rows,
                                void* y, float* pair_out, int max_tiles, int n_experts, int D, int F, int top, float limit, float alpha,
-                               float up_shift, const float* in_weight, const float* out_weight, int act, cudaStream_t stream) {
+                               float up_shift, const float* in_weight, const float* out_weight, int act, long long wait_cycles, int stop_tile,
+                               cudaStream_t stream) {
     if (max_tiles <= 0) return 0;
     if (D <= 0 || F <= 0 || D % 8 || F % 8 || top <= 0 || n_experts <= 0 ||
         (((uintptr_t)h | (uintptr_t)W_up | (uintptr_t)W_down | (uintptr_t)rows | (uintptr_t)y | (uintptr_t)pair_out) & 15))
@@ -260,11 +257,12 @@ extern "C" int hos_moe_grouped(const void* h, const void* W_up, const void* W_do
     launch_pdl(moe_gather_kernel, dim3((unsigned)max_tiles * (XM / 8)), dim3(256), 0, stream, (const bf16*)h, listed, tile_expert, (bf16*)rows, D, top);
     int rc = check_launch("moe_grouped (gather)");
     if (rc) return rc;
-    GroupedArgs up = {listed, tile_expert, in_weight, y, max_tiles, F, D, limit, alpha, up_shift};
+    if (wait_cycles <= 0) wait_cycles = kXWaitCycles;
+    GroupedArgs up = {listed, tile_expert, in_weight, y, max_tiles, F, D, limit, alpha, up_shift, wait_cycles, stop_tile};
     if (act == kGatedSwish) rc = launch_grouped<kGroupedGatedUp>(rows, W_up, 2ll * n_experts * F, up, stream);
     else if (act == kReluSquare) rc = launch_grouped<kGroupedUp>(rows, W_up, (long long)n_experts * F, up, stream);
     else HOS_REFUSE("moe_grouped: unknown activation %d", act);
     if (rc) return rc;
-    GroupedArgs down = {listed, tile_expert, out_weight, pair_out, max_tiles, D, F, 0.f, 0.f, 0.f};
+    GroupedArgs down = {listed, tile_expert, out_weight, pair_out, max_tiles, D, F, 0.f, 0.f, 0.f, wait_cycles, stop_tile};
     return launch_grouped<kGroupedDown>(y, W_down, (long long)n_experts * D, down, stream);
 }

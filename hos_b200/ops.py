@@ -812,9 +812,11 @@ MOE_GROUPED_ROWS = 128      # rows of a tile of the lists that moe_grouped takes
 
 
 def moe_grouped(h, w_up, w_down, listed, tile_expert, rows, y, pair_out, top: int, limit: float, alpha: float, up_shift: float,
-                in_weight: Optional[torch.Tensor], out_weight: Optional[torch.Tensor], act: int) -> None:
+                in_weight: Optional[torch.Tensor], out_weight: Optional[torch.Tensor], act: int, wait_cycles: int = 0,
+                stop_tile: int = -1) -> None:
     """Both products of the experts over lists padded to MOE_GROUPED_ROWS; rows [places, D] and y [places, F] are scratch.  The
-    other arguments as moe_gate_up's and moe_down's.  bfloat16, D and F multiples of 8."""
+    other arguments as moe_gate_up's and moe_down's.  bfloat16, D and F multiples of 8.  wait_cycles, stop_tile: for tests of a
+    wait that runs out (the limit of the waits; a CTA's tile at which one does)."""
     for t, what in ((h, "rows"), (w_up, "expert gate/up weights"), (w_down, "expert down weights"), (rows, "gathered rows"), (y, "inner rows")):
         _check(t, what, torch.bfloat16)
     e, d, f = w_down.shape
@@ -823,7 +825,7 @@ def moe_grouped(h, w_up, w_down, listed, tile_expert, rows, y, pair_out, top: in
         raise KernelError("moe_grouped: sizes disagree")
     experts().call("hos_moe_grouped", _ptr(h), _ptr(w_up), _ptr(w_down), _ptr(listed), _ptr(tile_expert), _ptr(rows), _ptr(y),
                   _ptr(pair_out), tile_expert.numel(), e, d, f, int(top), float(limit), float(alpha), float(up_shift),
-                  _ptr(in_weight), _ptr(out_weight), int(act), _stream())
+                  _ptr(in_weight), _ptr(out_weight), int(act), int(wait_cycles), int(stop_tile), _stream())
 
 
 def moe_gate_up(h, w, listed, tile_expert, y, top: int, limit: float, alpha: float, up_shift: float = 1.0,

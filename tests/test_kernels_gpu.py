@@ -1357,6 +1357,37 @@ def test_moe_grouped(act, sizes):
             assert err <= 6 * 2.0 ** -8 * (z @ down[e].double().T).square().mean().sqrt().item() + 1e-6, (on_input, e, err)
 
 
+@pytest.mark.parametrize("stop_tile", [0, 1])
+def test_moe_grouped_ends_when_a_wait_runs_out(stop_tile):
+    """An epilogue warp takes its wait at a CTA's first or second tile as run out: the kernels end, the host hears of it and the
+    next call gives what it gave before.  46 tiles of rows in slices of 128 and 256 columns: more than one tile to a CTA."""
+    from hos_b200 import ops
+    from hos_b200.errors import KernelError
+    n, top, E, D, F = 1500, 2, 4, 1032, 1536
+    pairs, tile = n * top, ops.MOE_GROUPED_ROWS
+    h = torch.randn(n, D, device=DEV).bfloat16()
+    up = (torch.randn(E, 2 * F, D, device=DEV) / math.sqrt(D)).bfloat16()
+    down = (torch.randn(E, D, F, device=DEV) / math.sqrt(F)).bfloat16()
+    choice = torch.randint(0, E, (pairs,), dtype=torch.int32, device=DEV)
+    tiles = min(pairs, E) + pairs // tile
+    listed, owner = (torch.empty(k, dtype=torch.int32, device=DEV) for k in (tiles * tile, tiles))
+    ops.moe_align(choice, E, listed, owner, tile)
+
+    def run(**kw):
+        rows, y = (torch.zeros(tiles * tile, k, device=DEV).bfloat16() for k in (D, F))
+        out = torch.zeros(pairs, D, device=DEV)
+        ops.moe_grouped(h, up, down, listed, owner, rows, y, out, top, 0.0, 1.0, 0.0, None, None, ops.EXPERT_ACTIVATIONS["gated_swish"], **kw)
+        torch.cuda.synchronize()
+        return out
+    want = run()
+    ops.check_errors()
+    run(wait_cycles=1 << 20, stop_tile=stop_tile)
+    with pytest.raises(KernelError, match="routed experts gave up a wait"):
+        ops.check_errors()
+    assert torch.equal(run(), want)
+    ops.check_errors()
+
+
 @pytest.mark.parametrize("many", [False, True])
 @pytest.mark.parametrize("dim,vdim", [(64, 36), (128, 128), (256, 20)])
 def test_long_delta_walk(dim, vdim, many):
