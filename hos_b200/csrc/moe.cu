@@ -281,9 +281,9 @@ moe_choose_kernel(const float* __restrict__ logits, const float* __restrict__ co
 }
 
 // One block.  listed: [cap] pair ids (row * top + choice) expert by expert, -1 where a tile is padded;
-// tile_expert: [max_tiles], -1 beyond the real tiles.
+// tile_expert: [max_tiles], -1 beyond the real tiles; tile_row (or null): how many pairs the tiles before each one hold.
 __global__ void moe_align_kernel(const int* __restrict__ choice, int n_pairs, int n_experts, int* __restrict__ listed,
-                                 int cap, int* __restrict__ tile_expert, int max_tiles, int tile_rows) {
+                                 int cap, int* __restrict__ tile_expert, int max_tiles, int tile_rows, int* __restrict__ tile_row) {
     pdl_enter();
     extern __shared__ int sh[];                // count[n_experts], start[n_experts + 1], cursor[n_experts]
     int* count = sh;
@@ -297,13 +297,17 @@ __global__ void moe_align_kernel(const int* __restrict__ choice, int n_pairs, in
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        int at = 0;
+        int at = 0, held = 0;
         for (int e = 0; e < n_experts; ++e) {
             start[e] = at;
             const int tiles = (count[e] + tile_rows - 1) / tile_rows;
             for (int t = 0; t < tiles; ++t)
-                if (at / tile_rows + t < max_tiles) tile_expert[at / tile_rows + t] = e;
+                if (at / tile_rows + t < max_tiles) {
+                    tile_expert[at / tile_rows + t] = e;
+                    if (tile_row != nullptr) tile_row[at / tile_rows + t] = held + t * tile_rows;
+                }
             at += tiles * tile_rows;
+            held += count[e];
         }
         start[n_experts] = at;
         for (int t = at / tile_rows; t < max_tiles; ++t) tile_expert[t] = -1;
@@ -781,13 +785,13 @@ extern "C" int hos_moe_route(const void* h, int dtype, const float* router, cons
 }
 
 extern "C" int hos_moe_align(const int* choice, int n_pairs, int n_experts, int* listed, int cap, int* tile_expert,
-                             int max_tiles, int tile_rows, cudaStream_t stream) {
+                             int max_tiles, int tile_rows, int* tile_row, cudaStream_t stream) {
     if (n_pairs <= 0) return 0;
     if (tile_rows <= 0) HOS_REFUSE("moe_align: tiles of %d rows", tile_rows);
     const size_t smem = (size_t)(3 * n_experts + 1) * sizeof(int);
     if (smem > 48 * 1024) HOS_REFUSE("moe_align: %d experts are more than a block's shared memory holds", n_experts);
     launch_pdl(moe_align_kernel, dim3(1), dim3(1024), smem, stream, choice, n_pairs, n_experts, listed, cap, tile_expert,
-               max_tiles, tile_rows);
+               max_tiles, tile_rows, tile_row);
     return check_launch("moe_align");
 }
 

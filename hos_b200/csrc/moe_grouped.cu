@@ -1,9 +1,11 @@
 // The routed experts' two products on the 5th-generation tensor cores, bfloat16, over lists of (row, choice) pairs that
 // are padded to tiles of 128 for every expert (moe.cu, align).
 //
-//   gather    the listed rows, one after another (a tile's operand is then a box that TMA can fetch)
+//   gather    the listed rows, one after another (a tile's operand is then a box that TMA can fetch).  Tiles are padded, rows are not: a
+//             box goes on into the next expert's rows, and what comes of those is not stored, so the rows take as much memory as
+//             there are pairs, however many experts share them
 //   up        per tile and 256 rows of the expert's W (128 gate rows and their 128 up rows where the activation has a gate): tcgen05.mma
-//             M = 128, N = 256, the activation in the epilogue, rows of bfloat16 by list place
+//             M = 128, N = 256, the activation in the epilogue, rows of bfloat16 in the same order
 //   down      the same product over the inner numbers, times the pair's weight, to the pair's row of a 32-bit buffer
 //
 // A persistent kernel, one CTA per SM: a TMA warp, a warp that issues the products, eight epilogue warps (two for every
@@ -46,14 +48,15 @@ __device__ __forceinline__ void grouped_give_up() {
 // A warp per list place.
 __global__ void __launch_bounds__(256)
 moe_gather_kernel(const bf16* __restrict__ h, const int* __restrict__ listed, const int* __restrict__ tile_expert,
-                  bf16* __restrict__ rows, int D, int top) {
+                  const int* __restrict__ tile_row, bf16* __restrict__ rows, int D, int top) {
     pdl_enter();
     const int place = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (tile_expert[place / XM] < 0) return;
     const int id = listed[place];
     if (id < 0) return;
     const uint4* from = reinterpret_cast<const uint4*>(h + (size_t)(id / top) * D);
-    uint4* to = reinterpret_cast<uint4*>(rows + (size_t)place * D);
+    const int tile = place / XM;
+    uint4* to = reinterpret_cast<uint4*>(rows + ((size_t)(tile_row != nullptr ? tile_row[tile] : tile * XM) + place % XM) * D);
 #pragma unroll 4
     for (int i = threadIdx.x & 31; i < D / 8; i += 32) to[i] = from[i];
 }
@@ -61,6 +64,7 @@ moe_gather_kernel(const bf16* __restrict__ h, const int* __restrict__ listed, co
 struct GroupedArgs {
     const int* listed;
     const int* tile_expert;
+    const int* tile_row;        // where a tile's rows begin (null: at 128 times its number)
     const float* weight;        // by pair: on the expert's input (up) or its output (down), or null
     void* out;
     int max_tiles, N, K;        // N: numbers of an output row
@@ -106,6 +110,7 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap map_a,      // list place
     }
     const int n_tiles = (p.N + COLS - 1) / COLS, total = used * n_tiles, k_blocks = (p.K + XK - 1) / XK;
     const int rows_per_expert = (GATED ? 2 : 1) * p.N;
+    auto first_row = [&](int mt) { return p.tile_row != nullptr ? p.tile_row[mt] : mt * XM; };
     bool ok = true;                             // false: a wait of this thread (in the epilogue: of its warp) ran out
     auto wait = [&](uint64_t* bar, uint32_t parity) { return mbar_wait_cycles(bar, parity, p.wait_cycles); };
 
@@ -113,14 +118,14 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap map_a,      // list place
         if (lane == 0) {
             int it = 0;
             for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x) {
-                const int mt = tile % used, n0 = tile / used * COLS;
+                const int mt = tile % used, n0 = tile / used * COLS, row0 = first_row(mt);
                 const int w0 = p.tile_expert[mt] * rows_per_expert + n0, w1 = w0 + (GATED ? p.N : XN / 2);
                 for (int kb = 0; kb < k_blocks; ++kb, ++it) {
                     const int s = it % kXStages;
                     if (it >= kXStages && !wait(&empty[s], ((it / kXStages) - 1) & 1)) { ok = false; break; }
                     unsigned char* a_dst = stages + s * kXStageBytes;
                     mbar_expect_tx(&full[s], kXStageBytes);
-                    tc_tma_2d(a_dst, &map_a, kb * XK, mt * XM, &full[s]);
+                    tc_tma_2d(a_dst, &map_a, kb * XK, row0, &full[s]);
                     tc_tma_2d(a_dst + kXABytes, &map_w, kb * XK, w0, &full[s]);
                     tc_tma_2d(a_dst + kXABytes + kXBBytes / 2, &map_w, kb * XK, w1, &full[s]);
                 }
@@ -158,6 +163,7 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap map_a,      // list place
         for (int tile = blockIdx.x; tile < total; tile += gridDim.x, ++local) {
             const int mt = tile % used, n_first = tile / used * COLS;
             const int id = p.listed[mt * XM + r];
+            const size_t row = STEP == kGroupedDown ? (size_t)max(id, 0) : (size_t)first_row(mt) + r;      // of the output
             const float wt = id >= 0 && p.weight != nullptr ? p.weight[id] : 1.f;
             const int acc = local & 1;
             ok = __all_sync(0xffffffffu, wait(&acc_full[acc], (local >> 1) & 1)) && !(local == p.stop_tile && warp == 2);
@@ -174,7 +180,7 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap map_a,      // list place
                 if (id >= 0) {
                     const int n0 = n_first + c0, left = p.N - n0;                // N is a multiple of 8
                     if (STEP == kGroupedDown) {
-                        float4* dst = reinterpret_cast<float4*>((float*)p.out + (size_t)id * p.N + n0);
+                        float4* dst = reinterpret_cast<float4*>((float*)p.out + row * p.N + n0);
 #pragma unroll
                         for (int q = 0; q < 8; ++q)
                             if (4 * q < left)
@@ -182,7 +188,7 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap map_a,      // list place
                                                      __uint_as_float(v[4 * q + 2]) * wt, __uint_as_float(v[4 * q + 3]) * wt);
                     } else {
                         constexpr int ACT = GATED ? kGatedSwish : kReluSquare;
-                        uint4* dst = reinterpret_cast<uint4*>((bf16*)p.out + (size_t)(mt * XM + r) * p.N + n0);
+                        uint4* dst = reinterpret_cast<uint4*>((bf16*)p.out + row * p.N + n0);
 #pragma unroll
                         for (int q = 0; q < 4; ++q) {
                             uint32_t w[4];
@@ -216,10 +222,10 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap map_a,      // list place
 }
 
 template <int STEP>
-int launch_grouped(const void* rows, const void* W, long long w_rows, const GroupedArgs& p, cudaStream_t stream) {
+int launch_grouped(const void* rows, long long n_rows, const void* W, long long w_rows, const GroupedArgs& p, cudaStream_t stream) {
     CUtensorMap ma, mw;
     int rc;
-    if ((rc = tc_make_map(&ma, rows, (long long)p.max_tiles * XM, p.K, p.K, XM))) return rc;
+    if ((rc = tc_make_map(&ma, rows, n_rows, p.K, p.K, XM))) return rc;
     if ((rc = tc_make_map(&mw, W, w_rows, p.K, p.K, XN / 2))) return rc;
     if (cudaFuncSetAttribute(moe_grouped_kernel<STEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, kXSmem) != cudaSuccess)
         HOS_REFUSE("moe_grouped: cannot get %d bytes of shared memory", kXSmem);
@@ -240,29 +246,33 @@ extern "C" int hos_moe_grouped_set_error_word(int* word) {
     return 0;
 }
 
-// Both products of `max_tiles` listed tiles of 128: rows [max_tiles * 128][D] and y [max_tiles * 128][F] bfloat16 are scratch, pair_out
-// [pairs][D] 32-bit by pair id.  W_up: [experts][2F or F][D], W_down: [experts][D][F].  in_weight or out_weight (by pair, or null).  wait_cycles, stop_tile:
+// Both products of `max_tiles` listed tiles of 128.  rows [n_rows][D] and y [n_rows][F] bfloat16 are scratch: tile t's rows begin at
+// tile_row[t] (null: at 128 t), so n_rows is the number of pairs (or 128 max_tiles).  pair_out [pairs][D] 32-bit by pair id.
+// W_up: [experts][2F or F][D], W_down: [experts][D][F].  in_weight or out_weight (by pair, or null).  wait_cycles, stop_tile:
 // for tests of what happens when a wait runs out (GroupedArgs); 0 and -1 otherwise.
-extern "C" int hos_moe_grouped(const void* h, const void* W_up, const void* W_down, const int* listed, const int* tile_expert, void* rows,
-                               void* y, float* pair_out, int max_tiles, int n_experts, int D, int F, int top, float limit, float alpha,
-                               float up_shift, const float* in_weight, const float* out_weight, int act, long long wait_cycles, int stop_tile,
+extern "C" int hos_moe_grouped(const void* h, const void* W_up, const void* W_down, const int* listed, const int* tile_expert,
+                               const int* tile_row, void* rows, void* y, float* pair_out, int n_rows, int max_tiles, int n_experts,
+                               int D, int F, int top, float limit, float alpha, float up_shift, const float* in_weight, const float* out_weight, int act, long long wait_cycles, int stop_tile,
                                cudaStream_t stream) {
     if (max_tiles <= 0) return 0;
+    if (n_rows <= 0 || (tile_row == nullptr && n_rows < (long long)max_tiles * XM))
+        HOS_REFUSE("moe_grouped: %d rows do not hold %d tiles", n_rows, max_tiles);
     if (D <= 0 || F <= 0 || D % 8 || F % 8 || top <= 0 || n_experts <= 0 ||
         (((uintptr_t)h | (uintptr_t)W_up | (uintptr_t)W_down | (uintptr_t)rows | (uintptr_t)y | (uintptr_t)pair_out) & 15))
         HOS_REFUSE("moe_grouped: rows of %d and %d numbers must be multiples of 8, and the operands 16-byte aligned", D, F);
     const long long wide = D > F ? D : F;
     if (2 * wide * n_experts + XN > (1ll << 31) - 1 || max_tiles * (wide / 128 + 1) > (1ll << 30) || (long long)max_tiles * XM > (1ll << 30))
         HOS_REFUSE("moe_grouped: %d experts and %d tiles are more than one launch takes", n_experts, max_tiles);
-    launch_pdl(moe_gather_kernel, dim3((unsigned)max_tiles * (XM / 8)), dim3(256), 0, stream, (const bf16*)h, listed, tile_expert, (bf16*)rows, D, top);
+    launch_pdl(moe_gather_kernel, dim3((unsigned)max_tiles * (XM / 8)), dim3(256), 0, stream, (const bf16*)h, listed, tile_expert, tile_row, (bf16*)rows,
+               D, top);
     int rc = check_launch("moe_grouped (gather)");
     if (rc) return rc;
     if (wait_cycles <= 0) wait_cycles = kXWaitCycles;
-    GroupedArgs up = {listed, tile_expert, in_weight, y, max_tiles, F, D, limit, alpha, up_shift, wait_cycles, stop_tile};
-    if (act == kGatedSwish) rc = launch_grouped<kGroupedGatedUp>(rows, W_up, 2ll * n_experts * F, up, stream);
-    else if (act == kReluSquare) rc = launch_grouped<kGroupedUp>(rows, W_up, (long long)n_experts * F, up, stream);
+    GroupedArgs up = {listed, tile_expert, tile_row, in_weight, y, max_tiles, F, D, limit, alpha, up_shift, wait_cycles, stop_tile};
+    if (act == kGatedSwish) rc = launch_grouped<kGroupedGatedUp>(rows, n_rows, W_up, 2ll * n_experts * F, up, stream);
+    else if (act == kReluSquare) rc = launch_grouped<kGroupedUp>(rows, n_rows, W_up, (long long)n_experts * F, up, stream);
     else HOS_REFUSE("moe_grouped: unknown activation %d", act);
     if (rc) return rc;
-    GroupedArgs down = {listed, tile_expert, out_weight, pair_out, max_tiles, D, F, 0.f, 0.f, 0.f, wait_cycles, stop_tile};
-    return launch_grouped<kGroupedDown>(y, W_down, (long long)n_experts * D, down, stream);
+    GroupedArgs down = {listed, tile_expert, tile_row, out_weight, pair_out, max_tiles, D, F, 0.f, 0.f, 0.f, wait_cycles, stop_tile};
+    return launch_grouped<kGroupedDown>(y, n_rows, W_down, (long long)n_experts * D, down, stream);
 }

@@ -802,29 +802,34 @@ def moe_route(h, router, correction, token_seq, choice, weight, top: int, scorin
                   -1.0 if renormalise is None else float(renormalise), float(weight_scale), *(groups or (0, 0)), _stream())
 
 
-def moe_align(choice, n_experts: int, listed, tile_expert, tile_rows: Optional[int] = None) -> None:
-    """Every expert's pairs, its list padded to whole tiles of tile_rows (None: moe_tile_rows())."""
+def moe_align(choice, n_experts: int, listed, tile_expert, tile_rows: Optional[int] = None, tile_row=None) -> None:
+    """Every expert's pairs, its list padded to whole tiles of tile_rows (None: moe_tile_rows()); tile_row, if given, becomes the
+    number of pairs that the tiles before each one hold."""
+    if tile_row is not None and tile_row.numel() < tile_expert.numel():
+        raise KernelError("moe_align: sizes disagree")
     experts().call("hos_moe_align", _ptr(choice), choice.numel(), int(n_experts), _ptr(listed), listed.numel(),
-                  _ptr(tile_expert), tile_expert.numel(), int(tile_rows or moe_tile_rows()), _stream())
+                  _ptr(tile_expert), tile_expert.numel(), int(tile_rows or moe_tile_rows()), _ptr(tile_row), _stream())
 
 
 MOE_GROUPED_ROWS = 128      # rows of a tile of the lists that moe_grouped takes
 
 
 def moe_grouped(h, w_up, w_down, listed, tile_expert, rows, y, pair_out, top: int, limit: float, alpha: float, up_shift: float,
-                in_weight: Optional[torch.Tensor], out_weight: Optional[torch.Tensor], act: int, wait_cycles: int = 0,
-                stop_tile: int = -1) -> None:
-    """Both products of the experts over lists padded to MOE_GROUPED_ROWS; rows [places, D] and y [places, F] are scratch.  The
-    other arguments as moe_gate_up's and moe_down's.  bfloat16, D and F multiples of 8.  wait_cycles, stop_tile: for tests of a
-    wait that runs out (the limit of the waits; a CTA's tile at which one does)."""
+                in_weight: Optional[torch.Tensor], out_weight: Optional[torch.Tensor], act: int, tile_row=None,
+                wait_cycles: int = 0, stop_tile: int = -1) -> None:
+    """Both products of the experts over lists padded to MOE_GROUPED_ROWS; rows [., D] and y [., F] are scratch, of as many rows as
+    there are pairs with moe_align's tile_row, and without it of as many as the lists have places.  The other arguments as
+    moe_gate_up's and moe_down's.  bfloat16, D and F multiples of 8.  wait_cycles, stop_tile: for tests of a wait that runs
+    out (the limit of the waits; a CTA's tile at which one does)."""
     for t, what in ((h, "rows"), (w_up, "expert gate/up weights"), (w_down, "expert down weights"), (rows, "gathered rows"), (y, "inner rows")):
         _check(t, what, torch.bfloat16)
     e, d, f = w_down.shape
     if w_up.shape != (e, f * (2 if act == 0 else 1), d) or h.shape[1] != d or rows.shape[1] != d or y.shape[1] != f \
-            or min(rows.shape[0], y.shape[0], listed.numel()) < tile_expert.numel() * MOE_GROUPED_ROWS:
+            or listed.numel() < tile_expert.numel() * MOE_GROUPED_ROWS or rows.shape[0] != y.shape[0] \
+            or rows.shape[0] < (listed.numel() if tile_row is None else pair_out.shape[0]):
         raise KernelError("moe_grouped: sizes disagree")
-    experts().call("hos_moe_grouped", _ptr(h), _ptr(w_up), _ptr(w_down), _ptr(listed), _ptr(tile_expert), _ptr(rows), _ptr(y),
-                  _ptr(pair_out), tile_expert.numel(), e, d, f, int(top), float(limit), float(alpha), float(up_shift),
+    experts().call("hos_moe_grouped", _ptr(h), _ptr(w_up), _ptr(w_down), _ptr(listed), _ptr(tile_expert), _ptr(tile_row),
+                  _ptr(rows), _ptr(y), _ptr(pair_out), rows.shape[0], tile_expert.numel(), e, d, f, int(top), float(limit), float(alpha), float(up_shift),
                   _ptr(in_weight), _ptr(out_weight), int(act), int(wait_cycles), int(stop_tile), _stream())
 
 

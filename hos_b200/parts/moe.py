@@ -27,7 +27,11 @@ from ..registry import part_impl, register_part
 from .base import FeedForward, StepInfo, WeightSpec
 
 
-GROUPED = True          # bfloat16 with more pairs: the tcgen05 products of csrc/moe_grouped.cu; tests switch it off to compare
+# bfloat16 with more pairs: the tcgen05 products of csrc/moe_grouped.cu (tests switch it off to compare).  Measured against the tiles
+# of 64 rows, from 40 to 16,384 pairs: 4 experts of 2,048 x 2,304 1.4 to 5.5 times as fast, 8 of 1,024 x 1,024 1.1 to 3.9, 16 of 2,048 x
+# 512 1.4 to 3.2, 32 of 4,096 x 1,024 1.2 to 3.9, 64 of 2,048 x 512 1.2 to 2.6, 128 of 2,048 x 768 1.2 to 2.6, 256 of 2,048 x 512 1.2 to
+# 1.9, 256 of 7,168 x 2,048 1.5 to 2.2: nowhere slower.
+GROUPED = True
 FEW_PAIRS = 32          # up to this many (row, choice) pairs take the kernels without lists and tiles
 
 
@@ -126,13 +130,14 @@ class RoutedExperts(FeedForward):
                 max_tiles = min(pairs, self.n_experts) + pairs // tile
                 listed = torch.empty(max_tiles * tile, dtype=torch.int32, device=dev)
                 tile_expert = torch.empty(max_tiles, dtype=torch.int32, device=dev)
-                ops.moe_align(choice, self.n_experts, listed, tile_expert, tile)
-                y = torch.empty((max_tiles * tile, self.inner), dtype=h.dtype, device=dev)
+                tile_row = torch.empty(max_tiles, dtype=torch.int32, device=dev) if grouped else None
+                ops.moe_align(choice, self.n_experts, listed, tile_expert, tile, tile_row)
+                y = torch.empty((pairs if grouped else max_tiles * tile, self.inner), dtype=h.dtype, device=dev)
                 weights = (weight, None) if self.weight_on_input else (None, weight)
                 if grouped:
-                    rows = torch.empty((max_tiles * tile, self.width), dtype=h.dtype, device=dev)
+                    rows = torch.empty((pairs, self.width), dtype=h.dtype, device=dev)
                     ops.moe_grouped(h, self.w_gate_up, self.w_down, listed, tile_expert, rows, y, pair_out, top, self.limit,
-                                    self.alpha, self.up_shift, *weights, self.act)
+                                    self.alpha, self.up_shift, *weights, self.act, tile_row)
                 else:
                     ops.moe_gate_up(h, self.w_gate_up, listed, tile_expert, y, top, self.limit, self.alpha, self.up_shift,
                                     weights[0], self.act)

@@ -1357,6 +1357,42 @@ def test_moe_grouped(act, sizes):
             assert err <= 6 * 2.0 ** -8 * (z @ down[e].double().T).square().mean().sqrt().item() + 1e-6, (on_input, e, err)
 
 
+@pytest.mark.parametrize("act,weight_on", [("gated_swish", "output"), ("gated_swish", "input"), ("relu_square", "output")])
+@pytest.mark.parametrize("sizes", [(24, 2, 5, 136, 264), (64, 8, 96, 256, 128), (700, 2, 3, 72, 520)])
+def test_routed_experts_on_both_products(act, weight_on, sizes, monkeypatch):
+    """A layer of routed experts over the grouped products and over the tiles of 64 rows, padding rows among its rows: few and many
+    experts, a few rows to an expert and some hundred.  Both round inner rows of F numbers to bfloat16 (2^-9 of each, the last
+    bit not always the same), so with random signs they differ by a few 2^-9 of the result's root mean square.  The grouped
+    products' memory follows the pairs, not the experts: below what the tiles of 64 take where each expert has a few rows."""
+    from types import SimpleNamespace
+    from hos_b200.config.base import PartSpec
+    from hos_b200.parts import moe
+    from hos_b200.parts.base import Runtime
+    n, top, E, D, F = sizes
+    spec = PartSpec("routed_experts", dict(width=D, inner=F, experts=E, top=top, activation=act, weight_on=weight_on),
+                    {"router": "r", "expert": "{}.", "gate": "g", "up": "u", "down": "d"})
+    layer = moe.RoutedExperts(spec, Runtime(torch.device(DEV, torch.cuda.current_device()), torch.bfloat16))
+    layer.bind({w.name: torch.randn(w.shape, device=DEV).to(torch.float32 if w.name == "r" else torch.bfloat16) / math.sqrt(w.shape[1])
+                for w in layer.weight_specs()})
+    h = torch.randn(n, D, device=DEV).bfloat16()
+    seq = torch.zeros(n, dtype=torch.int32, device=DEV)
+    seq[-2:] = -1
+    step, out, held = SimpleNamespace(token_seq=seq), {}, {}
+    for grouped in (True, False):
+        monkeypatch.setattr(moe, "GROUPED", grouped)
+        layer.forward(h, step)
+        torch.cuda.synchronize()
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        out[grouped] = layer.forward(h, step)
+        torch.cuda.synchronize()
+        held[grouped] = torch.cuda.max_memory_allocated() - before
+    a, b = out[True][:-2].double(), out[False][:-2].double()
+    assert (a - b).abs().max().item() <= 6 * 2.0 ** -9 * b.square().mean().sqrt().item() * math.sqrt(top)
+    if E > 50:
+        assert held[True] < held[False], held
+
+
 @pytest.mark.parametrize("stop_tile", [0, 1])
 def test_moe_grouped_ends_when_a_wait_runs_out(stop_tile):
     """An epilogue warp takes its wait at a CTA's first or second tile as run out: the kernels end, the host hears of it and the
