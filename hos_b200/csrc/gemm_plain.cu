@@ -132,11 +132,13 @@ static int launch_plain(const void* A, const void* W, void* out, int M, int N, i
 // and more with fewer sums, so the four warps split a stage's k instead of the tile: with tiles of 16 rows a thread still
 // holds 8 x 4 sums, with tiles of 32 rows 8 x 8.  Where few rows leave too few tiles for the GPU's SMs, the CTAs of a cluster
 // share one tile by k and add their sums through distributed shared memory, each a slice of the rows, in the order of the
-// ranks.  In what order a sum is added up hangs on N and K alone: a row's results are the same bits whatever rows stand
+// ranks; where there are tiles enough, one CTA walks over the same parts of k and adds their sums in the same order (f32_walks).
+// In what order a sum is added up hangs on N and K alone: a row's results are the same bits whatever rows stand
 // beside it (padding, another batch), so k is always cut for one tile of rows, and there are no tiles of more rows, whose
-// warps would have to share k differently (up to 128 rows by one such tile were 10% faster at 121 rows).
-// Measured (B200): the gated product of 2 x 9,216 rows of W, K 2,304: 48 us at 16 rows (3.6 TB/s of weights), 79 at 30 (the tiles above: 621
-// at 121 rows).  The logits' error against 64 bits of a float32 prompt went from 9e-6 to 4e-6 (sums of several parts, not a long one).
+// warps would have to share k differently.
+// Measured (B200): the gated product of 2 x 9,216 rows of W, K 2,304: 48 us at 16 rows (3.6 TB/s of weights), 79 at 32, 285 at 121, 2,178 at
+// 1,000 (39 TFLOP/s); the tiles above take 510, 509, 621 and 3,476.  The logits' error against 64 bits of a float32 prompt went from 9.1e-6 to
+// 3.7e-6 (sums of several parts, not a long one).
 constexpr int kF32Threads = 128, kF32Cols = 64, kF32Depth = 32;
 
 struct F32Gemm {
@@ -167,23 +169,26 @@ struct F32Tile {
     static constexpr int RM = BM / LR, RN = kF32Cols / LC;         // sums of a thread
     static constexpr int STAGE = (BM + kF32Cols) * kF32Depth;        // numbers of a stage
     static constexpr int STAGES = 6;
+    static constexpr int LD = kF32Cols + 1;                          // a row of the sums' tiles, which take the stages' place ...
     static constexpr int SMEM = STAGES * STAGE * 4;
-    static constexpr int LD = kF32Cols + 1;                          // a row of the sums' tile, which takes the stages' place
+    static constexpr int WALK_SMEM = SMEM + WK * BM * LD * 4;        // ... but for a CTA that goes on after adding them up
     static_assert(WK * BM * LD <= STAGES * STAGE && RM * LR == BM && RM <= 8, "tile");
 };
 
-template <int BM, int EPI>
+template <int BM, int EPI, bool WALK>
 __global__ void __launch_bounds__(kF32Threads, BM <= 16 ? 3 : 2) gemm_f32_kernel(F32Gemm p) {
     using T = F32Tile<BM>;
     constexpr int STAGE = T::STAGE, STAGES = T::STAGES, RM = T::RM, RN = T::RN, LD = T::LD;
     extern __shared__ __align__(128) float smem[];
     const int lane = threadIdx.x & 31, kg = threadIdx.x >> 5;
     const int tx = lane % T::LC, ty = lane / T::LC;                  // columns tx + LC j, rows ty + LR i
-    const int rank = p.splits > 1 ? blockIdx.x % p.splits : 0;       // a cluster is `splits` CTAs along x
-    const int tile = blockIdx.x / p.splits, mt = (p.M + BM - 1) / BM;            // tiles of rows side by side: they share W in L2
-    const int n0 = tile / mt * (EPI == kEpiGated ? kF32Cols / 2 : kF32Cols), m0 = tile % mt * BM;
+    constexpr int COLS = EPI == kEpiGated ? kF32Cols / 2 : kF32Cols;
+    const int rank = !WALK && p.splits > 1 ? blockIdx.x % p.splits : 0;          // a cluster is `splits` CTAs along x
+    const int tile = WALK ? blockIdx.x : blockIdx.x / p.splits, mt = (p.M + BM - 1) / BM;            // tiles of rows side by side: they share W in L2
+    const int n0 = tile / mt * COLS, m0 = tile % mt * BM;
     const int blocks = (p.K + kF32Depth - 1) / kF32Depth;
-    const int first = (int)((long long)blocks * rank / p.splits), last = (int)((long long)blocks * (rank + 1) / p.splits);
+    auto part_begin = [&](int part) { return (int)((long long)blocks * part / p.splits); };
+    const int first = WALK ? 0 : part_begin(rank), last = WALK ? blocks : part_begin(rank + 1);
 
     // This thread's pieces of a stage: 8 pieces a row, so 16 rows a round of the block; piece and row parity are fixed.
     const int piece = threadIdx.x & 7, row0 = threadIdx.x >> 3;
@@ -219,7 +224,16 @@ __global__ void __launch_bounds__(kF32Threads, BM <= 16 ? 3 : 2) gemm_f32_kernel
         if (first + s < last) load(s, first + s);
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
-    int stage = 0;
+    float* sums = WALK ? smem + STAGES * STAGE : smem;               // a tile for each warp along k
+    auto keep_sums = [&] {
+#pragma unroll
+        for (int i = 0; i < RM; ++i)
+#pragma unroll
+            for (int j = 0; j < RN; ++j) sums[(kg * BM + ty + T::LR * i) * LD + tx + T::LC * j] = pair_sum(acc[i][j]);
+    };
+    constexpr int OUTS = WALK ? BM * COLS / kF32Threads : 1;         // results of a thread
+    float v_out[OUTS] = {}, up_out[OUTS] = {};
+    int stage = 0, part = 0;
     for (int block = first; block < last; ++block) {
         asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
         __syncthreads();                                             // this stage is there, and the one before it is read
@@ -247,23 +261,44 @@ __global__ void __launch_bounds__(kF32Threads, BM <= 16 ? 3 : 2) gemm_f32_kernel
             }
         }
         stage = stage == STAGES - 1 ? 0 : stage + 1;
+        if (WALK && block + 1 == part_begin(part + 1)) {             // the end of a part: its sums join the results
+            keep_sums();
+            __syncthreads();                                         // they are read before the next block's barrier
+#pragma unroll
+            for (int o = 0; o < OUTS; ++o) {
+                const int e = threadIdx.x + o * kF32Threads, at = e / COLS * LD + e % COLS;
+#pragma unroll
+                for (int g = 0; g < T::WK; ++g) {
+                    v_out[o] += sums[g * BM * LD + at];
+                    if (EPI == kEpiGated) up_out[o] += sums[g * BM * LD + at + 32];
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < RM; ++i)
+#pragma unroll
+                for (int j = 0; j < RN; ++j) acc[i][j] = 0;
+            ++part;
+        }
+    }
+    if constexpr (WALK) {
+#pragma unroll
+        for (int o = 0; o < OUTS; ++o) {
+            const int e = threadIdx.x + o * kF32Threads, m = m0 + e / COLS, n = n0 + e % COLS;
+            if (m < p.M && n < p.N) p.out[(size_t)m * p.ldo + n] = plain_epilogue<EPI>(v_out[o], up_out[o], p.bias, n, p.cap, p.act);
+        }
+        return;
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
 
-    // The sums to shared memory (a tile for each warp along k), the cluster's added, the rows' slices stored.
-#pragma unroll
-    for (int i = 0; i < RM; ++i)
-#pragma unroll
-        for (int j = 0; j < RN; ++j)
-            smem[(kg * BM + ty + T::LR * i) * LD + tx + T::LC * j] = pair_sum(acc[i][j]);
+    // The sums to shared memory, the cluster's added, the rows' slices stored.
+    keep_sums();
     if (p.splits > 1) {
         asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     } else {
         __syncthreads();
     }
-    constexpr int COLS = EPI == kEpiGated ? kF32Cols / 2 : kF32Cols;
     const int rows = (min(BM, p.M - m0) + p.splits - 1) / p.splits, lo = rank * rows;
     for (int e = threadIdx.x; e < rows * COLS; e += kF32Threads) {
         const int r = lo + e / COLS, c = e % COLS;
@@ -318,14 +353,14 @@ const int* f32_clusters() {
     };
     static const Counts counts = [] {
         Counts c = {};
-        c.ok = cudaFuncSetAttribute(gemm_f32_kernel<BM, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, F32Tile<BM>::SMEM) == cudaSuccess;
+        c.ok = cudaFuncSetAttribute(gemm_f32_kernel<BM, EPI, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, F32Tile<BM>::SMEM) == cudaSuccess;
         int per_sm = 0;
-        c.ok = c.ok && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gemm_f32_kernel<BM, EPI>, kF32Threads, F32Tile<BM>::SMEM) == cudaSuccess;
+        c.ok = c.ok && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gemm_f32_kernel<BM, EPI, false>, kF32Threads, F32Tile<BM>::SMEM) == cudaSuccess;
         c.n[1] = per_sm * sm_count_cached();
         for (int s = 2; s <= kF32MaxSplits && c.ok; ++s) {
             cudaLaunchAttribute attr[1];
             cudaLaunchConfig_t cfg = f32_config<BM, EPI>(1024, s, attr, 0);
-            if (cudaOccupancyMaxActiveClusters(&c.n[s], gemm_f32_kernel<BM, EPI>, &cfg) != cudaSuccess) c.n[s] = 0;
+            if (cudaOccupancyMaxActiveClusters(&c.n[s], gemm_f32_kernel<BM, EPI, false>, &cfg) != cudaSuccess) c.n[s] = 0;
         }
         cudaGetLastError();                                          // a size that does not fit is none to choose, not an error
         c.ok = c.ok && c.n[1] > 0;
@@ -352,6 +387,28 @@ inline int f32_splits(const int* clusters, int tiles, int K) {
     return best;
 }
 
+// Whether one CTA had better walk over a tile's parts of k, one after another, than a cluster share them (the bits are the same).
+// A cluster fills and empties its rings for every part, about 5.5 blocks' worth, but gives few tiles to many SMs; a CTA that walks
+// fills its ring once, and adding up a part costs it about a block.  A lone CTA takes 0.65 of what two on an SM take.
+// Measured, cluster / walk in us, for rows of K 2,304 to 4,096 results: 121 rows 89 / 85, 160 rows 109 / 125, 512 rows 312 / 274, 4,096
+// rows 2,397 / 2,092; K 1,024 to 1,024: 64 rows 14 / 30, 160 rows 29 / 30, 300 rows 48 / 46, 2,048 rows 264 / 149 (the tiles above 244);
+// K 9,216 to 2,304: 300 rows 433 / 467, 512 rows 683 / 604.
+inline bool f32_walks(const int* clusters, long long tiles, int splits, int K) {
+    const int blocks = (K + kF32Depth - 1) / kF32Depth, sms = sm_count_cached();
+    auto per_sm = [&](long long ctas) { return ctas == 0 ? 0.f : fmaxf(1.3f, (float)((ctas + sms - 1) / sms)); };
+    auto rounds = [&](int slots, int ctas) {
+        return (float)(tiles / slots) * per_sm((long long)slots * ctas) + per_sm(tiles % slots * ctas);
+    };
+    return rounds(clusters[1], 1) * (float)(blocks + 4 + splits) < rounds(clusters[splits], splits) * ((float)blocks / splits + 5.5f);
+}
+
+template <int EPI>
+bool f32_walk_ready() {
+    static const bool ok = cudaFuncSetAttribute(gemm_f32_kernel<32, EPI, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                F32Tile<32>::WALK_SMEM) == cudaSuccess;
+    return ok;
+}
+
 template <int BM, int EPI>
 int launch_f32(F32Gemm p, cudaStream_t stream) {
     const int cols = EPI == kEpiGated ? kF32Cols / 2 : kF32Cols;
@@ -359,9 +416,16 @@ int launch_f32(F32Gemm p, cudaStream_t stream) {
     const int* clusters = f32_clusters<32, EPI>();       // the larger tiles' for both heights: the same cut of k
     if (clusters == nullptr || f32_clusters<BM, EPI>() == nullptr) HOS_REFUSE("gemm_f32: the kernel does not fit on this GPU");
     p.splits = f32_splits(clusters, nt, p.K);
+    if constexpr (BM == 32) {
+        if (p.splits > 1 && f32_walks(clusters, (long long)nt * mt, p.splits, p.K)) {
+            if (!f32_walk_ready<EPI>()) HOS_REFUSE("gemm_f32: the kernel does not fit on this GPU");
+            gemm_f32_kernel<32, EPI, true><<<(unsigned)((long long)nt * mt), kF32Threads, F32Tile<32>::WALK_SMEM, stream>>>(p);
+            return check_launch("gemm_f32");
+        }
+    }
     cudaLaunchAttribute attr[1];
     cudaLaunchConfig_t cfg = f32_config<BM, EPI>((long long)nt * mt, p.splits, attr, stream);
-    cudaLaunchKernelEx(&cfg, gemm_f32_kernel<BM, EPI>, p);
+    cudaLaunchKernelEx(&cfg, gemm_f32_kernel<BM, EPI, false>, p);
     return check_launch("gemm_f32");
 }
 

@@ -1212,6 +1212,13 @@ def test_gemm_f32(shape):
             assert torch.equal(few, out[: min(rows, M)]), (kw, rows)
 
 
+@pytest.mark.parametrize("shape", [(1000, 200, 256), (2100, 130, 1028), (4200, 96, 4100), (700, 1024, 1024)])
+def test_gemm_f32_of_many_rows(shape):
+    """As test_gemm_f32, where a tile's parts of k are walked over by one CTA instead of shared by a cluster: a row alone, 16 and
+    33 rows (which are shared) must give the same bits."""
+    test_gemm_f32(shape)
+
+
 @pytest.mark.parametrize("sizes", [(64, 64, 128, 512, 0), (64, 64, 128, 512, 100), (48, 32, 64, 72, 0), (8, 16, 40, 64, 65)])
 @pytest.mark.parametrize("lens", [(64,), (1, 63, 130, 257), (500, 128)])
 def test_latent_prompt(sizes, lens):
