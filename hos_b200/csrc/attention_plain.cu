@@ -8,6 +8,8 @@
 // prompt from position 0: nothing is read from the cache), or the paged cache.
 // Scores: (q.k) * scale, soft-capped, keys t in [max(0, pos + 1 - window), pos]
 // (window <= 0: all keys up to pos), softmax, weighted sum of values.
+#include <type_traits>
+
 #include "common.cuh"
 #include "kv_layout.cuh"
 
@@ -53,16 +55,18 @@ attn_plain_kernel(const T* __restrict__ q, int q_stride, const T* __restrict__ k
     const int slot = PAGED ? seq_slot[seq] : 0;
     const size_t row0 = PAGED ? 0 : (size_t)cu_seqlens[seq];
 
-    // Keys four at a time (two of large heads): their loads, dot products and exponentials do not wait for one another, and the
-    // running sums are scaled once for all of them.  The 121-token prompt of an 8-head layer with 256 numbers a head
-    // takes 47 us so and 114 us with one key at a time, which is one chain of load, warp sum and exponential per key (165 us
-    // where the values are only asked for once the weights are there).
-    constexpr int KEYS = PL <= 8 ? 4 : 2;
-    for (int t = lo; t <= pos; t += KEYS) {
-        float s[KEYS], p[KEYS], v[KEYS][PL];
+    // COUNT keys from t on: their loads, dot products and exponentials do not wait for one another, and the running sums are scaled
+    // once for all of them.  The 121-token prompt of an 8-head layer with 256 numbers a head takes 43 us with four keys at a time,
+    // 47 with two and 96 with one after another (one chain of load, warp sum and exponential per key, and the values asked for
+    // when the weights are there).  Heads of up to 128 numbers are visited two keys at a time: with four, the registers leave an
+    // SM too few warps (16 heads of 128, 121 / 2,048 tokens: two 40 / 3,634 us, four 71 / 5,602, one after another 84 / 4,036).
+    constexpr int KEYS = PL <= 4 ? 2 : 4;
+    auto visit = [&](int t, auto count) {
+        constexpr int COUNT = decltype(count)::value;
+        float s[COUNT], p[COUNT], v[COUNT][PL];
 #pragma unroll
-        for (int u = 0; u < KEYS; ++u) {
-            const int key = min(t + u, pos);       // beyond the last: read again, weight 0
+        for (int u = 0; u < COUNT; ++u) {
+            const int key = t + u;
             const T* kp;
             const T* vp;
             int r = 0;
@@ -92,26 +96,28 @@ attn_plain_kernel(const T* __restrict__ q, int q_stride, const T* __restrict__ k
         }
         float m_new = m;
 #pragma unroll
-        for (int u = 0; u < KEYS; ++u) {
+        for (int u = 0; u < COUNT; ++u) {
             s[u] = softcap_precise(warp_sum(s[u]) * scale, cap);
             m_new = fmaxf(m_new, s[u]);
         }
         const float corr = expf(m - m_new);      // exp(-inf) = 0 on the first keys
         l *= corr;
 #pragma unroll
-        for (int u = 0; u < KEYS; ++u) {
-            p[u] = t + u <= pos ? expf(s[u] - m_new) : 0.f;
+        for (int u = 0; u < COUNT; ++u) {
+            p[u] = expf(s[u] - m_new);
             l += p[u];
         }
 #pragma unroll
         for (int i = 0; i < per_lane; ++i) {
             acc[i] *= corr;
 #pragma unroll
-            for (int u = 0; u < KEYS; ++u)
-                if (t + u <= pos) acc[i] = fmaf(p[u], v[u][i], acc[i]);
+            for (int u = 0; u < COUNT; ++u) acc[i] = fmaf(p[u], v[u][i], acc[i]);
         }
         m = m_new;
-    }
+    };
+    int t = lo;
+    for (; t + KEYS <= pos + 1; t += KEYS) visit(t, std::integral_constant<int, KEYS>{});
+    for (; t <= pos; ++t) visit(t, std::integral_constant<int, 1>{});
     const float inv = l > 0.f ? 1.f / l : 0.f;
 #pragma unroll
     for (int i = 0; i < per_lane; ++i) {

@@ -196,6 +196,27 @@ def _ref_attention(q, k, v, pos, scale, cap, window):
     return out
 
 
+@pytest.mark.parametrize("window", [None, 3, 6])
+@pytest.mark.parametrize("hd", [5, 40, 100, 250, 500, 1000])
+def test_attention_plain_of_few_keys(hd, window):
+    """Every number of keys from one to nine, so every remainder of the keys that are visited together, at every number of
+    numbers to a lane, against 64 bits: sums of up to 1,000 products and of nine values in 32-bit."""
+    from hos_b200 import ops
+    nh, nkv, n, scale = 4, 2, 9, 0.5 / math.sqrt(hd)
+    rows = torch.randn(n, (nh + 2 * nkv) * hd, device=DEV)
+    out = torch.full((n, nh * hd), 7.0, device=DEV)
+    pos, seq = torch.arange(n, dtype=torch.int32, device=DEV), torch.zeros(n, dtype=torch.int32, device=DEV)
+    ops.attn_plain(rows, rows.shape[1], out, pos, seq, n, nh, nkv, hd, scale, 3.0, window, k_rows=rows[:, nh * hd:],
+                   v_rows=rows[:, (nh + nkv) * hd:], kv_stride=rows.shape[1], cu_seqlens=torch.tensor([0, n], dtype=torch.int32, device=DEV))
+    q, k, v = (x.double().view(n, -1, hd) for x in rows.split([nh * hd, nkv * hd, nkv * hd], 1))
+    k, v = (x.repeat_interleave(nh // nkv, 1) for x in (k, v))
+    s = 3.0 * torch.tanh(torch.einsum("ihd,jhd->hij", q, k) * scale / 3.0)
+    d = torch.arange(n, device=DEV)[:, None] - torch.arange(n, device=DEV)[None]
+    s = s.masked_fill((d < 0) | ((d >= window) if window else torch.zeros_like(d, dtype=torch.bool)), -math.inf)
+    want = torch.einsum("hij,jhd->ihd", s.softmax(2), v).flatten(1)
+    assert (out.double() - want).abs().max().item() <= 1e-5
+
+
 @pytest.mark.parametrize("cfg", [dict(nh=4, nkv=2, hd=16, window=8, cap=50.0, slack=40),
                                  dict(nh=6, nkv=1, hd=48, window=37, cap=20.0, slack=100),
                                  dict(nh=3, nkv=1, hd=64, window=None, cap=0.0, slack=0),
