@@ -866,13 +866,16 @@ segment_starts_kernel(const float* __restrict__ state, Segments sg, const int* _
 
 // raw: float32 [N][ld]: q (Gk * dim) | k (Gk * dim) | v (H * vdim) | b (H) | a (H) | ... ; conv_w: [C][taps] over
 // the first C = 2 Gk dim + H vdim columns; conv_state: [slots][taps - 1][C], row j the input taps - 1 - j tokens back.
-// A warp per (row, head): the head's convolutions are independent loads, its length a warp sum, and a single token's row is
-// spread over as many blocks as it has eight heads (a block per row walked its channels in turns, each a chain of loads:
-// 24 rows of 4,096 channels 31.1 -> 5.6 us, and a decode step of 24 sequences 0.79 -> 0.66 ms; 2,048 rows the same time).
+// Two kernels, the same bits.  conv_prep: a warp per (row, head), the head's convolutions independent loads, its length a warp sum; a
+// single token's row is spread over as many blocks as it has eight heads.  A lane holds HELD numbers, so heads of up to 32 HELD.
+// conv_prep_rows: a block per row walks its channels in turns, each a chain of loads, which many rows hide.
+// Measured (B200, warp per head / block per row): 16 heads of 128 on 8 key heads, 4 taps, 24 rows 3.7 / 17.7 us, 2,048 rows 29 / 54; 8 of 256
+// 47 / 88; 4 heads of 32 and 48, 97 rows 3.0 / 4.9, 2,048 rows 11.2 / 11.7.  Other numbers of taps than 2 to 4 are not held: 16 heads of 128, 8
+// taps, 300 rows 18 / 32, 700 rows 34 / 36, 2,048 rows 95 / 86; 4 of 32 and 48, 300 rows 5.9 / 6.8, 512 rows 7.6 / 7.1.
 constexpr int kConvHeads = 8;       // heads, and warps, of a block
-constexpr int kConvHeld = 8;        // numbers of a head that a lane holds between the sum and the division
+constexpr int kConvFewRows = 400;   // the most rows of a warp per head where the taps are not held
 
-template <int TAPS>                 // 0: any number
+template <int TAPS, int HELD>       // TAPS 0: any number
 __global__ void __launch_bounds__(32 * kConvHeads)
 conv_prep_kernel(const float* __restrict__ raw, long long ld, const float* __restrict__ conv_w, int taps,
                  const float* conv_state,      // may be written through keep_here: neither is __restrict__
@@ -912,26 +915,23 @@ conv_prep_kernel(const float* __restrict__ raw, long long ld, const float* __res
     // keep_here: every sequence of the step brings one token, so a lane alone reads and writes its channels' kept inputs:
     // they move on by one here instead of in a launch of their own
     float* keep_w = keep_here != nullptr ? keep_here + (size_t)seq_slot[seq] * (taps - 1) * C : nullptr;
-    auto channel = [&](int d) {
-        return silu_precise(short_conv(raw + first + d, ld, 0.f, conv_w, taps, keep, keep_w, C, first + d, n, r0, fresh));
-    };
-    float y[kConvHeld];
+    float y[HELD];
     if constexpr (TAPS > 0) {
         // all inputs of the lane's channels are read before any kept one is written: no read waits for a write
-        float x[kConvHeld][TAPS];
+        float x[HELD][TAPS];
 #pragma unroll
         for (int j = 0; j < TAPS; ++j) {
             const int src = n - (TAPS - 1) + j;          // the row of this step that holds the input, if it is one
             const float* from = src >= r0 ? raw + (size_t)src * ld + first : keep + (size_t)((TAPS - 1) + (src - r0)) * C + first;
             const bool zero = src < r0 && fresh;
 #pragma unroll
-            for (int i = 0; i < kConvHeld; ++i) {
+            for (int i = 0; i < HELD; ++i) {
                 const int d = lane + 32 * i;
                 x[i][j] = d < size && !zero ? from[d] : 0.f;
             }
         }
 #pragma unroll
-        for (int i = 0; i < kConvHeld; ++i) {
+        for (int i = 0; i < HELD; ++i) {
             const int d = lane + 32 * i;
             float acc = 0.f;
             if (d < size) {
@@ -945,30 +945,79 @@ conv_prep_kernel(const float* __restrict__ raw, long long ld, const float* __res
         }
     } else {
 #pragma unroll
-        for (int i = 0; i < kConvHeld; ++i) {
+        for (int i = 0; i < HELD; ++i) {
             const int d = lane + 32 * i;
-            y[i] = d < size ? channel(d) : 0.f;
+            y[i] = d < size ? silu_precise(short_conv(raw + first + d, ld, 0.f, conv_w, taps, keep, keep_w, C, first + d, n, r0, fresh)) : 0.f;
         }
     }
     float ss = 0.f;
     if (normed) {
 #pragma unroll
-        for (int i = 0; i < kConvHeld; ++i) ss = fmaf(y[i], y[i], ss);
-    }
-    for (int d = lane + 32 * kConvHeld; d < size; d += 32) {         // large heads: the rest waits in the output
-        const float v = channel(d);
-        out[d] = v;
-        ss = fmaf(v, v, ss);
+        for (int i = 0; i < HELD; ++i) ss = fmaf(y[i], y[i], ss);
     }
     float f = 1.f;
     if (normed) f = (1.f / sqrtf(warp_sum(ss) + 1e-6f)) * (hd < Gk ? 1.f / sqrtf((float)dim) : 1.f);
 #pragma unroll
-    for (int i = 0; i < kConvHeld; ++i) {
+    for (int i = 0; i < HELD; ++i) {
         const int d = lane + 32 * i;
         if (d < size) out[d] = y[i] * f;
     }
-    if (normed)
-        for (int d = lane + 32 * kConvHeld; d < size; d += 32) out[d] *= f;
+}
+
+__global__ void __launch_bounds__(256)
+conv_prep_rows_kernel(const float* __restrict__ raw, long long ld, const float* __restrict__ conv_w, int taps,
+                      const float* conv_state,      // may be written through keep_here: neither is __restrict__
+                      const float* __restrict__ a_log, const float* __restrict__ dt_bias,
+                      const int* __restrict__ token_pos, const int* __restrict__ token_seq, const int* __restrict__ cu_seqlens,
+                      const int* __restrict__ seq_slot, float* __restrict__ act, float* __restrict__ beta_out,
+                      float* __restrict__ g_out, int H, int Gk, int dim, int vdim, float* keep_here) {
+    pdl_enter();
+    extern __shared__ float qk[];                // [2 Gk dim] after the activation
+    __shared__ float inv_len[64];
+    const int n = blockIdx.x;
+    const int seq = token_seq[n];
+    const int QK = 2 * Gk * dim, C = QK + H * vdim;
+    float* arow = act + (size_t)n * C;
+    if (seq < 0) {
+        for (int i = threadIdx.x; i < C; i += blockDim.x) arow[i] = 0.f;
+        for (int i = threadIdx.x; i < H; i += blockDim.x) {
+            beta_out[(size_t)n * H + i] = 0.f;
+            g_out[(size_t)n * H + i] = 1.f;
+        }
+        return;
+    }
+    const int r0 = cu_seqlens[seq];
+    const bool fresh = token_pos[r0] == 0;
+    const float* keep = conv_state + (size_t)seq_slot[seq] * (taps - 1) * C;
+    // keep_here: every sequence of the step brings one token, so this block alone reads and writes its slot's kept
+    // inputs (a thread the channels it convolves): they move on by one here instead of in a launch of their own
+    float* keep_w = keep_here != nullptr ? keep_here + (size_t)seq_slot[seq] * (taps - 1) * C : nullptr;
+    for (int ch = threadIdx.x; ch < C; ch += blockDim.x) {
+        const float acc = short_conv(raw + ch, ld, 0.f, conv_w, taps, keep, keep_w, C, ch, n, r0, fresh);
+        const float y = silu_precise(acc);
+        if (ch < QK) qk[ch] = y;
+        else arow[ch] = y;
+    }
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+    for (int hd0 = 0; hd0 < 2 * Gk; hd0 += 64) {         // the heads' lengths, a warp per head
+        for (int hd = hd0 + warp; hd < min(2 * Gk, hd0 + 64); hd += nwarps) {
+            float ss = 0.f;
+            for (int d = lane; d < dim; d += 32) ss = fmaf(qk[hd * dim + d], qk[hd * dim + d], ss);
+            ss = warp_sum(ss);
+            if (lane == 0) inv_len[hd - hd0] = (1.f / sqrtf(ss + 1e-6f)) * (hd < Gk ? 1.f / sqrtf((float)dim) : 1.f);
+        }
+        __syncthreads();
+        for (int i = hd0 * dim + threadIdx.x; i < min(2 * Gk, hd0 + 64) * dim; i += blockDim.x)
+            arow[i] = qk[i] * inv_len[i / dim - hd0];
+        __syncthreads();
+    }
+    for (int h = threadIdx.x; h < H; h += blockDim.x) {
+        const float b = raw[(size_t)n * ld + C + h], a = raw[(size_t)n * ld + C + H + h] + dt_bias[h];
+        beta_out[(size_t)n * H + h] = 1.f / (1.f + expf(-b));
+        const float sp = a > 20.f ? a : log1pf(expf(a));
+        g_out[(size_t)n * H + h] = expf(-expf(a_log[h]) * sp);
+    }
 }
 
 // act(x): 0 none, 1 x logistic(x)
@@ -1272,11 +1321,34 @@ extern "C" int hos_conv_prep(const float* raw, long long ld, const float* conv_w
                              int H, int Gk, int dim, int vdim, int keep_here, cudaStream_t stream) {
     if (N <= 0) return 0;
     if (taps < 1 || taps > kMaxTaps) HOS_REFUSE("conv_prep: %d taps are outside 1..%d", taps, kMaxTaps);
-    if (2ll * Gk * dim > 40960) HOS_REFUSE("conv_prep: %d query and key channels do not fit", 2 * Gk * dim);
+    const size_t smem = (size_t)2 * Gk * dim * sizeof(float);
+    if (smem > 160 * 1024) HOS_REFUSE("conv_prep: %d query and key channels do not fit", 2 * Gk * dim);
+    float* keep = keep_here ? const_cast<float*>(conv_state) : (float*)nullptr;
+    const int largest = dim > vdim ? dim : vdim;
+    const int held = largest <= 32 ? 1 : largest <= 64 ? 2 : largest <= 128 ? 4 : 8;
+    if (largest > 256 || (N > kConvFewRows && (taps < 2 || taps > 4))) {
+        if (smem > 48 * 1024) cudaFuncSetAttribute(conv_prep_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        launch_pdl(conv_prep_rows_kernel, dim3(N), dim3(256), smem, stream, raw, ld, conv_w, taps, conv_state, a_log, dt_bias,
+                   token_pos, token_seq, cu_seqlens, seq_slot, act, beta_out, g_out, H, Gk, dim, vdim, keep);
+        return check_launch("conv_prep");
+    }
     const dim3 grid(N, (2 * Gk + H + kConvHeads - 1) / kConvHeads);
-    launch_pdl(taps == 4 ? conv_prep_kernel<4> : conv_prep_kernel<0>, grid, dim3(32 * kConvHeads), 0, stream, raw, ld, conv_w, taps,
-               conv_state, a_log, dt_bias, token_pos, token_seq, cu_seqlens, seq_slot, act, beta_out, g_out, H, Gk, dim, vdim,
-               keep_here ? const_cast<float*>(conv_state) : (float*)nullptr);
+#define HOS_CONV(T, HD)                                                                                              \
+    launch_pdl(conv_prep_kernel<T, HD>, grid, dim3(32 * kConvHeads), 0, stream, raw, ld, conv_w, taps, conv_state, a_log, dt_bias, token_pos, \
+               token_seq, cu_seqlens, seq_slot, act, beta_out, g_out, H, Gk, dim, vdim, keep)
+#define HOS_CONV_T(T)                                                                                                \
+    do {                                                                                                             \
+        if (held == 1) HOS_CONV(T, 1);                                                                               \
+        else if (held == 2) HOS_CONV(T, 2);                                                                          \
+        else if (held == 4) HOS_CONV(T, 4);                                                                          \
+        else HOS_CONV(T, 8);                                                                                         \
+    } while (0)
+    if (taps == 2) HOS_CONV_T(2);
+    else if (taps == 3) HOS_CONV_T(3);
+    else if (taps == 4) HOS_CONV_T(4);
+    else HOS_CONV_T(0);
+#undef HOS_CONV_T
+#undef HOS_CONV
     return check_launch("conv_prep");
 }
 

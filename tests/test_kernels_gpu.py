@@ -1498,6 +1498,44 @@ def test_long_delta_walk(dim, vdim, many):
     assert (state[slot.long()].double() - S).abs().max().item() <= 2e-5
 
 
+@pytest.mark.parametrize("taps", [1, 2, 3, 4, 7])
+@pytest.mark.parametrize("dim,vdim", [(20, 32), (64, 33), (128, 100), (200, 256), (300, 40)])
+def test_conv_prep_of_few_and_many_rows(dim, vdim, taps):
+    """A warp per head and a block per row (many rows of taps that are not held, larger heads): the first rows of a long sequence have
+    the same bits alone and with the others behind them, at every number of numbers to a lane, and stand where 64 bits put them: a
+    convolution of seven products of numbers of size one, a length and a factor, each rounded to 2^-24 of itself."""
+    from types import SimpleNamespace
+    from hos_b200 import ops
+    H, Gk = 6, 3
+    C = 2 * Gk * dim + H * vdim
+    raw, w = torch.randn(700, C + 2 * H + 3, device=DEV), torch.randn(C, taps, device=DEV) / math.sqrt(taps)
+    a_log, dt_bias, kept = torch.randn(H, device=DEV), torch.randn(H, device=DEV), torch.randn(2, taps - 1, C, device=DEV)
+
+    def run(n, fresh):
+        step = SimpleNamespace(token_pos=torch.arange(n, dtype=torch.int32, device=DEV) + (0 if fresh else 9),
+                               token_seq=torch.zeros(n, dtype=torch.int32, device=DEV),
+                               cu_seqlens=torch.tensor([0, n], dtype=torch.int32, device=DEV), seq_slot=torch.ones(1, dtype=torch.int32, device=DEV))
+        act, beta, g = torch.full((n, C), 7.0, device=DEV), torch.empty(n, H, device=DEV), torch.empty(n, H, device=DEV)
+        ops.conv_prep(raw[:n], w, kept, a_log, dt_bias, step, act, beta, g, H, Gk, dim, vdim)
+        return act, beta, g
+    for fresh in (True, False):
+        many = run(700, fresh)
+        for few in (1, 9, 400):
+            assert all(torch.equal(a, b[:few]) for a, b in zip(run(few, fresh), many)), (fresh, few)
+        x = raw[:, :C].double()
+        x = torch.cat([torch.zeros_like(x[: taps - 1]) if fresh else kept[1].double(), x])
+        y = sum(x[j:j + 700] * w[:, j].double() for j in range(taps))
+        y = y * torch.sigmoid(y)
+        qk = y[:, : 2 * Gk * dim].view(700, 2 * Gk, dim)
+        qk = qk / torch.sqrt((qk * qk).sum(-1, keepdim=True) + 1e-6)
+        qk[:, :Gk] *= dim ** -0.5
+        want = torch.cat([qk.flatten(1), y[:, 2 * Gk * dim:]], 1)
+        assert (many[0].double() - want).abs().max().item() <= 1e-5
+        dt = torch.nn.functional.softplus(raw[:, C + H:C + 2 * H].double() + dt_bias.double())
+        assert (many[2].double() - torch.exp(-torch.exp(a_log.double()) * dt)).abs().max().item() <= 1e-5
+        assert (many[1].double() - torch.sigmoid(raw[:, C:C + H].double())).abs().max().item() <= 1e-5
+
+
 @pytest.mark.parametrize("rule", ["decay", "delta"])
 @pytest.mark.parametrize("dim,vdim,B,H", [(64, 36, 3, 4), (128, 128, 24, 16), (128, 20, 9, 4), (256, 72, 40, 4)])
 def test_state_of_single_tokens(rule, dim, vdim, B, H):
