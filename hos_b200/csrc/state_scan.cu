@@ -1208,9 +1208,10 @@ extern "C" int hos_state_scan(const float* q, const float* k, const float* v, lo
     if (smem > 200 * 1024) HOS_REFUSE("state_scan: heads of %d x %d do not fit a block's shared memory", dim, vdim);
     const bool pieces = aligned && (dim == 64 || dim == 128 || dim == 256) && (uintptr_t)state % 16 == 0 && rot_dims == 0 && k_mult == 1.f;
     if (rule != kChannelRule && !segments && pieces && n_rows <= n_seqs) {
-        // single tokens: as many columns to a thread as leave two blocks to an SM
+        // single tokens: as many columns to a thread as there are and as leave two blocks to an SM
         const int stride = 256 / (dim / 8);
         int nc = 8;
+        while (nc > 1 && stride * (nc / 2) >= vdim) nc /= 2;
         while (nc > 1 && (long long)n_seqs * H * ((vdim + stride * nc - 1) / (stride * nc)) < 2 * sm_count_cached()) nc /= 2;
         const dim3 blocks(n_seqs, H, (vdim + stride * nc - 1) / (stride * nc));
 #define HOS_STEP(Rv, NCv)                                                                                            \

@@ -1576,3 +1576,10 @@ def test_state_of_single_tokens(rule, dim, vdim, B, H):
     tol = dim * 2.0 ** -24 * 10
     assert (out.double() - want)[live].abs().max().item() <= tol
     assert (state[slot.long()].double() - S)[live].abs().max().item() <= tol
+
+
+@pytest.mark.parametrize("rule", ["decay", "delta"])
+@pytest.mark.parametrize("dim,vdim,B,H", [(64, 20, 64, 8), (64, 64, 128, 4), (128, 8, 300, 2), (256, 16, 90, 4)])
+def test_state_of_single_tokens_of_few_columns(rule, dim, vdim, B, H):
+    """As test_state_of_single_tokens, with so many sequences that a thread would hold more columns than there are."""
+    test_state_of_single_tokens(rule, dim, vdim, B, H)
