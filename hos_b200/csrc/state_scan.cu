@@ -35,7 +35,7 @@
 namespace hos {
 
 constexpr int kScanChunk = 8;       // tokens staged at a time
-constexpr int kDeepRing = 6;        // chunks in shared memory of a walk that has its SM to itself
+constexpr int kDeepRing = 6;        // chunks in shared memory of a delta walk that has its SM to itself
 constexpr int kPad = 4;             // floats after every DR staged numbers: 16-byte reads of R neighbours miss each other's banks
 
 __device__ __forceinline__ float silu_precise(float x) { return x / (1.f + expf(-x)); }
@@ -124,6 +124,23 @@ __device__ __forceinline__ uint64_t mul_pair(uint64_t a, uint64_t b) {
     return d;
 }
 
+// Eight tokens' sums over R >= 8 threads side by side, p[t] this thread's part of token t's: with every turn a thread hands on half of
+// the tokens it still has.  The thread r < 8 gets the sum of token token_of_eight(r).
+template <int R>
+__device__ __forceinline__ float sum_of_eight(const float (&p)[kScanChunk], int r) {
+    static_assert(kScanChunk == 8 && R >= 8, "three turns");
+    float four[4], two[2];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) four[i] = ((r & 1) ? p[i + 4] : p[i]) + __shfl_xor_sync(0xffffffffu, (r & 1) ? p[i] : p[i + 4], 1);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) two[i] = ((r & 2) ? four[i + 2] : four[i]) + __shfl_xor_sync(0xffffffffu, (r & 2) ? four[i] : four[i + 2], 2);
+    float acc = ((r & 4) ? two[1] : two[0]) + __shfl_xor_sync(0xffffffffu, (r & 4) ? two[0] : two[1], 4);
+#pragma unroll
+    for (int o = 8; o < R; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    return acc;
+}
+__device__ __forceinline__ int token_of_eight(int r) { return (r & 1) * 4 + (r & 2) + ((r & 4) >> 2); }
+
 enum ScanRule : int { kDecayRule = 0, kDeltaRule = 1, kChannelRule = 2 };
 
 // What a walk by segments needs: seg_len rows to a segment, `count` segments to a sequence at most (blockIdx.x is sequence x
@@ -136,16 +153,18 @@ struct Segments {
 };
 
 // A thread's cells: DR rows of DC neighbouring columns (DC > 1, the walks by segments: what is read of k, q and the decays
-// serves DC columns).
-template <int DR, int R, int DC, int RULE, bool LOCAL>
+// serves DC columns; not with the delta rule).  BUF buffers of staged tokens (2 or, with the delta rule, kDeepRing).  PAIRED: the delta
+// rule on pairs of rows, two in one instruction (the same bits).
+template <int DR, int R, int DC, int RULE, bool LOCAL, int BUF, bool PAIRED>
 __global__ void __launch_bounds__(256)
 state_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v, long long ld,
                   int aligned, int act_in_walk, const float* __restrict__ g, long long g_ld, const float* __restrict__ beta,
                   long long beta_ld, float* __restrict__ state, const int* __restrict__ token_pos,
                   const int* __restrict__ token_seq, const int* __restrict__ cu_seqlens, const int* __restrict__ seq_slot,
                   float* __restrict__ out, int H, int Gk, int dim, int vdim, int CC, const float* __restrict__ rot_freq,
-                  int rot_dims, int rot_style, float k_mult, float o_mult, Segments sg, int n_buf) {
+                  int rot_dims, int rot_style, float k_mult, float o_mult, Segments sg) {
     constexpr bool DELTA = RULE == kDeltaRule, CHANNEL = RULE == kChannelRule;
+    static_assert((!DELTA || DC == 1) && (DELTA || !PAIRED), "the delta rule's walk");
     pdl_enter();
     extern __shared__ __align__(16) float sm[];
     const int seq = blockIdx.x / sg.count, seg = blockIdx.x % sg.count, head = blockIdx.y, col0 = blockIdx.z * CC;
@@ -169,7 +188,7 @@ state_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
     const int n_cols = CC / DC;                  // threads' columns of this block
     auto live = [&](int j) { return c < n_cols && col + j < vdim; };
     const int dpad = R * (DR + kPad);
-    // a ring of n_buf (2 or kDeepRing) buffers of staged tokens: while one chunk is walked the next ones' rows are on their way (cp.async)
+    // a ring of buffers of staged tokens: while one chunk is walked the next ones' rows are on their way (cp.async)
     const int per_buf = kScanChunk * ((CHANNEL ? 3 : 2) * dpad + 2 * CC) + 2 * kScanChunk;      // q, k, (g,) v, o, g, beta
     const bool v_aligned = DC == 4 && (vdim & 3) == 0 && (ld & 3) == 0 && ((uintptr_t)v & 15) == 0;
     const bool v_scaled = RULE == kDecayRule && beta != nullptr;
@@ -199,8 +218,8 @@ state_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
             for (int i = 0; i < DR; ++i) S[j][i] = (!zero && live(j) && r * DR + i < dim) ? from[i] : 0.f;
         }
     }
-    uint64_t P[DC][DR / 2];                      // four columns, and the delta rule: the cells as pairs of rows
-    if (DC == 4 || DELTA) {
+    uint64_t P[DC][DR / 2];                      // four columns, and the paired delta rule: the cells as pairs of rows
+    if (DC == 4 || PAIRED) {
 #pragma unroll
         for (int j = 0; j < DC; ++j)
 #pragma unroll
@@ -208,7 +227,7 @@ state_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
     }
     // rows beyond dim and columns beyond vdim are read by the walk and never staged: they stay zero for good
     if (R * DR != dim || col0 + CC > vdim) {
-        for (int i = threadIdx.x; i < n_buf * per_buf; i += blockDim.x) sm[i] = 0.f;
+        for (int i = threadIdx.x; i < BUF * per_buf; i += blockDim.x) sm[i] = 0.f;
         __syncthreads();
     }
 
@@ -255,21 +274,28 @@ state_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
         }
     };
 
-    for (int b = 0; b < n_buf - 1; ++b) {
-        const int t0 = lo + b * kScanChunk;
-        if (t0 < hi) stage(t0, min(kScanChunk, hi - t0), sm + b * per_buf);
-        cp_async_commit_all();
+    stage(lo, min(kScanChunk, hi - lo), sm);
+    cp_async_commit_all();
+    if constexpr (BUF > 2) {
+#pragma unroll
+        for (int b = 1; b < BUF - 1; ++b) {
+            const int t0 = lo + b * kScanChunk;
+            if (t0 < hi) stage(t0, min(kScanChunk, hi - t0), sm + b * per_buf);
+            cp_async_commit_all();
+        }
     }
     int which = 0;
     float dec[kDecayPerThread] = {1.f, 1.f, 1.f, 1.f};       // first walks: the product of the segment's decays
-    for (int t0 = lo; t0 < hi; t0 += kScanChunk, which = which + 1 == n_buf ? 0 : which + 1) {
+    for (int t0 = lo; t0 < hi; t0 += kScanChunk, which = BUF == 2 ? which ^ 1 : which + 1 == BUF ? 0 : which + 1) {
         const int nt = min(kScanChunk, hi - t0);
-        if (n_buf == 2) cp_async_wait<0>();
-        else cp_async_wait<kDeepRing - 2>();
+        cp_async_wait<BUF - 2>();
         __syncthreads();            // this chunk has landed; everyone is done with the buffer before it
-        const int ahead = t0 + (n_buf - 1) * kScanChunk;
-        if (ahead < hi) stage(ahead, min(kScanChunk, hi - ahead), sm + (which == 0 ? n_buf - 1 : which - 1) * per_buf);
-        cp_async_commit_all();
+        const int ahead = t0 + (BUF - 1) * kScanChunk;
+        if (ahead < hi) {
+            stage(ahead, min(kScanChunk, hi - ahead), sm + (BUF == 2 ? which ^ 1 : which == 0 ? BUF - 1 : which - 1) * per_buf);
+            if (BUF == 2) cp_async_commit_all();
+        }
+        if (BUF > 2) cp_async_commit_all();      // the waits count groups
         float* qs = sm + which * per_buf;
         float* ks = qs + kScanChunk * dpad;
         if (!LOCAL && rot_in_walk) {
@@ -360,13 +386,14 @@ state_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
                 for (int o = R / 8; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
                 if ((r & (R / 4 - 1)) == 0 && c < n_cols) os[t * CC + c * DC + (up ? 2 : 0) + (up2 ? 1 : 0)] = acc * o_mult;
             }
-        } else if constexpr (DELTA) {
+        } else if constexpr (PAIRED) {
             // Every thread walks (a warp's shuffles want all its lanes); only live columns are written.  A chain per token: the
             // dot product over the column's threads, then the update.  Whole chunks have no branch in them, so that the
             // tokens' reads and the products with q run beside the chain.
             auto walk = [&](auto whole_chunk) {
                 constexpr bool FULL = decltype(whole_chunk)::value;
-                float part[DC][kScanChunk];   // the read-outs' partial sums: added up after the walk, off its chain
+                float part[kScanChunk];       // the read-outs' partial sums: added up after the walk, off its chain
+                uint64_t(&C)[DR / 2] = P[0];
 #pragma unroll
                 for (int t = 0; t < kScanChunk; ++t) {
                     if (!FULL && t >= nt) continue;
@@ -374,79 +401,49 @@ state_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
                     const ulonglong2* q4 = (const ulonglong2*)(qs + t * dpad + r * (DR + kPad));
                     const uint64_t gt = pair_of(gs[t], gs[t]);
                     ulonglong2 kk[DR / 4];
-                    float dot[DC];
-                    uint64_t d01[DC], d23[DC];          // four chains a column, not one of DR links
+                    uint64_t d01 = 0, d23 = 0;          // four chains, not one of DR links
 #pragma unroll
                     for (int i = 0; i < DR / 4; ++i) {
                         kk[i] = k4[i];
-#pragma unroll
-                        for (int j = 0; j < DC; ++j) {
-                            P[j][2 * i] = mul_pair(gt, P[j][2 * i]);
-                            P[j][2 * i + 1] = mul_pair(gt, P[j][2 * i + 1]);
-                            d01[j] = fma_pair(P[j][2 * i], kk[i].x, i == 0 ? 0 : d01[j]);
-                            d23[j] = fma_pair(P[j][2 * i + 1], kk[i].y, i == 0 ? 0 : d23[j]);
-                        }
+                        C[2 * i] = mul_pair(gt, C[2 * i]);
+                        C[2 * i + 1] = mul_pair(gt, C[2 * i + 1]);
+                        d01 = fma_pair(C[2 * i], kk[i].x, d01);
+                        d23 = fma_pair(C[2 * i + 1], kk[i].y, d23);
                     }
+                    float d0, d1, d2, d3;
+                    halves_of(d01, d0, d1);
+                    halves_of(d23, d2, d3);
+                    float dot = (d0 + d1) + (d2 + d3);
 #pragma unroll
-                    for (int j = 0; j < DC; ++j) {
-                        float d0, d1, d2, d3;
-                        halves_of(d01[j], d0, d1);
-                        halves_of(d23[j], d2, d3);
-                        dot[j] = (d0 + d1) + (d2 + d3);
+                    for (int o = 1; o < R; o <<= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+                    const float u = bs[t] * ((c < n_cols ? vs[t * CC + c] : 0.f) - dot);
+                    const uint64_t uu = pair_of(u, u);
+                    uint64_t a01 = 0, a23 = 0;
+#pragma unroll
+                    for (int i = 0; i < DR / 4; ++i) {
+                        const ulonglong2 qq = q4[i];
+                        C[2 * i] = fma_pair(kk[i].x, uu, C[2 * i]);
+                        C[2 * i + 1] = fma_pair(kk[i].y, uu, C[2 * i + 1]);
+                        a01 = fma_pair(C[2 * i], qq.x, a01);
+                        a23 = fma_pair(C[2 * i + 1], qq.y, a23);
                     }
-#pragma unroll
-                    for (int o = 1; o < R; o <<= 1)
-#pragma unroll
-                        for (int j = 0; j < DC; ++j) dot[j] += __shfl_xor_sync(0xffffffffu, dot[j], o);
-#pragma unroll
-                    for (int j = 0; j < DC; ++j) {
-                        const float u = bs[t] * ((c < n_cols ? vs[t * CC + c * DC + j] : 0.f) - dot[j]);
-                        const uint64_t uu = pair_of(u, u);
-                        uint64_t a01 = 0, a23 = 0;
-#pragma unroll
-                        for (int i = 0; i < DR / 4; ++i) {
-                            const ulonglong2 qq = q4[i];
-                            P[j][2 * i] = fma_pair(kk[i].x, uu, P[j][2 * i]);
-                            P[j][2 * i + 1] = fma_pair(kk[i].y, uu, P[j][2 * i + 1]);
-                            a01 = fma_pair(P[j][2 * i], qq.x, a01);
-                            a23 = fma_pair(P[j][2 * i + 1], qq.y, a23);
-                        }
-                        float a0, a1, a2, a3;
-                        halves_of(a01, a0, a1);
-                        halves_of(a23, a2, a3);
-                        part[j][t] = (a0 + a1) + (a2 + a3);
-                    }
+                    float a0, a1, a2, a3;
+                    halves_of(a01, a0, a1);
+                    halves_of(a23, a2, a3);
+                    part[t] = (a0 + a1) + (a2 + a3);
                 }
                 if constexpr (FULL && R >= kScanChunk) {
-                    // eight tokens' sums over R threads: with every turn a thread hands on half of the tokens it still has
-                    static_assert(kScanChunk == 8, "three turns");
-#pragma unroll
-                    for (int j = 0; j < DC; ++j) {
-                        const float(&p)[kScanChunk] = part[j];
-                        float four[4], two[2];
-#pragma unroll
-                        for (int i = 0; i < 4; ++i)
-                            four[i] = ((r & 1) ? p[i + 4] : p[i]) + __shfl_xor_sync(0xffffffffu, (r & 1) ? p[i] : p[i + 4], 1);
-#pragma unroll
-                        for (int i = 0; i < 2; ++i)
-                            two[i] = ((r & 2) ? four[i + 2] : four[i]) + __shfl_xor_sync(0xffffffffu, (r & 2) ? four[i] : four[i + 2], 2);
-                        float acc = ((r & 4) ? two[1] : two[0]) + __shfl_xor_sync(0xffffffffu, (r & 4) ? two[0] : two[1], 4);
-#pragma unroll
-                        for (int o = 8; o < R; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-                        const int t = (r & 1) * 4 + (r & 2) + ((r & 4) >> 2);
-                        if (r < 8 && c < n_cols) os[t * CC + c * DC + j] = acc * o_mult;
-                    }
+                    const float acc = sum_of_eight<R>(part, r);
+                    if (r < 8 && c < n_cols) os[token_of_eight(r) * CC + c] = acc * o_mult;
                 } else {
 #pragma unroll
-                    for (int j = 0; j < DC; ++j)
+                    for (int t = 0; t < kScanChunk; ++t) {
+                        if (!FULL && t >= nt) break;
+                        float acc = part[t];
 #pragma unroll
-                        for (int t = 0; t < kScanChunk; ++t) {
-                            if (!FULL && t >= nt) break;
-                            float acc = part[j][t];
-#pragma unroll
-                            for (int o = 1; o < R; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-                            if (r == 0 && c < n_cols) os[t * CC + c * DC + j] = acc * o_mult;
-                        }
+                        for (int o = 1; o < R; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+                        if (r == 0 && c < n_cols) os[t * CC + c] = acc * o_mult;
+                    }
                 }
             };
             if (nt == kScanChunk) walk(std::true_type{});
@@ -464,6 +461,22 @@ state_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
                 float u = c < n_cols ? vs[t * CC + c] : 0.f;
                 if (RULE == kDecayRule && act_in_walk) u = silu_precise(u);      // single tokens: the activation rides here
                 if (v_scaled) u *= bs[t];
+                if (DELTA) {
+                    float d0 = 0.f, d1 = 0.f, d2 = 0.f, d3 = 0.f;       // four chains, not one of DR links
+#pragma unroll
+                    for (int i = 0; i < DR / 4; ++i) {
+                        const float4 kk = k4[i];
+                        S[0][4 * i] *= gt; S[0][4 * i + 1] *= gt; S[0][4 * i + 2] *= gt; S[0][4 * i + 3] *= gt;
+                        d0 = fmaf(S[0][4 * i], kk.x, d0);
+                        d1 = fmaf(S[0][4 * i + 1], kk.y, d1);
+                        d2 = fmaf(S[0][4 * i + 2], kk.z, d2);
+                        d3 = fmaf(S[0][4 * i + 3], kk.w, d3);
+                    }
+                    float dot = (d0 + d1) + (d2 + d3);
+#pragma unroll
+                    for (int o = 1; o < R; o <<= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+                    u = bs[t] * (u - dot);
+                }
                 float a[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
                 for (int i = 0; i < DR / 4; ++i) {
@@ -474,10 +487,17 @@ state_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
                     }
                     const float4 gg = CHANNEL ? g4[i] : make_float4(gt, gt, gt, gt);
                     float* s4 = &S[0][4 * i];
-                    s4[0] = fmaf(gg.x, s4[0], kk.x * u);
-                    s4[1] = fmaf(gg.y, s4[1], kk.y * u);
-                    s4[2] = fmaf(gg.z, s4[2], kk.z * u);
-                    s4[3] = fmaf(gg.w, s4[3], kk.w * u);
+                    if (DELTA) {
+                        s4[0] = fmaf(kk.x, u, s4[0]);
+                        s4[1] = fmaf(kk.y, u, s4[1]);
+                        s4[2] = fmaf(kk.z, u, s4[2]);
+                        s4[3] = fmaf(kk.w, u, s4[3]);
+                    } else {
+                        s4[0] = fmaf(gg.x, s4[0], kk.x * u);
+                        s4[1] = fmaf(gg.y, s4[1], kk.y * u);
+                        s4[2] = fmaf(gg.z, s4[2], kk.z * u);
+                        s4[3] = fmaf(gg.w, s4[3], kk.w * u);
+                    }
                     if (LOCAL) continue;
                     a[0] = fmaf(s4[0], qq.x, a[0]);
                     a[1] = fmaf(s4[1], qq.y, a[1]);
@@ -525,7 +545,7 @@ state_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
     } else if (!last) {
         return;                                  // only the last segment's state is the sequence's
     }
-    if (DC == 4 || DELTA) {
+    if (DC == 4 || PAIRED) {
 #pragma unroll
         for (int j = 0; j < DC; ++j)
 #pragma unroll
@@ -688,22 +708,10 @@ delta_walk_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
                     part[j][t] = (a0 + a1) + (a2 + a3);
                 }
             }
-            // eight tokens' sums over R threads: with every turn a thread hands on half of the tokens it still has
-            static_assert(kScanChunk == 8 && R >= 8, "three turns");
 #pragma unroll
             for (int j = 0; j < DC; ++j) {
-                const float(&p)[kScanChunk] = part[j];
-                float four[4], two[2];
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    four[i] = ((r & 1) ? p[i + 4] : p[i]) + __shfl_xor_sync(0xffffffffu, (r & 1) ? p[i] : p[i + 4], 1);
-#pragma unroll
-                for (int i = 0; i < 2; ++i)
-                    two[i] = ((r & 2) ? four[i + 2] : four[i]) + __shfl_xor_sync(0xffffffffu, (r & 2) ? four[i] : four[i + 2], 2);
-                float acc = ((r & 4) ? two[1] : two[0]) + __shfl_xor_sync(0xffffffffu, (r & 4) ? two[0] : two[1], 4);
-#pragma unroll
-                for (int o = 8; o < R; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-                const int t = (r & 1) * 4 + (r & 2) + ((r & 4) >> 2);
+                const float acc = sum_of_eight<R>(part[j], r);
+                const int t = token_of_eight(r);
                 if (r < 8 && live && (FULL || t < nt)) out[((size_t)(t0 + t) * H + head) * vdim + col + j] = acc * o_mult;
             }
         };
@@ -1197,11 +1205,14 @@ extern "C" int hos_state_scan(const float* q, const float* k, const float* v, lo
     const int aligned = (dim % 4 == 0 && ld % 4 == 0 && (uintptr_t)q % 16 == 0 && (uintptr_t)k % 16 == 0 &&
                          (rule != kChannelRule || (g_ld % 4 == 0 && (uintptr_t)g % 16 == 0))) ? 1 : 0;
     const dim3 grid(n_seqs * sg.count, H, (vdim + CC - 1) / CC);
-    // Few long walks have an SM (almost) to themselves, and nothing but the ring hides the way of their rows from memory: two
-    // chunks of eight tokens are not enough (the delta rule, 16 heads of 128 x 128, 2,048 tokens, before it had a kernel of its own
-    // for such sizes: with a deeper ring and pairs of rows in one instruction 723 -> 504 us).  More walks than that hide one another's loads, and shared memory for more of
-    // them at once is worth more.
-    const bool alone = (long long)grid.x * grid.y * grid.z <= 2ll * sm_count_cached() && long_walk;
+    // The delta rule walks on pairs of rows from a chunk of tokens a sequence on (32 sequences of 300 tokens, 8 heads of 100 x 60: 320 -> 272
+    // us); shorter walks lose by the longer code (8 sequences of two tokens, 4 heads of 512 x 64: 7.5 -> 8.0).
+    // Few long walks of it have an SM (almost) to themselves, and nothing but the ring hides the way of their rows from
+    // memory: two chunks of eight tokens are not enough (pairs and ring, 2,000 tokens, 8 heads of 32 x 64: 537 -> 470 us).  More walks than that hide one another's loads, and shared memory for more
+    // of them at once is worth more.  The other rules' long walks go by segments, and short ones lose by filling a ring (33
+    // tokens, 16 heads of 64: 13.8 us, with a ring of six chunks 15.3).
+    const bool paired = rule == kDeltaRule && n_rows >= (long long)kScanChunk * n_seqs;
+    const bool alone = rule == kDeltaRule && (long long)grid.x * grid.y * grid.z <= 2ll * sm_count_cached() && long_walk;
     const int n_buf = alone && kDeepRing * per_buf <= 100 * 1024 ? kDeepRing : 2;
     const size_t smem = n_buf * per_buf;
     if (rule != kDecayRule && act_in_walk) HOS_REFUSE("state_scan: the activation in the walk is the decay rule's");
@@ -1244,29 +1255,31 @@ extern "C" int hos_state_scan(const float* q, const float* k, const float* v, lo
         HOS_DELTA(32);
 #undef HOS_DELTA
     }
-#define HOS_SCAN(DRv, Rv, DCv, DL, LOC)                                                                                   \
+#define HOS_SCAN(DRv, Rv, DCv, DL, LOC, BUF, PR)                                                                     \
     do {                                                                                                             \
         if (smem > 48 * 1024)                                                                                        \
-            cudaFuncSetAttribute(state_scan_kernel<DRv, Rv, DCv, DL, LOC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-        launch_pdl(state_scan_kernel<DRv, Rv, DCv, DL, LOC>, grid, dim3(threads), smem, stream, q, k, v, ld, aligned, act_in_walk, g, g_ld, beta, \
-                   beta_ld, state, token_pos, token_seq, cu_seqlens, seq_slot, out, H, Gk, dim, vdim, CC, rot_freq,  \
-                   rot_dims, rot_style, k_mult, o_mult, sg, n_buf);                                                         \
+            cudaFuncSetAttribute(state_scan_kernel<DRv, Rv, DCv, DL, LOC, BUF, PR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+        launch_pdl(state_scan_kernel<DRv, Rv, DCv, DL, LOC, BUF, PR>, grid, dim3(threads), smem, stream, q, k, v, ld, aligned, act_in_walk, g, g_ld, \
+                   beta, beta_ld, state, token_pos, token_seq, cu_seqlens, seq_slot, out, H, Gk, dim, vdim, CC, rot_freq, \
+                   rot_dims, rot_style, k_mult, o_mult, sg);                                                         \
     } while (0)
 #define HOS_SCAN_S(DRv, Rv, DL)                                                                                      \
     do {                                                                                                             \
         constexpr int DCs = DRv == 8 ? 4 : 1;                                                                        \
         if (segments) {                                                                                              \
-            HOS_SCAN(DRv, Rv, DCs, DL, true);                                                                           \
+            HOS_SCAN(DRv, Rv, DCs, DL, true, 2, false);                                                              \
             launch_pdl(segment_starts_kernel, dim3((unsigned)(((long long)H * vdim * dim + 255) / 256), n_seqs), dim3(256), 0, stream, \
                        (const float*)state, sg, token_pos, token_seq, cu_seqlens, seq_slot, H, dim, vdim, DL == kChannelRule ? 1 : 0); \
-            HOS_SCAN(DRv, Rv, DCs, DL, false);                                                                       \
+            HOS_SCAN(DRv, Rv, DCs, DL, false, 2, false);                                                             \
         } else {                                                                                                     \
-            HOS_SCAN(DRv, Rv, 1, DL, false);                                                                         \
+            HOS_SCAN(DRv, Rv, 1, DL, false, 2, false);                                                               \
         }                                                                                                            \
     } while (0)
 #define HOS_SCAN_D(DRv, Rv)                                                                                          \
     do {                                                                                                             \
-        if (rule == kDeltaRule) HOS_SCAN(DRv, Rv, 1, kDeltaRule, false);                                              \
+        if (rule == kDeltaRule && !paired) HOS_SCAN(DRv, Rv, 1, kDeltaRule, false, 2, false);                        \
+        else if (rule == kDeltaRule && n_buf == 2) HOS_SCAN(DRv, Rv, 1, kDeltaRule, false, 2, true);                 \
+        else if (rule == kDeltaRule) HOS_SCAN(DRv, Rv, 1, kDeltaRule, false, kDeepRing, true);                       \
         else if (rule == kChannelRule) HOS_SCAN_S(DRv, Rv, kChannelRule);                                            \
         else HOS_SCAN_S(DRv, Rv, kDecayRule);                                                                        \
     } while (0)
