@@ -1208,7 +1208,7 @@ def test_product_on_pairs_of_sms_with_k_split(shape):
 @pytest.mark.parametrize("shape", [(1, 64, 32), (2, 1, 4), (16, 65, 132), (17, 2304, 512), (33, 130, 36), (49, 31, 1028), (95, 200, 260),
                                    (97, 33, 2052), (128, 64, 4096), (129, 100, 68), (300, 96, 128)])
 def test_gemm_f32(shape):
-    """The 32-bit product with rows of whole 16-byte pieces: every tile height, remainders of rows, columns and k, tiles
+    """The 32-bit product with rows of whole 16-byte pieces: both tile heights, remainders of rows, columns and k, tiles
     shared by a cluster.  A sum of K products of numbers of size 1 and K^-1/2, each rounded to 2^-24 of it, is off by less than
     2^-24 K of sum |a w| <= 2^-24 K x (some) K^1/2; 3e-6 x sqrt(K) is far above what random signs leave of it."""
     from hos_b200 import ops
