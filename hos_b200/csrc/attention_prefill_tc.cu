@@ -149,6 +149,12 @@ struct PrefillTcArgs {
     const int* seq_slot;
     const int* page_table;
     int table_stride, ring_pages;
+    // the pair kernel's walks in shares (gridDim.z of them at most, each of share_tiles tiles or so; 0: every walk whole): what a
+    // share leaves, [block of queries][head][share] times [THD / 4][128 rows] four sums, not divided, and [128 rows] (maximum in
+    // units of log2, sum of weights)
+    int share_tiles;
+    float4* part_o;
+    float2* part_ml;
     long long wait_cycles;      // the limit of every wait
     int stop_tile;              // for tests of the give-up path: the tile at which a softmax warp takes its wait as run out (-1: none)
 };
@@ -493,10 +499,42 @@ __device__ __forceinline__ bool mbar_wait_cluster_cycles(uint64_t* bar, uint32_t
     return true;
 }
 
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
-attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q,      // boxes of [128 rows x 64 columns]
-                         const __grid_constant__ CUtensorMap map_k,      // boxes of [64 rows x 64 columns]
-                         PrefillTcArgs a) {
+// Which sequence and which block of 128 queries a block of the grid is (long walks first), and the tiles of PK keys it walks over.
+struct PairWalk {
+    int seq, row0, len, q0, p0;         // the sequence, its first row and its rows, the block's first row among them and its position
+    int last_q, lo, tiles, shares;      // the last query's position; the first tile, their number, the shares they are cut into
+};
+template <bool PAGED>
+__device__ __forceinline__ bool pair_walk(const PrefillTcArgs& a, int tile, int most_shares, PairWalk& w) {
+    int nt = 0;
+    for (w.seq = 0; w.seq < a.n_seqs; ++w.seq) {
+        w.row0 = a.cu_seqlens[w.seq] - (PAGED ? a.row_base : 0);
+        w.len = a.cu_seqlens[w.seq + 1] - (PAGED ? a.row_base : 0) - w.row0;
+        nt = (w.len + TQ - 1) / TQ;
+        if (tile < nt) break;
+        tile -= nt;
+    }
+    if (w.seq >= a.n_seqs) return false;
+    w.q0 = (nt - 1 - tile) * TQ;
+    w.p0 = w.q0 + (PAGED ? a.token_pos[w.row0] : 0);
+    w.last_q = w.p0 + min(w.len - 1 - w.q0, TQ - 1);
+    const int first_key = a.window > 0 ? max(0, w.p0 + 1 - a.window) : 0;
+    w.lo = first_key / PK;
+    w.tiles = w.last_q / PK - w.lo + 1;
+    w.shares = most_shares > 1 ? min(most_shares, (w.tiles + a.share_tiles - 1) / a.share_tiles) : 1;
+    return true;
+}
+
+// PAGED, as in the one-CTA kernel: the queries are the step's rows at the positions it gives them, and map_k and map_v cover the
+// cache's pages (a tile is two of them); without PAGED the values come through map_q and map_v is not used.  A paged walk may be cut
+// into shares, one to a pair (gridDim.z; attn_prefill_merge_kernel adds them up): a piece of 739 tokens has six blocks of
+// queries, which with four pairs of heads are 24 pairs of SMs for 74.
+// Measured (B200, 8 heads of 256, 739 tokens on top of 2,901, us): one CTA a block 84, pairs 72, pairs in 2 / 3 / 4 shares 52 / 42 / 58 (4: more
+// than run at once).  Prompts from position 0 are not cut: 2,048 tokens 44 whole, 51 in two shares of up to ten tiles, 4,096 79 and 109.
+template <bool PAGED>
+__device__ __forceinline__ void pair_attention(const CUtensorMap& map_q,      // boxes of [128 rows x 64 columns]
+                                               const CUtensorMap& map_k,      // boxes of [64 rows x 64 columns]
+                                               const CUtensorMap& map_v, const PrefillTcArgs& a) {
     pdl_launch_dependents();      // as in the one-CTA kernel: set-up first, the producers wait before their first copy
     extern __shared__ unsigned char smem_unaligned[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~(uintptr_t)1023);
@@ -515,31 +553,29 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q,      // boxe
     uint64_t* v_full = bars + 13;
     uint64_t* v_empty = bars + 15;
     uint32_t* tmem_base_smem = reinterpret_cast<uint32_t*>(bars + 17);
+    int* out_rows = reinterpret_cast<int*>(bars + 18);           // the block's first row and its rows: the epilogue's, no registers' until then
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();
     const bool leader = rank == 0;
 
-    // which sequence and which block of 128 queries: the same for both CTAs of a pair (they differ in the head)
-    int seq = 0, tile = blockIdx.y, row0 = 0, len = 0, nt = 0;
-    for (; seq < a.n_seqs; ++seq) {
-        row0 = a.cu_seqlens[seq];
-        len = a.cu_seqlens[seq + 1] - row0;
-        nt = (len + TQ - 1) / TQ;
-        if (tile < nt) break;
-        tile -= nt;
-    }
-    if (seq >= a.n_seqs) return;                                 // both CTAs of the pair alike
-    const int q0 = (nt - 1 - tile) * TQ;
+    // the same block of queries and share for both CTAs of a pair (they differ in the head)
+    PairWalk w;
+    if (!pair_walk<PAGED>(a, blockIdx.y, PAGED ? gridDim.z : 1, w)) return;
+    const int share = PAGED ? blockIdx.z : 0;
+    if (share >= w.shares) return;
+    const int p0 = w.p0;
     const int head = blockIdx.x, kvh = head / (a.n_heads / a.n_kv_heads);
-    const int last_q = min(len - 1, q0 + TQ - 1);
-    const int first_key = a.window > 0 ? max(0, q0 + 1 - a.window) : 0;
-    const int kt_lo = first_key / PK, kt_hi = last_q / PK;
-    const int n_tiles = kt_hi - kt_lo + 1;
+    const int even = w.shares == 1 ? w.tiles : w.tiles / w.shares, more = w.tiles - even * w.shares;    // the first `more` take one more
+    const int kt_lo = w.lo + even * share + min(share, more);
+    const int n_tiles = even + (share < more ? 1 : 0);
 
     if (threadIdx.x == 0) {
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_q)) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_k)) : "memory");
+        if (PAGED) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_v)) : "memory");
+        out_rows[0] = w.row0 + w.q0;
+        out_rows[1] = w.len - w.q0;
         mbar_init(q_full, 1);
         for (int s = 0; s < 2; ++s) {
             mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1);
@@ -569,22 +605,40 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q,      // boxe
             pdl_wait();       // the projection's rows are complete from here on
             if (leader) mbar_expect_tx(q_full, 2 * kQBytesTc);
             for (int c = 0; c < CBLK; ++c)
-                tma_load_2d_pair(q_s + c * kQBlockBytes, &map_q, a.q_col0 + head * THD + 64 * c, row0 + q0, q_full);
+                tma_load_2d_pair(q_s + c * kQBlockBytes, &map_q, a.q_col0 + head * THD + 64 * c, w.row0 + w.q0, q_full);
+            // paged: a tile is two pages, the second one clamped to the last that holds a key of these queries (its keys are
+            // masked where it stands for a later one); looked up one tile ahead of their use
+            PagedKV geo{nullptr, nullptr, a.page_table, a.table_stride, a.ring_pages, a.n_kv_heads, THD};
+            const int* table = PAGED ? a.page_table + (size_t)a.seq_slot[w.seq] * a.table_stride : nullptr;
+            auto page_row = [&](int lp) {
+                return (table[kv_table_entry(geo, min(lp, w.last_q / kPageTokens))] * a.n_kv_heads + kvh) * kPageTokens;
+            };
+            int next0 = PAGED ? page_row(2 * kt_lo) : 0, next1 = PAGED ? page_row(2 * kt_lo + 1) : 0;
             for (int j = 0; j < n_tiles && ok; ++j) {
                 const int s = j % kPairStages;
                 unsigned char* kd = kv_s + (size_t)s * kPairStageBytes;
                 unsigned char* vd = kd + kPairKBytes;
-                const int krow = row0 + (kt_lo + j) * PK;
+                // the rows of the tile's two halves in their tensor maps, and the first column of its keys and values
+                const int row_a = PAGED ? next0 : w.row0 + (kt_lo + j) * PK, row_b = PAGED ? next1 : row_a + 64;
+                const int kcol = PAGED ? 0 : a.k_col0 + kvh * THD, vcol = (PAGED ? 0 : a.v_col0 + kvh * THD) + (THD / 2) * (int)rank;
+                if (PAGED && j + 1 < n_tiles) {
+                    next0 = page_row(2 * (kt_lo + j + 1));
+                    next1 = page_row(2 * (kt_lo + j + 1) + 1);
+                }
                 if (j >= kPairStages && !tc_wait(&k_empty[s], ((j / kPairStages) - 1) & 1)) { ok = false; break; }
                 if (leader) mbar_expect_tx(&k_full[s], 2 * kPairKBytes);
                 for (int c = 0; c < CBLK; ++c)          // keys 64 rank .. 64 rank + 63 of the tile, all dimensions
-                    tma_load_2d_pair(kd + c * kPairKBlockBytes, &map_k, a.k_col0 + kvh * THD + 64 * c, krow + 64 * (int)rank,
-                                     &k_full[s]);
+                    tma_load_2d_pair(kd + c * kPairKBlockBytes, &map_k, kcol + 64 * c, rank == 0 ? row_a : row_b, &k_full[s]);
                 if (j >= kPairStages && !tc_wait(&v_empty[s], ((j / kPairStages) - 1) & 1)) { ok = false; break; }
                 if (leader) mbar_expect_tx(&v_full[s], 2 * kPairVBytes);
-                for (int c = 0; c < CBLK / 2; ++c)      // all 128 keys, this CTA's half of the dimensions
-                    tma_load_2d_pair(vd + c * kPairVBlockBytes, &map_q, a.v_col0 + kvh * THD + (THD / 2) * (int)rank + 64 * c, krow,
-                                     &v_full[s]);
+                for (int c = 0; c < CBLK / 2; ++c) {    // all 128 keys, this CTA's half of the dimensions
+                    if (PAGED) {
+                        tma_load_2d_pair(vd + c * kPairVBlockBytes, &map_v, vcol + 64 * c, row_a, &v_full[s]);
+                        tma_load_2d_pair(vd + c * kPairVBlockBytes + 64 * 128, &map_v, vcol + 64 * c, row_b, &v_full[s]);
+                    } else {
+                        tma_load_2d_pair(vd + c * kPairVBlockBytes, &map_q, vcol + 64 * c, row_a, &v_full[s]);
+                    }
+                }
             }
             if (!ok) record_give_up();
         }
@@ -639,7 +693,7 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q,      // boxe
         const int half = (warp - 2) >> 2;                        // which 64 of the tile's 128 keys
         const int r = quarter * 32 + lane;                       // row of the tile = TMEM lane
         const uint32_t t_lane = tmem_base + ((uint32_t)(quarter * 32) << 16);
-        const int qpos = q0 + r;
+        const int qpos = p0 + r;
         const bool capped = a.cap > 0.f;
         const float pre = capped ? a.scale / a.cap : 1.f;
         const float c_logit = capped ? a.cap : a.scale;          // logit = c_logit * t
@@ -667,7 +721,7 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q,      // boxe
                 __syncwarp();
                 if (lane == 0) mbar_arrive_leader(&s_empty[sb]);     // this warp has its part of the S buffer
                 if (capped) tanh_scores<64>(sc, pre);
-                const bool whole = kt0 + PK - 1 <= q0 && (a.window <= 0 || kt0 > q0 + TQ - 1 - a.window);
+                const bool whole = kt0 + PK - 1 <= p0 && (a.window <= 0 || kt0 > p0 + TQ - 1 - a.window);
                 if (whole) {
 #pragma unroll
                     for (int i = 0; i < 64; ++i) m_half = fmaxf(m_half, sc[i]);
@@ -748,14 +802,23 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q,      // boxe
         asm volatile("bar.sync 1, 256;" ::: "memory");
         if (ok) {
             const float l_row = l_run + xchg[(half ^ 1) * TQ + r];
+            const bool whole_walk = w.shares == 1, mine = r < out_rows[1];
+            const size_t row = (size_t)(out_rows[0] + r), part = ((size_t)blockIdx.y * a.n_heads + head) * gridDim.z + share;
             const float inv = l_row > 0.f ? 1.f / l_row : 0.f;
-            bf16* orow = a.out + (size_t)(row0 + qpos) * a.out_stride + (size_t)head * THD;
+            bf16* orow = a.out + row * a.out_stride + (size_t)head * THD;
+            float4* po = a.part_o + part * (THD / 4) * TQ + r;
+            if (!whole_walk && half == 0) a.part_ml[part * TQ + r] = make_float2(m_ref * c2, l_row);
 #pragma unroll 1
             for (int c = half * (THD / 2); c < (half + 1) * (THD / 2); c += 32) {
                 uint32_t o[32];
                 tc_ld32(t_lane + kPairColO + c, o);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (qpos < len) {
+                if (!whole_walk) {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        po[(c / 4 + i) * TQ] = make_float4(__uint_as_float(o[4 * i]), __uint_as_float(o[4 * i + 1]),
+                                                           __uint_as_float(o[4 * i + 2]), __uint_as_float(o[4 * i + 3]));
+                } else if (mine) {
                     uint4* dst = reinterpret_cast<uint4*>(orow + c);
 #pragma unroll
                     for (int q4 = 0; q4 < 4; ++q4)
@@ -775,6 +838,53 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q,      // boxe
     cluster_sync_all();
     if (warp == 1) tmem_dealloc_pair(tmem_base, kPairTmemCols);
 }
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
+attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+                         const __grid_constant__ PrefillTcArgs a) {
+    pair_attention<false>(map_q, map_k, map_k, a);
+}
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
+attn_chunk_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+                       const __grid_constant__ CUtensorMap map_v, const __grid_constant__ PrefillTcArgs a) {
+    pair_attention<true>(map_q, map_k, map_v, a);
+}
+
+// The shares of a block of queries and a head, in the order of their keys: O = sum of 2^(m_s - M) O_s over sum of 2^(m_s - M) l_s.
+// A thread per row, 32 numbers of it; blocks whose walk was whole have been written.
+__global__ void __launch_bounds__(TQ) attn_prefill_merge_kernel(PrefillTcArgs a, int shares) {
+    pdl_enter();
+    PairWalk w;
+    if (!pair_walk<true>(a, blockIdx.y, shares, w) || w.shares == 1) return;
+    const int head = blockIdx.x, c0 = blockIdx.z * 32, r = threadIdx.x;
+    if (w.q0 + r >= w.len) return;
+    const size_t first = ((size_t)blockIdx.y * a.n_heads + head) * shares;
+    float top = -INFINITY, l = 0.f;
+    for (int s = 0; s < w.shares; ++s) top = fmaxf(top, a.part_ml[(first + s) * TQ + r].x);
+    float sum[32] = {};
+    for (int s = 0; s < w.shares; ++s) {
+        const float2 ml = a.part_ml[(first + s) * TQ + r];
+        if (ml.x == -INFINITY) continue;             // no key of this share is seen
+        const float f = exp2f(ml.x - top);
+        const float4* po = a.part_o + ((first + s) * (THD / 4) + c0 / 4) * TQ + r;
+        l = fmaf(f, ml.y, l);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float4 o = po[i * TQ];
+            sum[4 * i] = fmaf(f, o.x, sum[4 * i]);
+            sum[4 * i + 1] = fmaf(f, o.y, sum[4 * i + 1]);
+            sum[4 * i + 2] = fmaf(f, o.z, sum[4 * i + 2]);
+            sum[4 * i + 3] = fmaf(f, o.w, sum[4 * i + 3]);
+        }
+    }
+    const float inv = l > 0.f ? 1.f / l : 0.f;
+    uint4* dst = reinterpret_cast<uint4*>(a.out + (size_t)(w.row0 + w.q0 + r) * a.out_stride + (size_t)head * THD + c0);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        dst[i] = make_uint4(pack_bf16(sum[8 * i] * inv, sum[8 * i + 1] * inv), pack_bf16(sum[8 * i + 2] * inv, sum[8 * i + 3] * inv),
+                            pack_bf16(sum[8 * i + 4] * inv, sum[8 * i + 5] * inv), pack_bf16(sum[8 * i + 6] * inv, sum[8 * i + 7] * inv));
+}
+
 #endif   // head sizes with the pair kernel
 
 #endif   // head sizes with the kernel
@@ -792,6 +902,30 @@ static int& pair_state() {
 extern "C" int hos_attn_prefill_pair(int on) {
     pair_state() = on ? 1 : 0;
     return 0;
+}
+
+// How many pairs of SMs the prompts and long pieces of these heads run on at once; 0: they do not run on pairs.
+extern "C" int hos_attn_prefill_pairs(int n_heads, int n_kv_heads) {
+#if (HOS_HEAD_DIM == 128) || (HOS_HEAD_DIM == 256)
+    if (pair_state() == 0 || n_kv_heads <= 0 || n_heads % (2 * n_kv_heads) != 0) return 0;
+    static int at_once = 0;
+    if (at_once == 0) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(n_heads, 64, 1);
+        cfg.blockDim = dim3(kTcThreads);
+        cfg.dynamicSmemBytes = kPairSmem;
+        int n = 0;
+        if (cudaFuncSetAttribute(attn_chunk_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, attn_chunk_pair_kernel, &cfg) != cudaSuccess || n <= 0) {
+            cudaGetLastError();
+            n = sm_count_cached() / 2;
+        }
+        at_once = n;
+    }
+    return at_once;
+#else
+    return 0;
+#endif
 }
 
 // 1 if this library has the tensor-core prompt kernel (head sizes 64, 128, 256).
@@ -877,12 +1011,15 @@ extern "C" int hos_attn_prefill_tc(const void* rows, long long n_rows, int row_s
 // cores.  q: the step's projection rows of these sequences [n_rows, row_stride] (the q heads stand first in a row);
 // sequence s has the rows cu_seqlens[s] - row_base .. of q and out, at the consecutive positions token_pos[row], and
 // the page-table row seq_slot[s]; n_q_tiles is at least the sum over sequences of ceil(rows / 128).  The pages are
-// [n_pages][n_kv_heads][64][head_dim] arrays in the cache's permuted layout.
+// [n_pages][n_kv_heads][64][head_dim] arrays in the cache's permuted layout.  shares > 1: a block's walk over its keys may be cut into
+// up to that many, each of share_tiles tiles of 128 keys or so, where the heads run on pairs of SMs (hos_attn_prefill_pairs); part_o and
+// part_ml: n_q_tiles * n_heads * shares * 128 times head_dim and times two floats, 16-byte aligned.
 extern "C" int hos_attn_chunk_tc(const void* q, long long n_rows, int row_stride, void* out, int out_stride,
                                  const int* cu_seqlens, int row_base, const int* token_pos, const int* seq_slot,
                                  int n_seqs, int n_q_tiles, void* k_pages, void* v_pages, long long n_pages,
                                  const int* page_table, int table_stride, int ring_pages, int n_heads, int n_kv_heads,
-                                 int head_dim, float scale, float cap, int window, cudaStream_t stream) {
+                                 int head_dim, float scale, float cap, int window, int shares, int share_tiles, float* part_o,
+                                 float* part_ml, cudaStream_t stream) {
 #if (HOS_HEAD_DIM == 64) || (HOS_HEAD_DIM == 128) || (HOS_HEAD_DIM == 256)
     if (n_q_tiles <= 0 || n_seqs <= 0) return 0;
     if (head_dim != THD) HOS_REFUSE("attn_chunk_tc: built for head_dim %d, asked for %d", THD, head_dim);
@@ -899,12 +1036,6 @@ extern "C" int hos_attn_chunk_tc(const void* q, long long n_rows, int row_stride
     const long long page_rows = n_pages * n_kv_heads * kPageTokens;
     if ((rc = tc_make_map(&mk, k_pages, page_rows, THD, THD, TK, false))) return rc;
     if ((rc = tc_make_map(&mv, v_pages, page_rows, THD, THD, TK, false))) return rc;
-    static bool attr_set = false;
-    if (!attr_set) {
-        if (cudaFuncSetAttribute(attn_prefill_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem) != cudaSuccess)
-            HOS_REFUSE("attn_chunk_tc: cannot get %d bytes of shared memory", kTcSmem);
-        attr_set = true;
-    }
     PrefillTcArgs a = {};
     a.out = (bf16*)out; a.out_stride = out_stride; a.cu_seqlens = cu_seqlens; a.n_seqs = n_seqs;
     a.n_heads = n_heads; a.n_kv_heads = n_kv_heads;
@@ -913,6 +1044,29 @@ extern "C" int hos_attn_chunk_tc(const void* q, long long n_rows, int row_stride
     a.row_base = row_base; a.token_pos = token_pos; a.seq_slot = seq_slot;
     a.page_table = page_table; a.table_stride = table_stride; a.ring_pages = ring_pages;
     a.wait_cycles = kTcWaitCycles; a.stop_tile = -1;
+#if (HOS_HEAD_DIM == 128) || (HOS_HEAD_DIM == 256)
+    if (pair_state() != 0 && (n_heads / n_kv_heads) % 2 == 0) {
+        if (shares > 1 && (part_o == nullptr || part_ml == nullptr || share_tiles <= 0 || shares > 65535))
+            HOS_REFUSE("attn_chunk_tc: %d shares need their length and a workspace", shares);
+        if (shares > 1) { a.share_tiles = share_tiles; a.part_o = (float4*)part_o; a.part_ml = (float2*)part_ml; }
+        else shares = 1;
+        static bool pair_attr_set = false;
+        if (!pair_attr_set) {
+            if (cudaFuncSetAttribute(attn_chunk_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem) != cudaSuccess)
+                HOS_REFUSE("attn_chunk_tc: cannot get %d bytes of shared memory", kPairSmem);
+            pair_attr_set = true;
+        }
+        launch_pdl(attn_chunk_pair_kernel, dim3(n_heads, n_q_tiles, shares), dim3(kTcThreads), kPairSmem, stream, mq, mk, mv, a);
+        if (shares > 1) launch_pdl(attn_prefill_merge_kernel, dim3(n_heads, n_q_tiles, THD / 32), dim3(TQ), 0, stream, a, shares);
+        return check_launch("attn_chunk_tc (pairs of SMs)");
+    }
+#endif
+    static bool attr_set = false;
+    if (!attr_set) {
+        if (cudaFuncSetAttribute(attn_prefill_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem) != cudaSuccess)
+            HOS_REFUSE("attn_chunk_tc: cannot get %d bytes of shared memory", kTcSmem);
+        attr_set = true;
+    }
     launch_pdl(attn_prefill_tc_kernel<true>, dim3(n_heads, n_q_tiles), dim3(kTcThreads), kTcSmem, stream, mq, mk, mv, a);
     return check_launch("attn_chunk_tc");
 #else

@@ -7,6 +7,7 @@ import ctypes
 import os
 from typing import Dict, Optional
 
+import numpy as np
 import torch
 
 from .. import ops
@@ -222,6 +223,84 @@ def prompt_blocks(step, block: int):
     return len(cu) - 1, sum((cu[i + 1] - cu[i] + block - 1) // block for i in range(len(cu) - 1))
 
 
+PAIR_KEYS = 128             # keys of a tile of the pair kernel
+MAX_SHARES = 8
+SHARE_MIN_TILES = 2
+# What a walk costs besides its tiles, and what cut walks cost besides theirs, in tiles of 2.2 us (head size 256): set-up and epilogue
+# 5 to 8 us, partial sums written, read and merged 5.  Fits the times beside the kernel.
+SHARE_TILES_FIXED, SHARE_TILES_MERGE = 3.0, 2.5
+
+
+def cut_walks(tiles, pairs_per_block: int, pairs: int):
+    """(shares, tiles of a share) for blocks of queries whose walks over the keys are `tiles` long (tiles of PAIR_KEYS keys), each
+    walked by `pairs_per_block` pairs of SMs out of `pairs` at a time: (1, 0) where the walks stay whole.  A walk of n tiles is cut
+    into min(shares, ceil(n / tiles of a share)) parts.  The estimate, in tiles: a part costs its tiles and a fixed part, cut
+    walks a merge; parts that do not run at once share the pairs evenly, and end raggedly by half a part."""
+    tiles = np.asarray(tiles, dtype=np.int64)
+    longest = int(tiles.max()) if tiles.size else 0
+    if longest < 2 * SHARE_MIN_TILES or tiles.size * pairs_per_block >= 2 * pairs:
+        return 1, 0
+    best, best_cost = (1, 0), None
+    for shares in range(1, MAX_SHARES + 1):
+        length = -(-longest // shares)
+        if shares > 1 and length < SHARE_MIN_TILES:
+            break
+        parts = np.minimum(shares, -(-tiles // length))
+        most = int((-(-tiles // parts)).max())
+        n = int(parts.sum()) * pairs_per_block
+        cost = most + SHARE_TILES_FIXED
+        if n > pairs:
+            cost = max(cost, (int(tiles.sum()) * pairs_per_block + SHARE_TILES_FIXED * n) / pairs + 0.5 * most)
+        if shares > 1:
+            cost += SHARE_TILES_MERGE
+        if best_cost is None or cost < 0.95 * best_cost:
+            best, best_cost = ((shares, length) if shares > 1 else (1, 0)), cost
+    return best
+
+
+def _shares(part, n_heads: int, n_kv_heads: int, head_dim: int, window):
+    """cut_walks for the sequences of `part`, once per step and kind of layer."""
+    f = lib_for(head_dim).lib.hos_attn_prefill_pairs
+    f.restype, f.argtypes = ctypes.c_int, [ctypes.c_int, ctypes.c_int]
+    _set_pairs(head_dim, enabled["prefill_pair"])
+    pairs = int(f(n_heads, n_kv_heads))
+    if pairs == 0:
+        return 1, 0
+    key = ("attention shares", part.row_offset, part.n_tokens, n_heads, window)
+    got = part.shared.get(key)
+    if got is None:
+        w = int(window) if window else 0
+        if part.replayed or not part.cu_host:         # what the launches are planned for: every block as long as the longest
+            _, blocks = prompt_blocks(part, 128)
+            span = min(part.max_len_after, w + 127) if w else part.max_len_after
+            tiles = [-(-span // PAIR_KEYS)] * max(1, blocks - part.n_seqs + 1)
+        else:
+            tiles = []
+            starts = part.starts_host or [0] * (len(part.cu_host) - 1)
+            for i, start in enumerate(starts):
+                n = part.cu_host[i + 1] - part.cu_host[i]
+                for q0 in range(0, n, 128):
+                    first = max(0, start + q0 + 1 - w) if w else 0
+                    tiles.append((start + min(n, q0 + 128) - 1) // PAIR_KEYS - first // PAIR_KEYS + 1)
+        got = part.shared[key] = cut_walks(tiles, n_heads // 2, pairs)
+    return got
+
+
+def _share_workspace(blocks: int, n_heads: int, head_dim: int, shares: int, device):
+    """What the shares of cut walks leave: unnormalised sums, and (maximum, sum of weights) pairs."""
+    if shares <= 1:
+        return None, None
+    places = blocks * n_heads * shares * 128
+    return (torch.empty(places * head_dim, dtype=torch.float32, device=device),
+            torch.empty(places * 2, dtype=torch.float32, device=device))
+
+
+def _set_pairs(head_dim: int, want: bool) -> None:
+    if _pair_state.get(head_dim) != want:
+        lib_for(head_dim).call("hos_attn_prefill_pair", 1 if want else 0)
+        _pair_state[head_dim] = want
+
+
 def prefill_tc(rows: torch.Tensor, out, cu_seqlens, n_seqs: int, blocks: int, n_heads, n_kv_heads, head_dim, scale, cap,
                window, pairs: bool = True, wait_cycles: int = 0, stop_tile: int = -1) -> None:
     """Attention of whole prompts from position 0 on the tcgen05 tensor cores; `rows` is the
@@ -230,10 +309,7 @@ def prefill_tc(rows: torch.Tensor, out, cu_seqlens, n_seqs: int, blocks: int, n_
     share their keys may run as one pair of SMs (head sizes 128 and 256, an even group).
     wait_cycles, stop_tile: for tests of a wait that runs out (the limit of the waits; the tile at which one does)."""
     lib = lib_for(head_dim)
-    want = bool(pairs and enabled["prefill_pair"])
-    if _pair_state.get(head_dim) != want:
-        lib.call("hos_attn_prefill_pair", 1 if want else 0)
-        _pair_state[head_dim] = want
+    _set_pairs(head_dim, bool(pairs and enabled["prefill_pair"]))
     lib.call("hos_attn_prefill_tc", ops._ptr(rows), rows.shape[0], rows.shape[1], ops._ptr(out), out.shape[1],
              ops._ptr(cu_seqlens), n_seqs, blocks, n_heads, n_kv_heads, head_dim, float(scale), float(cap),
              int(window) if window else 0, int(wait_cycles), int(stop_tile), ops._stream())
@@ -269,15 +345,18 @@ def chunk(q, q_stride, out, cu_seqlens, row_base: int, token_pos, seq_slot, n_se
 
 
 def chunk_tc(q, out, cu_seqlens, row_base: int, token_pos, seq_slot, n_seqs: int, blocks: int,
-             cache: ops.PagedKVArgs, n_heads, scale, cap, window) -> None:
+             cache: ops.PagedKVArgs, n_heads, scale, cap, window, pairs: bool = True, shares: int = 1, share_tiles: int = 0) -> None:
     """As `chunk`, on the tcgen05 tensor cores (head sizes 64, 128, 256): q is [rows, stride] with the q heads
-    first in a row; `blocks`: at least the sum over sequences of ceil(rows / 128)."""
+    first in a row; `blocks`: at least the sum over sequences of ceil(rows / 128); pairs: see prefill_tc; shares, share_tiles: pairs
+    of SMs walk over a block's keys in up to that many parts of about that many tiles (see cut_walks)."""
     lib = lib_for(cache.head_dim)
+    _set_pairs(cache.head_dim, bool(pairs and enabled["prefill_pair"]))
+    part_o, part_ml = _share_workspace(blocks, n_heads, cache.head_dim, shares, q.device)
     lib.call("hos_attn_chunk_tc", ops._ptr(q), q.shape[0], q.shape[1], ops._ptr(out), out.shape[1], ops._ptr(cu_seqlens),
              int(row_base), ops._ptr(token_pos), ops._ptr(seq_slot), n_seqs, blocks, ops._ptr(cache.k_pages),
              ops._ptr(cache.v_pages), cache.k_pages.shape[0], ops._ptr(cache.page_table), cache.table_stride,
              cache.ring_pages, n_heads, cache.n_kv_heads, cache.head_dim, float(scale), float(cap),
-             int(window) if window else 0, ops._stream())
+             int(window) if window else 0, int(shares), int(share_tiles), ops._ptr(part_o), ops._ptr(part_ml), ops._stream())
 
 
 def attend_chunks(mixer, qkv, att, part, cache) -> bool:
@@ -292,8 +371,9 @@ def attend_chunks(mixer, qkv, att, part, cache) -> bool:
     slots = part.seq_slot[part.seq_offset:]
     if enabled["chunk_tc"] and qkv.is_contiguous() and has_tc_prefill(mixer.head_dim):
         _, blocks = prompt_blocks(part, 128)
+        shares, share_tiles = _shares(part, mixer.n_heads, mixer.n_kv_heads, mixer.head_dim, mixer.window)
         chunk_tc(qkv, att, part.cu_seqlens, part.row_offset, part.token_pos, slots, part.n_seqs, blocks, cache,
-                 mixer.n_heads, mixer.scale, mixer.softcap, mixer.window)
+                 mixer.n_heads, mixer.scale, mixer.softcap, mixer.window, shares=shares, share_tiles=share_tiles)
         return True
     _, blocks = prompt_blocks(part, 64)
     chunk(qkv, qkv.shape[1], att, part.cu_seqlens, part.row_offset, part.token_pos, slots, part.n_seqs, blocks, cache,
