@@ -18,10 +18,17 @@
 // rows (fewer than 16 heads per kv head) cost nothing that matters: the kernel is bound by
 // the cache's bytes.
 //
-// The kernel has a second way to cut the work (attn_decode_kernel<true>, asked for with 0 shares): not every
+// The kernel has a second way to cut the work (attn_decode_kernel<true, ...>, asked for with 0 shares): not every
 // (token, kv head) into the same number of shares, but the row of all pages of all (token, kv head) into one
 // piece of equal length per CTA, wherever the borders fall (see EvenPlan).  That wins where equal shares would
-// leave a round of SMs mostly empty, and where the sequences are of unequal lengths.
+// leave a round of SMs mostly empty, and where the sequences are of unequal lengths.  There two groups of four consumer warps
+// take a CTA's pieces in turn (where shared memory has room for both): what a piece costs besides its pages (queries, merges, the ticket,
+// 3 to 4 us of latencies) then passes under the other group's pages.  The same two groups take whole (token, kv head) in turn where
+// there are more of them than CTAs and none is cut: there a CTA's items are handed out by length, the longest first and the next round
+// the other way round, so that the CTAs with the longest item get the shortest beside it.
+// Measured (B200, 8 heads of 256 over 4, us before / now; before: items as they come, one group, heads as the rows of the MMA): 64
+// sequences of 64 to 2,036 keys 48.6 (even shares) / 37.1, of 64 to 1,000 35.2 / 21.2, of 517 28.4 / 28.8; 8 of 8,184 in four shares 44.6 / 43.5; one
+// share of 8,184 keys, 128 pages after one another, 126 / 88.
 //
 // Compiled per head size: -DHOS_HEAD_DIM=N, N a multiple of 16 up to 256.
 #include "common.cuh"
@@ -39,12 +46,12 @@ static_assert(HD % 16 == 0 && HD >= 16 && HD <= 256, "head_dim must be a multipl
 
 constexpr int kTileBytes = kPageTokens * HD * 2;                    // one [64][HD] bf16 tile
 constexpr int kStageBytes = 2 * kTileBytes;                         // keys and values of one page
-constexpr int kQBytes = 16 * HD * 2;
 constexpr int kMaxHeadsPerCta = 16;
 constexpr int kMaxStages = 8;
 constexpr int kMaxSplits = 64;
 constexpr int kSmemBudget = 226 * 1024;
-constexpr int kConsumers = 128, kDecodeThreads = 160;
+constexpr int kConsumers = 128;                                      // threads of a group of consumers
+__host__ __device__ constexpr int decode_threads(int groups) { return groups * kConsumers + 32; }
 constexpr long long kWaitCycles = 1ll << 31;                        // about a second
 
 __device__ int g_decode_error = 0;     // set when a bounded wait gave up
@@ -87,7 +94,12 @@ __device__ __forceinline__ bool wait_timed(uint64_t* bar, uint32_t parity) {
         if (clock64() - t0 > kWaitCycles) return false;
     return true;
 }
-__device__ __forceinline__ void consumer_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+__device__ __forceinline__ void consumer_sync(int who) { asm volatile("bar.sync %0, 128;" ::"r"(1 + who) : "memory"); }
+// a / b of numbers that mostly fit 32 bits
+__device__ __forceinline__ long long quotient(long long a, long long b) {
+    if (((a | b) >> 31) == 0) return (uint32_t)a / (uint32_t)b;
+    return a / b;
+}
 __device__ __forceinline__ void cluster_barrier() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -175,8 +187,8 @@ __device__ __forceinline__ EvenWalk even_begin(const EvenPlan& e, int n_tokens) 
     const int pages = e.pre[lo + 1] - e.pre[lo];
     const long long rem = w.at - (long long)e.pre[lo] * e.per_token;
     w.n = lo;
-    w.y = (int)(rem / pages);
-    w.off = (int)(rem % pages);
+    w.y = (int)quotient(rem, pages);
+    w.off = (int)(rem - (long long)w.y * pages);
     return w;
 }
 // The next piece of this CTA's walk: false when there is none.
@@ -188,8 +200,8 @@ __device__ __forceinline__ bool even_next(const DecodeArgs& a, const EvenPlan& e
     it.lp_begin = it.lo / kPageTokens + w.off;
     it.n_tiles = take;
     const long long start = (long long)e.pre[w.n] * e.per_token + (long long)w.y * pages;
-    it.first_cta = (int)(start / e.per_cta);
-    it.n_parts = (int)((start + pages - 1) / e.per_cta) - it.first_cta + 1;
+    it.first_cta = (int)quotient(start, e.per_cta);
+    it.n_parts = (int)quotient(start + pages - 1, e.per_cta) - it.first_cta + 1;
     it.part = (int)blockIdx.x - it.first_cta;
     w.at += take;
     w.off += take;
@@ -203,32 +215,63 @@ __device__ __forceinline__ bool even_next(const DecodeArgs& a, const EvenPlan& e
     return true;
 }
 constexpr int kEvenMaxTokens = 2048;   // rows of a step with even shares (their running sums live in shared memory)
+constexpr int kSortedMaxTokens = 256;  // rows of a step whose items are sorted (every CTA ranks them for itself)
 constexpr int kEvenMaxParts = 32;      // a (token, y) lies in at most this many CTAs (the CTAs' shares grow if need be)
 
-template <bool EVEN>
-__global__ void __launch_bounds__(kDecodeThreads, 1) attn_decode_kernel(DecodeArgs a) {
+// Where a lane's row of the 16-byte chunks 2 kk + first lies in a tile: the permutation of a row repeats every eight chunks, so four
+// registers and an immediate name them all.
+struct LaneChunks {
+    uint32_t at[4];
+    __device__ __forceinline__ LaneChunks(int row, int first) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) at[j] = row * HD * 2 + (HD % 64 == 0 ? ((2 * j + first) ^ (row & 7)) << 4 : first << 4);
+    }
+    __device__ __forceinline__ uint32_t operator()(int kk) const { return HD % 64 == 0 ? at[kk & 3] + (kk >> 2) * 128 : at[0] + kk * 32; }
+};
+// Rows of the queries' tile in shared memory.
+__host__ __device__ constexpr int query_rows(int merge_rows) { return merge_rows <= 8 ? 8 : 16; }
+// Bytes of shared memory of one group of consumers: queries, the four warps' results, the shares' weights.
+__host__ __device__ constexpr int group_bytes(int merge_rows) {
+    return query_rows(merge_rows) * HD * 2 + 4 * merge_rows * (HD + 2) * 4 + (2 * merge_rows * kMaxSplits * 4 + 15) / 16 * 16;
+}
+
+// FEW: no more than eight query heads to a kv head.  The products are then formed the other way round, S^T = K Q^T and O^T = V^T P^T, so
+// that the heads are the MMA's eight columns and no row of it is idle: half as many MMAs and sums, and room for the queries to stay
+// in registers.  P^T comes from S^T's registers by two 8 x 8 transpositions.
+template <bool EVEN, int GROUPS, bool FEW>
+__global__ void __launch_bounds__(decode_threads(GROUPS), 1) attn_decode_kernel(DecodeArgs a) {
+    static_assert(FEW || GROUPS == 1, "many heads are one group's");
+    constexpr bool SORTED = !EVEN && GROUPS == 2;      // whole items, by their length
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const int stages = a.stages;
+    const int tid = threadIdx.x & (kConsumers - 1), warp = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31;    // within a group of consumers
+    const int who = threadIdx.x / kConsumers;                                   // which group; GROUPS: the producer
     bf16* stage_base = reinterpret_cast<bf16*>(smem_raw);                       // stages x (K tile, V tile)
-    bf16* q_s = reinterpret_cast<bf16*>(smem_raw + (size_t)stages * kStageBytes);  // [16][HD]
-    float* mo = reinterpret_cast<float*>(smem_raw + (size_t)stages * kStageBytes + kQBytes);   // [4][merge_rows][HD]
+    unsigned char* own = smem_raw + (size_t)stages * kStageBytes;
+    // A tile's arrival is told to the group that takes it, on a barrier of that group's own: a group knows its phases by its own tiles,
+    // however many of the other's pass through a stage between them.
+    uint64_t* full = reinterpret_cast<uint64_t*>(own + GROUPS * group_bytes(a.merge_rows));      // [groups][kMaxStages]
+    uint64_t* empty = full + GROUPS * kMaxStages;                               // [stages]
+    float* res = reinterpret_cast<float*>(empty + kMaxStages);                  // equal shares: [merge_rows][HD + 2], this share's result, for the cluster
+    int* pre = reinterpret_cast<int*>(empty + kMaxStages);                      // even shares: [n_tokens + 1]; sorted: [2][n_tokens]
+    own += (GROUPS > 1 ? min(who, GROUPS - 1) : 0) * group_bytes(a.merge_rows);
+    bf16* q_s = reinterpret_cast<bf16*>(own);                                   // [query_rows][HD]
+    float* mo = reinterpret_cast<float*>(own + query_rows(a.merge_rows) * HD * 2);   // [4][merge_rows][HD]
     float* mml = mo + 4 * a.merge_rows * HD;                                    // [4][merge_rows][2]
     float* wm = mml + 4 * a.merge_rows * 2;                                     // [merge_rows][kMaxSplits] share weights
     float* wl = wm + a.merge_rows * kMaxSplits;                                 // [merge_rows][kMaxSplits]
-    float* res = wl + a.merge_rows * kMaxSplits;                                // [merge_rows][HD + 2]: this share's result, for the cluster
-    uint64_t* full = reinterpret_cast<uint64_t*>(res + a.merge_rows * (HD + 2));   // [stages]
-    uint64_t* empty = full + kMaxStages;                                        // [stages]
-    int* pre = reinterpret_cast<int*>(empty + kMaxStages);                      // even shares: [n_tokens + 1]
-    __shared__ int last_flag;
+    __shared__ int last_flag[GROUPS];
     __shared__ int even_most;
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int group = a.n_heads / a.cache.n_kv_heads;
     const int chunks = (group + kMaxHeadsPerCta - 1) / kMaxHeadsPerCta;
     const int total_items = EVEN ? 0 : a.n_tokens * a.cache.n_kv_heads * chunks * a.n_splits;
 
-    if (tid == 0) {
-        for (int s = 0; s < stages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 4); }
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < stages; ++s) {
+            for (int g = 0; g < GROUPS; ++g) mbar_init(&full[g * kMaxStages + s], 1);
+            mbar_init(&empty[s], 4);
+        }
         mbar_fence_init();
         even_most = 1;
     }
@@ -238,7 +281,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) attn_decode_kernel(DecodeAr
         // pages per token (positions and sequences were written at the head of the step, long before this kernel),
         // their running sum, and the most pages of one token; padding rows have none
         int most = 0;
-        for (int n = tid; n < a.n_tokens; n += kDecodeThreads) {
+        for (int n = threadIdx.x; n < a.n_tokens; n += decode_threads(GROUPS)) {
             int pages = 0;
             if (a.token_seq[n] >= 0) {
                 const int pos = a.token_pos[n];
@@ -250,7 +293,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) attn_decode_kernel(DecodeAr
         }
         if (most > 1) atomicMax(&even_most, most);
         __syncthreads();
-        if (warp == 0) {                       // running sum, 32 tokens at a time
+        if (threadIdx.x < 32) {                // running sum, 32 tokens at a time
             int carry = 0;
             for (int n0 = 0; n0 < a.n_tokens; n0 += 32) {
                 const int n = n0 + lane;
@@ -267,10 +310,33 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) attn_decode_kernel(DecodeAr
         }
         __syncthreads();
         plan.total = (long long)pre[a.n_tokens] * plan.per_token;
-        const long long even = (plan.total + gridDim.x - 1) / gridDim.x;
+        const long long even = quotient(plan.total + gridDim.x - 1, gridDim.x);
         const int least = (even_most + kEvenMaxParts - 2) / (kEvenMaxParts - 1);     // so that no (token, y) lies in too many CTAs
         plan.per_cta = (int)max(even, (long long)max(1, least));
     }
+    if (SORTED) {                              // pages per token, then the tokens by their number
+        int* order = pre + a.n_tokens;
+        for (int n = threadIdx.x; n < a.n_tokens; n += decode_threads(GROUPS)) {
+            const int pos = a.token_pos[n], lo = a.window > 0 ? max(0, pos + 1 - a.window) : 0;
+            pre[n] = a.token_seq[n] >= 0 ? pos / kPageTokens - lo / kPageTokens + 1 : 0;
+        }
+        __syncthreads();
+        for (int n = threadIdx.x; n < a.n_tokens; n += decode_threads(GROUPS)) {
+            int rank = 0;
+            for (int m = 0; m < a.n_tokens; ++m) rank += pre[m] > pre[n] || (pre[m] == pre[n] && m < n) ? 1 : 0;
+            order[rank] = n;
+        }
+        __syncthreads();
+    }
+    const int per_token = a.cache.n_kv_heads * chunks;
+    // item `round` of this CTA: total_items or more where there is none
+    auto item_of = [&](int round) {
+        if (!SORTED) return (int)(blockIdx.x + round * gridDim.x);
+        return (int)(round & 1 ? (round + 1) * gridDim.x - 1 - blockIdx.x : blockIdx.x + round * gridDim.x);
+    };
+    auto item_at = [&](int index) {
+        return make_item(a, SORTED ? pre[a.n_tokens + index / per_token] * per_token + index % per_token : index, group, chunks);
+    };
     pdl_launch_dependents();
     // This kernel is launched so that it may start while the projection before it still runs.  That
     // kernel writes q and the step's new keys and values, nothing else that is read here: the
@@ -279,22 +345,25 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) attn_decode_kernel(DecodeAr
     // at least two kernels earlier.  In a ring the oldest tile of the window can share its page
     // with the newest positions: the rows that are being written are masked in that tile.)
 
-    if (warp == 4) {
+    if (who == GROUPS) {
         // ---------------- producer: one thread feeds the ring, item after item ----------------
         if (lane == 0) {
             const bf16* k_pages = reinterpret_cast<const bf16*>(a.cache.k_pages);
             const bf16* v_pages = reinterpret_cast<const bf16*>(a.cache.v_pages);
             int t = 0;            // tiles issued so far by this CTA
             bool ok = true, waited = false;
+            int turn = 0;
             EvenWalk walk = even_begin(plan, a.n_tokens);
-            for (int index = blockIdx.x; ok; index += gridDim.x) {
+            for (int round = 0; ok; ++round) {
                 Item it;
                 if (EVEN) {
                     if (!even_next(a, plan, walk, it, group, chunks)) break;
                 } else {
+                    const int index = item_of(round);
                     if (index >= total_items) break;
-                    it = make_item(a, index, group, chunks);
+                    it = item_at(index);
                 }
+                uint64_t* arrive = full + (GROUPS > 1 ? (turn++ & 1) * kMaxStages : 0);
                 if (it.n_tiles == 0) continue;
                 const int* table = a.cache.page_table + (size_t)it.slot * a.cache.table_stride;
                 for (int tile = 0; tile < it.n_tiles; ++tile, ++t) {
@@ -307,9 +376,9 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) attn_decode_kernel(DecodeAr
                     const int page = table[kv_table_entry(a.cache, it.lp_begin + tile)];
                     const size_t off = kv_tile_offset(a.cache, page, it.kvh);
                     bf16* dst = stage_base + (size_t)s * (kStageBytes / 2);
-                    mbar_expect_tx(&full[s], kStageBytes);
-                    bulk_g2s(dst, k_pages + off, kTileBytes, &full[s]);
-                    bulk_g2s(dst + kTileBytes / 2, v_pages + off, kTileBytes, &full[s]);
+                    mbar_expect_tx(&arrive[s], kStageBytes);
+                    bulk_g2s(dst, k_pages + off, kTileBytes, &arrive[s]);
+                    bulk_g2s(dst + kTileBytes / 2, v_pages + off, kTileBytes, &arrive[s]);
                 }
             }
             if (!ok) record_give_up();
@@ -325,28 +394,39 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) attn_decode_kernel(DecodeAr
         return;
     }
 
-    // ---------------- consumers: warps 0..3 ----------------
+    // ---------------- consumers: groups of four warps ----------------
     pdl_wait();                   // q and the newest keys are complete from here on
     if (EVEN) {                   // padding rows are nobody's work here: a defined output for them
         for (int n = blockIdx.x; n < a.n_tokens; n += gridDim.x)
             if (pre[n + 1] == pre[n])
-                for (int i = tid; i < a.n_heads * HD; i += kConsumers)
+                for (int i = threadIdx.x; i < a.n_heads * HD; i += GROUPS * kConsumers)
                     a.out[(size_t)n * a.out_stride + i] = __float2bfloat16(0.f);
     }
     const int g = lane >> 2, t4 = lane & 3;
     const float inv_cap = a.cap > 0.f ? 1.f / a.cap : 0.f;
     const uint32_t q_base = smem_u32(q_s);
-    int t = 0;                    // tiles consumed so far by this CTA
+    const int upper = (lane >> 3) & 1, right = lane >> 4;
+    const LaneChunks k_at(FEW ? warp * 16 + (lane & 7) + upper * 8 : warp * 16 + (lane & 7) + right * 8, FEW ? right : upper);
+    const LaneChunks v_at(FEW ? warp * 16 + (lane & 7) + right * 8 : warp * 16 + (lane & 7) + upper * 8, FEW ? upper : right);
+    int t = 0;                    // tiles of the pieces so far, this group's and the other's
     bool gave_up = false;
+    int turn = 0;
+    uint32_t phases = 0;          // bit s: the parity of this group's next tile in stage s
+    full += (GROUPS > 1 ? who : 0) * kMaxStages;
 
     EvenWalk walk = even_begin(plan, a.n_tokens);
-    for (int index = blockIdx.x;; index += gridDim.x) {
+    for (int round = 0;; ++round) {
         Item it;
         if (EVEN) {
             if (!even_next(a, plan, walk, it, group, chunks)) break;
         } else {
+            const int index = item_of(round);
             if (index >= total_items) break;
-            it = make_item(a, index, group, chunks);
+            it = item_at(index);
+        }
+        if (GROUPS > 1 && (turn++ & 1) != who) {          // the other group's piece
+            t += it.n_tiles;
+            continue;
         }
         const int n = it.n;
         const int mr = a.merge_rows;
@@ -363,101 +443,113 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) attn_decode_kernel(DecodeAr
             continue;
         }
         // Q rows (zero beyond the real heads), permuted like the key tiles
-        consumer_sync();                       // the last item's readers of q_s and of the merge area are done
+        consumer_sync(who);                       // the last item's readers of q_s and of the merge area are done
         {
             const bf16* qp = a.q + (size_t)n * a.q_stride + (size_t)it.head0 * HD;
             constexpr int chunks_per_row = HD / 8;
-            for (int i = tid; i < 16 * chunks_per_row; i += kConsumers) {
+            for (int i = tid; i < query_rows(mr) * chunks_per_row; i += kConsumers) {
                 const int r = i / chunks_per_row, c = i % chunks_per_row;
                 uint4 v = make_uint4(0, 0, 0, 0);
                 if (r < it.n_rows) v = *reinterpret_cast<const uint4*>(qp + (size_t)r * HD + c * 8);
                 *reinterpret_cast<uint4*>(q_s + tile_chunk_offset<HD>(r, c)) = v;
             }
         }
-        consumer_sync();
+        consumer_sync(who);
 
-        float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
-        float o[HD / 8][4];
+        uint32_t qf[FEW ? HD / 16 : 1][2];         // FEW: rows 0 to 7 of the queries, 16 numbers at a time
+        if constexpr (FEW) {
 #pragma unroll
-        for (int i = 0; i < HD / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+            for (int kk = 0; kk < HD / 16; ++kk)
+                ldmatrix_x2(qf[kk], q_base + 2 * tile_chunk_offset<HD>(lane & 7, kk * 2 + ((lane >> 3) & 1)));
+        }
+        float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
+        // sums: tiles of 8 columns (rows g and g + 8: heads); FEW: of 16 (rows g and g + 8: numbers of a head; columns 2 t4, 2 t4 + 1: heads)
+        constexpr int O_TILES = FEW ? HD / 16 : HD / 8;
+        float o[O_TILES][4] = {};
 
         for (int tile = 0; tile < it.n_tiles; ++tile, ++t) {
             const int s = t % stages;
-            if (!wait_timed(&full[s], (t / stages) & 1)) { gave_up = true; break; }      // (the whole CTA: the barrier is one)
+            if (!wait_timed(&full[s], (phases >> s) & 1)) { gave_up = true; break; }      // (the whole group: the barrier is one)
+            phases ^= 1u << s;
             const bf16* k_s = stage_base + (size_t)s * (kStageBytes / 2);
             const bf16* v_s = k_s + kTileBytes / 2;
             const uint32_t k_base = smem_u32(k_s), v_base = smem_u32(v_s);
 
-            // ---- S = Q K^T for this warp's 16 keys ----
-            float sc[2][4] = {};
+            const int key0 = (it.lp_begin + tile) * kPageTokens + warp * 16;
+            // ---- S = Q K^T for this warp's 16 keys: two sums of every score, so that a chain is half as long ----
+            // (rows g and g + 8, columns 2 t4 and 2 t4 + 1: heads and keys, or FEW: keys and heads)
+            float sc[FEW ? 1 : 2][4] = {}, sd[FEW ? 1 : 2][4] = {};
 #pragma unroll
             for (int kk = 0; kk < HD / 16; ++kk) {
-                uint32_t qa[4], kb[4];
-                {
-                    const int row = (lane & 7) + ((lane >> 3) & 1) * 8;
-                    const int ch = kk * 2 + (lane >> 4);
-                    ldmatrix_x4(qa, q_base + 2 * tile_chunk_offset<HD>(row, ch));
+                auto& to = kk & 1 ? sd : sc;
+                uint32_t kb[4];
+                if constexpr (FEW) {
+                    ldmatrix_x4(kb, k_base + k_at(kk));
+                    mma_bf16(to[0], kb, qf[kk][0], qf[kk][1]);
+                } else {
+                    uint32_t qa[4];
+                    ldmatrix_x4(qa, q_base + 2 * tile_chunk_offset<HD>((lane & 7) + upper * 8, kk * 2 + right));
+                    ldmatrix_x4(kb, k_base + k_at(kk));
+                    mma_bf16(to[0], qa, kb[0], kb[1]);
+                    mma_bf16(to[1], qa, kb[2], kb[3]);
                 }
-                {
-                    const int row = warp * 16 + (lane & 7) + (lane >> 4) * 8;
-                    const int ch = kk * 2 + ((lane >> 3) & 1);
-                    ldmatrix_x4(kb, k_base + 2 * tile_chunk_offset<HD>(row, ch));
-                }
-                mma_bf16(sc[0], qa, kb[0], kb[1]);
-                mma_bf16(sc[1], qa, kb[2], kb[3]);
             }
-            // ---- scale, soft-cap, mask, running softmax ----
-            const int key0 = (it.lp_begin + tile) * kPageTokens + warp * 16;
+            // ---- scale, soft-cap, mask, running softmax: of the heads g and g + 8, or FEW: 2 t4 and 2 t4 + 1 ----
             float m_new[2] = {m_run[0], m_run[1]};
 #pragma unroll
-            for (int nt = 0; nt < 2; ++nt)
+            for (int nt = 0; nt < (FEW ? 1 : 2); ++nt)
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    const int key = key0 + nt * 8 + 2 * t4 + (i & 1);
-                    float v = softcap_fast(sc[nt][i] * a.scale, a.cap, inv_cap);
+                    const int key = FEW ? key0 + g + 8 * (i >> 1) : key0 + nt * 8 + 2 * t4 + (i & 1);
+                    const int r = FEW ? i & 1 : i >> 1;
+                    float v = softcap_fast((sc[nt][i] + sd[nt][i]) * a.scale, a.cap, inv_cap);
                     v = (key >= it.lo && key <= it.pos) ? v : -INFINITY;
                     sc[nt][i] = v;
-                    m_new[i >> 1] = fmaxf(m_new[i >> 1], v);
+                    m_new[r] = fmaxf(m_new[r], v);
                 }
             float corr[2], m_use[2];
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
-                m_new[r] = fmaxf(m_new[r], __shfl_xor_sync(0xffffffffu, m_new[r], 1));
-                m_new[r] = fmaxf(m_new[r], __shfl_xor_sync(0xffffffffu, m_new[r], 2));
+#pragma unroll
+                for (int x = FEW ? 4 : 1; x < (FEW ? 32 : 4); x <<= 1) m_new[r] = fmaxf(m_new[r], __shfl_xor_sync(0xffffffffu, m_new[r], x));
                 m_use[r] = m_new[r] == -INFINITY ? 0.f : m_new[r];
                 corr[r] = __expf(m_run[r] - m_use[r]);
                 m_run[r] = m_new[r];
                 l_run[r] *= corr[r];
             }
-            uint32_t pa[4];
-            {
-                float p[2][4];
 #pragma unroll
-                for (int nt = 0; nt < 2; ++nt)
+            for (int nt = 0; nt < (FEW ? 1 : 2); ++nt)
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        p[nt][i] = __expf(sc[nt][i] - m_use[i >> 1]);
-                        l_run[i >> 1] += p[nt][i];
-                    }
-                pa[0] = pack_bf16(p[0][0], p[0][1]);
-                pa[1] = pack_bf16(p[0][2], p[0][3]);
-                pa[2] = pack_bf16(p[1][0], p[1][1]);
-                pa[3] = pack_bf16(p[1][2], p[1][3]);
-            }
-            // ---- O = O * corr + P V ----
-#pragma unroll
-            for (int dd = 0; dd < HD / 16; ++dd) {
-                uint32_t vb[4];
-                const int row = warp * 16 + (lane & 7) + ((lane >> 3) & 1) * 8;
-                const int ch = dd * 2 + (lane >> 4);
-                ldmatrix_x4_trans(vb, v_base + 2 * tile_chunk_offset<HD>(row, ch));
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    float* acc = o[dd * 2 + h];
-                    acc[0] *= corr[0]; acc[1] *= corr[0]; acc[2] *= corr[1]; acc[3] *= corr[1];
+                for (int i = 0; i < 4; ++i) {
+                    const int r = FEW ? i & 1 : i >> 1;
+                    sc[nt][i] = __expf(sc[nt][i] - m_use[r]);
+                    l_run[r] += sc[nt][i];
                 }
-                mma_bf16(o[dd * 2], pa, vb[0], vb[1]);
-                mma_bf16(o[dd * 2 + 1], pa, vb[2], vb[3]);
+            // ---- O = O * corr + P V ----
+            if constexpr (FEW) {
+                const uint32_t pb[2] = {transposed_8x8(pack_bf16(sc[0][0], sc[0][1])), transposed_8x8(pack_bf16(sc[0][2], sc[0][3]))};
+#pragma unroll
+                for (int dd = 0; dd < HD / 16; ++dd) {
+                    uint32_t va[4];
+                    ldmatrix_x4_trans(va, v_base + v_at(dd));
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) o[dd][i] *= corr[i & 1];
+                    mma_bf16(o[dd], va, pb[0], pb[1]);
+                }
+            } else {
+                const uint32_t pa[4] = {pack_bf16(sc[0][0], sc[0][1]), pack_bf16(sc[0][2], sc[0][3]), pack_bf16(sc[1][0], sc[1][1]),
+                                        pack_bf16(sc[1][2], sc[1][3])};
+#pragma unroll
+                for (int dd = 0; dd < HD / 16; ++dd) {
+                    uint32_t vb[4];
+                    ldmatrix_x4_trans(vb, v_base + v_at(dd));
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) o[dd * 2 + h][i] *= corr[i >> 1];
+                    mma_bf16(o[dd * 2], pa, vb[0], vb[1]);
+                    mma_bf16(o[dd * 2 + 1], pa, vb[2], vb[3]);
+                }
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(&empty[s]);      // this warp is done with the stage
@@ -466,27 +558,31 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) attn_decode_kernel(DecodeAr
 
         // ---- merge the four warps (each saw other keys) through shared memory ----
 #pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            l_run[r] += __shfl_xor_sync(0xffffffffu, l_run[r], 1);
-            l_run[r] += __shfl_xor_sync(0xffffffffu, l_run[r], 2);
-        }
+        for (int r = 0; r < 2; ++r)
+#pragma unroll
+            for (int x = FEW ? 4 : 1; x < (FEW ? 32 : 4); x <<= 1) l_run[r] += __shfl_xor_sync(0xffffffffu, l_run[r], x);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const int row = g + 8 * h;
+            const int row = FEW ? 2 * t4 + h : g + 8 * h;
             if (row < it.n_rows) {
+                float* b = mo + ((size_t)warp * mr + row) * HD;
 #pragma unroll
-                for (int i = 0; i < HD / 8; ++i) {
-                    float* b = mo + ((size_t)warp * mr + row) * HD + i * 8 + 2 * t4;
-                    b[0] = o[i][2 * h];
-                    b[1] = o[i][2 * h + 1];
+                for (int i = 0; i < O_TILES; ++i) {
+                    if (FEW) {
+                        b[i * 16 + g] = o[i][h];
+                        b[i * 16 + g + 8] = o[i][2 + h];
+                    } else {
+                        b[i * 8 + 2 * t4] = o[i][2 * h];
+                        b[i * 8 + 2 * t4 + 1] = o[i][2 * h + 1];
+                    }
                 }
-                if (t4 == 0) {
+                if ((FEW ? g : t4) == 0) {
                     mml[(warp * mr + row) * 2 + 0] = m_run[h];
                     mml[(warp * mr + row) * 2 + 1] = l_run[h];
                 }
             }
         }
-        consumer_sync();
+        consumer_sync(who);
         for (int idx = tid; idx < it.n_rows * HD; idx += kConsumers) {
             const int r = idx / HD, d = idx % HD;
             float M = -INFINITY;
@@ -545,14 +641,14 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) attn_decode_kernel(DecodeAr
 
         // ---- the share is written: take a ticket; the last share of (token, kv head) merges all ----
         __threadfence();
-        consumer_sync();
+        consumer_sync(who);
         int* ticket = a.tickets + (size_t)n * a.cache.n_kv_heads * chunks + it.y;
         if (tid == 0) {
-            last_flag = atomicAdd(ticket, 1) == it.n_parts - 1;
-            if (last_flag) *ticket = 0;        // left at zero for the next launch
+            last_flag[who] = atomicAdd(ticket, 1) == it.n_parts - 1;
+            if (last_flag[who]) *ticket = 0;        // left at zero for the next launch
         }
-        consumer_sync();
-        if (!last_flag) continue;
+        consumer_sync(who);
+        if (!last_flag[who]) continue;
         __threadfence();
         // weights of the shares, once per row: w_s = e^{M_s - M} / sum_s L_s e^{M_s - M} (0 for a share without keys)
         for (int i = tid; i < it.n_rows * it.n_parts; i += kConsumers) {
@@ -561,7 +657,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) attn_decode_kernel(DecodeAr
             wm[r * kMaxSplits + s] = __ldcg(&a.part_ml[at * 2]);
             wl[r * kMaxSplits + s] = __ldcg(&a.part_ml[at * 2 + 1]);
         }
-        consumer_sync();
+        consumer_sync(who);
         if (tid < it.n_rows) {
             float M = -INFINITY, L = 0.f;
             for (int s = 0; s < it.n_parts; ++s) M = fmaxf(M, wm[tid * kMaxSplits + s]);
@@ -574,7 +670,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) attn_decode_kernel(DecodeAr
             const float inv = L > 0.f ? 1.f / L : 0.f;
             for (int s = 0; s < it.n_parts; ++s) wm[tid * kMaxSplits + s] *= inv;
         }
-        consumer_sync();
+        consumer_sync(who);
         for (int idx = tid; idx < it.n_rows * HD; idx += kConsumers) {
             const int r = idx / HD, d = idx % HD;
             const int head = it.head0 + r;
@@ -662,23 +758,37 @@ extern "C" int hos_attn_decode_set_error_word(int* word) {
     return 0;
 }
 
+// The kernels for a group of query heads: equal shares (sorted: whole items by their length), and even shares with one or two groups of consumers.
+static void (*decode_kernel_equal(int group, bool sorted = false))(DecodeArgs) {
+    if (sorted) return attn_decode_kernel<false, 2, true>;
+    return group <= 8 ? attn_decode_kernel<false, 1, true> : attn_decode_kernel<false, 1, false>;
+}
+static void (*decode_kernel_even(int group, int groups))(DecodeArgs) {
+    if (groups == 2) return attn_decode_kernel<true, 2, true>;
+    return group <= 8 ? attn_decode_kernel<true, 1, true> : attn_decode_kernel<true, 1, false>;
+}
+
 // How many clusters of `size` CTAs with `smem` bytes each run on the GPU at once (0: such clusters cannot be had).
-static int clusters_that_fit(int size, int smem) {
-    static int known[17][2] = {};             // [cluster size]: (smem asked about, answer)
+static int clusters_that_fit(int size, int smem, int group) {
+    static int known_of[2][17][2] = {};       // [few heads or many][cluster size]: (smem asked about, answer)
+    const int few = group <= 8 ? 1 : 0;
+    auto& known = known_of[few];
     if (size < 1 || size > 16) return 0;
     if (known[size][0] == smem) return known[size][1];
-    static bool wide = false;
+    static bool wide_of[2] = {false, false};
+    bool& wide = wide_of[few];
     if (size > 8 && !wide) {
-        wide = cudaFuncSetAttribute(attn_decode_kernel<false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+        wide = cudaFuncSetAttribute(decode_kernel_equal(group), cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
         cudaGetLastError();
     }
-    static int attr_smem = 0;
+    static int attr_smem_of[2] = {0, 0};
+    int& attr_smem = attr_smem_of[few];
     if (smem > attr_smem &&
-        cudaFuncSetAttribute(attn_decode_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess)
+        cudaFuncSetAttribute(decode_kernel_equal(group), cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess)
         attr_smem = smem;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)size);
-    cfg.blockDim = dim3(kDecodeThreads);
+    cfg.blockDim = dim3(decode_threads(1));
     cfg.dynamicSmemBytes = smem;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -686,16 +796,16 @@ static int clusters_that_fit(int size, int smem) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int n = 0;
-    if ((size > 8 && !wide) || cudaOccupancyMaxActiveClusters(&n, attn_decode_kernel<false>, &cfg) != cudaSuccess) n = 0;
+    if ((size > 8 && !wide) || cudaOccupancyMaxActiveClusters(&n, decode_kernel_equal(group), &cfg) != cudaSuccess) n = 0;
     cudaGetLastError();
     known[size][0] = smem;
     known[size][1] = n;
     return n;
 }
-static int decode_smem(int group, int* stages_out, int even_tokens = 0) {
+static int decode_smem(int group, int* stages_out, int ints = 0, int groups = 1) {
     const int merge_rows = group < kMaxHeadsPerCta ? group : kMaxHeadsPerCta;
-    const int fixed = kQBytes + 5 * merge_rows * (HD + 2) * 4 + 2 * merge_rows * kMaxSplits * 4 + 2 * kMaxStages * 8 + 128 +
-                      (even_tokens > 0 ? ((even_tokens + 1) * 4 + 15) / 16 * 16 : 0);
+    const int fixed = groups * group_bytes(merge_rows) + (groups + 1) * kMaxStages * 8 + 64 +
+                      (ints > 0 ? (ints * 4 + 15) / 16 * 16 : merge_rows * (HD + 2) * 4);
     int stages = (kSmemBudget - fixed) / kStageBytes;
     if (stages > kMaxStages) stages = kMaxStages;
     if (stages_out) *stages_out = stages;
@@ -707,7 +817,7 @@ extern "C" int hos_attn_decode_clusters(int n_heads, int n_kv_heads, int n_split
     if (n_kv_heads <= 0 || n_heads % n_kv_heads != 0 || n_splits < 2 || n_splits > 16) return 0;
     int stages = 0;
     const int smem = decode_smem(n_heads / n_kv_heads, &stages);
-    return stages < 2 ? 0 : clusters_that_fit(n_splits, smem);
+    return stages < 2 ? 0 : clusters_that_fit(n_splits, smem, n_heads / n_kv_heads);
 }
 
 extern "C" int hos_attn_decode(const void* q, int q_stride, void* out, int out_stride, float* workspace,
@@ -734,16 +844,30 @@ extern "C" int hos_attn_decode(const void* q, int q_stride, void* out, int out_s
     DecodeArgs a;
     a.merge_rows = group < kMaxHeadsPerCta ? group : kMaxHeadsPerCta;
     int stages = 0;
-    const int smem = decode_smem(group, &stages, even ? n_tokens : 0);
+    const int smem = decode_smem(group, &stages, even ? n_tokens + 1 : 0);
     if (stages < 2) HOS_REFUSE("attn_decode: shared memory holds fewer than two stages for head_dim %d", HD);
     a.stages = stages;
-    static int attr_smem[2] = {0, 0};
-    if (smem > attr_smem[even]) {
-        const cudaError_t e = even
-            ? cudaFuncSetAttribute(attn_decode_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)
-            : cudaFuncSetAttribute(attn_decode_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) HOS_REFUSE("attn_decode: cannot get %d bytes of shared memory", smem);
-        attr_smem[even] = smem;
+    // Two groups of consumers where they leave the ring three stages, or as many as it has beside one: with even shares, and with whole
+    // items that are more than the CTAs (so that a CTA has several, to be handed out by their length).
+    const bool several = n_splits == 1 && items > sm_count() && n_tokens <= kSortedMaxTokens;
+    int groups = 1, smem_used = smem;
+    if ((even || several) && group <= 8) {
+        int with_two = 0;
+        const int smem_two = decode_smem(group, &with_two, even ? n_tokens + 1 : 2 * n_tokens, 2);
+        if (with_two >= 3 || (with_two >= 2 && with_two == stages)) {
+            groups = 2;
+            smem_used = smem_two;
+            a.stages = with_two;
+        }
+    }
+    const bool sorted = several && groups == 2;
+    static int attr_smem[2][4] = {};            // [few heads or many][equal shares, even shares with one or two groups, sorted]
+    const int few = group <= 8 ? 1 : 0, kind = even ? groups : sorted ? 3 : 0;
+    if (smem_used > attr_smem[few][kind]) {
+        const cudaError_t e = cudaFuncSetAttribute(even ? decode_kernel_even(group, groups) : decode_kernel_equal(group, sorted),
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, smem_used);
+        if (e != cudaSuccess) HOS_REFUSE("attn_decode: cannot get %d bytes of shared memory", smem_used);
+        attr_smem[few][kind] = smem_used;
     }
     a.q = (const bf16*)q; a.q_stride = q_stride;
     a.out = (bf16*)out; a.out_stride = out_stride;
@@ -760,7 +884,7 @@ extern "C" int hos_attn_decode(const void* q, int q_stride, void* out, int out_s
     if (n_splits > 1 && n_splits <= 16 && items <= sm_count() && cluster_merge_enabled()) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)items);
-        cfg.blockDim = dim3(kDecodeThreads);
+        cfg.blockDim = dim3(decode_threads(1));
         cfg.dynamicSmemBytes = smem;
         cfg.stream = stream;
         cudaLaunchAttribute attr[2];
@@ -769,20 +893,24 @@ extern "C" int hos_attn_decode(const void* q, int q_stride, void* out, int out_s
         attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
-        const int fit = clusters_that_fit(n_splits, smem);
+        const int fit = clusters_that_fit(n_splits, smem, group);
         if ((long long)fit * n_splits >= items) {
             a.cluster_merge = 1;
             cfg.numAttrs = 2;
-            cudaLaunchKernelEx(&cfg, attn_decode_kernel<false>, a);
+            cudaLaunchKernelEx(&cfg, decode_kernel_equal(group), a);
             return check_launch("attn_decode (clusters)");
         }
     }
     if (even) {
-        launch_ahead(true, attn_decode_kernel<true>, dim3(sm_count()), dim3(kDecodeThreads), smem, stream, a);
+        launch_ahead(true, decode_kernel_even(group, groups), dim3(sm_count()), dim3(decode_threads(groups)), smem_used, stream, a);
         return check_launch("attn_decode (even shares)");
     }
+    if (sorted) {
+        launch_ahead(true, decode_kernel_equal(group, true), dim3(sm_count()), dim3(decode_threads(2)), smem_used, stream, a);
+        return check_launch("attn_decode (by length)");
+    }
     const int grid = items < sm_count() ? (int)items : sm_count();
-    launch_ahead(true, attn_decode_kernel<false>, dim3(grid), dim3(kDecodeThreads), smem, stream, a);
+    launch_ahead(true, decode_kernel_equal(group), dim3(grid), dim3(decode_threads(1)), smem, stream, a);
     return check_launch("attn_decode");
 }
 

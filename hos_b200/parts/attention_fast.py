@@ -95,10 +95,10 @@ def decode_splits(n_tokens: int, n_kv_heads: int, group: int, max_len: int, wind
     return best
 
 
-# Fitted to measurements at head size 256, 8192 keys: one sequence takes 43.0 / 29.7 / 24.7 / 26.6 us with
-# 4 / 8 / 16 / 32 shares (launch included), eight sequences 130 / 76 / 65.5 / 72.6 us with 1 / 2 / 4 / 9;
-# at 64 sequences two shares instead of one cost 27 us more per layer.
-_ITEM_US, _PAGE_US, _MERGE_US, _MERGE_PER_SHARE_US = 6.0, 0.9, 1.0, 0.275
+# Fitted to measurements at head size 256, 8192 keys: one share of a sequence alone on its SM takes 0.67 us a page (0.76 with neighbours at work) and 3 to 5 us
+# besides (88 / 50 / 36 / 28 us with 1 / 2 / 3 / 4 shares of 128 pages); at 64 sequences of 2,036 keys two shares
+# instead of one cost 22 us more per layer.
+_ITEM_US, _PAGE_US, _MERGE_US, _MERGE_PER_SHARE_US = 4.5, 0.76, 1.0, 0.275
 # Up to 16 shares of at most one wave of items merge as a cluster through shared memory: 2.3 to 2.8 us less
 # than through the workspace (one sequence, 8,192 keys, 16 shares: 17.4 -> 14.6 us; a window of 4,096: 13.5 -> 10.7).
 CLUSTER_SHARES = 16
@@ -112,7 +112,9 @@ _CLUSTER_MERGE_US, _CLUSTER_MERGE_PER_SHARE_US = 0.3, 0.03
 # Sequences of unequal lengths (8,100 / 4,000 / 2,000 / 1,000 / 500 / 500 / 250 / 250 keys, repeated): equal shares
 # take as long as the longest sequence's share, even shares follow the sum: 8 sequences 1.96 -> 1.86 ms a step, 16
 # sequences 2.69 -> 2.22, 32 sequences 4.05 -> 3.00.
-_EVEN_US = 22.0
+# (A page by itself then took 0.9 us and even shares 22 us; with two groups of consumers a CTA they take 17: 64 sequences of 64 to
+# 2,036 keys 40 us a layer, 12 of 700 to 5,000 32.)
+_EVEN_US = 16.0
 _ROUND_US = 8.0
 _PAGE_SHARED_US = 0.0085
 EVEN_MAX_ROWS = 2048
@@ -120,6 +122,25 @@ EVEN_MOST_PARTS = 20
 
 
 _fit_known: Dict[tuple, int] = {}
+
+
+def whole_items_by_length(n_rows: int, per_token: int, pages: int, fill: float) -> bool:
+    """Whether whole (token, kv head), handed out by their length, finish before even shares do (both with two groups of consumers; see
+    csrc/attention_decode.cu): `pages` of the longest row's keys, `fill` as for decode_splits.  The longest item alone, or what an SM
+    has on average, and a second item that is the longer the more alike the rows are; even shares: the average, and what cutting
+    costs.  64 rows of 64 to 2,036 keys 37 / 40 us, 48 of 200 to 1,500 29 / 32, 64 of 64 to 1,000 21 / 30; 40 rows of 8,192 keys,
+    whose 160 items are two rounds of 148 SMs: even shares."""
+    sms = ops.sm_count()
+    items = n_rows * per_token
+    if items <= sms or n_rows > SORTED_MAX_ROWS:
+        return False
+    mean = pages * fill
+    average = items * mean / sms
+    whole = _ITEM_US + max(_PAGE_US * (max(pages, average) + mean * fill), average * sms * _PAGE_SHARED_US)
+    return whole < _EVEN_US + average * sms * _PAGE_SHARED_US
+
+
+SORTED_MAX_ROWS = 256
 
 
 def clusters_fit(head_dim: int, n_heads: int, n_kv_heads: int, n_splits: int) -> int:
@@ -177,7 +198,13 @@ def decode(q: torch.Tensor, q_stride: int, out: torch.Tensor, token_pos, token_s
         _cluster_state[hd] = want
     if n_splits is None:
         fit = (lambda s: clusters_fit(hd, n_heads, nkv, s)) if want else None
-        n_splits = decode_splits(n_tokens, nkv, n_heads // nkv, max_len, window, min_live, fit, max_live, fill)
+        group = n_heads // nkv
+        n_splits = decode_splits(n_tokens, nkv, group, max_len, window, min_live, fit, max_live, fill)
+        if n_splits == 0 and group <= 8:
+            span = min(max_len, window) if window else max_len
+            live = min(n_tokens, max_live) if max_live else n_tokens
+            if whole_items_by_length(live, nkv, -(-span // ops.PAGE_TOKENS) + (1 if window else 0), fill):
+                n_splits = 1
     ws = tickets = None
     if n_splits == 0:            # even shares: every CTA the same number of pages, two places per CTA for what is cut
         f = lib.lib.hos_attn_decode_even_workspace
