@@ -794,6 +794,24 @@ static int launch_attn_tc(const float* q_lat, const LatentQuery<bf16>& q, const 
 #undef HOS_TC
 }
 
+// How many blocks of the tensor-core kernel (one row of the step each) an SM holds; 0: it does not take rows of these sizes.
+extern "C" int hos_latent_attn_blocks(int R, int D, int rot_dims) {
+    if (R <= 0 || R > 1024 || D < R || D % 8 != 0 || rot_dims < 0) return 0;
+    const int NT = R <= 128 ? 2 : R <= 256 ? 4 : R <= 512 ? 8 : 16;
+    const int Ds = max((D + 15) / 16 * 16, 64 * NT) + 8;
+    const size_t smem = (size_t)(2 * 16 * Ds + 2 * kTK * Ds + 2 * 16 * 40) * 2 + (size_t)(8 * 16 * 36 + 32 + 2 * rot_dims) * 4;
+    const void* kernel = NT == 2 ? (const void*)latent_attn_tc_kernel<true, 2> : NT == 4 ? (const void*)latent_attn_tc_kernel<true, 4>
+                         : NT == 8 ? (const void*)latent_attn_tc_kernel<true, 8> : (const void*)latent_attn_tc_kernel<true, 16>;
+    int n = 0;
+    if (smem > 200 * 1024 ||
+        (smem > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kAttnThreads, smem) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return n;
+}
+
 // Rows per block: four where many rows share keys (prompts), fewer where the sums would not fit the registers;
 // one with shares of the keys (decoding).
 template <typename T, bool PAGED>

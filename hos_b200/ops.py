@@ -668,6 +668,18 @@ def latent_prep(step, rank: int, rot: int, eps: float, inv_freq: Optional[torch.
                   cache.table_stride if cache else 0, cache.ring_pages if cache else 0, n, _stream())
 
 
+_latent_blocks: dict = {}
+
+
+def latent_attn_blocks(rank: int, row: int, rot_dims: int) -> int:
+    """Blocks of the tensor-core kernel over latent rows that an SM holds at once (asked once per shape); 0: not its sizes."""
+    key = (rank, row, rot_dims)
+    n = _latent_blocks.get(key)
+    if n is None:
+        n = _latent_blocks[key] = int(blocks().fn("hos_latent_attn_blocks")(rank, row, rot_dims))
+    return n
+
+
 def latent_attn(q_lat: torch.Tensor, q: torch.Tensor, dq: int, inv_freq: Optional[torch.Tensor], rot_dims: int, style: int, kc: Optional[torch.Tensor], cache: Optional[PagedKVArgs], sink: Optional[torch.Tensor],
                 o_lat: torch.Tensor, step, row0: int, rows: int, rank: int, scale: float, window: Optional[int],
                 paged: bool, n_splits: int = 1, rows_per_block: int = 1, tensor_cores: bool = True) -> None:

@@ -132,14 +132,18 @@ class LatentAttention(Mixer):
     def plan(self, rows: int, step: StepInfo):
         """(shares of the keys, rows per block) for `rows` rows of a step.  Rows of one sequence that follow one another
         share the keys they read: four to a block (prompts, long pieces).  Few rows, or rows of different sequences
-        (decoding), run one to a block, and their keys are cut into shares so that the GPU is filled about twice: at
-        least two tiles of 32 keys per share, at most 32 shares."""
+        (decoding), run one to a block, and their keys are cut into shares so that the blocks fill the GPU once, or twice
+        where an SM holds several of them: at least two tiles of 32 keys per share, at most 32 shares.  (Rows of 576 numbers: one
+        block to an SM; 8 rows of 16 heads, 300 to 1,024 keys, in 16 shares, which are two rounds, 22.6 us; in 9 18.0, and the merge 4.7 for 5.8.)"""
         if not step.single_token and rows >= 64:
             return 1, 4
         blocks = rows * ((self.n_heads + 7) // 8)
         sms = ops.sm_count()
         longest = step.max_len_after
         keys = min(int(self.window), longest) if self.window else longest
+        rot_dims = self.position.kernel_args()[1] if self.position else 0
+        if self.use_tensor_cores and not self.rt.is_fp32 and ops.latent_attn_blocks(self.rank, self.row, rot_dims) == 1:
+            return max(1, min(32, (keys + 63) // 64, sms // blocks)), 1
         return max(1, min(32, (keys + 63) // 64, (2 * sms + blocks - 1) // blocks)), 1
 
     def _prompt_sizes_fit(self) -> bool:
