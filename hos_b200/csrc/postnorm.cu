@@ -164,6 +164,51 @@ group_norm_gate_kernel(const float* __restrict__ o, const float* __restrict__ w,
     }
 }
 
+// Wide groups (one root mean square over all heads): a block per row and group whose threads ask for everything they need, four
+// neighbours at a time, before any of it is used; the kernel above, a number at a time and twice over o, is what other widths and
+// unaligned rows take.  Bound by the latency of one round of loads at few rows.
+template <typename TH, int NV>
+__global__ void __launch_bounds__(256)
+group_norm_gate_vec_kernel(const float* __restrict__ o, const float* __restrict__ w, int w_per_group,
+                           const float* __restrict__ gate, long long gate_stride, int act, const int* __restrict__ token_seq,
+                           TH* __restrict__ out, long long ldo, float eps, int G, int gs) {
+    pdl_enter();
+    __shared__ float scratch[32];
+    const int n = blockIdx.x, g = blockIdx.y;
+    const size_t base = ((size_t)n * G + g) * gs, obase = (size_t)n * ldo + (size_t)g * gs;
+    const bool padding = token_seq != nullptr && token_seq[n] < 0;        // a defined row, nothing read
+    const float* wg = w + (w_per_group ? 0 : (size_t)g * gs);
+    const float* gt = gate + (size_t)n * gate_stride + (size_t)g * gs;
+    float4 v[NV], z[NV], m[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const int d = (threadIdx.x + 256 * i) * 4;
+        v[i] = z[i] = m[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (d < gs && !padding) {
+            v[i] = *reinterpret_cast<const float4*>(o + base + d);
+            z[i] = *reinterpret_cast<const float4*>(gt + d);
+            m[i] = *reinterpret_cast<const float4*>(wg + d);
+        }
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) ss += (v[i].x * v[i].x + v[i].y * v[i].y) + (v[i].z * v[i].z + v[i].w * v[i].w);
+    ss = block_sum(ss, scratch);
+    const float inv = 1.f / sqrtf(ss / (float)gs + eps);
+    auto gated = [&](float x, float y, float weight) {
+        const float s = 1.f / (1.f + expf(-y));
+        return x * inv * weight * (act == 1 ? y * s : s);
+    };
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const int d = (threadIdx.x + 256 * i) * 4;
+        if (d >= gs) break;
+        const float r[4] = {gated(v[i].x, z[i].x, m[i].x), gated(v[i].y, z[i].y, m[i].y), gated(v[i].z, z[i].z, m[i].z),
+                            gated(v[i].w, z[i].w, m[i].w)};
+        store4(out + obase + d, padding ? make_float4(0.f, 0.f, 0.f, 0.f) : make_float4(r[0], r[1], r[2], r[3]));
+    }
+}
+
 // The same with a warp to a group (heads of up to 2,048 numbers, a multiple of 4): a block takes a row, its warps the
 // row's groups in turn; 16-byte reads, the group read twice (the second time from L1).
 template <typename TH>
@@ -340,6 +385,24 @@ extern "C" int hos_group_norm_gate(const float* o, const float* w, int w_per_gro
         else
             launch_pdl(group_norm_gate_warp_kernel<float>, dim3(N), dim3(256), 0, stream, o, w, w_per_group, gate, gate_stride,
                        act, token_seq, (float*)out, ldo, eps, G, gs);
+        return check_launch("group_norm_gate");
+    }
+    if (gs > 512 && gs <= 8192 && gs % 4 == 0 && gate_stride % 4 == 0 && ldo % 4 == 0 &&
+        (((uintptr_t)o | (uintptr_t)gate | (uintptr_t)w | (uintptr_t)out) & 15) == 0) {
+#define HOS_GNG(TH, NV)                                                                                              \
+    launch_pdl(group_norm_gate_vec_kernel<TH, NV>, dim3(N, G), dim3(256), 0, stream, o, w, w_per_group, gate, gate_stride, act, token_seq, \
+               (TH*)out, ldo, eps, G, gs)
+#define HOS_GNG_T(TH)                                                                                                \
+    do {                                                                                                             \
+        if (gs <= 1024) HOS_GNG(TH, 1);                                                                              \
+        else if (gs <= 2048) HOS_GNG(TH, 2);                                                                         \
+        else if (gs <= 4096) HOS_GNG(TH, 4);                                                                         \
+        else HOS_GNG(TH, 8);                                                                                         \
+    } while (0)
+        if (out_dtype == kBF16) HOS_GNG_T(bf16);
+        else HOS_GNG_T(float);
+#undef HOS_GNG_T
+#undef HOS_GNG
         return check_launch("group_norm_gate");
     }
     if (out_dtype == kBF16)
