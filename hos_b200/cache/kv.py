@@ -46,6 +46,7 @@ class KVGroup:
         v_shape = (n_pages, need.n_kv_heads, PAGE, need.v_head_dim or need.head_dim)
         self.v = [None if need.keys_only else torch.zeros(v_shape, dtype=dtype, device=device) for _ in range(n_entries)]
         self.table_host = torch.zeros((n_slots, self.table_stride), dtype=torch.int32)
+        self._table_np = self.table_host.numpy()       # the same memory: an entry is written without a tensor operation
         self.table_dev = torch.zeros((n_slots, self.table_stride), dtype=torch.int32, device=device)
         self._slot_pages: Dict[int, List[int]] = {}
         self._dirty: set = set()
@@ -73,9 +74,10 @@ class KVGroup:
         if self.ring_pages == 0 and (new_len + PAGE - 1) // PAGE > self.table_stride:
             raise CacheError(f"a sequence of {new_len} tokens is longer than the cache's tables "
                              f"hold ({self.table_stride * PAGE})")
+        row = self._table_np[slot]
         while len(held) < want:
             page = self.pages.take()
-            self.table_host[slot, len(held)] = page
+            row[len(held)] = page
             held.append(page)
             self._dirty.add(slot)
 

@@ -230,6 +230,9 @@ class Runner:
 
     def _check_ids(self, token_lists) -> None:
         for toks in token_lists:
+            ids = np.asarray(toks)
+            if ids.dtype.kind in "iu" and ids.size and int(ids.min()) >= 0 and int(ids.max()) < self.vocab_size:
+                continue                     # integers, all of them inside: no look at each
             for t in toks:
                 if not (0 <= int(t) < self.vocab_size):
                     raise HosError(f"token id {t} is outside the vocabulary (0..{self.vocab_size - 1})")
