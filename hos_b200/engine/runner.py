@@ -230,9 +230,8 @@ class Runner:
 
     def _check_ids(self, token_lists) -> None:
         for toks in token_lists:
-            ids = np.asarray(toks)
-            if ids.dtype.kind in "iu" and ids.size and int(ids.min()) >= 0 and int(ids.max()) < self.vocab_size:
-                continue                     # integers, all of them inside: no look at each
+            if isinstance(toks, (list, tuple)) and set(map(type, toks)) == {int} and min(toks) >= 0 and max(toks) < self.vocab_size:
+                continue                     # plain integers, all of them inside: no look at each
             for t in toks:
                 if not (0 <= int(t) < self.vocab_size):
                     raise HosError(f"token id {t} is outside the vocabulary (0..{self.vocab_size - 1})")
