@@ -598,17 +598,15 @@ state_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
 // What the four tokens make of one another without S (28 numbers per head) delta_fours_kernel leaves beforehand, for all of them at
 // once.  Products of decays, not differences of logarithms: a decay of zero stays one.
 // Where a thread stages is known once, the ring is deep, a chunk of eight tokens has one barrier, and the read-outs go from the
-// registers that hold them straight to memory.  A thread holds ROWS rows (every R-th piece
-// of four) of DC columns.
+// registers that hold them straight to memory.  A thread holds ROWS rows (every R-th piece of four) of
+// DC columns.
 // What bounds it: the SM's reads of k and q from shared memory (a thread's row pieces serve DC = 2 columns), then the latency of the
-// one chain, with few warps to hide it.  8 rows of two columns to a thread measured 241 us
-// where 16 rows of one column took 308 and 8 rows of one 387; where blocks fill the SMs several times over, 16 rows of two columns.
-// Measured (B200, us, token by token / this, both kernels): 16 heads of 128 x 128, 2,048 tokens 408 / 232, 128 tokens 28.5 / 19.9, 33 tokens
-// 9.9 / 9.9, 4 x 300 116 / 93; 8 heads of 256 x 256, 2,048 tokens 983 / 442; 16 heads of 64 x 64 352 / 228, 24 x 35 tokens 21.6 / 25.8.
-// Error against 64 bits (2-norm, 2,048 tokens, 128 x 128): read-outs 1.02e-7 / 8.3e-8, state 5.2e-8 / 4.5e-8: the fours' numbers are made in
-// 64 bits and rounded once.
+// one chain, with few warps to hide it.  8 rows to a thread measured 241 us where 16 rows of one column took 308 and 8 rows of one 387.
+// Measured (B200, us, token by token / this, both kernels): 16 heads of 128 x 128, 2,048 tokens 408 / 243, 128 tokens 28.5 / 20.8, 33 tokens
+// 9.9 / 10.2, 4 x 300 116 / 94; 8 heads of 256 x 256, 2,048 tokens 983 / 445; 16 heads of 64 x 64 352 / 227, 24 x 35 tokens 21.6 / 26.9.
+// Read-outs' error against 64 bits (2-norm, 2,048 tokens) 1.02e-7 / 8.7e-8: the fours' numbers are made in 64 bits and rounded once.
 constexpr int kDeltaThreads = 128, kDeltaRing = 6;
-constexpr int kFour = 4, kFourNumbers = 28;      // G [4], beta [4], D[3][.] [4], beta_j D (k_i . k_j) terms 10 20 21 30 31 32, D (k_i . q_j) terms 00 10 11 20 21 22 30 31 32 33
+constexpr int kFour = 4, kFourNumbers = 28;      // G [4], beta [4], D[3][.] [4], (k_i . k_j) terms 10 20 21 30 31 32, (k_i . q_j) terms 00 10 11 20 21 22 30 31 32 33
 
 // Where the numbers of four tokens lie: no two sequences' places meet, however the rows are shared out.
 __device__ __forceinline__ float* four_place(float* ws, int seq, int first_row, int four, int H, int head) {
