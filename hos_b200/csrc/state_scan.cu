@@ -107,11 +107,6 @@ rotate_rows_kernel(float* __restrict__ x, long long ld, int Hq, int Hk, int dim,
 constexpr int kDecayPerThread = 4;
 
 // Two 32-bit multiply-adds (or products) in one instruction: each half is the plain operation with one rounding.
-__device__ __forceinline__ uint64_t add_pair(uint64_t a, uint64_t b) {
-    uint64_t r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
 __device__ __forceinline__ uint64_t pair_of(float x, float y) {
     uint64_t d;
     asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
@@ -145,23 +140,6 @@ __device__ __forceinline__ float sum_of_eight(const float (&p)[kScanChunk], int 
     return acc;
 }
 __device__ __forceinline__ int token_of_eight(int r) { return (r & 1) * 4 + (r & 2) + ((r & 4) >> 2); }
-
-// The same among R >= 4 threads: a thread r < 8 gets the sums of token (the value returned) and, of four threads, of the one after it too.
-template <int R>
-__device__ __forceinline__ int sums_of_eight(const float (&p)[kScanChunk], int r, float (&sums)[2]) {
-    if constexpr (R >= 8) {
-        sums[0] = sum_of_eight<R>(p, r);
-        return token_of_eight(r);
-    } else {
-        static_assert(R == 4, "two turns");
-        float four[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) four[i] = ((r & 1) ? p[i + 4] : p[i]) + __shfl_xor_sync(0xffffffffu, (r & 1) ? p[i] : p[i + 4], 1);
-#pragma unroll
-        for (int i = 0; i < 2; ++i) sums[i] = ((r & 2) ? four[i + 2] : four[i]) + __shfl_xor_sync(0xffffffffu, (r & 2) ? four[i] : four[i + 2], 2);
-        return (r & 1) * 4 + (r & 2);
-    }
-}
 
 enum ScanRule : int { kDecayRule = 0, kDeltaRule = 1, kChannelRule = 2 };
 
@@ -590,117 +568,33 @@ state_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
 }
 
 // ---- the delta rule's long walks ---------------------------------------------------------------------------------------
-// Heads of ROWS x R key numbers whose rows are whole 16-byte pieces, four tokens at a time.  A token's u hangs on the state its predecessor
-// leaves, but only through scalars: with S the state before the four, G_j = g_0 .. g_j and D[j][i] = g_{i+1} .. g_j,
-//   u_j = beta_j (v_j - G_j S^T k_j - sum over i < j of D[j][i] (k_i . k_j) u_i),
-//   o_j = G_j S^T q_j + sum over i <= j of D[j][i] (k_i . q_j) u_i,      S <- G_3 S + sum of D[3][i] k_i u_i^T,
-// so the four dot products with S, whose sums over the column's R threads are what a walk token by token waits for, go side by side.
-// What the four tokens make of one another without S (28 numbers per head) delta_fours_kernel leaves beforehand, for all of them at
-// once.  Products of decays, not differences of logarithms: a decay of zero stays one.
-// Where a thread stages is known once, the ring is deep, a chunk of eight tokens has one barrier, and the read-outs go from the
-// registers that hold them straight to memory.  A thread holds ROWS rows (every R-th piece of four) of
-// DC columns.
-// What bounds it: the SM's reads of k and q from shared memory (a thread's row pieces serve DC = 2 columns), then the latency of the
-// one chain, with few warps to hide it.  8 rows to a thread measured 241 us where 16 rows of one column took 308 and 8 rows of one 387.
-// Measured (B200, us, token by token / this, both kernels): 16 heads of 128 x 128, 2,048 tokens 408 / 243, 128 tokens 28.5 / 20.8, 33 tokens
-// 9.9 / 10.2, 4 x 300 116 / 94; 8 heads of 256 x 256, 2,048 tokens 983 / 445; 16 heads of 64 x 64 352 / 227, 24 x 35 tokens 21.6 / 26.9.
-// Read-outs' error against 64 bits (2-norm, 2,048 tokens) 1.02e-7 / 8.7e-8: the fours' numbers are made in 64 bits and rounded once.
-constexpr int kDeltaThreads = 128, kDeltaRing = 6;
-constexpr int kFour = 4, kFourNumbers = 28;      // G [4], beta [4], D[3][.] [4], (k_i . k_j) terms 10 20 21 30 31 32, (k_i . q_j) terms 00 10 11 20 21 22 30 31 32 33
+// Heads of 8 R key numbers whose rows are whole 16-byte pieces: the same walk as above (and the same bits), with nothing in a
+// chunk of eight tokens but the tokens.  What bounds it is the chain of a token (scale, dot product, sum over the column's R
+// threads, update), about 160 cycles, so everything else has to stay off it: where a thread stages is known once, the ring is
+// deep, a chunk has one barrier, whole chunks have no branch, and the read-outs go from the registers that hold them
+// straight to memory.  A thread holds 8 rows of DC columns.
+// Measured (B200, 16 heads of 128 x 128, 2,048 tokens): 399 us, 195 ns a token; in the general kernel 504, before its ring and pairs 723.
+// Vagonex, prompt of 2,048 tokens 5.05 -> 4.63 ms, four of 300 to 1,000 tokens 5.67 -> 5.43 (two columns to a thread in both).
+constexpr int kDeltaRing = 6;
 
-// Where the numbers of four tokens lie: no two sequences' places meet, however the rows are shared out.
-__device__ __forceinline__ float* four_place(float* ws, int seq, int first_row, int four, int H, int head) {
-    return ws + ((size_t)(first_row / kFour + 2 * seq + four) * H + head) * kFourNumbers;
-}
-
-// A warp per (four tokens, key head); blockIdx: (eight fours, key head, sequence).  The walk's last chunk is whole: fours behind the end
-// keep the state and write nothing.
-template <int DIM>
-__global__ void __launch_bounds__(256)
-delta_fours_kernel(const float* __restrict__ q, const float* __restrict__ k, long long ld, const float* __restrict__ g, long long g_ld,
-                   const float* __restrict__ beta, long long beta_ld, const int* __restrict__ token_seq, const int* __restrict__ cu_seqlens,
-                   float* __restrict__ ws, int H, int Gk) {
-    pdl_enter();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, seq = blockIdx.z, kh = blockIdx.y, four = blockIdx.x * 8 + warp;
-    const int first = cu_seqlens[seq], lo = first + four * kFour, hi = cu_seqlens[seq + 1];
-    if (lo >= hi + ((first - hi) & (kScanChunk - 1)) || hi <= first || token_seq[first] < 0) return;
-    constexpr int E = DIM / 32;                  // numbers of a row to a lane
-    float kk[kFour][E], qq[kFour][E];
-#pragma unroll
-    for (int j = 0; j < kFour; ++j)
-#pragma unroll
-        for (int e = 0; e < E; ++e) {
-            const size_t at = (size_t)min(lo + j, hi - 1) * ld + (size_t)kh * DIM + lane + 32 * e;
-            kk[j][e] = lo + j < hi ? k[at] : 0.f;
-            qq[j][e] = lo + j < hi ? q[at] : 0.f;
-        }
-    double dot[16];                              // in 64 bits: what enters the walk is rounded once
-    auto product = [&](const float (&x)[E], const float (&y)[E]) {
-        double a = 0.;
-#pragma unroll
-        for (int e = 0; e < E; ++e) a = fma((double)x[e], (double)y[e], a);
-#pragma unroll
-        for (int x = 16; x > 0; x >>= 1) a += __shfl_xor_sync(0xffffffffu, a, x);
-        return a;
-    };
-    {
-        int at = 0;
-#pragma unroll
-        for (int j = 1; j < kFour; ++j)
-#pragma unroll
-            for (int i = 0; i < j; ++i) dot[at++] = product(kk[i], kk[j]);
-#pragma unroll
-        for (int j = 0; j < kFour; ++j)
-#pragma unroll
-            for (int i = 0; i <= j; ++i) dot[at++] = product(kk[i], qq[j]);
-    }
-    const int per = H / Gk;                      // heads that share these keys: a lane each
-    for (int h = kh * per + lane; h < (kh + 1) * per; h += 32) {
-        float bb[kFour];
-        double gg[kFour], D[kFour][kFour], G[kFour];
-#pragma unroll
-        for (int j = 0; j < kFour; ++j) {        // behind the sequence's end: no decay, nothing written
-            gg[j] = lo + j < hi ? g[(size_t)(lo + j) * g_ld + h] : 1.f;
-            bb[j] = lo + j < hi ? beta[(size_t)(lo + j) * beta_ld + h] : 0.f;
-            G[j] = j == 0 ? gg[0] : G[j - 1] * gg[j];
-#pragma unroll
-            for (int i = 0; i <= j; ++i) D[j][i] = i == j ? 1. : D[j - 1][i] * gg[j];
-        }
-        float4* to = reinterpret_cast<float4*>(four_place(ws, seq, first, four, H, h));
-        to[0] = make_float4(G[0], G[1], G[2], G[3]);
-        to[1] = make_float4(bb[0], bb[1], bb[2], bb[3]);
-        to[2] = make_float4(D[3][0], D[3][1], D[3][2], 1.f);
-        to[3] = make_float4(bb[1] * (D[1][0] * dot[0]), bb[2] * (D[2][0] * dot[1]), bb[2] * (D[2][1] * dot[2]), bb[3] * (D[3][0] * dot[3]));
-        to[4] = make_float4(bb[3] * (D[3][1] * dot[4]), bb[3] * (D[3][2] * dot[5]), dot[6], D[1][0] * dot[7]);
-        to[5] = make_float4(dot[8], D[2][0] * dot[9], D[2][1] * dot[10], dot[11]);
-        to[6] = make_float4(D[3][0] * dot[12], D[3][1] * dot[13], D[3][2] * dot[14], dot[15]);
-    }
-}
-
-template <int R, int DC, int ROWS>
+template <int R, int DC>
 struct DeltaTile {
-    static constexpr int COLS = kDeltaThreads / R * DC;              // columns of a block
-    static constexpr int ROW = ROWS * R;                             // a staged row of q or k
-    static constexpr int FOURS = kScanChunk / kFour * kFourNumbers;  // numbers of a chunk's fours
-    static constexpr int CHUNK = kScanChunk * (2 * ROW + COLS) + FOURS;  // numbers of a chunk: q, k, v, the fours
+    static constexpr int COLS = 256 / R * DC;                        // columns of a block
+    static constexpr int ROW = R * (8 + kPad);                       // a staged row of q or k
+    static constexpr int CHUNK = kScanChunk * (2 * ROW + COLS + 2);  // numbers of a chunk: q, k, v, g, beta
     static constexpr int SMEM = kDeltaRing * CHUNK * 4;
-    static constexpr int PER_ROW = ROWS / 4 * R;                            // 16-byte pieces of a row
+    static constexpr int PER_ROW = 2 * R;                            // 16-byte pieces of a row
 };
 
-// 16 bytes to shared memory, zeros where `there` is false (`from` is then any readable address).
-__device__ __forceinline__ void cp_async16_or_zero(void* dst, const void* from, bool there) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(from), "r"(there ? 16 : 0)
-                 : "memory");
-}
-
-template <int R, int DC, int ROWS>
-__global__ void __launch_bounds__(kDeltaThreads)
-delta_walk_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v, long long ld, float* __restrict__ ws,
+template <int R, int DC>
+__global__ void __launch_bounds__(256)
+delta_walk_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v, long long ld,
+                  const float* __restrict__ g, long long g_ld, const float* __restrict__ beta, long long beta_ld,
                   float* __restrict__ state, const int* __restrict__ token_pos, const int* __restrict__ token_seq,
                   const int* __restrict__ cu_seqlens, const int* __restrict__ seq_slot, float* __restrict__ out, int H, int Gk,
                   int vdim, float o_mult) {
-    using T = DeltaTile<R, DC, ROWS>;
-    constexpr int DIM = ROWS * R, PIECES = ROWS / 4;
+    using T = DeltaTile<R, DC>;
+    constexpr int DIM = 8 * R;
     pdl_enter();
     extern __shared__ __align__(16) float sm[];
     const int seq = blockIdx.x, head = blockIdx.y, col0 = blockIdx.z * T::COLS;
@@ -711,45 +605,44 @@ delta_walk_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
     const int r = threadIdx.x % R, c = threadIdx.x / R, col = col0 + c * DC;       // vdim is a multiple of 4, so of DC
     const bool live = col < vdim;
 
-    // what this thread stages of every chunk: a piece of some of its q and k rows, of its v rows, of the fours' numbers; rows behind the
-    // sequence's end are zeros (their u is zero, but zero times what lay there before might not be)
+    // what this thread stages of every chunk: a piece of some of its q and k rows, of its v rows, a decay or a beta
     const int piece = threadIdx.x % T::PER_ROW, row = threadIdx.x / T::PER_ROW;
-    const int at = row * T::ROW + piece * 4;
+    const int at = row * T::ROW + piece / 2 * (8 + kPad) + piece % 2 * 4;
     const int vrow = threadIdx.x / (T::COLS / 4), vcol = threadIdx.x % (T::COLS / 4) * 4;
     const bool stages_v = vrow < kScanChunk && col0 + vcol < vdim;
-    const int tail = kDeltaThreads - 1 - threadIdx.x;                              // the last threads: the numbers of two fours, seven pieces each
+    const int tail = 255 - threadIdx.x;                              // the last threads: 8 decays, 8 betas
     const float* from_q = q + (size_t)kh * DIM + piece * 4;
     const float* from_k = k + (size_t)kh * DIM + piece * 4;
     const float* from_v = v + (size_t)head * vdim + col0 + vcol;
     auto stage = [&](int t0, float* buf) {
 #pragma unroll
-        for (int t = 0; t < kScanChunk; t += kDeltaThreads / T::PER_ROW) {
+        for (int t = 0; t < kScanChunk; t += 256 / T::PER_ROW) {
             const int n = t0 + t + row;
-            if (t + row < kScanChunk) {
-                const size_t step = (size_t)min(n, hi - 1) * ld;
-                cp_async16_or_zero(buf + t * T::ROW + at, from_q + step, n < hi);
-                cp_async16_or_zero(buf + (kScanChunk + t) * T::ROW + at, from_k + step, n < hi);
+            if (t + row < kScanChunk && n < hi) {
+                cp_async16(buf + t * T::ROW + at, from_q + (size_t)n * ld);
+                cp_async16(buf + (kScanChunk + t) * T::ROW + at, from_k + (size_t)n * ld);
             }
         }
         float* rest = buf + 2 * kScanChunk * T::ROW;
-        if (stages_v) cp_async16_or_zero(rest + vrow * T::COLS + vcol, from_v + (size_t)min(t0 + vrow, hi - 1) * ld, t0 + vrow < hi);
-        if (tail < 14) {
-            const int f = tail / 7;
-            cp_async16(rest + kScanChunk * T::COLS + tail * 4, four_place(ws, seq, lo, (t0 - lo) / kFour + f, H, head) + tail % 7 * 4);
+        if (stages_v && t0 + vrow < hi) cp_async16(rest + vrow * T::COLS + vcol, from_v + (size_t)(t0 + vrow) * ld);
+        if (tail < 16) {
+            const int n = t0 + (tail & 7);
+            float* to = rest + kScanChunk * T::COLS + tail;
+            if (n < hi) cp_async4(to, tail < 8 ? g + (size_t)n * g_ld + head : beta + (size_t)n * beta_ld + head);
         }
     };
 
-    float* st = state + (((size_t)seq_slot[seq] * H + head) * vdim + (live ? col : 0)) * DIM + r * 4;
-    uint64_t P[DC][2 * PIECES];
+    float* st = state + (((size_t)seq_slot[seq] * H + head) * vdim + (live ? col : 0)) * DIM + r * 8;
+    uint64_t P[DC][4];
 #pragma unroll
-    for (int j = 0; j < DC; ++j)
-#pragma unroll
-        for (int p = 0; p < PIECES; ++p) {
-            float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (!fresh && live) a = *reinterpret_cast<const float4*>(st + (size_t)j * DIM + 4 * R * p);
-            P[j][2 * p] = pair_of(a.x, a.y);
-            P[j][2 * p + 1] = pair_of(a.z, a.w);
+    for (int j = 0; j < DC; ++j) {
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+        if (!fresh && live) {
+            a = *reinterpret_cast<const float4*>(st + (size_t)j * DIM);
+            b = *reinterpret_cast<const float4*>(st + (size_t)j * DIM + 4);
         }
+        P[j][0] = pair_of(a.x, a.y); P[j][1] = pair_of(a.z, a.w); P[j][2] = pair_of(b.x, b.y); P[j][3] = pair_of(b.z, b.w);
+    }
 #pragma unroll
     for (int b = 0; b < kDeltaRing - 1; ++b) {
         if (lo + b * kScanChunk < hi) stage(lo + b * kScanChunk, sm + b * T::CHUNK);
@@ -762,125 +655,80 @@ delta_walk_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
         const int ahead = t0 + (kDeltaRing - 1) * kScanChunk;
         if (ahead < hi) stage(ahead, sm + (which == 0 ? kDeltaRing - 1 : which - 1) * T::CHUNK);
         cp_async_commit_all();
-        const float* qs = sm + which * T::CHUNK + r * 4;
+        const float* qs = sm + which * T::CHUNK + r * (8 + kPad);
         const float* ks = qs + kScanChunk * T::ROW;
         const float* vs = sm + which * T::CHUNK + 2 * kScanChunk * T::ROW + c * DC;
-        const float4* fs = reinterpret_cast<const float4*>(sm + which * T::CHUNK + 2 * kScanChunk * T::ROW + kScanChunk * T::COLS);
+        const float* gs = sm + which * T::CHUNK + 2 * kScanChunk * T::ROW + kScanChunk * T::COLS;
         which = which + 1 == kDeltaRing ? 0 : which + 1;
-        // the read-outs' partial sums with the state before their four (added up after the walk, off its chain); what the four's own writes
-        // add to this thread's read-outs, and the decay of the state in them
-        constexpr int OWN = R < 8 ? 2 : 1;
-        const int mine = R < 8 ? (r & 1) * 4 + (r & 2) : token_of_eight(r);
-        float part[DC][kScanChunk], own[DC][OWN], decay[OWN];
+        auto walk = [&](auto whole_chunk) {
+            constexpr bool FULL = decltype(whole_chunk)::value;
+            const int nt = FULL ? kScanChunk : hi - t0;
+            float part[DC][kScanChunk];       // the read-outs' partial sums: added up after the walk, off its chain
 #pragma unroll
-        for (int i = 0; i < OWN; ++i) decay[i] = reinterpret_cast<const float*>(fs)[(mine + i) / kFour * kFourNumbers + (mine + i) % kFour];
+            for (int t = 0; t < kScanChunk; ++t) {
+                if (!FULL && t >= nt) {
 #pragma unroll
-        for (int f = 0; f < kScanChunk / kFour; ++f) {
-            ulonglong2 kr[kFour][PIECES];
-            float G[kFour], be[kFour], E[kFour], kk[6], kq[10];
-            {
-                const float4 n0 = fs[7 * f], n1 = fs[7 * f + 1], n2 = fs[7 * f + 2], n3 = fs[7 * f + 3], n4 = fs[7 * f + 4], n5 = fs[7 * f + 5],
-                             n6 = fs[7 * f + 6];
-                G[0] = n0.x; G[1] = n0.y; G[2] = n0.z; G[3] = n0.w;
-                be[0] = n1.x; be[1] = n1.y; be[2] = n1.z; be[3] = n1.w;
-                E[0] = n2.x; E[1] = n2.y; E[2] = n2.z; E[3] = n2.w;
-                kk[0] = n3.x; kk[1] = n3.y; kk[2] = n3.z; kk[3] = n3.w; kk[4] = n4.x; kk[5] = n4.y;
-                kq[0] = n4.z; kq[1] = n4.w; kq[2] = n5.x; kq[3] = n5.y; kq[4] = n5.z; kq[5] = n5.w;
-                kq[6] = n6.x; kq[7] = n6.y; kq[8] = n6.z; kq[9] = n6.w;
-            }
-            float a[DC][kFour], o[DC][kFour];
-#pragma unroll
-            for (int i = 0; i < kFour; ++i) {
-                const float* ki = ks + (f * kFour + i) * T::ROW;
-                const float* qi = qs + (f * kFour + i) * T::ROW;
-                ulonglong2 qr[PIECES];
-#pragma unroll
-                for (int p = 0; p < PIECES; ++p) {
-                    kr[i][p] = *reinterpret_cast<const ulonglong2*>(ki + 4 * R * p);
-                    qr[p] = *reinterpret_cast<const ulonglong2*>(qi + 4 * R * p);
+                    for (int j = 0; j < DC; ++j) part[j][t] = 0.f;
+                    continue;
                 }
+                const ulonglong2* k4 = (const ulonglong2*)(ks + t * T::ROW);
+                const ulonglong2* q4 = (const ulonglong2*)(qs + t * T::ROW);
+                const ulonglong2 k0 = k4[0], k1 = k4[1], q0 = q4[0], q1 = q4[1];
+                const float gt = gs[t], bt = gs[8 + t];
+                const uint64_t gg = pair_of(gt, gt);
+                float dot[DC];
 #pragma unroll
                 for (int j = 0; j < DC; ++j) {
-                    auto dot = [&](const ulonglong2 (&x)[PIECES]) {                       // four chains
-                        uint64_t d0 = mul_pair(P[j][0], x[0].x), d1 = mul_pair(P[j][1], x[0].y);
-                        uint64_t d2 = mul_pair(P[j][2], x[1].x), d3 = mul_pair(P[j][3], x[1].y);
-                        if constexpr (PIECES == 4) {
-                            d0 = fma_pair(P[j][4], x[2].x, d0);
-                            d1 = fma_pair(P[j][5], x[2].y, d1);
-                            d2 = fma_pair(P[j][6], x[3].x, d2);
-                            d3 = fma_pair(P[j][7], x[3].y, d3);
-                        }
-                        d0 = add_pair(d0, d2);
-                        d1 = add_pair(d1, d3);
-                        float e0, e1, e2, e3;
-                        halves_of(d0, e0, e1);
-                        halves_of(d1, e2, e3);
-                        return (e0 + e1) + (e2 + e3);
-                    };
-                    a[j][i] = dot(kr[i]);
-                    o[j][i] = dot(qr);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) P[j][i] = mul_pair(gg, P[j][i]);
+                    const uint64_t d01 = fma_pair(P[j][2], k1.x, fma_pair(P[j][0], k0.x, 0));       // four chains
+                    const uint64_t d23 = fma_pair(P[j][3], k1.y, fma_pair(P[j][1], k0.y, 0));
+                    float d0, d1, d2, d3;
+                    halves_of(d01, d0, d1);
+                    halves_of(d23, d2, d3);
+                    dot[j] = (d0 + d1) + (d2 + d3);
+                }
+#pragma unroll
+                for (int o = 1; o < R; o <<= 1)
+#pragma unroll
+                    for (int j = 0; j < DC; ++j) dot[j] += __shfl_xor_sync(0xffffffffu, dot[j], o);
+#pragma unroll
+                for (int j = 0; j < DC; ++j) {
+                    const float u = bt * (vs[t * T::COLS + j] - dot[j]);
+                    const uint64_t uu = pair_of(u, u);
+                    P[j][0] = fma_pair(k0.x, uu, P[j][0]);
+                    P[j][1] = fma_pair(k0.y, uu, P[j][1]);
+                    P[j][2] = fma_pair(k1.x, uu, P[j][2]);
+                    P[j][3] = fma_pair(k1.y, uu, P[j][3]);
+                    const uint64_t a01 = fma_pair(P[j][2], q1.x, fma_pair(P[j][0], q0.x, 0));
+                    const uint64_t a23 = fma_pair(P[j][3], q1.y, fma_pair(P[j][1], q0.y, 0));
+                    float a0, a1, a2, a3;
+                    halves_of(a01, a0, a1);
+                    halves_of(a23, a2, a3);
+                    part[j][t] = (a0 + a1) + (a2 + a3);
                 }
             }
-#pragma unroll
-            for (int x = 1; x < R; x <<= 1)
-#pragma unroll
-                for (int j = 0; j < DC; ++j)
-#pragma unroll
-                    for (int i = 0; i < kFour; ++i) a[j][i] += __shfl_xor_sync(0xffffffffu, a[j][i], x);
-            const uint64_t gg = pair_of(G[3], G[3]);
 #pragma unroll
             for (int j = 0; j < DC; ++j) {
-                const float* vj = vs + f * kFour * T::COLS + j;
-                float u[kFour];
-                // (beta is in kk; the terms of one another are small beside the rest and added up first)
-                u[0] = be[0] * fmaf(-G[0], a[j][0], vj[0]);
-                u[1] = fmaf(-kk[0], u[0], be[1] * fmaf(-G[1], a[j][1], vj[T::COLS]));
-                u[2] = be[2] * fmaf(-G[2], a[j][2], vj[2 * T::COLS]) - fmaf(kk[2], u[1], kk[1] * u[0]);
-                u[3] = be[3] * fmaf(-G[3], a[j][3], vj[3 * T::COLS]) - fmaf(kk[5], u[2], fmaf(kk[4], u[1], kk[3] * u[0]));
-#pragma unroll
-                for (int p = 0; p < 2 * PIECES; ++p) P[j][p] = mul_pair(gg, P[j][p]);
-#pragma unroll
-                for (int i = 0; i < kFour; ++i) {
-                    const float w = E[i] * u[i];
-                    const uint64_t ww = pair_of(w, w);
-#pragma unroll
-                    for (int p = 0; p < PIECES; ++p) {
-                        P[j][2 * p] = fma_pair(kr[i][p].x, ww, P[j][2 * p]);
-                        P[j][2 * p + 1] = fma_pair(kr[i][p].y, ww, P[j][2 * p + 1]);
-                    }
-                }
-                const float y[kFour] = {kq[0] * u[0], fmaf(kq[2], u[1], kq[1] * u[0]), fmaf(kq[5], u[2], fmaf(kq[4], u[1], kq[3] * u[0])),
-                                        fmaf(kq[9], u[3], fmaf(kq[8], u[2], fmaf(kq[7], u[1], kq[6] * u[0])))};
-#pragma unroll
-                for (int i = 0; i < OWN; ++i) {
-                    const int t = mine + i;
-                    const float lower = t & 1 ? y[1] : y[0], upper = t & 1 ? y[3] : y[2], picked = t & 2 ? upper : lower;
-                    own[j][i] = f == 0 || t >= kFour ? picked : own[j][i];
-                }
-#pragma unroll
-                for (int i = 0; i < kFour; ++i) part[j][f * kFour + i] = o[j][i];
+                const float acc = sum_of_eight<R>(part[j], r);
+                const int t = token_of_eight(r);
+                if (r < 8 && live && (FULL || t < nt)) out[((size_t)(t0 + t) * H + head) * vdim + col + j] = acc * o_mult;
             }
-        }
-#pragma unroll
-        for (int j = 0; j < DC; ++j) {
-            float acc[2];
-            sums_of_eight<R>(part[j], r, acc);
-#pragma unroll
-            for (int i = 0; i < OWN; ++i)
-                if (r < 8 && live && t0 + mine + i < hi)
-                    out[((size_t)(t0 + mine + i) * H + head) * vdim + col + j] = fmaf(decay[i], acc[i], own[j][i]) * o_mult;
-        }
+        };
+        if (hi - t0 >= kScanChunk) walk(std::true_type{});
+        else walk(std::false_type{});
     }
     if (!live) return;
 #pragma unroll
-    for (int j = 0; j < DC; ++j)
-#pragma unroll
-        for (int p = 0; p < PIECES; ++p) {
-            float4 a;
-            halves_of(P[j][2 * p], a.x, a.y);
-            halves_of(P[j][2 * p + 1], a.z, a.w);
-            *reinterpret_cast<float4*>(st + (size_t)j * DIM + 4 * R * p) = a;
-        }
+    for (int j = 0; j < DC; ++j) {
+        float4 a, b;
+        halves_of(P[j][0], a.x, a.y);
+        halves_of(P[j][1], a.z, a.w);
+        halves_of(P[j][2], b.x, b.y);
+        halves_of(P[j][3], b.z, b.w);
+        *reinterpret_cast<float4*>(st + (size_t)j * DIM) = a;
+        *reinterpret_cast<float4*>(st + (size_t)j * DIM + 4) = b;
+    }
 }
 
 // ---- single tokens ---------------------------------------------------------------------------------------------------------
@@ -1285,17 +1133,15 @@ struct ScanShape {
     int threads() const { return (CC / DC * R + 31) / 32 * 32; }
 };
 constexpr int kMinSegment = 64;       // tokens
-template <int R, int DC, int ROWS>
+template <int R, int DC>
 int launch_delta(const float* q, const float* k, const float* v, long long ld, const float* g, long long g_ld, const float* beta,
                  long long beta_ld, float* state, const int* token_pos, const int* token_seq, const int* cu_seqlens, const int* seq_slot,
-                 float* out, int n_seqs, int H, int Gk, int vdim, int max_new, float o_mult, float* ws, cudaStream_t stream) {
-    using T = DeltaTile<R, DC, ROWS>;
-    if (cudaFuncSetAttribute(delta_walk_kernel<R, DC, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM) != cudaSuccess)
+                 float* out, int n_seqs, int H, int Gk, int vdim, float o_mult, cudaStream_t stream) {
+    using T = DeltaTile<R, DC>;
+    if (cudaFuncSetAttribute(delta_walk_kernel<R, DC>, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM) != cudaSuccess)
         HOS_REFUSE("state_scan: cannot get %d bytes of shared memory", T::SMEM);
-    launch_pdl(delta_fours_kernel<ROWS * R>, dim3((max_new + 8 * kFour - 1) / (8 * kFour), Gk, n_seqs), dim3(256), 0, stream, q, k, ld, g, g_ld, beta,
-               beta_ld, token_seq, cu_seqlens, ws, H, Gk);
-    launch_pdl(delta_walk_kernel<R, DC, ROWS>, dim3(n_seqs, H, (vdim + T::COLS - 1) / T::COLS), dim3(kDeltaThreads), T::SMEM, stream, q, k, v, ld, ws, state,
-               token_pos, token_seq, cu_seqlens, seq_slot, out, H, Gk, vdim, o_mult);
+    launch_pdl(delta_walk_kernel<R, DC>, dim3(n_seqs, H, (vdim + T::COLS - 1) / T::COLS), dim3(256), T::SMEM, stream, q, k, v, ld, g, g_ld, beta,
+               beta_ld, state, token_pos, token_seq, cu_seqlens, seq_slot, out, H, Gk, vdim, o_mult);
     return check_launch("state_scan (delta rule)");
 }
 }  // namespace hos
@@ -1317,13 +1163,6 @@ extern "C" int hos_state_scan_segment(int n_seqs, int H, int dim, int vdim, int 
     return (len + kScanChunk - 1) / kScanChunk * kScanChunk;
 }
 
-// Floats of workspace (fours) that a long walk of the delta rule wants: 0 where hos_state_scan walks token by token.
-extern "C" long long hos_state_scan_fours(int n_rows, int n_seqs, int H, int dim, int vdim, int max_new) {
-    if (n_seqs <= 0 || n_seqs > 65535 || (dim != 64 && dim != 128 && dim != 256) || vdim % 4 != 0 || n_rows < 4ll * kScanChunk * n_seqs || max_new <= 0)
-        return 0;
-    return ((long long)n_rows / kFour + 2 * n_seqs) * H * kFourNumbers;
-}
-
 // q, k: rows of Gk heads of `dim` numbers; v: rows of H heads of `vdim`; all float32 with `ld` numbers between rows.
 // rule: 0 decay, 1 delta, 2 channel.  g: [.][H] (channel rule: [.][H * dim]) with g_ld between rows (0: one row of constants).
 // beta: the delta rule's; with the decay rule, if given, the factor on v; o_mult: a constant on the read-outs.  state: [slots][H][vdim][dim].
@@ -1331,14 +1170,12 @@ extern "C" long long hos_state_scan_fours(int n_rows, int n_seqs, int H, int dim
 // x logistic(x) as they are read, instead of by hos_act_rows before.  rot_freq ([rot_dims / 2], or null), rot_style, k_mult:
 // the staged q and k are turned by their tokens' positions and the keys multiplied, as hos_rotate_rows would have done
 // before (meant for single-token steps; it follows the rows as they are, so it does not go with act_in_walk).  seg_len, seg_count > 1: the
-// walk in segments (hos_state_scan_segment), seg_count of them to a sequence at most, with its workspace.  fours, max_new: the workspace of
-// hos_state_scan_fours (or null: token by token) and the most tokens of a sequence.
+// walk in segments (hos_state_scan_segment), seg_count of them to a sequence at most, with its workspace.
 extern "C" int hos_state_scan(const float* q, const float* k, const float* v, long long ld, int act_in_walk, int rule,
                               float o_mult, const float* g, long long g_ld, const float* beta, long long beta_ld, float* state, const int* token_pos,
                               const int* token_seq, const int* cu_seqlens, const int* seq_slot, float* out, int n_rows,
                               int n_seqs, int H, int Gk, int dim, int vdim, const float* rot_freq, int rot_dims, int rot_style,
-                              float k_mult, int seg_len, int seg_count, float* seg_states, float* seg_decays, float* fours, int max_new,
-                              cudaStream_t stream) {
+                              float k_mult, int seg_len, int seg_count, float* seg_states, float* seg_decays, cudaStream_t stream) {
     if (n_seqs <= 0) return 0;
     if (rot_freq == nullptr) rot_dims = 0;
     if (rot_dims < 0 || rot_dims % 2 != 0 || rot_dims > dim || (rot_style != 0 && rot_style != 1))
@@ -1405,21 +1242,17 @@ extern "C" int hos_state_scan(const float* q, const float* k, const float* v, lo
 #undef HOS_STEP
         return check_launch("state_scan (single tokens)");
     }
-    if (rule == kDeltaRule && fours != nullptr && hos_state_scan_fours(n_rows, n_seqs, H, dim, vdim, max_new) > 0 && pieces &&
-        (uintptr_t)v % 16 == 0 && (uintptr_t)fours % 16 == 0) {
+    if (rule == kDeltaRule && long_walk && pieces && vdim % 4 == 0 && (uintptr_t)v % 16 == 0) {
         // two columns to a thread where the blocks fill the SMs several times over anyway: the reads of k and q serve both
-        const bool many = (long long)n_seqs * H * vdim * (dim / 16) > 2ll * kDeltaThreads * sm_count_cached();
-#define HOS_DELTA(Rv, DCv, ROWSv)                                                                                    \
-    return launch_delta<Rv, DCv, ROWSv>(q, k, v, ld, g, g_ld, beta, beta_ld, state, token_pos, token_seq, cu_seqlens, seq_slot, out, n_seqs, H, Gk, \
-                                        vdim, max_new, o_mult, fours, stream)
-        if (many) {
-            if (dim == 64) HOS_DELTA(4, 2,16);
-            if (dim == 128) HOS_DELTA(8, 2,16);
-            HOS_DELTA(16, 2,16);
-        }
-        if (dim == 64) HOS_DELTA(8, 2,8);
-        if (dim == 128) HOS_DELTA(16, 2,8);
-        HOS_DELTA(32, 2,8);
+        const bool many = (long long)n_seqs * H * vdim * (dim / 8) > 2ll * 256 * sm_count_cached();
+#define HOS_DELTA(Rv)                                                                                                \
+    return many ? launch_delta<Rv, 2>(q, k, v, ld, g, g_ld, beta, beta_ld, state, token_pos, token_seq, cu_seqlens, seq_slot, out, n_seqs, H, Gk, \
+                                      vdim, o_mult, stream)                                                          \
+                : launch_delta<Rv, 1>(q, k, v, ld, g, g_ld, beta, beta_ld, state, token_pos, token_seq, cu_seqlens, seq_slot, out, n_seqs, H, Gk, \
+                                      vdim, o_mult, stream)
+        if (dim == 64) HOS_DELTA(8);
+        if (dim == 128) HOS_DELTA(16);
+        HOS_DELTA(32);
 #undef HOS_DELTA
     }
 #define HOS_SCAN(DRv, Rv, DCv, DL, LOC, BUF, PR)                                                                     \

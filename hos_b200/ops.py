@@ -1214,7 +1214,6 @@ def gated_attn_mma_decode(q: torch.Tensor, cache: PagedKVArgs, sink: Optional[to
 
 
 segmented_scans = True        # tests switch it off to compare the walk by segments with the whole one
-fours_of_tokens = True        # and this one to compare the delta rule four tokens at a time with its walk token by token
 
 
 def state_scan(rows: torch.Tensor, q_col: int, k_col: int, v_col: int, silu_on_load: bool, g: torch.Tensor,
@@ -1253,13 +1252,6 @@ def state_scan(rows: torch.Tensor, q_col: int, k_col: int, v_col: int, silu_on_l
             places = int(step.n_seqs) * seg_count * heads
             seg_states = torch.empty(places * vdim * dim, dtype=torch.float32, device=rows.device)
             seg_decays = torch.empty(places * (dim if channel_g else 1), dtype=torch.float32, device=rows.device)
-    fours = None                             # long walks of the delta rule go four tokens at a time, with a workspace
-    if rule == 1 and fours_of_tokens:
-        f = mixers().lib.hos_state_scan_fours
-        f.restype, f.argtypes = ctypes.c_longlong, [ctypes.c_int] * 6
-        floats = int(f(n, int(step.n_seqs), int(heads), int(dim), int(vdim), int(step.max_new)))
-        if floats > 0:
-            fours = torch.empty(floats, dtype=torch.float32, device=rows.device)
     in_walk = bool(silu_on_load) and beta is None and step.max_new == 1      # single tokens: no launch of its own for it
     if silu_on_load and not in_walk:        # q, k, v lie side by side from q_col on: x logistic(x) in place, once, before the walk
         if not (q_col < k_col < v_col) or v_col + heads * vdim - q_col != 2 * key_heads * dim + heads * vdim:
@@ -1270,8 +1262,7 @@ def state_scan(rows: torch.Tensor, q_col: int, k_col: int, v_col: int, silu_on_l
                   _ptr(second), heads if second is not None else 0, _ptr(state), _ptr(step.token_pos), _ptr(step.token_seq),
                   _ptr(step.cu_seqlens), _ptr(step.seq_slot), _ptr(out), n, int(step.n_seqs), int(heads), int(key_heads),
                   int(dim), int(vdim), _ptr(rot[0]) if rot else None, int(rot[1]) if rot else 0, int(rot[2]) if rot else 0,
-                  float(rot[3]) if rot else 1.0, seg_len, seg_count, _ptr(seg_states), _ptr(seg_decays), _ptr(fours),
-                  int(step.max_new), _stream(),
+                  float(rot[3]) if rot else 1.0, seg_len, seg_count, _ptr(seg_states), _ptr(seg_decays), _stream(),
                   label="hos_state_scan/channel" if channel_g else ("hos_state_scan/v_factor" if v_factor is not None else None))
 
 
