@@ -606,12 +606,14 @@ __device__ __forceinline__ void pair_attention(const CUtensorMap& map_q,      //
             if (leader) mbar_expect_tx(q_full, 2 * kQBytesTc);
             for (int c = 0; c < CBLK; ++c)
                 tma_load_2d_pair(q_s + c * kQBlockBytes, &map_q, a.q_col0 + head * THD + 64 * c, w.row0 + w.q0, q_full);
-            // paged: a tile is two pages, the second one clamped to the last that holds a key of these queries (its keys are
-            // masked where it stands for a later one); looked up one tile ahead of their use
+            // paged: a tile is two pages, both clamped to those that hold a key of these queries (a page that stands for an earlier
+            // or a later one is masked: no page is read of which no key is seen, whose values times 0 might be NaN); looked up one
+            // tile ahead of their use
             PagedKV geo{nullptr, nullptr, a.page_table, a.table_stride, a.ring_pages, a.n_kv_heads, THD};
             const int* table = PAGED ? a.page_table + (size_t)a.seq_slot[w.seq] * a.table_stride : nullptr;
+            const int first_page = a.window > 0 ? max(0, w.p0 + 1 - a.window) / kPageTokens : 0;
             auto page_row = [&](int lp) {
-                return (table[kv_table_entry(geo, min(lp, w.last_q / kPageTokens))] * a.n_kv_heads + kvh) * kPageTokens;
+                return (table[kv_table_entry(geo, min(max(lp, first_page), w.last_q / kPageTokens))] * a.n_kv_heads + kvh) * kPageTokens;
             };
             int next0 = PAGED ? page_row(2 * kt_lo) : 0, next1 = PAGED ? page_row(2 * kt_lo + 1) : 0;
             for (int j = 0; j < n_tiles && ok; ++j) {

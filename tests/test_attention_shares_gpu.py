@@ -62,3 +62,31 @@ def test_walks_in_shares(cfg, shares, length):
             if l - n <= p < l:
                 want = _ref_attention(qs[i][p], ks[i].to(dt).float(), vs[i], p, scale, cap, window)
                 close(out[cu[i] + p - (l - n)].reshape(nh, hd), want.to(dt), dt)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("hd", [128, 256])
+@pytest.mark.parametrize("pairs,shares,length", [(False, 1, 0), (True, 1, 0), (True, 2, 1)])
+def test_a_page_below_the_window_is_not_read(hd, pairs, shares, length):
+    """A window of 200 keys of which the first query's begins in the second page of a tile of 128: the page before it holds
+    infinities (which times a weight of 0 would be NaN), and so does everything below it."""
+    from hos_b200.parts import attention_fast as af
+    dt, nh, nkv, window, start, n = torch.bfloat16, 4, 2, 200, 400, 150
+    torch.manual_seed(5)
+    total = start + n
+    ks, vs = (torch.randn(total, nkv, hd).to(dt).float() for _ in range(2))
+    first = start + 1 - window
+    assert (first // 64) % 2 == 1
+    ks[:first // 64 * 64] = math.inf
+    vs[:first // 64 * 64] = math.inf
+    q = (torch.randn(n, nh, hd) * 0.5).to(dt).float()
+    scale = 0.9 / math.sqrt(hd)
+    cache, slots = _fill_cache([ks.to(DEV)], [vs.to(DEV)], [total], nkv, hd, 0, dt, fill=0.0)
+    out = torch.full((n, nh * hd), 7.0, device=DEV, dtype=dt)
+    af.chunk_tc(q.reshape(n, -1).to(DEV).to(dt), out, torch.tensor([0, n], dtype=torch.int32, device=DEV), 0,
+                torch.arange(start, total, dtype=torch.int32, device=DEV), torch.tensor(slots, dtype=torch.int32, device=DEV), 1,
+                (n + 127) // 128, cache, nh, scale, 0.0, window, pairs=pairs, shares=shares, share_tiles=length)
+    assert not af.prefill_tc_gave_up(hd)
+    for i in (0, 1, 63, 127, 128, n - 1):
+        want = _ref_attention(q[i], ks, vs, start + i, scale, 0.0, window)
+        close(out[i].reshape(nh, hd), want.to(dt), dt)
