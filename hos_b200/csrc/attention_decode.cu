@@ -758,14 +758,23 @@ extern "C" int hos_attn_decode_set_error_word(int* word) {
     return 0;
 }
 
+// A kernel that may take all the shared memory there is, or null.  That is asked for once and for every group of heads: what a launch takes
+// hangs on the group, and an attribute set for one replaces what was set for another.
+template <bool EVEN, int GROUPS, bool FEW>
+static void (*decode_kernel())(DecodeArgs) {
+    static bool allowed = false;
+    if (!allowed)
+        allowed = cudaFuncSetAttribute(attn_decode_kernel<EVEN, GROUPS, FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget) == cudaSuccess;
+    return allowed ? attn_decode_kernel<EVEN, GROUPS, FEW> : nullptr;
+}
 // The kernels for a group of query heads: equal shares (sorted: whole items by their length), and even shares with one or two groups of consumers.
 static void (*decode_kernel_equal(int group, bool sorted = false))(DecodeArgs) {
-    if (sorted) return attn_decode_kernel<false, 2, true>;
-    return group <= 8 ? attn_decode_kernel<false, 1, true> : attn_decode_kernel<false, 1, false>;
+    if (sorted) return decode_kernel<false, 2, true>();
+    return group <= 8 ? decode_kernel<false, 1, true>() : decode_kernel<false, 1, false>();
 }
 static void (*decode_kernel_even(int group, int groups))(DecodeArgs) {
-    if (groups == 2) return attn_decode_kernel<true, 2, true>;
-    return group <= 8 ? attn_decode_kernel<true, 1, true> : attn_decode_kernel<true, 1, false>;
+    if (groups == 2) return decode_kernel<true, 2, true>();
+    return group <= 8 ? decode_kernel<true, 1, true>() : decode_kernel<true, 1, false>();
 }
 
 // How many clusters of `size` CTAs with `smem` bytes each run on the GPU at once (0: such clusters cannot be had).
@@ -775,17 +784,13 @@ static int clusters_that_fit(int size, int smem, int group) {
     auto& known = known_of[few];
     if (size < 1 || size > 16) return 0;
     if (known[size][0] == smem) return known[size][1];
+    const auto kernel = decode_kernel_equal(group);
     static bool wide_of[2] = {false, false};
     bool& wide = wide_of[few];
-    if (size > 8 && !wide) {
-        wide = cudaFuncSetAttribute(decode_kernel_equal(group), cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+    if (kernel != nullptr && size > 8 && !wide) {
+        wide = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
         cudaGetLastError();
     }
-    static int attr_smem_of[2] = {0, 0};
-    int& attr_smem = attr_smem_of[few];
-    if (smem > attr_smem &&
-        cudaFuncSetAttribute(decode_kernel_equal(group), cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess)
-        attr_smem = smem;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)size);
     cfg.blockDim = dim3(decode_threads(1));
@@ -796,7 +801,7 @@ static int clusters_that_fit(int size, int smem, int group) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int n = 0;
-    if ((size > 8 && !wide) || cudaOccupancyMaxActiveClusters(&n, decode_kernel_equal(group), &cfg) != cudaSuccess) n = 0;
+    if (kernel == nullptr || (size > 8 && !wide) || cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) n = 0;
     cudaGetLastError();
     known[size][0] = smem;
     known[size][1] = n;
@@ -861,14 +866,8 @@ extern "C" int hos_attn_decode(const void* q, int q_stride, void* out, int out_s
         }
     }
     const bool sorted = several && groups == 2;
-    static int attr_smem[2][4] = {};            // [few heads or many][equal shares, even shares with one or two groups, sorted]
-    const int few = group <= 8 ? 1 : 0, kind = even ? groups : sorted ? 3 : 0;
-    if (smem_used > attr_smem[few][kind]) {
-        const cudaError_t e = cudaFuncSetAttribute(even ? decode_kernel_even(group, groups) : decode_kernel_equal(group, sorted),
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, smem_used);
-        if (e != cudaSuccess) HOS_REFUSE("attn_decode: cannot get %d bytes of shared memory", smem_used);
-        attr_smem[few][kind] = smem_used;
-    }
+    const auto kernel = even ? decode_kernel_even(group, groups) : decode_kernel_equal(group, sorted);
+    if (kernel == nullptr) HOS_REFUSE("attn_decode: cannot get %d bytes of shared memory", smem_used);
     a.q = (const bf16*)q; a.q_stride = q_stride;
     a.out = (bf16*)out; a.out_stride = out_stride;
     a.part_o = workspace;
@@ -897,20 +896,20 @@ extern "C" int hos_attn_decode(const void* q, int q_stride, void* out, int out_s
         if ((long long)fit * n_splits >= items) {
             a.cluster_merge = 1;
             cfg.numAttrs = 2;
-            cudaLaunchKernelEx(&cfg, decode_kernel_equal(group), a);
+            cudaLaunchKernelEx(&cfg, kernel, a);
             return check_launch("attn_decode (clusters)");
         }
     }
     if (even) {
-        launch_ahead(true, decode_kernel_even(group, groups), dim3(sm_count()), dim3(decode_threads(groups)), smem_used, stream, a);
+        launch_ahead(true, kernel, dim3(sm_count()), dim3(decode_threads(groups)), smem_used, stream, a);
         return check_launch("attn_decode (even shares)");
     }
     if (sorted) {
-        launch_ahead(true, decode_kernel_equal(group, true), dim3(sm_count()), dim3(decode_threads(2)), smem_used, stream, a);
+        launch_ahead(true, kernel, dim3(sm_count()), dim3(decode_threads(2)), smem_used, stream, a);
         return check_launch("attn_decode (by length)");
     }
     const int grid = items < sm_count() ? (int)items : sm_count();
-    launch_ahead(true, decode_kernel_equal(group), dim3(grid), dim3(decode_threads(1)), smem, stream, a);
+    launch_ahead(true, kernel, dim3(grid), dim3(decode_threads(1)), smem, stream, a);
     return check_launch("attn_decode");
 }
 
