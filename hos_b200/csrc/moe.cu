@@ -551,13 +551,11 @@ moe_down_tc_kernel(const bf16* __restrict__ y, const bf16* __restrict__ W, const
 // lane 16 bytes of each of its weight rows at a time against the activation row in shared memory.  A warp walks its
 // QF features' rows together, so that 2 QF (gate and up) or QF independent 16-byte loads are under way per lane and
 // step, and the loads of several steps are issued together (16 a lane): the launch is bound by the weights it
-// streams, and a lone load per step leaves the memory idle.  QF is the largest of 4, 2, 1 that still gives two
-// blocks to an SM (fewer blocks of more features leave SMs idle or with twice the work of others; more blocks of
-// fewer features read the activation row more often).  Pairs of one expert share its weights: the block of the first of them (within
-// 32 neighbours) takes the others along, up to kFewRows of their rows at a time, and their blocks leave at once; a pair's sums are the same
-// bits with others or alone.  Measured (B200, both products of 16 experts of 2,048 x 2,304, two to a row, squared relu, us, a block per pair /
-// a block per expert): 1 row 14.8 / 15.0, 4 rows 29.2 / 28.9, 8 rows (10.6 experts on average) 49.9 / 44.9, 16 rows (13.9) 84.9 / 65.0; gated 8
-// rows 73.4 / 66.7, 16 rows 131 / 106.  bfloat16, K a multiple of 8.
+// streams, and a lone load per step leaves the memory idle.  ROWS = 1: every pair for itself, the weights of an expert that several
+// chose are read again from L2.  ROWS = kFewRows: the block of an expert's first pair (within 32 neighbours) takes the others along, up to
+// ROWS of their rows at a time, and their blocks leave at once; a pair's sums are the same bits with others or alone.  That pays where the
+// weights' way in is what takes the time and the blocks that stay still fill the GPU; the caller chooses ROWS and QF (ops.moe_few_plan,
+// with what both measured).  bfloat16, K a multiple of 8.
 constexpr int kFewRows = 4;
 
 // The pairs among this one's 32 neighbours that chose expert e, as bits; 0 if an earlier one takes this one along.
@@ -567,10 +565,11 @@ __device__ __forceinline__ unsigned pairs_to_take(const int* choice, int pair, i
     return (same & ((1u << (pair & 31)) - 1u)) != 0 ? 0u : same;
 }
 // Takes up to `most` pairs off the list.
-__device__ __forceinline__ int take_pairs(unsigned& list, int base, int most, int (&ids)[kFewRows]) {
+template <int ROWS>
+__device__ __forceinline__ int take_pairs(unsigned& list, int base, int most, int (&ids)[ROWS]) {
     int n = 0;
 #pragma unroll
-    for (int p = 0; p < kFewRows; ++p) {
+    for (int p = 0; p < ROWS; ++p) {
         ids[p] = base;
         if (p < most && list != 0) {
             ids[p] = base + __ffs(list) - 1;
@@ -592,8 +591,8 @@ __device__ __forceinline__ float dot8(const uint4& a, const uint4& b) {
     return s;
 }
 
-// y[pair][F] = act(gate, up) of row pair / top under expert choice[pair]; `most` rows fit into shared memory
-template <int QF, int ACT>
+// y[pair][F] = act(gate, up) of row pair / top under expert choice[pair]; `most` rows (of ROWS) fit into shared memory
+template <int QF, int ACT, int ROWS>
 __global__ void __launch_bounds__(256)
 moe_gate_up_few_kernel(const bf16* __restrict__ h, const bf16* __restrict__ W, const int* __restrict__ choice,
                        bf16* __restrict__ y, int D, int F, int top, int n_experts, float limit, float alpha,
@@ -603,7 +602,8 @@ moe_gate_up_few_kernel(const bf16* __restrict__ h, const bf16* __restrict__ W, c
     uint4* rows = reinterpret_cast<uint4*>(raw);                // the activation rows, 8 numbers a group
     const int pair = blockIdx.y, e = choice[pair];
     if (e < 0 || e >= n_experts) return;
-    unsigned list = pairs_to_take(choice, pair, gridDim.y, e);
+    unsigned list = ROWS > 1 ? pairs_to_take(choice, pair, gridDim.y, e) : 1u;
+    if (list == 0) return;
     const int groups = D >> 3, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr bool GATED = ACT == kGatedSwish;
     const bf16* Wg = W + (size_t)e * (GATED ? 2 : 1) * F * D;
@@ -618,17 +618,17 @@ moe_gate_up_few_kernel(const bf16* __restrict__ h, const bf16* __restrict__ W, c
     }
     constexpr int U = (GATED ? 8 : 16) / QF;                    // steps whose loads are issued together: 16 loads a lane
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-    while (list != 0) {
-        int ids[kFewRows];
-        const int n = take_pairs(list, pair & ~31, most, ids);
+    do {
+        int ids[ROWS] = {pair};
+        const int n = ROWS > 1 ? take_pairs(list, pair & ~31, most, ids) : 1;
 #pragma unroll
-        for (int p = 0; p < kFewRows; ++p) {
+        for (int p = 0; p < ROWS; ++p) {
             if (p >= n) break;
             const uint4* src = reinterpret_cast<const uint4*>(h + (size_t)(ids[p] / top) * D);
             for (int g = threadIdx.x; g < groups; g += 256) rows[p * groups + g] = src[g];
         }
         __syncthreads();
-        float sg[kFewRows][QF] = {}, su[kFewRows][QF] = {};
+        float sg[ROWS][QF] = {}, su[ROWS][QF] = {};
         if (f0 < F) {
             for (int g0 = lane; g0 < groups; g0 += 32 * U) {
                 uint4 wg[U][QF], wu[U][QF];
@@ -646,7 +646,7 @@ moe_gate_up_few_kernel(const bf16* __restrict__ h, const bf16* __restrict__ W, c
                     const int g = g0 + 32 * u;
                     if (g >= groups) break;
 #pragma unroll
-                    for (int p = 0; p < kFewRows; ++p) {
+                    for (int p = 0; p < ROWS; ++p) {
                         if (p >= n) break;
                         const uint4 x = rows[p * groups + g];
 #pragma unroll
@@ -658,7 +658,7 @@ moe_gate_up_few_kernel(const bf16* __restrict__ h, const bf16* __restrict__ W, c
                 }
             }
 #pragma unroll
-            for (int p = 0; p < kFewRows; ++p) {
+            for (int p = 0; p < ROWS; ++p) {
                 if (p >= n) break;
                 const float wt = in_weight ? in_weight[ids[p]] : 1.f;
 #pragma unroll
@@ -669,12 +669,13 @@ moe_gate_up_few_kernel(const bf16* __restrict__ h, const bf16* __restrict__ W, c
                 }
             }
         }
+        if (ROWS == 1) break;
         __syncthreads();                                        // the rows are read before the next ones take their place
-    }
+    } while (list != 0);
 }
 
 // pair_out[pair][D] = weight[pair] * (W_down[e] . y[pair])
-template <int QF>
+template <int QF, int ROWS>
 __global__ void __launch_bounds__(256)
 moe_down_few_kernel(const bf16* __restrict__ y, const bf16* __restrict__ W, const int* __restrict__ choice,
                     const float* __restrict__ weight, float* __restrict__ pair_out, int D, int F, int n_experts, int most) {
@@ -683,7 +684,8 @@ moe_down_few_kernel(const bf16* __restrict__ y, const bf16* __restrict__ W, cons
     uint4* rows = reinterpret_cast<uint4*>(raw);
     const int pair = blockIdx.y, e = choice[pair];
     if (e < 0 || e >= n_experts) return;
-    unsigned list = pairs_to_take(choice, pair, gridDim.y, e);
+    unsigned list = ROWS > 1 ? pairs_to_take(choice, pair, gridDim.y, e) : 1u;
+    if (list == 0) return;
     const int groups = F >> 3, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const bf16* Wd = W + (size_t)e * D * F;
     const int n0 = (blockIdx.x * 8 + warp) * QF;
@@ -692,17 +694,17 @@ moe_down_few_kernel(const bf16* __restrict__ y, const bf16* __restrict__ W, cons
     for (int q = 0; q < QF; ++q) w_row[q] = reinterpret_cast<const uint4*>(Wd + (size_t)min(n0 + q, D - 1) * F);
     constexpr int U = 16 / QF;                                  // steps whose loads are issued together: 16 loads a lane
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-    while (list != 0) {
-        int ids[kFewRows];
-        const int n = take_pairs(list, pair & ~31, most, ids);
+    do {
+        int ids[ROWS] = {pair};
+        const int n = ROWS > 1 ? take_pairs(list, pair & ~31, most, ids) : 1;
 #pragma unroll
-        for (int p = 0; p < kFewRows; ++p) {
+        for (int p = 0; p < ROWS; ++p) {
             if (p >= n) break;
             const uint4* src = reinterpret_cast<const uint4*>(y + (size_t)ids[p] * F);
             for (int g = threadIdx.x; g < groups; g += 256) rows[p * groups + g] = src[g];
         }
         __syncthreads();
-        float s[kFewRows][QF] = {};
+        float s[ROWS][QF] = {};
         if (n0 < D) {
             for (int g0 = lane; g0 < groups; g0 += 32 * U) {
                 uint4 w[U][QF];
@@ -717,7 +719,7 @@ moe_down_few_kernel(const bf16* __restrict__ y, const bf16* __restrict__ W, cons
                     const int g = g0 + 32 * u;
                     if (g >= groups) break;
 #pragma unroll
-                    for (int p = 0; p < kFewRows; ++p) {
+                    for (int p = 0; p < ROWS; ++p) {
                         if (p >= n) break;
                         const uint4 x = rows[p * groups + g];
 #pragma unroll
@@ -726,7 +728,7 @@ moe_down_few_kernel(const bf16* __restrict__ y, const bf16* __restrict__ W, cons
                 }
             }
 #pragma unroll
-            for (int p = 0; p < kFewRows; ++p) {
+            for (int p = 0; p < ROWS; ++p) {
                 if (p >= n) break;
                 const float wt = weight ? weight[ids[p]] : 1.f;
 #pragma unroll
@@ -736,8 +738,9 @@ moe_down_few_kernel(const bf16* __restrict__ y, const bf16* __restrict__ W, cons
                 }
             }
         }
+        if (ROWS == 1) break;
         __syncthreads();
-    }
+    } while (list != 0);
 }
 
 // A block per row and per 256 * VEC columns: the chosen pairs' rows are independent loads, so a row of any width
@@ -946,58 +949,74 @@ static int few_rows(int K) {
     return fit < 1 ? 1 : fit < kFewRows ? fit : kFewRows;
 }
 
-// The same two products for a handful of pairs (see the kernels): y is [pairs][F] by pair id.  Returns 1 (and
+static int check_few_plan(int qf, int together) {
+    if ((qf != 1 && qf != 2 && qf != 4) || (together != 1 && together != kFewRows))
+        HOS_REFUSE("moe few pairs: %d features to a warp, %d pairs at a time", qf, together);
+    return 0;
+}
+
+// The same two products for a handful of pairs (see the kernels): y is [pairs][F] by pair id.  qf: output features to a warp (1, 2, 4);
+// together: 1, or 4 where an expert's pairs share its weights.  Returns 1 (and
 // launches nothing) where the sizes are not the kernels' (K no multiple of 8, rows that do not fit shared memory).
 extern "C" int hos_moe_gate_up_few(const void* h, const void* W, const int* choice, void* y, int n_pairs, int D, int F,
                                    int top, int n_experts, float limit, float alpha, float up_shift, const float* in_weight,
-                                   int act, cudaStream_t stream) {
+                                   int act, int qf, int together, cudaStream_t stream) {
     if (n_pairs <= 0) return 0;
     if (D % 8 || F % 8 || D * 2 > 96 * 1024 || ((uintptr_t)h | (uintptr_t)W | (uintptr_t)y) % 16) return 1;
     if (act != kGatedSwish && act != kReluSquare) HOS_REFUSE("moe_gate_up_few: unknown activation %d", act);
-    const long long want = 2LL * sm_count();
-    // gate and up rows: four features a warp are 181 registers a thread, one block to an SM (4 rows of 16 experts of 2,048 x 2,304, all
-    // different: both products 49 us, with two features 44; 8 rows 74 and 67, 16 rows 113 and 106)
-    const int most_qf = act == kReluSquare ? 4 : 2;
-    const int qf = most_qf == 4 && (long long)((F + 31) / 32) * n_pairs >= want ? 4 : (long long)((F + 15) / 16) * n_pairs >= want ? 2 : 1;
-    const int most = few_rows(D), smem = most * D * 2;
-#define HOS_GU_FEW_A(QF, ACT)                                                                                        \
+    if (const int rc = check_few_plan(qf, together)) return rc;
+    const int most = together == 1 ? 1 : few_rows(D), smem = most * D * 2;
+#define HOS_GU_FEW_A(QF, ACT, ROWS)                                                                                  \
     do {                                                                                                             \
         if (smem > 48 * 1024)                                                                                        \
-            cudaFuncSetAttribute(moe_gate_up_few_kernel<QF, ACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); \
-        launch_pdl(moe_gate_up_few_kernel<QF, ACT>, dim3((F + 8 * QF - 1) / (8 * QF), n_pairs), dim3(256), (size_t)smem, \
+            cudaFuncSetAttribute(moe_gate_up_few_kernel<QF, ACT, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); \
+        launch_pdl(moe_gate_up_few_kernel<QF, ACT, ROWS>, dim3((F + 8 * QF - 1) / (8 * QF), n_pairs), dim3(256), (size_t)smem, \
                    stream, (const bf16*)h, (const bf16*)W, choice, (bf16*)y, D, F, top, n_experts, limit, alpha,     \
                    up_shift, in_weight, most);                                                                       \
     } while (0)
-#define HOS_GU_FEW(QF)                                                                                               \
+#define HOS_GU_FEW(QF, ROWS)                                                                                         \
     do {                                                                                                             \
-        if (act == kReluSquare) HOS_GU_FEW_A(QF, kReluSquare);                                                       \
-        else HOS_GU_FEW_A(QF, kGatedSwish);                                                                          \
+        if (act == kReluSquare) HOS_GU_FEW_A(QF, kReluSquare, ROWS);                                                 \
+        else HOS_GU_FEW_A(QF, kGatedSwish, ROWS);                                                                    \
     } while (0)
-    if (qf == 4) HOS_GU_FEW(4);
-    else if (qf == 2) HOS_GU_FEW(2);
-    else HOS_GU_FEW(1);
+    if (together == 1) {
+        if (qf == 4) HOS_GU_FEW(4, 1);
+        else if (qf == 2) HOS_GU_FEW(2, 1);
+        else HOS_GU_FEW(1, 1);
+    } else if (qf == 4 && act == kReluSquare) {
+        HOS_GU_FEW_A(4, kReluSquare, kFewRows);
+    } else if (qf >= 2) {               // four gate and four up rows for four pairs would be 181 registers a thread, one block to an SM
+        HOS_GU_FEW(2, kFewRows);
+    } else {
+        HOS_GU_FEW(1, kFewRows);
+    }
 #undef HOS_GU_FEW_A
 #undef HOS_GU_FEW
     return check_launch("moe_gate_up_few");
 }
 
 extern "C" int hos_moe_down_few(const void* y, const void* W, const int* choice, const float* weight, float* pair_out,
-                                int n_pairs, int D, int F, int n_experts, cudaStream_t stream) {
+                                int n_pairs, int D, int F, int n_experts, int qf, int together, cudaStream_t stream) {
     if (n_pairs <= 0) return 0;
     if (D % 8 || F % 8 || F * 2 > 96 * 1024 || ((uintptr_t)y | (uintptr_t)W) % 16) return 1;
-    const long long want = 2LL * sm_count();
-    const int qf = (long long)((D + 31) / 32) * n_pairs >= want ? 4 : (long long)((D + 15) / 16) * n_pairs >= want ? 2 : 1;
-    const int most = few_rows(F), smem = most * F * 2;
-#define HOS_DOWN_FEW(QF)                                                                                             \
+    if (const int rc = check_few_plan(qf, together)) return rc;
+    const int most = together == 1 ? 1 : few_rows(F), smem = most * F * 2;
+#define HOS_DOWN_FEW(QF, ROWS)                                                                                       \
     do {                                                                                                             \
         if (smem > 48 * 1024)                                                                                        \
-            cudaFuncSetAttribute(moe_down_few_kernel<QF>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);        \
-        launch_pdl(moe_down_few_kernel<QF>, dim3((D + 8 * QF - 1) / (8 * QF), n_pairs), dim3(256), (size_t)smem,     \
+            cudaFuncSetAttribute(moe_down_few_kernel<QF, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);  \
+        launch_pdl(moe_down_few_kernel<QF, ROWS>, dim3((D + 8 * QF - 1) / (8 * QF), n_pairs), dim3(256), (size_t)smem, \
                    stream, (const bf16*)y, (const bf16*)W, choice, weight, pair_out, D, F, n_experts, most);         \
     } while (0)
-    if (qf == 4) HOS_DOWN_FEW(4);
-    else if (qf == 2) HOS_DOWN_FEW(2);
-    else HOS_DOWN_FEW(1);
+    if (together == 1) {
+        if (qf == 4) HOS_DOWN_FEW(4, 1);
+        else if (qf == 2) HOS_DOWN_FEW(2, 1);
+        else HOS_DOWN_FEW(1, 1);
+    } else {
+        if (qf == 4) HOS_DOWN_FEW(4, kFewRows);
+        else if (qf == 2) HOS_DOWN_FEW(2, kFewRows);
+        else HOS_DOWN_FEW(1, kFewRows);
+    }
 #undef HOS_DOWN_FEW
     return check_launch("moe_down_few");
 }

@@ -9,6 +9,7 @@ built, loading it raises `ExtensionMissingError`.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 import re
 from dataclasses import dataclass
@@ -864,13 +865,49 @@ def moe_down(y, w, listed, tile_expert, weight, pair_out) -> None:
                   _ptr(pair_out), tile_expert.numel(), w.shape[1], w.shape[2], _stream())
 
 
+MOE_FEW_ROWS = 4            # pairs of an expert that share its weights at a time
+
+
+@functools.lru_cache(maxsize=1024)
+def moe_few_plan(features: int, k: int, pairs: int, n_experts: int, gated: bool = False) -> tuple:
+    """(features to a warp, pairs of an expert at a time) for one of moe_few's products: `features` outputs of `k` numbers each for `pairs`
+    pairs.  A block per pair and 8 features a warp's worth: the most features that still give two blocks to an SM (fewer blocks
+    leave SMs idle or with twice the work of others, more of them read the activation row more often).  An expert's pairs share
+    its weights, a block for all of them, where its first pair is expected to have company (11 pairs to 9 experts) and the weights are more
+    than what passes in the latencies, or they are so large that nothing else counts (the shared form is no slower then), if a block holds
+    two rows and the blocks that stay still fill the GPU.
+    Measured (us, a block per pair / per expert; pairs, the experts they were drawn from): 2,304 outputs of 2,048, 16 of 16 24.7 / 21.8, 32 of 16
+    42.5 / 32.2, gated 8 of 16 26.4 / 25.3 and 32 of 16 88 / 65; 2,048 outputs of 5,632, 32 of 4 70 / 54.  Small weights or few blocks: 512 outputs of
+    2,048, 32 of 8 9.2 / 14.2; of 16,384 (one row to a block) 56 / 144; 1,024 of 512, 2 of 8 2.6 / 2.9; gated 512 of 1,024, 32 of 8 10.7 / 13.0.
+    Gate and up together are twice the loads: two features where the weights are large (2,048 x 768 gated, 16 pairs 23.7 / 21.0)."""
+    sms = sm_count()
+    met = n_experts * (1.0 - (1.0 - 1.0 / max(1, n_experts)) ** pairs)             # experts that the pairs are expected to meet
+    weights = met * features * k * (4 if gated else 2)
+
+    def widest(live: float, least: float, most: int) -> int:
+        return next((q for q in (4, 2) if q <= most and -(-features // (8 * q)) * live >= least), 1)
+    fit = min(MOE_FEW_ROWS, 48 * 1024 // (2 * k))                          # rows that a block holds
+    large = weights >= 80e6
+    if fit >= 2 and (large or (pairs >= 1.22 * met and weights >= 30e6)):
+        qf = widest(met, 1.62 * sms, 2 if gated else 4)
+        blocks = -(-features // (8 * qf)) * met
+        if blocks >= 2 * sms or (large and blocks >= 1.5 * sms):
+            return qf, MOE_FEW_ROWS
+    return widest(pairs, 2 * sms, 2 if gated and weights >= 25e6 else 4), 1
+
+
 def moe_few(h, w_gate_up, w_down, choice, weight, y, pair_out, top: int, n_experts: int, limit: float, alpha: float,
-            up_shift: float = 1.0, weight_on_input: bool = False, act: int = 0) -> bool:
+            up_shift: float = 1.0, weight_on_input: bool = False, act: int = 0, plans: Optional[tuple] = None) -> bool:
     """Both expert products for a handful of (row, choice) pairs, without lists or tiles (decoding at small batch):
-    y [pairs, F] and pair_out [pairs, D] by pair id.  False: the sizes are not these kernels' and nothing ran."""
+    y [pairs, F] and pair_out [pairs, D] by pair id.  False: the sizes are not these kernels' and nothing ran.
+    plans: moe_few_plan's answers for the two products, or None."""
     lib = experts()
     global launch_count
     pairs, d, f = choice.numel(), h.shape[1], w_down.shape[2]
+    if pairs == 0:
+        return True
+    up, down = plans or (moe_few_plan(f, d, pairs, n_experts, act == EXPERT_ACTIVATIONS["gated_swish"]),
+                         moe_few_plan(d, f, pairs, n_experts))
 
     def timed(name, *args):                 # these calls may answer 1 (not their sizes), so they do not go through call()
         if _call_times is None:
@@ -884,12 +921,12 @@ def moe_few(h, w_gate_up, w_down, choice, weight, y, pair_out, top: int, n_exper
         return rc
 
     rc = timed("hos_moe_gate_up_few", _ptr(h), _ptr(w_gate_up), _ptr(choice), _ptr(y), pairs, d, f, int(top), int(n_experts),
-               float(limit), float(alpha), float(up_shift), _ptr(weight) if weight_on_input else None, int(act), _stream())
+               float(limit), float(alpha), float(up_shift), _ptr(weight) if weight_on_input else None, int(act), *up, _stream())
     if rc == 1:
         return False
     if rc == 0:
         rc = timed("hos_moe_down_few", _ptr(y), _ptr(w_down), _ptr(choice), None if weight_on_input else _ptr(weight),
-                   _ptr(pair_out), pairs, d, f, int(n_experts), _stream())
+                   _ptr(pair_out), pairs, d, f, int(n_experts), *down, _stream())
     launch_count += 2
     if rc != 0:
         msg = lib._last_error() if lib._last_error else b""
