@@ -31,6 +31,7 @@ rotation are this one's.
 from __future__ import annotations
 
 import functools
+import math
 from typing import List, Mapping, Optional
 
 import torch
@@ -48,6 +49,29 @@ from .base import CallStore, KVNeed, Mixer, StepInfo, WeightSpec
 # layer's attention at 256 rows with rank 512, 256 and 128: 69 / 51, 43 / 37 and 37 / 43 us; at 1,024 rows with rank 24: 161 / 53.
 PROMPT_ROWS = 64
 PROMPT_WORK = 64 * 512
+
+
+@functools.lru_cache(maxsize=256)
+def key_shares(rows: int, heads: int, rank: int, keys: int, fill: float, sms: int) -> int:
+    """The shares that the keys of `rows` single rows are cut into, eight heads to a block and one block to an SM: those with the least
+    estimated time.  `keys`: the most that a row sees; `fill`: what the rows see over rows x keys.
+    The estimate, us: a block takes 3.0 and 2.55 a tile of 32 keys; blocks that do not run at once come in rounds, whole ones where the rows
+    are alike, as SMs come free where they are not; a merge takes 5.1, 0.16 a share, and its way through memory.  Fitted to rows of 512 + 64 numbers
+    (B200, 1 to 128 rows of 8, 16 and 32 heads, 300 to 4,096 keys; deviation 6%).  Against the best of all shares, as many as run at once take
+    1.14 times as long on average over 159 such batches, shares that fill the GPU twice 1.12 times and these 1.01; us, in that order:
+    8 rows of 300 to 1,024 keys 21.5 / 26 / 21, 33 of 1,024 51 / 65 / 51, 48 of 1,024 89 / 82 / 72, 40 of 64 to 4,096 330 / 118 / 100."""
+    tiles = -(-keys // 32)
+    groups = (heads + 7) // 8
+    best, best_cost = 1, None
+    for shares in range(1, min(32, (keys + 63) // 64) + 1):
+        more = max(0.0, rows * groups * shares / sms - 1.0)             # rounds after the first
+        rounds = fill * math.ceil(more) + (1.0 - fill) * more
+        cost = 3.0 + 2.55 * -(-tiles // shares) + rounds * (3.0 + 2.55 * max(1.0, fill * tiles / shares))
+        if shares > 1:
+            cost += 5.1 + 0.16 * shares + 0.024 * rows * shares * heads * rank / 8192
+        if best_cost is None or cost < 0.99 * best_cost:
+            best, best_cost = shares, cost
+    return best
 
 
 class LatentAttention(Mixer):
@@ -132,9 +156,8 @@ class LatentAttention(Mixer):
     def plan(self, rows: int, step: StepInfo):
         """(shares of the keys, rows per block) for `rows` rows of a step.  Rows of one sequence that follow one another
         share the keys they read: four to a block (prompts, long pieces).  Few rows, or rows of different sequences
-        (decoding), run one to a block, and their keys are cut into shares so that the blocks fill the GPU once, or twice
-        where an SM holds several of them: at least two tiles of 32 keys per share, at most 32 shares.  (Rows of 576 numbers: one
-        block to an SM; 8 rows of 16 heads, 300 to 1,024 keys, in 16 shares, which are two rounds, 22.6 us; in 9 18.0, and the merge 4.7 for 5.8.)"""
+        (decoding), run one to a block, and their keys are cut into shares: see key_shares where an SM holds one block, and
+        where it holds several, shares that fill the GPU about twice; at least two tiles of 32 keys per share, at most 32 shares."""
         if not step.single_token and rows >= 64:
             return 1, 4
         blocks = rows * ((self.n_heads + 7) // 8)
@@ -143,7 +166,8 @@ class LatentAttention(Mixer):
         keys = min(int(self.window), longest) if self.window else longest
         rot_dims = self.position.kernel_args()[1] if self.position else 0
         if self.use_tensor_cores and not self.rt.is_fp32 and ops.latent_attn_blocks(self.rank, self.row, rot_dims) == 1:
-            return max(1, min(32, (keys + 63) // 64, sms // blocks)), 1
+            live = min(rows, step.max_live) if step.max_live else rows
+            return key_shares(live, self.n_heads, self.rank, keys, step.fill_for(self.window), sms), 1
         return max(1, min(32, (keys + 63) // 64, (2 * sms + blocks - 1) // blocks)), 1
 
     def _prompt_sizes_fit(self) -> bool:
