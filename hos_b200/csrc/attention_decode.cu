@@ -825,11 +825,30 @@ extern "C" int hos_attn_decode_clusters(int n_heads, int n_kv_heads, int n_split
     return stages < 2 ? 0 : clusters_that_fit(n_splits, smem, n_heads / n_kv_heads);
 }
 
+// Bytes and stages of a launch with two groups of consumers, or 0: they are for up to eight heads to a kv head and where they leave the ring
+// three stages, or as many as it has beside one (at head size 256 three stages become two from three heads to a kv head on).
+static int two_groups_smem(int group, int n_tokens, bool even, int* stages) {
+    const int ints = even ? n_tokens + 1 : 2 * n_tokens;
+    int beside_one = 0;
+    decode_smem(group, &beside_one, ints);
+    const int smem = decode_smem(group, stages, ints, 2);
+    return group <= 8 && (*stages >= 3 || (*stages >= 2 && *stages == beside_one)) ? smem : 0;
+}
+// The groups of consumers that a launch of n_tokens rows takes: with even shares, or with whole items handed out by their length
+// (1: such a launch takes them as they come).
+extern "C" int hos_attn_decode_groups(int n_tokens, int n_heads, int n_kv_heads, int even) {
+    if (n_tokens <= 0 || n_kv_heads <= 0 || n_heads <= 0 || n_heads % n_kv_heads != 0) return 1;
+    if (n_tokens > (even ? kEvenMaxTokens : kSortedMaxTokens)) return 1;
+    int stages = 0;
+    return two_groups_smem(n_heads / n_kv_heads, n_tokens, even != 0, &stages) > 0 ? 2 : 1;
+}
+
+// by_length: with one share, whether whole items are handed out by their length where there are more of them than CTAs.
 extern "C" int hos_attn_decode(const void* q, int q_stride, void* out, int out_stride, float* workspace,
                                int* tickets, const int* token_pos, const int* token_seq, const int* seq_slot,
                                const int* token_slot, void* k_pages, void* v_pages, const int* page_table, int table_stride,
                                int ring_pages, int n_tokens, int n_heads, int n_kv_heads, int head_dim,
-                               float scale, float cap, int window, int n_splits, int max_new, cudaStream_t stream) {
+                               float scale, float cap, int window, int n_splits, int max_new, int by_length, cudaStream_t stream) {
     if (n_tokens <= 0) return 0;
     if (max_new < 1) HOS_REFUSE("attn_decode: max_new %d (the most new tokens of a sequence in this step) must be at least 1", max_new);
     if (head_dim != HD) HOS_REFUSE("attn_decode: built for head_dim %d, asked for %d", HD, head_dim);
@@ -852,14 +871,13 @@ extern "C" int hos_attn_decode(const void* q, int q_stride, void* out, int out_s
     const int smem = decode_smem(group, &stages, even ? n_tokens + 1 : 0);
     if (stages < 2) HOS_REFUSE("attn_decode: shared memory holds fewer than two stages for head_dim %d", HD);
     a.stages = stages;
-    // Two groups of consumers where they leave the ring three stages, or as many as it has beside one: with even shares, and with whole
-    // items that are more than the CTAs (so that a CTA has several, to be handed out by their length).
-    const bool several = n_splits == 1 && items > sm_count() && n_tokens <= kSortedMaxTokens;
+    // (whole items handed out by their length want several to a CTA)
+    const bool several = by_length && n_splits == 1 && items > sm_count() && n_tokens <= kSortedMaxTokens;
     int groups = 1, smem_used = smem;
-    if ((even || several) && group <= 8) {
+    if (even || several) {
         int with_two = 0;
-        const int smem_two = decode_smem(group, &with_two, even ? n_tokens + 1 : 2 * n_tokens, 2);
-        if (with_two >= 3 || (with_two >= 2 && with_two == stages)) {
+        const int smem_two = two_groups_smem(group, n_tokens, even, &with_two);
+        if (smem_two > 0) {
             groups = 2;
             smem_used = smem_two;
             a.stages = with_two;
@@ -961,5 +979,5 @@ extern "C" int hos_attn_decode_noalloc(const void* q, int q_stride, void* out, i
     }
     return hos_attn_decode(q, q_stride, out, out_stride, workspace, tickets, token_pos, token_seq, seq_slot, nullptr, k_pages,
                            v_pages, page_table, table_stride, ring_pages, n_tokens, n_heads, n_kv_heads, head_dim,
-                           scale, cap, window, n_splits, /*max_new: nothing is fetched ahead*/ 1 << 30, stream);
+                           scale, cap, window, n_splits, /*max_new: nothing is fetched ahead*/ 1 << 30, /*by_length*/ 1, stream);
 }

@@ -4,8 +4,10 @@ csrc/attention_prefill.cu).  They are compiled per head size (a multiple of 16, 
 from __future__ import annotations
 
 import ctypes
+import functools
+import math
 import os
-from typing import Dict, Optional
+from typing import Dict, NamedTuple, Optional
 
 import numpy as np
 import torch
@@ -36,111 +38,203 @@ def lib_for(head_dim: int) -> ops.Library:
 
 
 def decode_splits(n_tokens: int, n_kv_heads: int, group: int, max_len: int, window: Optional[int],
-                  min_live: int = 0, clusters_fit=None, max_live: int = 0, fill: float = 1.0) -> int:
-    """How many shares the keys of one (token, kv head) are cut into.  The kernel's CTAs (one per
-    SM) take items one after another; an item costs a fixed part (look-ups, first loads, the merge)
-    and a part per page.  The number of shares is the one that makes the step shortest by that
-    model (constants measured at head size 256), for all `n_tokens` rows live and, if the step is
+                  min_live: int = 0, clusters_fit=None, max_live: int = 0, fill: float = 1.0, head_dim: int = 256,
+                  groups: int = 2) -> int:
+    """How many shares the keys of one (token, kv head) are cut into; 0: even shares.  The kernel's CTAs (one per
+    SM) take items one after another; the answer is the cut that makes the step shortest by the estimate below, for
+    all `n_tokens` rows live and, if the step is
     a replayed one whose last rows may be padding, for `min_live` live rows and half-way as well
     (`max_live`: no more than that many of the rows are live; 0: all may be).  `fill`: the sequences' lengths add
     up to at most this fraction of live rows x what the longest holds (in this layer: of its window, if it has one):
     equal shares follow the longest sequence whatever the others hold, even shares follow the sum.
     `clusters_fit(s)`: how many clusters of s CTAs of the kernel run at once (None: no cluster merge); with
-    all of a step's clusters on the GPU at once the shares merge through shared memory, which is cheaper."""
-    chunks = (group + 15) // 16
+    all of a step's clusters on the GPU at once the shares merge through shared memory, which is cheaper.
+    `groups`: the groups of consumers that even shares have with these heads (consumer_groups)."""
+    return _decode_splits(_heads(n_kv_heads, group, head_dim), n_tokens, _pages(max_len, window), min_live, clusters_fit, max_live,
+                          round(fill, 2), groups, enabled["decode_even"] and n_tokens <= EVEN_MAX_ROWS, ops.sm_count())
+
+
+class _Heads(NamedTuple):
+    per_token: int              # items of a row
+    weight: float               # query heads of an item x head size / 512
+    page: float                 # bytes of a page's keys and values / 64 KB
+    alone: float                # us that a page takes a CTA by itself
+
+
+def _heads(n_kv_heads: int, group: int, head_dim: int) -> _Heads:
+    page = head_dim / 256
+    return _Heads(max(1, n_kv_heads * ((group + 15) // 16)), min(group, 16) * head_dim / 512, page,
+                  (0.41 + 0.26 * page) * (1.23 if group > 8 or group * head_dim > 1280 else 1.0))
+
+
+def _pages(max_len: int, window: Optional[int]) -> int:
     span = min(max_len, window) if window else max_len
-    pages = (span + ops.PAGE_TOKENS - 1) // ops.PAGE_TOKENS + (1 if window else 0)
-    per_token = max(1, n_kv_heads * chunks)
+    return -(-span // ops.PAGE_TOKENS) + (1 if window else 0)
+
+
+@functools.lru_cache(maxsize=1024)
+def _decode_splits(h: _Heads, n_tokens, pages, min_live, clusters_fit, max_live, fill, groups, may_even, sms) -> int:
     hi = max(1, min(n_tokens, max_live) if max_live else n_tokens)
     lo = min(max(1, min_live), hi) if min_live else hi
     lives = (lo, (lo + hi) // 2, hi, hi) if lo < hi else (hi,)      # fewest, middle and most live rows (a full batch counts twice)
+
+    def cluster(s: int) -> bool:
+        return 1 < s <= CLUSTER_SHARES and hi * h.per_token * s <= sms and clusters_fit is not None and clusters_fit(s) >= hi * h.per_token
+
     best, best_cost = 1, None
-    sms = ops.sm_count()
-
-    def merge_us(s: int) -> float:
-        if s == 1:
-            return 0.0
-        if clusters_fit is not None and s <= CLUSTER_SHARES and hi * per_token * s <= sms \
-                and clusters_fit(s) >= hi * per_token:
-            return _CLUSTER_MERGE_US + _CLUSTER_MERGE_PER_SHARE_US * s      # the shares are one cluster
-        return _MERGE_US + _MERGE_PER_SHARE_US * s
-
     for s in range(1, min(MAX_SPLITS, max(1, (pages + 1) // 2)) + 1):
-        per_item = _ITEM_US + _PAGE_US * -(-pages // s) + merge_us(s)
-        cost = sum(-(-live * per_token * s // sms) * per_item for live in lives)
-        if best_cost is None or cost < 0.97 * best_cost:          # more shares only for a clear gain
+        if s > 1 and lo * h.per_token * (s - 1) > 2 * sms:          # more rounds than that never pay
+            break
+        merged = cluster(s)
+        cost = sum(_equal_us(h, live, pages, fill, s, merged, sms) for live in lives)
+        if s == 1:                                                  # (a round of whole items against even shares: see _whole)
+            cost += sum(8.0 * ((live * h.per_token - 1) // sms) for live in lives)
+        if best_cost is None or cost < 0.995 * best_cost:           # more shares only for a gain
             best, best_cost = s, cost
-    # Even shares (0): every CTA the same number of pages, wherever the borders of the (token, kv head) fall.  They
-    # cost a fixed part more (the running sums of the pages, a second piece of work per CTA, a merge of almost
-    # every (token, kv head) through the workspace) and save the last round that equal items leave mostly empty.
-    # Weighed with a model that knows that many CTAs at once share the memory's speed: a round of all SMs is
-    # slower per page than a last round of a few.
-    # Only while the longest (token, kv head) lies in at most EVEN_MOST_PARTS CTAs: the last CTA of each merges all
-    # of its parts (one sequence at 32,768 keys in 37 parts: 1.90 ms a step against 1.75 ms in clusters).
-    held = max(1.0, pages * fill)             # pages an average (token, kv head) holds in this layer
-    if enabled["decode_even"] and n_tokens <= EVEN_MAX_ROWS and \
-            pages <= EVEN_MOST_PARTS * max(1, -(-int(lo * per_token * held) // sms)):
-        def page_us(active: int) -> float:
-            return max(_PAGE_US, active * _PAGE_SHARED_US)
-        share, equal, even = -(-pages // best), 0.0, 0.0
-        for live in lives:
-            full, rest = divmod(live * per_token * best, sms)      # rounds of all SMs, and what is left for a last one
-            equal += full * (_ITEM_US + share * page_us(sms) + merge_us(best))
-            if rest:
-                equal += _ITEM_US + share * page_us(rest) + merge_us(best)
-            equal += _ROUND_US * max(0, full + (1 if rest else 0) - 1)
-            even += _EVEN_US + -(-int(live * per_token * held) // sms) * page_us(sms)
-        if even < 0.95 * equal:
-            return 0
+    if may_even and sum(_even_us(h, live, pages, fill, groups, sms) for live in lives) < best_cost:
+        return 0
     return best
 
 
-# Fitted to measurements at head size 256, 8192 keys: one share of a sequence alone on its SM takes 0.67 us a page (0.76 with neighbours at work) and 3 to 5 us
-# besides (88 / 50 / 36 / 28 us with 1 / 2 / 3 / 4 shares of 128 pages); at 64 sequences of 2,036 keys two shares
-# instead of one cost 22 us more per layer.
-_ITEM_US, _PAGE_US, _MERGE_US, _MERGE_PER_SHARE_US = 4.5, 0.76, 1.0, 0.275
+# The estimate, us a launch (weight, page, alone: see _Heads).
+#   a page takes a CTA `alone`: 0.41 + 0.26 page, with more than eight heads to a kv head (the MMA's rows) or a ring of two stages (six
+#   heads of 256) 1.23 times that; and the memory's speed is shared: 0.00964 page for every CTA that streams (6.8 TB/s);
+#   an item 3.5 + 1.25 weight, a further round of items 3.45 less (its first pages come during the last one's merge);
+#   a merge through a cluster 0.59 + weight (0.41 + 1.66 a CTA of it) and 0.45 + 0.25 weight more where the shares are no power of two, through
+#   the workspace and a ticket 2.66 + weight (1.08 + 0.087 a share, 1.23 more likewise);
+#   even shares 5.2 (one group of consumers: 6.5) + 6.3 weight, 0.21 weight for every CTA that the longest item lies in, and 1.2 for each of
+#   the shortest rows' items, of which a CTA may have to do as many as a row has;
+#   whole items by their length 6.3, 0.66 weight for every round after the first.
+# Fitted to 1,017 batches of 1 to 128 rows of 200 to 8,184 keys, alike and not, with windows and without, head sizes 64, 128 and 256, 2 to 16
+# query heads a kv head, each cut in up to 20 ways (B200, replayed launches on cold caches; deviation 7%).
+# Examples of 8 heads of 256 over 4, us with even shares / one / two / four: 8 rows of 2,000 to
+# 8,184 keys 39.6 / 89.6 / 50.0 / 33.9, 24 of 4,096 72.4 / 62.5 / 80.2 / 75.8, 40 of 8,184 205 / 246 / 221 / 223, 16 of 64 to 8,184 34.5 / 89.8 /
+# 50.9 / 34.4, 36 of 1,024 30.3 / 27.9 / 35.1 / 45.8; of 32 heads of 256 over 2: 32 of 64 to 2,036 83 / 42 / 38 / 67.
+def _page_us(h: _Heads, active: int) -> float:
+    return max(h.alone, 0.00964 * h.page * active)
+
+
+@functools.lru_cache(maxsize=256)
+def _lengths(rows: int, fill: float) -> np.ndarray:
+    """Lengths of `rows` rows, the longest (1) first, that fill `fill` of rows x the longest: evenly spread over their logarithm."""
+    lo, hi = 1e-9, 1.0
+    for _ in range(40):
+        mid = math.sqrt(lo * hi)
+        lo, hi = (mid, hi) if (mid - 1.0) / math.log(mid) < fill else (lo, mid)
+    return hi ** (np.arange(rows) / max(1, rows - 1))
+
+
+def _walks_us(h: _Heads, lengths: np.ndarray, per_row: int, sms: int, by_length: bool) -> float:
+    """The time that CTAs take for the pages of items which are handed out in turn (by_length: every other round backwards), while the
+    memory's speed is shared by those that are not done."""
+    items = np.repeat(lengths, per_row)
+    rounds = -(-items.size // sms)
+    held = np.zeros((rounds, sms))
+    held.reshape(-1)[:items.size] = items
+    if by_length:
+        held[1::2] = held[1::2, ::-1]
+    held = np.sort(held.sum(axis=0))
+    us = np.maximum(h.alone, 0.00964 * h.page * np.arange(sms, 0, -1))
+    return float(np.dot(np.diff(held, prepend=0.0), us))
+
+
+def _equal_us(h: _Heads, rows: int, pages: int, fill: float, s: int, cluster: bool, sms: int) -> float:
+    full, rest = divmod(rows * h.per_token * s, sms)
+    if fill > 0.99 or rows == 1:
+        walks = -(-pages // s) * (full * _page_us(h, sms) + (_page_us(h, rest) if rest else 0.0))
+    else:
+        lengths = np.maximum(1.0, np.maximum(1.0, pages * _lengths(rows, fill)) / s)
+        walks = _walks_us(h, lengths[np.argsort(np.arange(rows) * 0.6180339887 % 1.0)], h.per_token * s, sms, False)     # in no order
+    rounds = full + (1 if rest else 0)
+    odd = 1.0 if s & (s - 1) else 0.0
+    if cluster:
+        merge = 0.59 + h.weight * (0.41 + 1.66 / s) + (0.45 + 0.25 * h.weight) * odd
+    else:
+        merge = 2.66 + h.weight * (1.08 + 0.087 * s + 1.23 * odd) if s > 1 else 0.0
+    return walks + rounds * (3.5 + 1.25 * h.weight + merge) - 3.45 * (rounds - 1)
+
+
+def _even_us(h: _Heads, rows: int, pages: int, fill: float, groups: int, sms: int) -> float:
+    share = max(1, -(-int(rows * h.per_token * max(1.0, pages * fill)) // sms), -(-pages // (EVEN_MOST_PARTS - 1)))
+    short = max(1.0, pages * float(_lengths(rows, fill)[int(0.8 * (rows - 1))]))        # pages of a short row
+    items = min(h.per_token, share / short) if rows > 1 else 0.0
+    return ((5.2 if groups == 2 else 6.5) + 6.3 * h.weight + min(EVEN_MOST_PARTS, pages / share) * 0.21 * h.weight + 1.2 * items +
+            share * _page_us(h, sms))
+
+
+def _by_length_us(h: _Heads, rows: int, pages: int, fill: float, sms: int) -> float:
+    rounds = -(-rows * h.per_token // sms)
+    return _walks_us(h, np.maximum(1.0, pages * _lengths(rows, fill)), h.per_token, sms, True) + 6.3 + 0.66 * h.weight * (rounds - 1)
+
+
 # Up to 16 shares of at most one wave of items merge as a cluster through shared memory: 2.3 to 2.8 us less
 # than through the workspace (one sequence, 8,192 keys, 16 shares: 17.4 -> 14.6 us; a window of 4,096: 13.5 -> 10.7).
 CLUSTER_SHARES = 16
-_CLUSTER_MERGE_US, _CLUSTER_MERGE_PER_SHARE_US = 0.3, 0.03
-# Even shares against the best equal shares, a step of Gemma-2 2B sizes at 8,192 keys (ms): 20 sequences 3.63 / 3.81,
-# 40: 5.80 / 6.92, 56: 7.28 / 8.15, 64: 8.04 / 8.02; but 8: 2.41 / 2.11, 16: 3.16 / 2.94, 32: 4.82 / 4.58.
-# The model that fits these: 22 us more per launch than one round of equal shares, 8 us for every further round of
-# equal shares, and a page costs a CTA 0.9 us alone but 0.0085 us times the number of CTAs that stream at once (64 KB
-# per page at head size 256: 7.7 TB/s between them).  At Gemma-2 9B sizes, 16 sequences of 64 to 2,300 keys (0.64 of
-# what 16 of the longest would hold) lose 0.15 ms a step with even shares: the model has to say no there.
-# Sequences of unequal lengths (8,100 / 4,000 / 2,000 / 1,000 / 500 / 500 / 250 / 250 keys, repeated): equal shares
-# take as long as the longest sequence's share, even shares follow the sum: 8 sequences 1.96 -> 1.86 ms a step, 16
-# sequences 2.69 -> 2.22, 32 sequences 4.05 -> 3.00.
-# (A page by itself then took 0.9 us and even shares 22 us; with two groups of consumers a CTA they take 17: 64 sequences of 64 to
-# 2,036 keys 40 us a layer, 12 of 700 to 5,000 32.)
-_EVEN_US = 16.0
-_ROUND_US = 8.0
-_PAGE_SHARED_US = 0.0085
 EVEN_MAX_ROWS = 2048
-EVEN_MOST_PARTS = 20
+EVEN_MOST_PARTS = 32        # CTAs that a (token, kv head) lies in, at most (csrc/attention_decode.cu: kEvenMaxParts)
+SORTED_MAX_ROWS = 256
 
 
+def whole_items_by_length(n_rows: int, per_token: int, pages: int, fill: float, weight: float = 1.0, page: float = 1.0) -> bool:
+    """Whether whole (token, kv head), handed out by their length, finish before even shares do (both with two groups of consumers; see
+    csrc/attention_decode.cu): `pages` of the longest row's keys, `fill` as for decode_splits.  64 rows of 16 heads of 128 over 4, 64 to
+    2,036 keys, 25.6 / 32.5 us; 40 of 8,184 keys, whose 160 items are two rounds of 148 SMs, 166 / 114."""
+    sms = ops.sm_count()
+    if n_rows * per_token <= sms or n_rows > SORTED_MAX_ROWS:
+        return False
+    h = _Heads(per_token, weight, page, 0.41 + 0.26 * page)
+    return _by_length_us(h, n_rows, pages, fill, sms) < _even_us(h, n_rows, pages, fill, 2, sms)
+
+
+@functools.lru_cache(maxsize=1024)
+def _whole(h: _Heads, splits: int, rows: int, pages: int, fill: float, even_groups: int, groups: int, sms: int) -> tuple:
+    """(shares, by their length) where decode_splits chose even shares or whole items (`splits`: 0 or 1) and the items are more than the SMs:
+    even shares (of `even_groups` groups of consumers), whole items as they come (one group, nothing sorted: rows all alike), or by
+    their length (where `groups`, which that launch would have, are two).  64 rows of 8 heads of 256 over 4, us as they come / by length: 517
+    keys each 28.8 / 30.1, 2,048 81.8 / 85.2; 16 heads of 128 over 4, 64 to 2,036 keys 31.9 / 25.6."""
+    best = (splits, False)
+    cost = _even_us(h, rows, pages, fill, even_groups, sms) if splits == 0 else None
+    whole = _equal_us(h, rows, pages, fill, 1, False, sms)
+    if cost is None or whole < 0.97 * cost:
+        best, cost = (1, False), whole
+    if groups == 2 and rows <= SORTED_MAX_ROWS and _by_length_us(h, rows, pages, fill, sms) < 0.97 * cost:
+        best = (1, True)
+    return best
+
+
+def plan(head_dim: int, n_tokens: int, n_heads: int, n_kv_heads: int, max_len: int, window: Optional[int], min_live: int, clusters_fit,
+         max_live: int, fill: float, groups_of) -> tuple:
+    """(shares as decode_splits, whole items by their length) for a launch of n_tokens rows, of which as many are live as decode_splits is
+    told; groups_of: consumer_groups.  Over the 1,017 batches beside the estimate the choice takes 1.01 times as long as the best of all cuts;
+    one fitted at head size 256 with two query heads to a kv head took 1.05 times, up to 3.5 times."""
+    group, heads = n_heads // n_kv_heads, _heads(n_kv_heads, n_heads // n_kv_heads, head_dim)
+    even_groups = groups_of(head_dim, n_tokens, n_heads, n_kv_heads, True)
+    splits = decode_splits(n_tokens, n_kv_heads, group, max_len, window, min_live, clusters_fit, max_live, fill, head_dim, even_groups)
+    live = min(n_tokens, max_live) if max_live else n_tokens
+    if splits > 1 or live * heads.per_token <= ops.sm_count():
+        return splits, False
+    return _whole(heads, splits, live, _pages(max_len, window), round(fill, 2), even_groups,
+                  groups_of(head_dim, n_tokens, n_heads, n_kv_heads, False), ops.sm_count())
+
+
+_groups_known: Dict[tuple, int] = {}
 _fit_known: Dict[tuple, int] = {}
 
 
-def whole_items_by_length(n_rows: int, per_token: int, pages: int, fill: float) -> bool:
-    """Whether whole (token, kv head), handed out by their length, finish before even shares do (both with two groups of consumers; see
-    csrc/attention_decode.cu): `pages` of the longest row's keys, `fill` as for decode_splits.  The longest item alone, or what an SM
-    has on average, and a second item that is the longer the more alike the rows are; even shares: the average, and what cutting
-    costs.  64 rows of 64 to 2,036 keys 37 / 40 us, 48 of 200 to 1,500 29 / 32, 64 of 64 to 1,000 21 / 30; 40 rows of 8,192 keys,
-    whose 160 items are two rounds of 148 SMs: even shares."""
-    sms = ops.sm_count()
-    items = n_rows * per_token
-    if items <= sms or n_rows > SORTED_MAX_ROWS:
-        return False
-    mean = pages * fill
-    average = items * mean / sms
-    whole = _ITEM_US + max(_PAGE_US * (max(pages, average) + mean * fill), average * sms * _PAGE_SHARED_US)
-    return whole < _EVEN_US + average * sms * _PAGE_SHARED_US
+def consumer_groups(head_dim: int, n_tokens: int, n_heads: int, n_kv_heads: int, even: bool) -> int:
+    """Groups of consumers of a launch with even shares, or with whole items by their length (asked once per shape)."""
+    key = (head_dim, n_tokens, n_heads, n_kv_heads, even)
+    n = _groups_known.get(key)
+    if n is None:
+        f = lib_for(head_dim).lib.hos_attn_decode_groups
+        f.restype, f.argtypes = ctypes.c_int, [ctypes.c_int] * 4
+        n = _groups_known[key] = int(f(n_tokens, n_heads, n_kv_heads, int(even)))
+    return n
 
 
-SORTED_MAX_ROWS = 256
+@functools.lru_cache(maxsize=64)
+def _fits(head_dim: int, n_heads: int, n_kv_heads: int):
+    return functools.partial(clusters_fit, head_dim, n_heads, n_kv_heads)
 
 
 def clusters_fit(head_dim: int, n_heads: int, n_kv_heads: int, n_splits: int) -> int:
@@ -182,14 +276,15 @@ def decode(q: torch.Tensor, q_stride: int, out: torch.Tensor, token_pos, token_s
            cache: ops.PagedKVArgs, n_tokens: int, n_heads: int, scale: float, cap: float,
            window: Optional[int], max_len: int, n_splits: Optional[int] = None,
            max_new: Optional[int] = None, min_live: int = 0, token_slot=None, cluster: bool = True,
-           max_live: int = 0, fill: float = 1.0) -> None:
+           max_live: int = 0, fill: float = 1.0, by_length: bool = True) -> None:
     """Attention of n_tokens single queries over the paged cache (each token at its own
     position in its own sequence).  `max_new`: the most tokens any sequence brings in this step;
     the kernel may fetch keys that lie below them while the kernel before it (which writes the
     step's new keys) still runs.  None: it fetches nothing ahead.  `token_slot`: each token's cache slot
     (seq_slot[token_seq]) if the step has it: the kernel then finds its first page one look-up sooner.
     `cluster`: up to 16 shares of at most one wave of work items may run as clusters that merge through
-    shared memory (False: always through the workspace)."""
+    shared memory (False: always through the workspace).  `by_length`, with n_splits 1: more items than SMs are handed out by
+    their length."""
     hd, nkv = cache.head_dim, cache.n_kv_heads
     lib = lib_for(hd)
     want = bool(cluster and enabled["decode_cluster"])
@@ -197,14 +292,8 @@ def decode(q: torch.Tensor, q_stride: int, out: torch.Tensor, token_pos, token_s
         lib.call("hos_attn_decode_cluster", 1 if want else 0)
         _cluster_state[hd] = want
     if n_splits is None:
-        fit = (lambda s: clusters_fit(hd, n_heads, nkv, s)) if want else None
-        group = n_heads // nkv
-        n_splits = decode_splits(n_tokens, nkv, group, max_len, window, min_live, fit, max_live, fill)
-        if n_splits == 0 and group <= 8:
-            span = min(max_len, window) if window else max_len
-            live = min(n_tokens, max_live) if max_live else n_tokens
-            if whole_items_by_length(live, nkv, -(-span // ops.PAGE_TOKENS) + (1 if window else 0), fill):
-                n_splits = 1
+        n_splits, by_length = plan(hd, n_tokens, n_heads, nkv, max_len, window, min_live, _fits(hd, n_heads, nkv) if want else None,
+                                   max_live, fill, consumer_groups)
     ws = tickets = None
     if n_splits == 0:            # even shares: every CTA the same number of pages, two places per CTA for what is cut
         f = lib.lib.hos_attn_decode_even_workspace
@@ -219,7 +308,7 @@ def decode(q: torch.Tensor, q_stride: int, out: torch.Tensor, token_pos, token_s
              ops._ptr(cache.k_pages),
              ops._ptr(cache.v_pages), ops._ptr(cache.page_table), cache.table_stride, cache.ring_pages,
              n_tokens, n_heads, nkv, hd, float(scale), float(cap), int(window) if window else 0,
-             int(n_splits), int(max_new) if max_new else 1 << 30, ops._stream())
+             int(n_splits), int(max_new) if max_new else 1 << 30, int(by_length), ops._stream())
     # one or two sequences' worth of CTAs leave most SMs free: the product after this kernel may be placed beside it
     ctas = ops.sm_count() if n_splits == 0 else n_tokens * nkv * ((n_heads // nkv + 15) // 16) * n_splits
     ops.note_room_left(2 * ctas <= ops.sm_count())
