@@ -54,7 +54,7 @@ PROMPT_WORK = 64 * 512
 @functools.lru_cache(maxsize=256)
 def key_shares(rows: int, heads: int, rank: int, keys: int, fill: float, sms: int) -> int:
     """The shares that the keys of `rows` single rows are cut into, eight heads to a block and one block to an SM: those with the least
-    estimated time.  `keys`: the most that a row sees; `fill`: what the rows see over rows x keys.
+    estimated time, and of near ties the most (a replayed step's rows grow beyond what its launches were planned with).  `keys`: the most that a row sees; `fill`: what the rows see over rows x keys.
     The estimate, us: a block takes 3.0 and 2.55 a tile of 32 keys; blocks that do not run at once come in rounds, whole ones where the rows
     are alike, as SMs come free where they are not; a merge takes 5.1, 0.16 a share, and its way through memory.  Fitted to rows of 512 + 64 numbers
     (B200, 1 to 128 rows of 8, 16 and 32 heads, 300 to 4,096 keys; deviation 6%).  Against the best of all shares, as many as run at once take
@@ -62,16 +62,16 @@ def key_shares(rows: int, heads: int, rank: int, keys: int, fill: float, sms: in
     8 rows of 300 to 1,024 keys 21.5 / 26 / 21, 33 of 1,024 51 / 65 / 51, 48 of 1,024 89 / 82 / 72, 40 of 64 to 4,096 330 / 118 / 100."""
     tiles = -(-keys // 32)
     groups = (heads + 7) // 8
-    best, best_cost = 1, None
+    costs = {}
     for shares in range(1, min(32, (keys + 63) // 64) + 1):
         more = max(0.0, rows * groups * shares / sms - 1.0)             # rounds after the first
         rounds = fill * math.ceil(more) + (1.0 - fill) * more
         cost = 3.0 + 2.55 * -(-tiles // shares) + rounds * (3.0 + 2.55 * max(1.0, fill * tiles / shares))
         if shares > 1:
             cost += 5.1 + 0.16 * shares + 0.024 * rows * shares * heads * rank / 8192
-        if best_cost is None or cost < 0.99 * best_cost:
-            best, best_cost = shares, cost
-    return best
+        costs[shares] = cost
+    near = 1.02 * min(costs.values())
+    return max(shares for shares, cost in costs.items() if cost <= near)
 
 
 class LatentAttention(Mixer):
