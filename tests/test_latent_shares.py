@@ -17,7 +17,7 @@ MEASURED = [
     ((64, 16, 1024, 1.0), {1: 90.0, 2: 98.1, 3: 103.2, 4: 107.8}),
     ((96, 16, 1024, 1.0), {1: 178.3, 2: 147.2, 3: 139.4, 4: 161.5, 5: 154.9}),
     ((96, 16, 4096, 1.0), {1: 663.5, 2: 512.4, 3: 465.6, 4: 529.0, 5: 501.8}),
-    ((24, 32, 4096, 0.24), {1: 328.4, 7: 111.4, 6: 113.2, 8: 118.1, 9: 113.0, 10: 115.8}),
+    ((24, 32, 4096, 0.24), {1: 328.4, 7: 111.4, 6: 112.6, 8: 117.7, 9: 112.1, 10: 115.0, 12: 117.4, 14: 118.8}),
 ]
 
 
