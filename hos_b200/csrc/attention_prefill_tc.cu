@@ -1014,7 +1014,8 @@ extern "C" int hos_attn_prefill_tc(const void* rows, long long n_rows, int row_s
 // sequence s has the rows cu_seqlens[s] - row_base .. of q and out, at the consecutive positions token_pos[row], and
 // the page-table row seq_slot[s]; n_q_tiles is at least the sum over sequences of ceil(rows / 128).  The pages are
 // [n_pages][n_kv_heads][64][head_dim] arrays in the cache's permuted layout.  shares > 1: a block's walk over its keys may be cut into
-// up to that many, each of share_tiles tiles of 128 keys or so, where the heads run on pairs of SMs (hos_attn_prefill_pairs); part_o and
+// up to that many, each of share_tiles tiles of 128 keys or so, where the heads run on pairs of SMs (hos_attn_prefill_pairs; 0: one SM a block
+// and head, which is sooner done where walks are short); part_o and
 // part_ml: n_q_tiles * n_heads * shares * 128 times head_dim and times two floats, 16-byte aligned.
 extern "C" int hos_attn_chunk_tc(const void* q, long long n_rows, int row_stride, void* out, int out_stride,
                                  const int* cu_seqlens, int row_base, const int* token_pos, const int* seq_slot,
@@ -1047,7 +1048,7 @@ extern "C" int hos_attn_chunk_tc(const void* q, long long n_rows, int row_stride
     a.page_table = page_table; a.table_stride = table_stride; a.ring_pages = ring_pages;
     a.wait_cycles = kTcWaitCycles; a.stop_tile = -1;
 #if (HOS_HEAD_DIM == 128) || (HOS_HEAD_DIM == 256)
-    if (pair_state() != 0 && (n_heads / n_kv_heads) % 2 == 0) {
+    if (shares != 0 && pair_state() != 0 && (n_heads / n_kv_heads) % 2 == 0) {
         if (shares > 1 && (part_o == nullptr || part_ml == nullptr || share_tiles <= 0 || shares > 65535))
             HOS_REFUSE("attn_chunk_tc: %d shares need their length and a workspace", shares);
         if (shares > 1) { a.share_tiles = share_tiles; a.part_o = (float4*)part_o; a.part_ml = (float2*)part_ml; }

@@ -374,32 +374,65 @@ def cut_walks(tiles, pairs_per_block: int, pairs: int):
     return best
 
 
-def _shares(part, n_heads: int, n_kv_heads: int, head_dim: int, window):
-    """cut_walks for the sequences of `part`, once per step and kind of layer."""
-    f = lib_for(head_dim).lib.hos_attn_prefill_pairs
-    f.restype, f.argtypes = ctypes.c_int, [ctypes.c_int, ctypes.c_int]
+def on_one_sm(pages, tiles, pairs_per_block: int, pairs: int, shares: int, share_tiles: int) -> bool:
+    """Whether blocks of queries whose walks over the keys are `pages` tiles of 64 keys long, or `tiles` of PAIR_KEYS, are done sooner by the
+    kernel on one SM a block and head than by pairs of SMs with cut_walks' answer.  The estimate, us: a walk on one SM 5.0 and 1.33 a tile
+    of 64 keys, on a pair 7.0 and 2.12 a tile of 128, in shares 3.7 and 1.2 a share more; walks that do not run at once as in cut_walks.
+    Measured (B200, us one SM / pairs as planned): 17 tokens on top of 40, 8 heads of 256, 6.2 / 9.1, of 500 16.8 / 18.7, of 1,500 36.8 / 22.2; 32
+    heads of 128 over 16, 739 tokens on top of 40 22.9 / 27.0, of 500 40.3 / 38.9.  Over 504 such pieces the choice takes 1.00 times the best;
+    always pairs 1.06 times, up to 1.54."""
+    pages, tiles = np.asarray(pages, dtype=np.int64), np.asarray(tiles, dtype=np.int64)
+    if pages.size == 0:
+        return False
+    alone = 5.0 + 1.33 * int(pages.max())
+    walks = 2 * pairs_per_block * pages.size
+    if walks > 2 * pairs:
+        alone = max(alone, (1.33 * 2 * pairs_per_block * int(pages.sum()) + 5.0 * walks) / (2 * pairs) + 0.55 * int(pages.max()))
+    parts = np.minimum(shares, -(-tiles // share_tiles)) if shares > 1 else np.ones_like(tiles)
+    longest, n = int((-(-tiles // parts)).max()), int(parts.sum()) * pairs_per_block
+    paired = 7.0 + 2.12 * longest
+    if n > pairs:
+        paired = max(paired, (2.12 * int(tiles.sum()) * pairs_per_block + 7.0 * n) / pairs + 1.08 * longest)
+    if int(parts.max()) > 1:
+        paired += 3.7 + 1.2 * int(parts.max())
+    return alone < paired
+
+
+def _walk_plan(part, n_heads: int, n_kv_heads: int, head_dim: int, window):
+    """(pairs of SMs, shares, tiles of a share) for the sequences of `part`, once per step and kind of layer: see cut_walks and on_one_sm."""
     _set_pairs(head_dim, enabled["prefill_pair"])
-    pairs = int(f(n_heads, n_kv_heads))
+    pairs = _pairs_at_once(head_dim, n_heads, n_kv_heads, enabled["prefill_pair"])
     if pairs == 0:
-        return 1, 0
-    key = ("attention shares", part.row_offset, part.n_tokens, n_heads, window)
+        return False, 1, 0
+    key = ("attention walks", part.row_offset, part.n_tokens, n_heads, head_dim, window)
     got = part.shared.get(key)
     if got is None:
         w = int(window) if window else 0
+        pages, tiles = [], []
         if part.replayed or not part.cu_host:         # what the launches are planned for: every block as long as the longest
             _, blocks = prompt_blocks(part, 128)
-            span = min(part.max_len_after, w + 127) if w else part.max_len_after
-            tiles = [-(-span // PAIR_KEYS)] * max(1, blocks - part.n_seqs + 1)
+            span, n = min(part.max_len_after, w + 127) if w else part.max_len_after, max(1, blocks - part.n_seqs + 1)
+            pages, tiles = [-(-span // ops.PAGE_TOKENS)] * n, [-(-span // PAIR_KEYS)] * n
         else:
-            tiles = []
             starts = part.starts_host or [0] * (len(part.cu_host) - 1)
             for i, start in enumerate(starts):
                 n = part.cu_host[i + 1] - part.cu_host[i]
                 for q0 in range(0, n, 128):
-                    first = max(0, start + q0 + 1 - w) if w else 0
-                    tiles.append((start + min(n, q0 + 128) - 1) // PAIR_KEYS - first // PAIR_KEYS + 1)
-        got = part.shared[key] = cut_walks(tiles, n_heads // 2, pairs)
+                    first, last = max(0, start + q0 + 1 - w) if w else 0, start + min(n, q0 + 128) - 1
+                    pages.append(last // ops.PAGE_TOKENS - first // ops.PAGE_TOKENS + 1)
+                    tiles.append(last // PAIR_KEYS - first // PAIR_KEYS + 1)
+        shares, share_tiles = cut_walks(tiles, n_heads // 2, pairs)
+        got = (False, 1, 0) if on_one_sm(pages, tiles, n_heads // 2, pairs, shares, share_tiles) else (True, shares, share_tiles)
+        part.shared[key] = got
     return got
+
+
+@functools.lru_cache(maxsize=64)
+def _pairs_at_once(head_dim: int, n_heads: int, n_kv_heads: int, on: bool) -> int:
+    """How many pairs of SMs the pieces of these heads run on at once; 0: they do not (asked once per shape and state of the switch)."""
+    f = lib_for(head_dim).lib.hos_attn_prefill_pairs
+    f.restype, f.argtypes = ctypes.c_int, [ctypes.c_int, ctypes.c_int]
+    return int(f(n_heads, n_kv_heads))
 
 
 def _share_workspace(blocks: int, n_heads: int, head_dim: int, shares: int, device):
@@ -463,10 +496,11 @@ def chunk(q, q_stride, out, cu_seqlens, row_base: int, token_pos, seq_slot, n_se
 def chunk_tc(q, out, cu_seqlens, row_base: int, token_pos, seq_slot, n_seqs: int, blocks: int,
              cache: ops.PagedKVArgs, n_heads, scale, cap, window, pairs: bool = True, shares: int = 1, share_tiles: int = 0) -> None:
     """As `chunk`, on the tcgen05 tensor cores (head sizes 64, 128, 256): q is [rows, stride] with the q heads
-    first in a row; `blocks`: at least the sum over sequences of ceil(rows / 128); pairs: see prefill_tc; shares, share_tiles: pairs
-    of SMs walk over a block's keys in up to that many parts of about that many tiles (see cut_walks)."""
+    first in a row; `blocks`: at least the sum over sequences of ceil(rows / 128); pairs: as prefill_tc's, False: one SM a block and head; shares,
+    share_tiles: pairs of SMs walk over a block's keys in up to that many parts of about that many tiles (see cut_walks)."""
     lib = lib_for(cache.head_dim)
-    _set_pairs(cache.head_dim, bool(pairs and enabled["prefill_pair"]))
+    _set_pairs(cache.head_dim, enabled["prefill_pair"])
+    shares = max(1, int(shares)) if pairs else 0
     part_o, part_ml = _share_workspace(blocks, n_heads, cache.head_dim, shares, q.device)
     lib.call("hos_attn_chunk_tc", ops._ptr(q), q.shape[0], q.shape[1], ops._ptr(out), out.shape[1], ops._ptr(cu_seqlens),
              int(row_base), ops._ptr(token_pos), ops._ptr(seq_slot), n_seqs, blocks, ops._ptr(cache.k_pages),
@@ -487,9 +521,9 @@ def attend_chunks(mixer, qkv, att, part, cache) -> bool:
     slots = part.seq_slot[part.seq_offset:]
     if enabled["chunk_tc"] and qkv.is_contiguous() and has_tc_prefill(mixer.head_dim):
         _, blocks = prompt_blocks(part, 128)
-        shares, share_tiles = _shares(part, mixer.n_heads, mixer.n_kv_heads, mixer.head_dim, mixer.window)
+        pairs, shares, share_tiles = _walk_plan(part, mixer.n_heads, mixer.n_kv_heads, mixer.head_dim, mixer.window)
         chunk_tc(qkv, att, part.cu_seqlens, part.row_offset, part.token_pos, slots, part.n_seqs, blocks, cache,
-                 mixer.n_heads, mixer.scale, mixer.softcap, mixer.window, shares=shares, share_tiles=share_tiles)
+                 mixer.n_heads, mixer.scale, mixer.softcap, mixer.window, pairs=pairs, shares=shares, share_tiles=share_tiles)
         return True
     _, blocks = prompt_blocks(part, 64)
     chunk(qkv, qkv.shape[1], att, part.cu_seqlens, part.row_offset, part.token_pos, slots, part.n_seqs, blocks, cache,
