@@ -1,22 +1,21 @@
 // Attention of single tokens over the paged cache (decoding), bfloat16, split over the keys.
 //
-// A work item is one token, one kv head (with the up to 16 query heads that share it, stacked
-// as the rows of one MMA tile) and one contiguous share of the sequence's pages.  The kernel
-// is persistent: one CTA per SM walks over the items.  A page's [64][HD] key tile and value
+// A work item is one token, one kv head (with the up to 16 query heads that share it) and one contiguous share of the
+// sequence's pages.  The kernel is persistent: one CTA per SM walks over the items.  A page's [64][HD] key tile and value
 // tile are contiguous in the cache, so the producer warp brings each on chip with a single
 // bulk copy (TMA) counted on an mbarrier, running ahead of the math through a ring of stages
 // and across item boundaries, so that the memory pipe does not drain while an item is
-// finished.  Four consumer warps take 16 keys of a tile each: S = Q K^T (m16n8k16, bf16, 32-bit
-// accumulators), scale, soft-cap, mask, running max/sum in 32-bit, O += P V.  The four warps'
+// finished.  A group of four consumer warps takes 16 keys of a tile each: scores (m16n8k16, bf16, 32-bit
+// accumulators), scale, soft-cap, mask, running max/sum in 32-bit, weighted values.  Up to eight heads are the eight columns of the MMAs (FEW:
+// S^T = K Q^T, O^T = V^T P^T), nine to sixteen their rows (S = Q K^T, O = P V): with the rows mostly empty the MMAs and sums of a page
+// took a CTA longer than its bytes, 128 pages after one another 126 us, now 88.  The four warps'
 // partial results are merged through shared memory.  The shares of a (token, kv head) are then
 // merged in one of two ways.  When there are at most 16 of them and all of a launch's items run
 // at once, the launch is made of clusters, one per (token, kv head): every CTA leaves its
 // unnormalised result and (max, sum) in its own shared memory, the cluster meets at a barrier,
 // and every CTA merges a slice of the columns, reading the others' results through distributed
 // shared memory.  Otherwise a share writes its result to the workspace and takes a ticket; the
-// CTA that takes the last ticket of a (token, kv head) merges the shares.  Unused MMA
-// rows (fewer than 16 heads per kv head) cost nothing that matters: the kernel is bound by
-// the cache's bytes.
+// CTA that takes the last ticket of a (token, kv head) merges the shares.
 //
 // The kernel has a second way to cut the work (attn_decode_kernel<true, ...>, asked for with 0 shares): not every
 // (token, kv head) into the same number of shares, but the row of all pages of all (token, kv head) into one
@@ -24,11 +23,12 @@
 // leave a round of SMs mostly empty, and where the sequences are of unequal lengths.  There two groups of four consumer warps
 // take a CTA's pieces in turn (where shared memory has room for both): what a piece costs besides its pages (queries, merges, the ticket,
 // 3 to 4 us of latencies) then passes under the other group's pages.  The same two groups take whole (token, kv head) in turn where
-// there are more of them than CTAs and none is cut: there a CTA's items are handed out by length, the longest first and the next round
-// the other way round, so that the CTAs with the longest item get the shortest beside it.
-// Measured (B200, 8 heads of 256 over 4, us before / now; before: items as they come, one group, heads as the rows of the MMA): 64
-// sequences of 64 to 2,036 keys 48.6 (even shares) / 37.1, of 64 to 1,000 35.2 / 21.2, of 517 28.4 / 28.8; 8 of 8,184 in four shares 44.6 / 43.5; one
-// share of 8,184 keys, 128 pages after one another, 126 / 88.
+// there are more of them than CTAs, none is cut and the caller asks for it (by_length): there a CTA's items are handed out by length, the
+// longest first and the next round the other way round, so that the CTAs with the longest item get the shortest beside it.  Which way is
+// asked for: parts/attention_fast.py (plan), with the times of all of them.
+// Measured (B200, us even shares / whole items as they come / by their length): 16 heads of 128 over 4, 64 sequences of 64 to 2,036 keys 32.5 /
+// 31.9 / 25.6, of 64 to 1,000 24.6 / 19.9 / 16.1; 8 heads of 256 over 4, the same 40.6 / 41.3 / 41.0 and 31.2 / 26.0 / 25.0; rows alike, 64 of 2,048
+// 92.7 / 81.8 / 85.2, 40 of 2,048 61.5 / 69.7 / 80.7 (a second round of 12 items, which by their length fall to neighbouring SMs).
 //
 // Compiled per head size: -DHOS_HEAD_DIM=N, N a multiple of 16 up to 256.
 #include "common.cuh"
